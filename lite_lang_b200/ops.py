@@ -1178,15 +1178,61 @@ def delta_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b_off:
         c_int(taps), c_int(1 if per_channel else 0), _stream())
 
 
+CHUNK = 64                 # tokens of a chunk (csrc/chunk_scan.cu)
+# Tokens of a portion, on average, from which on it is scanned by chunks.  Measured on a B200, 12 heads of 128 x 128, one
+# portion (the walk's time grows with the tokens, the chunks' three launches take 28 us down to the smallest):
+#   decay scan, bfloat16: 64 tokens 14 us by the walk, 29 by chunks; 128 tokens 27 and 28; 2,048 tokens 320 and 53
+#   delta rule:           64 tokens 31 us by the walk, 37 by chunks; 128 tokens 58 and 47; 2,048 tokens 872 and 185
+DECAY_CHUNKED_MIN = 128
+DELTA_CHUNKED_MIN = 96
+
+
+def chunked_scan(step, tokens: int, dk: int, dv: int, least: int) -> Optional[Tuple[int, int, int]]:
+    """How a step's recurrences are cut: None (all entries token by token), or (entries at the front that stay with the
+    walk by tokens, entries behind them that go by chunks, an upper bound of their chunks).
+
+    A step's single tokens come first and stay with the walk.  The portions behind them go by chunks when they bring
+    ``least`` tokens each on average."""
+    if dk not in (64, 128) or dv % 64:
+        return None
+    single = int(getattr(step, "num_single", 0) or 0)
+    rest = int(step.num_entries) - single
+    if rest <= 0 or tokens - single < least * rest:
+        return None
+    return single, rest, (tokens - single) // CHUNK + rest
+
+
+def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, cut) -> None:
+    single, rest, items = cut
+    f32 = dict(dtype=torch.float32, device=qn.device)
+    s0 = torch.empty(items * H * dv * dk, **f32)
+    u = torch.empty(items * H * CHUNK * dv, **f32)
+    w = torch.empty(items * H * CHUNK * dk, **f32)
+    small = torch.empty(items * H * (CHUNK + 1), **f32)
+    load_library("chunk_scan").call(
+        "ll_chunk_delta_scan", _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(g), _ptr(state), c_long(state.stride(0)),
+        c_int(state.shape[0]), _ptr(step.cu_q[single:]), _ptr(step.req_slot[single:]), _ptr(o), c_int(rest), c_int(H),
+        c_int(Hk), c_int(dk), c_int(dv), _ptr(s0), _ptr(u), _ptr(w), _ptr(small), _ptr(small[items * H * CHUNK:]),
+        c_int(items), _stream())
+
+
 def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta: torch.Tensor, g: torch.Tensor,
                      state: torch.Tensor, step, o: torch.Tensor, H: int, Hk: int, dk: int, dv: int,
                      per_channel: bool) -> None:
     """The scan of every entry's tokens through its request's state; o float32 [tokens, H, dv]."""
     _need_cuda(qn, kn, vc, beta, g, state, o)
     _need(dk <= 256, f"delta rule: key heads of {dk} channels are wider than the scan kernel takes (256)")
+    entries = step.num_entries
+    if not per_channel and dv <= 128 and state.stride(0) % 4 == 0 and all(t.data_ptr() % 16 == 0 for t in (qn, kn, vc, state, o)):
+        cut = chunked_scan(step, qn.shape[0], dk, dv, DELTA_CHUNKED_MIN)
+        if cut is not None:
+            _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H, Hk, dk, dv, cut)
+            entries = cut[0]
+    if entries == 0:
+        return
     load_library("delta_rule").call(
         "ll_delta_recurrence", _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(g), _ptr(state), c_long(state.stride(0)),
-        _ptr(step.cu_q), _ptr(step.req_slot), _ptr(o), c_int(step.num_entries), c_int(H), c_int(Hk), c_int(dk),
+        _ptr(step.cu_q), _ptr(step.req_slot), _ptr(o), c_int(entries), c_int(H), c_int(Hk), c_int(dk),
         c_int(dv), c_int(1 if per_channel else 0), _stream())
 
 
@@ -1579,12 +1625,30 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay: Op
           and (skip is None or skip.numel() == H) and state.shape[1] >= H * dk * dv
           and o.shape[1] == H * dv and o.is_contiguous() and H % heads_per_group == 0,
           "decay_scan: shapes (key heads of at most 256 channels)")
+    entries, size = step.num_entries, proj.element_size()
+    if (proj.stride(0) * size % 16 == 0 and all(x * size % 16 == 0 for x in (q_off, k_off, v_off))
+            and all(t_.data_ptr() % 16 == 0 for t_ in (proj, o))):
+        cut = chunked_scan(step, proj.shape[0], dk, dv, DECAY_CHUNKED_MIN)
+        if cut is not None:
+            single, rest, items = cut
+            ds = torch.empty(items * H * dv * dk, dtype=torch.float32, device=proj.device)
+            gam = torch.empty(items * H, dtype=torch.float32, device=proj.device)
+            load_library("chunk_scan").call(
+                "ll_chunk_decay_scan", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), c_int(q_off),
+                c_int(k_off), c_int(v_off), _ptr(decay), _ptr(state), c_long(state.stride(0)), c_int(state.shape[0]),
+                _ptr(step.cu_q[single:]), _ptr(step.req_slot[single:]), _ptr(o), c_int(rest), c_int(H), c_int(dk),
+                c_int(dv), c_int(1 if write_state else 0), _ptr(step.status), c_int(heads_per_group), _ptr(token_decay),
+                _ptr(token_scale), _ptr(skip), _ptr(ds), _ptr(gam), c_int(items), _stream())
+            entries = single
+    if entries == 0:
+        return
     load_library("linear_attn").call(
         "ll_decay_scan", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), c_int(q_off), c_int(k_off),
         c_int(v_off), _ptr(decay), _ptr(state), c_long(state.stride(0)), c_int(state.shape[0]), _ptr(step.cu_q),
-        _ptr(step.req_slot), _ptr(o), c_int(step.num_entries), c_int(H), c_int(dk), c_int(dv),
+        _ptr(step.req_slot), _ptr(o), c_int(entries), c_int(H), c_int(dk), c_int(dv),
         c_int(1 if write_state else 0), _ptr(step.status), c_int(heads_per_group), _ptr(token_decay),
-        _ptr(token_scale), _ptr(skip), c_int(1 if o.shape[0] >= 4 * step.num_entries + 128 else 0), _stream())
+        _ptr(token_scale), _ptr(skip), c_int(1 if entries == step.num_entries and o.shape[0] >= 4 * entries + 128 else 0),
+        _stream())
 
 
 def ssd_prepare(proj: torch.Tensor, x_off: int, dt_off: int, conv_w: torch.Tensor, conv_b: Optional[torch.Tensor],

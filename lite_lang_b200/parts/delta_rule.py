@@ -136,7 +136,7 @@ class GatedDeltaRule(Mixer):
         return StateNeed((self.state_floats + (self.taps - 1) * (2 * self.Cq + self.Cv),), "float32")
 
     def kernel_libraries(self):
-        libs = ["core", "delta_rule"]
+        libs = ["core", "delta_rule", "chunk_scan"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
         return libs

@@ -77,7 +77,7 @@ class DecayLinearAttention(Mixer):
         return StateNeed((self.H * self.dv * self.dk,), "float32")
 
     def kernel_libraries(self):
-        libs = ["core", "linear_attn"]
+        libs = ["core", "linear_attn", "chunk_scan"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
         return libs
@@ -146,7 +146,7 @@ class Retention(Mixer):
         return StateNeed((self.H * self.dv * self.dk,), "float32")
 
     def kernel_libraries(self):
-        libs = ["core", "linear_attn"]
+        libs = ["core", "linear_attn", "chunk_scan"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
         return libs

@@ -97,7 +97,7 @@ class StateSpaceDuality(Mixer):
         return StateNeed((self.state_floats + (self.taps - 1) * self.C,), "float32")
 
     def kernel_libraries(self):
-        libs = ["core", "ssd", "linear_attn"]
+        libs = ["core", "ssd", "linear_attn", "chunk_scan"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
         return libs
