@@ -34,6 +34,8 @@
 // product is issued.  A table entry of a key that a row does see must name a page of the pool; one that
 // does not sets LL_ERR_PAGE_RANGE.
 //
+// Sink: one more key a head, of a given score and without a value: its share joins the row's sum at the end.
+//
 // Pairs: neighbouring query heads (2a, 2a + 1) are two score maps over the same keys and values and come out as one head,
 // z = o_even - lambda o_odd, z / sqrt(mean(z^2) + eps) * post (float32, before the gate and the one rounding).  Their rows
 // are neighbouring lanes of a warp.
@@ -54,6 +56,10 @@ struct AttnTcParams {
   int n_entries, nkv, group, tpb;   // tpb: tokens a CTA (floor(128 / group))
   int page_size, num_pages, window;
   int box_rows;                     // keys a K/V box: min(page_size, 64)
+  // where K and V of (page, kv head) start in their tensor maps: row page * page_rows + head * head_rows, column
+  // head * head_cols (a cache plane has a head's rows below the other's; rows of all heads side by side have its columns)
+  int page_rows, head_rows, head_cols;
+  const float* sink;                // a number a head: the score of one more key without a value, or null
   float scale_log2;
   // the key blocks of a row block may be split over up to nsplit CTAs (long contexts, few row blocks):
   // partial results (unnormalised O, reference maximum, sum) meet in scratch memory, the last CTA to
@@ -195,7 +201,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
           set_status(p.status, LL_ERR_PAGE_RANGE);   // a key that a row sees has no page of the pool
         page = 0;
       }
-      return (page * p.nkv + kvh) * p.page_size + kp % p.page_size;
+      return page * p.page_rows + kvh * p.head_rows + kp % p.page_size;
     };
     // order of the copies: K(0), K(1), then V(j) before K(j + 2), the order in which the MMAs want them
     auto load = [&](int j, int row, bool is_v) {
@@ -208,7 +214,8 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
       __syncwarp();
       if (lane < boxes) {
         const unsigned dst = at_smem(kv_s) + s * STAGE_BYTES + (is_v ? KV_BYTES : 0) + lane * p.box_rows * 128;
-        for (int h = 0; h < HB; ++h) at_tma_2d(dst + h * (KV_BYTES / HB), is_v ? &vmap : &kmap, h * 64, row, full);
+        for (int h = 0; h < HB; ++h)
+          at_tma_2d(dst + h * (KV_BYTES / HB), is_v ? &vmap : &kmap, kvh * p.head_cols + h * 64, row, full);
       }
     };
     int row0 = page_of(0), row1 = page_of(1);   // cache rows of blocks j and j + 1
@@ -429,11 +436,13 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
           m_cur = m_new;
           ++round;
         }
-        inv = l_cur > 0.f ? 1.0f / l_cur : 0.f;
+        m_ref = m_cur;
+        l_run = l_cur;
       }
-    } else {
-      inv = l_run > 0.f ? 1.0f / l_run : 0.f;
     }
+    // (the sink's share of the sum is added once, to the whole row's; a row without keys has none to show)
+    if (p.sink != nullptr && row_ok && m_ref != -INFINITY) l_run += exp2f(p.sink[kvh * p.group + g] * 1.4426950408889634f - m_ref);
+    inv = l_run > 0.f ? 1.0f / l_run : 0.f;
     if (finish && p.pairs) {
       float ss = 0.f;
 #pragma unroll
@@ -534,7 +543,7 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
                   const int* req_slot, int n_entries, int row_blocks, int nh, int nkv, int hd, int page_size,
                   int num_pages, int window, float scale, int nsplit, int split_len, float* scratch, int* counters,
                   const void* gate, long gate_stride, int pairs, float lambda, float post, float pair_eps, int* status,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, const float* sink = nullptr, long kv_stride = 0) {
   if (row_blocks <= 0 || n_entries <= 0) return 0;
   if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv != 0 || nkv > 65535 || nh / nkv > 128 || (pairs && (nh / nkv) % 2 != 0))
     return (int)cudaErrorInvalidValue;
@@ -573,6 +582,11 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
   p.post = post;
   p.pair_eps = pair_eps;
   p.status = status;
+  p.sink = sink;
+  p.page_rows = kv_stride ? page_size : nkv * page_size;
+  p.head_rows = kv_stride ? 0 : page_size;
+  p.head_cols = kv_stride ? hd : 0;
+  if ((kv_stride % 8) != 0 || ((uintptr_t)k_cache % 16) != 0 || ((uintptr_t)v_cache % 16) != 0) return (int)cudaErrorInvalidValue;
 
   CUtensorMap qmap, kmap, vmap;
   const cuuint32_t estr3[3] = {1, 1, 1};
@@ -586,8 +600,8 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
       return (int)cudaErrorInvalidValue;
   }
   for (int which = 0; which < 2; ++which) {
-    const cuuint64_t dims[2] = {(cuuint64_t)hd, (cuuint64_t)num_pages * nkv * page_size};
-    const cuuint64_t strides[1] = {(cuuint64_t)hd * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)hd * (kv_stride ? nkv : 1), (cuuint64_t)num_pages * (kv_stride ? 1 : nkv) * page_size};
+    const cuuint64_t strides[1] = {(cuuint64_t)(kv_stride ? kv_stride : hd) * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)p.box_rows};
     if (enc(which ? &vmap : &kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(which ? v_cache : k_cache),
             dims, strides, box, estr3, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -645,4 +659,19 @@ extern "C" int ll_attn_prefill_tc_pairs(void* out, long out_stride, const void* 
   return at_run(out, out_stride, q, q_stride, num_tokens, k_cache, v_cache, block_table, bt_stride, cu_q, ctx_len, req_slot,
                 n_entries, row_blocks, nh, nkv, hd, page_size, num_pages, window, scale, nsplit, split_len, scratch,
                 counters, gate, gate_stride, 1, lambda, post, pair_eps, status, stream);
+}
+
+// Keys and values that are rows of a product instead of a cache plane: row j of k and v (kv_stride numbers apart) holds all
+// kv heads side by side, a page is page_size (a multiple of 64) of these rows.  sink: float32 [nh] or null (see the head of
+// this file).
+extern "C" int ll_attn_prefill_tc_rows(void* out, long out_stride, const void* q, long q_stride, int num_tokens,
+                                       const void* k, const void* v, long kv_stride, const int* block_table, int bt_stride,
+                                       const int* cu_q, const int* ctx_len, const int* req_slot, int n_entries,
+                                       int row_blocks, int nh, int nkv, int hd, int page_size, int num_pages, int window,
+                                       float scale, int nsplit, int split_len, float* scratch, int* counters,
+                                       const float* sink, int* status, cudaStream_t stream) {
+  if (kv_stride < (long)nkv * hd || page_size % 64 != 0) return (int)cudaErrorInvalidValue;
+  return at_run(out, out_stride, q, q_stride, num_tokens, k, v, block_table, bt_stride, cu_q, ctx_len, req_slot, n_entries,
+                row_blocks, nh, nkv, hd, page_size, num_pages, window, scale, nsplit, split_len, scratch, counters, nullptr, 0,
+                0, 0.f, 0.f, 0.f, status, stream, sink, kv_stride);
 }

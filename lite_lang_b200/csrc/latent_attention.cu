@@ -15,6 +15,8 @@
 //   latent_prepare    per token: RMS norm of the latent, rotation of k_r and of every head's q_r, cache write
 //   latent_attention  per (token, 8 heads): online softmax over the visible rows of the request, i.e.
 //                     positions lo..p with lo = max(0, p - window + 1) (window <= 0: all)
+//   latent_unpage     for prompt portions whose keys and values are expanded (parts/latent_attention.py): the rows the
+//                     entries see out of their pages, all entries in one launch
 //   latent_gather, latent_masked_softmax: the pieces between two library products for long prompt portions,
 //                     where all (token, head) rows of a block of queries meet the same run of cached rows:
 //                     the run is copied out of its pages, scores = Q K^T and sum = P C are products, and the
@@ -23,64 +25,85 @@
 // every sum depends on the position only, not on how the tokens were cut into steps or batched.
 #include "common.cuh"
 
-// number j of a rotated part whose numbers are src[0 .. r)
+#define LA_LATENT_PIECES 4        // latents of up to 512 numbers: 4 a thread
+
+// the r numbers at src turned into dst (dst may be src): pairs below `half` by their angle (cs, sn), the rest as they are.
+// Called with consecutive `first` of a group of `step` threads.
 template <typename T>
-__device__ __forceinline__ float la_rotated(const T* src, int j, float p, const float* freq, int half, int half_split,
-                                            float amplitude) {
-  if (j >= 2 * half) return to_f32<T>(src[j]);
-  const int i = half_split ? (j < half ? j : j - half) : j >> 1;            // the pair, its first and its second number
-  const int iu = half_split ? i : 2 * i, iv = half_split ? i + half : 2 * i + 1;
-  float sn, cs;
-  sincosf(p * freq[i], &sn, &cs);
-  sn *= amplitude;
-  cs *= amplitude;
-  const float u = to_f32<T>(src[iu]), v = to_f32<T>(src[iv]);
-  return j == iv ? v * cs + u * sn : u * cs - v * sn;
+__device__ __forceinline__ void la_turn(T* dst, const T* src, int first, int step, int r, int half, int half_split,
+                                        const float* cs, const float* sn) {
+  for (int i = first; i < half; i += step) {
+    const int iu = half_split ? i : 2 * i, iv = half_split ? i + half : 2 * i + 1;      // the pair's two numbers
+    const float u = to_f32<T>(src[iu]), v = to_f32<T>(src[iv]);
+    dst[iu] = from_f32<T>(u * cs[i] - v * sn[i]);
+    dst[iv] = from_f32<T>(v * cs[i] + u * sn[i]);
+  }
+  if (dst != src)
+    for (int j = 2 * half + first; j < r; j += step) dst[j] = src[j];
 }
 
 // qsrc row t (row stride q_stride; the projection itself, or the output of a second product when the queries go
 // through a latent of their own): q heads at q_off, head h's rotated part at q_off + h * (d + r) + d; proj row t:
 // the latent at kv_off (R wide), then the rotated key part (r wide).  Both cos and sin are multiplied by
-// `amplitude` (a scaled rotation's factor; 1 otherwise).
+// `amplitude` (a scaled rotation's factor; 1 otherwise).  Tokens from `inplace_from` on have their rotated query parts
+// turned where they lie instead of into q_full.
 template <typename T>
 __global__ void __launch_bounds__(128)
 latent_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, int kv_off, const float* __restrict__ norm_w,
                       float eps, const float* __restrict__ freq, int rot_dims, const int* __restrict__ positions,
                       const int* __restrict__ slot_map, T* __restrict__ cache, long num_slots,
                       T* __restrict__ q_full, int H, int d, int r, int R, int* status, float amplitude,
-                      const T* __restrict__ qsrc, long q_stride, int half_split) {
+                      T* qsrc, long q_stride, int half_split, int inplace_from) {
+  extern __shared__ float la_cs[];      // cos [half], sin [half]
   __shared__ float scratch[32];
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int t = blockIdx.x, tid = threadIdx.x;
-  const T* row = proj + (size_t)t * proj_stride;
   const float p = (float)positions[t];
-  // every head's rotated query part -> q_full [tokens, H, R + r] behind the R latent-space numbers
   const int half = rot_dims / 2;
-  for (int i = tid; i < H * r; i += blockDim.x) {
-    const int h = i / r, j = i % r;
-    const T* src = qsrc + (size_t)t * q_stride + q_off + (size_t)h * (d + r) + d;
-    const float out = la_rotated<T>(src, j, p, freq, half, half_split, amplitude);
-    q_full[((size_t)t * H + h) * (R + r) + R + j] = from_f32<T>(out);
+  float* la_sn = la_cs + half;
+  for (int i = tid; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf(p * freq[i], &sn, &cs);
+    la_cs[i] = cs * amplitude;
+    la_sn[i] = sn * amplitude;
   }
   const long slot = slot_map ? slot_map[t] : -1;
-  if (slot < 0) return;     // padding token, or a run-step that only reads this plane
-  if (slot >= num_slots) {
-    if (tid == 0) set_status(status, LL_ERR_SLOT_RANGE);
-    return;
-  }
-  const T* lat = row + kv_off;
+  const bool store = slot >= 0 && slot < num_slots;     // (else: a padding token, or a run-step that only reads this plane)
+  if (slot >= num_slots && tid == 0) set_status(status, LL_ERR_SLOT_RANGE);
+  const T* lat = proj + (size_t)t * proj_stride + kv_off;
+  float x[LA_LATENT_PIECES];
   float ss = 0.f;
-  for (int i = tid; i < R; i += blockDim.x) {
-    const float x = to_f32<T>(lat[i]);
-    ss = fmaf(x, x, ss);
+  if (store) {
+#pragma unroll
+    for (int k = 0; k < LA_LATENT_PIECES; ++k) {
+      const int i = tid + 128 * k;
+      x[k] = i < R ? to_f32<T>(lat[i]) : 0.f;
+      ss = fmaf(x[k], x[k], ss);
+    }
+    for (int i = tid + 128 * LA_LATENT_PIECES; i < R; i += 128) ss = fmaf(to_f32<T>(lat[i]), to_f32<T>(lat[i]), ss);
   }
+  __syncthreads();
+  // every head's rotated query part: a group of 16 threads a head
+  if (r > 0) {
+    T* qrow = qsrc + (size_t)t * q_stride + q_off + d;
+    for (int h = tid >> 4; h < H; h += 8) {
+      T* src = qrow + (size_t)h * (d + r);
+      T* dst = t >= inplace_from ? src : q_full + ((size_t)t * H + h) * (R + r) + R;
+      la_turn<T>(dst, src, tid & 15, 16, r, half, half_split, la_cs, la_sn);
+    }
+  }
+  if (!store) return;
   ss = block_sum(ss, scratch);
   const float inv = 1.0f / sqrtf(ss / (float)R + eps);
   T* dst = cache + (size_t)slot * (R + r);
-  for (int i = tid; i < R; i += blockDim.x) dst[i] = from_f32<T>(to_f32<T>(lat[i]) * inv * norm_w[i]);
-  for (int j = tid; j < r; j += blockDim.x)
-    dst[R + j] = from_f32<T>(la_rotated<T>(lat + R, j, p, freq, half, half_split, amplitude));
+#pragma unroll
+  for (int k = 0; k < LA_LATENT_PIECES; ++k) {
+    const int i = tid + 128 * k;
+    if (i < R) dst[i] = from_f32<T>(x[k] * inv * norm_w[i]);
+  }
+  for (int i = tid + 128 * LA_LATENT_PIECES; i < R; i += 128) dst[i] = from_f32<T>(to_f32<T>(lat[i]) * inv * norm_w[i]);
+  la_turn<T>(dst + R, lat + R, tid, 128, r, half, half_split, la_cs, la_sn);
 }
 
 #define LA_TK 32
@@ -491,14 +514,72 @@ latent_masked_softmax_kernel(T* __restrict__ P, const float* __restrict__ S, int
 extern "C" int ll_latent_prepare(int dtype, const void* proj, long proj_stride, int q_off, int kv_off,
                                  const float* norm_w, float eps, const float* freq, int rot_dims, const int* positions,
                                  const int* slot_map, void* cache, long num_slots, void* q_full, int num_tokens, int H,
-                                 int d, int r, int R, int* status, float amplitude, const void* qsrc, long q_stride,
-                                 int half_split, cudaStream_t stream) {
+                                 int d, int r, int R, int* status, float amplitude, void* qsrc, long q_stride,
+                                 int half_split, int inplace_from, cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || d < 0 || r < 0 || R <= 0 || rot_dims < 0 || rot_dims > r) return (int)cudaErrorInvalidValue;
-  LL_DISPATCH_DTYPE(dtype, ll_launch(latent_prepare_kernel<T>, dim3(num_tokens), dim3(128), 0, stream, (const T*)proj,
+  LL_DISPATCH_DTYPE(dtype, ll_launch(latent_prepare_kernel<T>, dim3(num_tokens), dim3(128), (size_t)(rot_dims / 2) * 8, stream, (const T*)proj,
                                      proj_stride, q_off, kv_off, norm_w, eps, freq, rot_dims, positions, slot_map,
                                      (T*)cache, num_slots, (T*)q_full, H, d, r, R, status, amplitude,
-                                     (const T*)qsrc, q_stride, half_split));
+                                     (T*)qsrc, q_stride, half_split, inplace_from));
+  return LL_LAUNCH_RESULT();
+}
+
+// The cached rows that the entries' queries may see, contiguous: entry e's rows are those of the positions
+// lo_e .. ctx_e + q_e - 1 (lo_e = max(0, ctx_e - window + 1) with a window, else 0) from row 64 p_e on, p_e the pages of 64
+// rows that the entries before take; the rest of its last page is zeros.  For attention over these rows: table [E][max_pages]
+// (an entry's pages), rel [E] (positions before its first query) and own [E] = e.  A block copies 8 rows of a page.
+__global__ void __launch_bounds__(128)
+latent_unpage_kernel(uint4* __restrict__ dst, const uint4* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
+                     const int* __restrict__ cu_q, const int* __restrict__ ctx_len, const int* __restrict__ req_slot, int E,
+                     int pieces, int page_size, int num_pages, int window, int* __restrict__ table, int max_pages,
+                     int* __restrict__ rel, int* __restrict__ own, int* status) {
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int page = blockIdx.x, part = blockIdx.y;
+  int at = 0, e = 0, lo = 0, rows = 0;
+  for (; e < E; ++e) {
+    const int ctx = ctx_len[e];
+    lo = window > 0 ? max(0, ctx - window + 1) : 0;
+    rows = ctx + cu_q[e + 1] - cu_q[e] - lo;
+    const int pages = (rows + 63) / 64;
+    if (page < at + pages) break;
+    at += pages;
+  }
+  if (e == E) return;
+  const int lp = page - at;
+  if (part == 0 && threadIdx.x == 0) {
+    if (lp < max_pages) table[(size_t)e * max_pages + lp] = page;
+    if (lp == 0) {
+      rel[e] = ctx_len[e] - lo;
+      own[e] = e;
+    }
+  }
+  const int slot = req_slot[e];
+  const int* bt = block_table + (size_t)max(slot, 0) * bt_stride;
+  for (int i = threadIdx.x; i < 8 * pieces; i += 128) {
+    const int j = lp * 64 + part * 8 + i / pieces, c = i % pieces;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (j < rows && slot >= 0) {
+      const int pos = lo + j, lpage = pos / page_size;
+      const int pg = lpage < bt_stride ? bt[lpage] : -1;
+      if (pg >= 0 && pg < num_pages) v = cache[((size_t)pg * page_size + pos % page_size) * pieces + c];
+      else set_status(status, LL_ERR_PAGE_RANGE);
+    }
+    dst[((size_t)page * 64 + part * 8 + i / pieces) * pieces + c] = v;
+  }
+}
+
+// dst: bfloat16 [pages * 64][KD], KD a multiple of 8; `pages`: the entries' pages together (or more: those stay as they are)
+extern "C" int ll_latent_unpage(void* dst, const void* cache, const int* block_table, int bt_stride, const int* cu_q,
+                                const int* ctx_len, const int* req_slot, int E, int KD, int page_size, int num_pages,
+                                int window, int pages, int* table, int max_pages, int* rel, int* own, int* status,
+                                cudaStream_t stream) {
+  if (E <= 0 || pages <= 0) return 0;
+  if (KD <= 0 || KD % 8 != 0 || page_size <= 0 || ((uintptr_t)dst % 16) != 0 || ((uintptr_t)cache % 16) != 0)
+    return (int)cudaErrorInvalidValue;
+  ll_launch(latent_unpage_kernel, dim3(pages, 8), dim3(128), 0, stream, (uint4*)dst, (const uint4*)cache, block_table, bt_stride,
+            cu_q, ctx_len, req_slot, E, KD / 8, page_size, num_pages, window, table, max_pages, rel, own, status);
   return LL_LAUNCH_RESULT();
 }
 

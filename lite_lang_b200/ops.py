@@ -466,6 +466,19 @@ def attn_prefill_tc_blocks(q_lens, group: int) -> int:
 _attn_tc_scratch = {}
 
 
+def _attn_tc_scratch_for(device, row_blocks: int, num_kv_heads: int, nsplit: int, head_dim: int):
+    """Scratch memory and counters of the split keys' partial results (None, None without splits)."""
+    if nsplit <= 1:
+        return None, None
+    floats = row_blocks * num_kv_heads * nsplit * 128 * (head_dim + 2)
+    have = _attn_tc_scratch.get(device)
+    if have is None or have[0].numel() < floats or have[1].numel() < row_blocks * num_kv_heads:
+        have = (torch.empty(max(floats, have[0].numel() if have else 0), dtype=torch.float32, device=device),
+                torch.zeros(max(row_blocks * num_kv_heads, 1024), dtype=torch.int32, device=device))
+        _attn_tc_scratch[device] = have
+    return have
+
+
 def attn_prefill_tc_plan(entries, group: int, window: Optional[int], num_kv_heads: int = 1, slots: int = 0):
     """(row blocks, nsplit, split_len) of a step for ``attn_prefill_tc``.  ``entries``: (cached tokens, new tokens)
     per entry; a row block takes floor(128 / group) tokens and walks n key blocks of 64.
@@ -543,15 +556,7 @@ def attn_prefill_tc(out: torch.Tensor, q: torch.Tensor, q_stride: int, k_cache: 
     if nsplit is None:
         nsplit = attn_prefill_tc_splits(row_blocks, num_kv_heads, q.device)
     _need(nsplit in (1, 2, 4, 8), "attn_prefill_tc: nsplit is 1, 2, 4 or 8")
-    scratch = counters = None
-    if nsplit > 1:
-        floats = row_blocks * num_kv_heads * nsplit * 128 * (head_dim + 2)
-        have = _attn_tc_scratch.get(q.device)
-        if have is None or have[0].numel() < floats or have[1].numel() < row_blocks * num_kv_heads:
-            have = (torch.empty(max(floats, have[0].numel() if have else 0), dtype=torch.float32, device=q.device),
-                    torch.zeros(max(row_blocks * num_kv_heads, 1024), dtype=torch.int32, device=q.device))
-            _attn_tc_scratch[q.device] = have
-        scratch, counters = have
+    scratch, counters = _attn_tc_scratch_for(q.device, row_blocks, num_kv_heads, nsplit, head_dim)
     args = (_ptr(out), c_long(out.stride(0)), _ptr(q), c_long(q_stride), c_int(q.shape[0]),
             _ptr(k_cache), _ptr(v_cache), _ptr(block_table), c_int(block_table.stride(0)), _ptr(cu_q), _ptr(ctx_len),
             _ptr(req_slot), c_int(num_entries), c_int(row_blocks), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
@@ -570,6 +575,34 @@ def attn_prefill_tc(out: torch.Tensor, q: torch.Tensor, q_stride: int, k_cache: 
                                      _stream())
         return
     load_library("attn_tc").call("ll_attn_prefill_tc", *args, _ptr(status), _stream())
+
+
+def attn_prefill_tc_rows(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, table: torch.Tensor,
+                         cu_q: torch.Tensor, ctx_len: torch.Tensor, own: torch.Tensor, plan, num_heads: int, head_dim: int,
+                         window: Optional[int], scale: float, sink: Optional[torch.Tensor],
+                         status: Optional[torch.Tensor]) -> None:
+    """``attn_prefill_tc`` over keys and values that are rows of a product: row j of ``k`` and ``v`` ([rows, num_heads *
+    head_dim], equal row strides) holds all heads side by side (a kv head each), an entry's rows are the pages of 64 rows in
+    ``table``.  ``plan`` from ``attn_prefill_tc_plan``; ``sink`` (float32 [heads]): one more key of that score without a value."""
+    _need_cuda(out, q, k, v, table, cu_q, ctx_len, own, sink)
+    for t, nm in ((table, "table"), (cu_q, "cu_q"), (ctx_len, "ctx_len"), (own, "own")):
+        _i32(t, nm)
+    _f32(sink, "sink")
+    E, width = table.shape[0], num_heads * head_dim
+    _need(head_dim in (64, 128) and all(t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0
+                                        for t in (out, q, k, v)), "attn_prefill_tc_rows: bfloat16 rows, heads of 64 or 128")
+    _need(k.shape == v.shape and k.stride(0) == v.stride(0) and k.shape[1] == width and k.shape[0] % 64 == 0
+          and out.shape[1] == width and q.shape[1] >= width, "attn_prefill_tc_rows: shapes")
+    _need(cu_q.numel() >= E + 1 and ctx_len.numel() >= E and own.numel() >= E and (sink is None or sink.numel() == num_heads),
+          "attn_prefill_tc_rows: entry arrays too short")
+    row_blocks, nsplit, split_len = plan
+    scratch, counters = _attn_tc_scratch_for(q.device, row_blocks, num_heads, nsplit, head_dim)
+    load_library("attn_tc").call(
+        "ll_attn_prefill_tc_rows", _ptr(out), c_long(out.stride(0)), _ptr(q), c_long(q.stride(0)), c_int(q.shape[0]), _ptr(k),
+        _ptr(v), c_long(k.stride(0)), _ptr(table), c_int(table.stride(0)), _ptr(cu_q), _ptr(ctx_len), _ptr(own), c_int(E),
+        c_int(row_blocks), c_int(num_heads), c_int(num_heads), c_int(head_dim), c_int(64), c_int(k.shape[0] // 64),
+        c_int(window or 0), c_float(scale), c_int(nsplit), c_int(max(1, int(split_len))), _ptr(scratch), _ptr(counters),
+        _ptr(sink), _ptr(status), _stream())
 
 
 _sample_scratch = {}
@@ -1254,12 +1287,16 @@ def delta_out(out: torch.Tensor, o: torch.Tensor, weight: torch.Tensor, gate: to
 def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, eps: float, freq: torch.Tensor,
                    rot_dims: int, positions: torch.Tensor, slot_map: Optional[torch.Tensor], cache: torch.Tensor,
                    q_full: torch.Tensor, H: int, d: int, r: int, R: int, status: Optional[torch.Tensor],
-                   amplitude: float = 1.0, q: Optional[torch.Tensor] = None, half_split: bool = False) -> None:
+                   amplitude: float = 1.0, q: Optional[torch.Tensor] = None, half_split: bool = False,
+                   inplace_from: Optional[int] = None) -> None:
     """Per token: the latent's RMS norm and the rotated key part into the cache row, and every head's rotated
     query part into ``q_full`` [tokens, H, R + r] behind the R latent-space numbers (which a product fills).
     ``q``: the rows that hold the query heads at ``q_off`` when they are not rows of ``proj`` (queries made by a
     second product); ``amplitude``: a factor on cos and sin; ``half_split``: pairs (i, i + rot_dims / 2) instead of
-    neighbours."""
+    neighbours.  ``inplace_from``: tokens from there on have their rotated query parts turned where they lie (``q_full``
+    holds the tokens before)."""
+    n = proj.shape[0]
+    first = n if inplace_from is None else int(inplace_from)
     _need_cuda(proj, norm_w, freq, positions, slot_map, cache, q_full, q)
     q = proj if q is None else q
     _need(q.dtype == proj.dtype and q.stride(1) == 1 and q.shape[0] == proj.shape[0], "latent_prepare: q rows")
@@ -1269,13 +1306,38 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Te
     _i32(slot_map, "slot_map")
     _need(proj.stride(1) == 1 and cache.is_contiguous() and cache.dtype == proj.dtype and cache.shape[-1] == R + r
           and cache.shape[1] == 1, "latent_prepare: the cache plane is [pages, 1, page, latent + rotated]")
-    _need(q_full.is_contiguous() and q_full.dtype == proj.dtype and tuple(q_full.shape[1:]) == (H, R + r),
-          "latent_prepare: q_full is [tokens, H, latent + rotated] of the projections' dtype")
+    _need(q_full.is_contiguous() and q_full.dtype == proj.dtype and tuple(q_full.shape[1:]) == (H, R + r)
+          and q_full.shape[0] >= min(first, n), "latent_prepare: q_full is [tokens, H, latent + rotated] of the projections' dtype")
     load_library("latent_attn").call(
         "ll_latent_prepare", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), c_int(q_off), c_int(kv_off),
         _ptr(norm_w), c_float(eps), _ptr(freq), c_int(rot_dims), _ptr(positions), _ptr(slot_map), _ptr(cache),
         c_long(cache.shape[0] * cache.shape[2]), _ptr(q_full), c_int(proj.shape[0]), c_int(H), c_int(d), c_int(r),
-        c_int(R), _ptr(status), c_float(amplitude), _ptr(q), c_long(q.stride(0)), c_int(1 if half_split else 0), _stream())
+        c_int(R), _ptr(status), c_float(amplitude), _ptr(q), c_long(q.stride(0)), c_int(1 if half_split else 0),
+        c_int(first), _stream())
+
+
+def latent_unpage(cache: torch.Tensor, block_table: torch.Tensor, cu_q: torch.Tensor, ctx_len: torch.Tensor,
+                  req_slot: torch.Tensor, spans, window: Optional[int], status: Optional[torch.Tensor]):
+    """The cached rows that entries' queries may see, contiguous and in pages of 64 rows: ``spans`` is (cached tokens, new
+    tokens) of each entry (host).  Returns (rows [pages * 64, width], table [entries, most pages of one], positions before
+    each entry's first query, its place): what attention over the rows takes for block table, context and slot."""
+    _need_cuda(cache, block_table, cu_q, ctx_len, req_slot)
+    for t, nm in ((block_table, "block_table"), (cu_q, "cu_q"), (ctx_len, "ctx_len"), (req_slot, "req_slot")):
+        _i32(t, nm)
+    E, KD = len(spans), cache.shape[-1]
+    _need(cache.dtype == torch.bfloat16 and cache.is_contiguous() and cache.shape[1] == 1 and KD % 8 == 0,
+          "latent_unpage: a bfloat16 plane [pages, 1, page, width], width a multiple of 8")
+    _need(cu_q.numel() >= E + 1 and ctx_len.numel() >= E and req_slot.numel() >= E, "latent_unpage: entry arrays too short")
+    pages = [(c + n - (max(0, c - window + 1) if window else 0) + CHUNK - 1) // CHUNK for c, n in spans]
+    total, most = sum(pages), max(pages)
+    rows = torch.empty((total * CHUNK, KD), dtype=cache.dtype, device=cache.device)
+    ints = torch.empty(E * (most + 2), dtype=torch.int32, device=cache.device)
+    table, rel, own = ints[:E * most].view(E, most), ints[E * most:E * (most + 1)], ints[E * (most + 1):]
+    load_library("latent_attn").call(
+        "ll_latent_unpage", _ptr(rows), _ptr(cache), _ptr(block_table), c_int(block_table.stride(0)), _ptr(cu_q), _ptr(ctx_len),
+        _ptr(req_slot), c_int(E), c_int(KD), c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window or 0), c_int(total),
+        _ptr(table), c_int(most), _ptr(rel), _ptr(own), _ptr(status), _stream())
+    return rows, table, rel, own
 
 
 def latent_attention(out: torch.Tensor, q_full: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, step,

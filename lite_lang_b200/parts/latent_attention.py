@@ -7,10 +7,12 @@ score = (q_plain . k_plain + q_rot . k_rot) * ``scale``; position i sees j with 
 (None: every earlier position); softmax; output projection over the concatenated heads.
 
 Only c and the rotated key part are cached: ``kv_rank + rot_dim`` numbers a token in one plane of a paged
-group with one kv head and no value plane.  Nothing per head is expanded from the cache either: since
+group with one kv head and no value plane.  For single tokens nothing per head is expanded from the cache either: since
 q_plain . (Uk_h c) = (Uk_h^T q_plain) . c, the queries are taken into the latent space by a batched product
 over heads, attention runs there (keys: the cached rows; values: their first ``kv_rank`` numbers), and a
-second batched product expands each head's weighted sum of latents with Uv_h.
+second batched product expands each head's weighted sum of latents with Uv_h.  That is kv_rank numbers a head, key and
+query where the expanded form has ``dim``; portions of prompts, whose queries share the keys, are served with the rows they
+see expanded once into every head's keys and values (one product, nothing of it kept) and the tcgen05 attention over them.
 
 Rotation: pairs of the rotated part's first ``rot_dims`` numbers (``rot_layout`` "interleaved": 2i with 2i+1;
 "half_split": i with i + rot_dims / 2) turn by position * ``rot_base``^(-2i / rot_dims); the rest passes unchanged.  Angles (float32 position times a
@@ -120,6 +122,15 @@ class LatentAttention(Mixer):
         self.w_uk = fetch("uk").to(dtype).to(device).contiguous().view(self.H, self.d, self.R)
         self.w_uv_t = fetch("uv").to(dtype).to(device).contiguous().view(self.H, self.dv, self.R).transpose(1, 2)
         self.w_o = fetch("o").to(dtype).to(device).contiguous()
+        # a cached row into every head's key [plain | rotated] and value: [Uk_h 0; 0 1] for the keys, [Uv_h 0] for the values
+        self.w_kv = None
+        if dtype == torch.bfloat16 and self.d + self.r == self.dv and self.dv in (64, 128) and (self.R + self.r) % 8 == 0:
+            wide = torch.zeros((2, self.H, self.dv, self.R + self.r), dtype=dtype, device=device)
+            wide[0, :, :self.d, :self.R] = self.w_uk
+            if self.r:
+                wide[0, :, self.d:, self.R:] = torch.eye(self.r, dtype=dtype, device=device)
+            wide[1, :, :, :self.R] = self.w_uv_t.transpose(1, 2)
+            self.w_kv = wide.view(2 * self.H * self.dv, self.R + self.r)
         # frequencies as the rotary part makes them (float64, the scaling's ramp, rounded once)
         rope = build_part("position", _PartSpec("rope_computed", {
             "rotary_dim": self.rot_dims, "theta": self.rot_base, "layout": self.rot_layout,
@@ -130,7 +141,7 @@ class LatentAttention(Mixer):
         self.freq = (freq.to(torch.float32) if freq.numel() else torch.zeros(1)).to(device).contiguous()
 
     def weight_bytes(self) -> int:
-        ts = [self.w_in, self.w_uk, self.w_uv_t, self.w_o, self.w_uq]
+        ts = [self.w_in, self.w_uk, self.w_uv_t, self.w_o, self.w_uq]      # (a step reads these or their expanded form)
         return sum(t.numel() * t.element_size() for t in ts if t is not None)
 
     def cache_need(self):
@@ -140,6 +151,8 @@ class LatentAttention(Mixer):
         libs = ["core", "latent_attn"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
+            if self.w_kv is not None:
+                libs.append("attn_tc")
         return libs
 
     # Prompt portions of at least this many tokens go through library products (scores and weighted sums of a
@@ -147,6 +160,40 @@ class LatentAttention(Mixer):
     # that walks each query's keys itself.
     PRODUCT_MIN_TOKENS = 32
     QUERY_BLOCK = 256
+    # Portions of at least this many tokens are served with expanded keys and values, as long as the rows to expand are at
+    # most so many times the step's tokens in them (a row costs (kv_rank + rot_dim) * 2 vdim multiply-adds a head to expand
+    # and saves kv_rank * 2 a head and query; below the line the step's time is its launches, which are fewer this way).
+    # Measured on a B200, 12 heads of 128, a latent of 512: 2,048 tokens in three requests with a window of 512, 237 us of
+    # kernels in 41 launches by the products over the latents, 76 us in 6 launches this way (690 and 131 us with the host).
+    EXPAND_MIN_TOKENS = 16
+    EXPAND_MAX_ROWS = 16
+
+    def _expanded(self, step, qrows):
+        """(cached, new) tokens of the step's portions if they are to be served with expanded keys and values, else None."""
+        entries = None if getattr(step, "captured", False) else getattr(step, "entries", None)
+        ctxs = getattr(step, "entry_ctx", None)
+        if self.w_kv is None or not ops.TC_ENABLED or entries is None or ctxs is None or qrows.stride(0) % 8:
+            return None
+        single = step.num_single
+        spans = [(c, len(e.tokens)) for e, c in zip(entries[single:], ctxs[single:])]
+        if not spans or min(q for _, q in spans) < self.EXPAND_MIN_TOKENS:
+            return None
+        rows = sum(q + (min(c, self.window - 1) if self.window else c) for c, q in spans)
+        return spans if rows <= self.EXPAND_MAX_ROWS * sum(q for _, q in spans) else None
+
+    def _attend_expanded(self, heads, qrows, step, cache, spans) -> None:
+        """The portions behind the step's single tokens: ``heads`` rows = attention over expanded keys and values."""
+        n1, H, hd = step.num_single, self.H, self.dv
+        rows, table, rel, own = ops.latent_unpage(cache.k, cache.block_table, step.cu_q[n1:], step.ctx_len[n1:],
+                                                  step.req_slot[n1:], spans, self.window, step.status)
+        kv = ops.linear(rows, self.w_kv)
+        key = ("latent_expanded", H, self.window)
+        plan = step.scratch.get(key)
+        if plan is None:
+            seen = [(min(c, self.window - 1) if self.window else c, q) for c, q in spans]
+            plan = step.scratch[key] = ops.attn_prefill_tc_plan(seen, 1, self.window, H, 2 * ops.sm_count(heads.device))
+        ops.attn_prefill_tc_rows(heads, qrows, kv[:, :H * hd], kv[:, H * hd:], table, step.cu_q[n1:], rel, own, plan, H, hd,
+                                 self.window, self.scale, self.sink_w, step.status)
 
     def forward(self, x, step, cache):
         n, dev, H, d, r, R = x.shape[0], x.device, self.H, self.d, self.r, self.R
@@ -156,17 +203,22 @@ class LatentAttention(Mixer):
             cq = torch.empty((n, self.q_rank), dtype=x.dtype, device=dev)
             ops.rmsnorm(cq, proj[:, :self.q_rank], self.q_norm_w, self.eps)
             qrows = ops.linear(cq, self.w_uq)
-        q_full = torch.empty((n, H, R + r), dtype=x.dtype, device=dev)
+        spans = self._expanded(step, qrows)
+        na = n if spans is None else step.num_single        # tokens that meet the latents themselves
+        q_full = torch.empty((na, H, R + r), dtype=x.dtype, device=dev)
         ops.latent_prepare(proj, 0, self.kv_off, self.norm_w, self.eps, self.freq, self.rot_dims, step.positions,
                            cache.slot_map if cache.writable else None, cache.k, q_full, H, d, r, R, step.status,
-                           amplitude=self.amplitude, q=qrows, half_split=self.half_split)
-        # queries into the latent space: a_h = Uk_h^T q_h, written in front of the rotated parts
-        q_plain = qrows[:, :H * (d + r)].view(n, H, d + r)[:, :, :d].permute(1, 0, 2)         # [H, n, d]
-        ops.batched_heads(q_plain, self.w_uk, out=q_full[:, :, :R].permute(1, 0, 2))            # [H, n, R]
-        lat = torch.empty((n, H, R), dtype=x.dtype, device=dev)
-        self.attend(lat, q_full, step, cache)
+                           amplitude=self.amplitude, q=qrows, half_split=self.half_split, inplace_from=na)
         heads = torch.empty((n, H * self.dv), dtype=x.dtype, device=dev)
-        ops.batched_heads(lat.permute(1, 0, 2), self.w_uv_t, out=heads.view(n, H, self.dv).permute(1, 0, 2))
+        if na:
+            # queries into the latent space: a_h = Uk_h^T q_h, written in front of the rotated parts
+            q_plain = qrows[:na, :H * (d + r)].view(na, H, d + r)[:, :, :d].permute(1, 0, 2)         # [H, na, d]
+            ops.batched_heads(q_plain, self.w_uk, out=q_full[:, :, :R].permute(1, 0, 2))            # [H, na, R]
+            lat = torch.empty((na, H, R), dtype=x.dtype, device=dev)
+            self.attend(lat, q_full, step, cache, spans is not None)
+            ops.batched_heads(lat.permute(1, 0, 2), self.w_uv_t, out=heads[:na].view(na, H, self.dv).permute(1, 0, 2))
+        if spans is not None:
+            self._attend_expanded(heads, qrows, step, cache, spans)
         if self.channel_gate:
             ops.gate_rows(heads, proj[:, self.gate_off:self.gate_off + H * self.dv])
         return ops.linear(heads, self.w_o, partial_ok=self.partial_ok)
@@ -185,11 +237,11 @@ class LatentAttention(Mixer):
         nsplit = max(1, min(tiles, (2 * ops.sm_count(device)) // max(1, ctas), 16))
         return nsplit, (tiles + nsplit - 1) // nsplit
 
-    def attend(self, lat, q_full, step, cache) -> None:
+    def attend(self, lat, q_full, step, cache, single_only: bool = False) -> None:
         n, H, R, r = q_full.shape[0], self.H, self.R, self.r
         args = (H, R, r, cache.page_size, self.window, self.scale)
         entries = None if getattr(step, "captured", False) else getattr(step, "entries", None)
-        if entries is None or all(len(e.tokens) < self.PRODUCT_MIN_TOKENS for e in entries):
+        if single_only or entries is None or all(len(e.tokens) < self.PRODUCT_MIN_TOKENS for e in entries):
             ops.latent_attention(lat, q_full, cache.k, cache.block_table, step, 0, n, *args,
                                  *self._splits(n, step, lat.device), sink=self.sink_w)
             return
