@@ -1,0 +1,284 @@
+// Paged attention in true float32 on tensor cores (head size 64 or 128, any page size and group): prompt portions and single
+// tokens.
+//
+// The float32 path's general kernel (attention_generic.cu) gives a block a (token, kv head) pair and reads the keys once for
+// its group of heads only: 337 us for two prompts of 262 and 439 tokens with 12 heads of 128 on 2 kv heads (71 us here), and
+// 704 us for 64 single tokens at contexts of 500 to 1,000, whose blocks walk their keys alone.  Here a CTA takes 64 rows
+// (a row = a (token, query head of the kv head's group) pair, token-major), so the keys are read once for 64 rows, and both
+// products run on mma.sync with every float32 operand as three bfloat16 terms that hold its 24 bits (mma_split.cuh):
+//   S [64 x 32]  = Q K^T     a warp 16 rows, 6 products a step of 16 channels
+//   O [64 x HD] += P V       P from the accumulators' registers
+// Two groups of four warps walk the tiles of 32 keys alternately, each with its own maximum, sum and O, and meet at the end in
+// shared memory: two tiles are on their way at a time and one group's softmax lies beside the other's products.  A tile's rows
+// of V are asked for before its scores and the next tile's rows of K before its second product (registers), and become terms
+// on their way into shared memory.
+//
+// Scores, softmax (expf) and sums are float32.  Keys that a row may not see get probability 0 by selection and their rows
+// of V are zeros, whatever the page holds.  The order of a row's sums depends on the tiles (which start at multiples of 32
+// positions) and, through the two groups, on the first tile that its row block sees.
+#include "mma_split.cuh"
+
+#define AF_THREADS 256
+#define AF_TK 32
+#define AF_ROWS 64
+
+struct AttnF32Params {
+  float* out;
+  long out_stride;
+  const float* q;
+  long q_stride;
+  const float* k_cache;      // [pages, nkv, page_size, HD]
+  const float* v_cache;
+  const int* block_table;
+  int bt_stride;
+  const int* cu_q;
+  const int* ctx_len;
+  const int* req_slot;
+  int n_entries, nkv, group, page_size, num_pages, window, row_blocks;
+  float scale;
+  int* status;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(AF_THREADS, 1)
+attn_f32_kernel(const AttnF32Params p) {
+  constexpr int P = HD + 8, NO = HD / 8, LOADS = AF_TK * HD / 4 / 128;      // 16-byte pieces of K (and of V) a thread brings
+  extern __shared__ __align__(16) unsigned char af_smem[];
+  bf16* qs = reinterpret_cast<bf16*>(af_smem);                 // [3][64][P]
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = warp >> 2, gt = tid & 127;
+  bf16* ks = qs + 3 * AF_ROWS * P + half * (6 * AF_TK * P);    // this group's tile: K [3][32][P], V [3][32][P]
+  bf16* vs = ks + 3 * AF_TK * P;
+  const int kvh = blockIdx.y;
+  int rb = p.row_blocks - 1 - blockIdx.x;                      // the later, heavier blocks of the step first
+  int entry = -1, rows = 0;
+  for (int e = 0; e < p.n_entries; ++e) {
+    const int n = (p.cu_q[e + 1] - p.cu_q[e]) * p.group, nb = (n + AF_ROWS - 1) / AF_ROWS;
+    if (rb < nb) {
+      entry = e;
+      rows = n;
+      break;
+    }
+    rb -= nb;
+  }
+  if (entry < 0) return;
+  const int slot = p.req_slot[entry], tok0 = p.cu_q[entry], ctx = p.ctx_len[entry];
+  const int r0 = rb * AF_ROWS, rl = min(rows, r0 + AF_ROWS) - 1;       // rows r0 .. rl of the entry
+  const int head0 = kvh * p.group;
+  if (slot < 0) {
+    for (int i = tid; i < (rl - r0 + 1) * HD; i += AF_THREADS) {
+      const int r = r0 + i / HD;
+      p.out[(size_t)(tok0 + r / p.group) * p.out_stride + (size_t)(head0 + r % p.group) * HD + i % HD] = 0.f;
+    }
+    return;
+  }
+  const int hi = ctx + rl / p.group, lo = p.window > 0 ? max(0, ctx + r0 / p.group - p.window + 1) : 0;
+  const int tile0 = lo / AF_TK, tiles = hi / AF_TK - tile0 + 1;
+  const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+
+  float4 in[LOADS];                                            // rows on their way
+  auto ask = [&](const float* cache, int tile) {
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) {
+      const int i = j * 128 + gt, kk = i / (HD / 4), c = (i % (HD / 4)) * 4, pos = (tile0 + tile) * AF_TK + kk;
+      in[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (pos >= lo && pos <= hi) {
+        const int lp = pos / p.page_size, page = lp < p.bt_stride ? bt[lp] : -1;
+        if (page >= 0 && page < p.num_pages)
+          in[j] = *reinterpret_cast<const float4*>(cache + (((size_t)page * p.nkv + kvh) * p.page_size + pos % p.page_size) * HD + c);
+        else
+          set_status(p.status, LL_ERR_PAGE_RANGE);
+      }
+    }
+  };
+  auto put4 = [](bf16* d, const float4& v, int plane) {
+    uint2 t0, t1, t2;
+    ms_split(v.x, v.y, t0.x, t1.x, t2.x);
+    ms_split(v.z, v.w, t0.y, t1.y, t2.y);
+    *reinterpret_cast<uint2*>(d) = t0;
+    *reinterpret_cast<uint2*>(d + plane) = t1;
+    *reinterpret_cast<uint2*>(d + 2 * plane) = t2;
+  };
+  auto put = [&](bf16* dst) {
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) {
+      const int i = j * 128 + gt, kk = i / (HD / 4), cc = (i % (HD / 4)) * 4;
+      put4(dst + kk * P + cc, in[j], AF_TK * P);
+    }
+  };
+  if (half < tiles) ask(p.k_cache, half);
+  for (int i = tid; i < AF_ROWS * (HD / 4); i += AF_THREADS) {
+    const int rr = i / (HD / 4), c = (i % (HD / 4)) * 4, r = r0 + rr;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r <= rl) v = *reinterpret_cast<const float4*>(p.q + (size_t)(tok0 + r / p.group) * p.q_stride + (size_t)(head0 + r % p.group) * HD + c);
+    put4(qs + rr * P + c, v, AF_ROWS * P);
+  }
+  __syncthreads();
+  const int m8 = lane >> 3, r8 = lane & 7, g = lane >> 2, c = lane & 3;
+  const int row = (warp & 3) * 16;
+  const unsigned qs_b = ms_smem(qs), ks_b = ms_smem(ks), vs_b = ms_smem(vs);
+  const int ra = r0 + row + g, rb8 = ra + 8;                   // the thread's two rows, their positions
+  const int pa = ra <= rl ? ctx + ra / p.group : -1, pb = rb8 <= rl ? ctx + rb8 / p.group : -1;
+  const int la = p.window > 0 ? pa - p.window + 1 : 0, lb = p.window > 0 ? pb - p.window + 1 : 0;
+  float o[NO][4], m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+#pragma unroll
+  for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  for (int tile = half; tile < tiles; tile += 2) {
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");      // the group is done with the tile before
+    put(ks);
+    ask(p.v_cache, tile);
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+    float s[4][4], low[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = low[i][j] = 0.f;
+#pragma unroll
+    for (int kt = 0; kt < HD / 16; ++kt) {
+      unsigned a[3][4], b[4][3][2];
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        ms_ldm4(a[q], qs_b + 2 * ((q * AF_ROWS + row + (m8 & 1) * 8 + r8) * P + kt * 16 + (m8 >> 1) * 8));
+      const unsigned at = ks_b + 2 * (((m8 >> 1) * 8 + r8) * P + kt * 16 + (m8 & 1) * 8);
+      ms_load_b<3, false>(b, at, 2 * AF_TK * P);
+      ms_load_b<3, false>(b + 2, at + 2 * 16 * P, 2 * AF_TK * P);
+      ms_terms<4, 3, 3>(s, low, a, b);
+    }
+    const int k0 = (tile0 + tile) * AF_TK;
+    float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int pos = k0 + i * 8 + 2 * c + (j & 1);
+        const bool seen = j < 2 ? (pos <= pa && pos >= la) : (pos <= pb && pos >= lb);
+        s[i][j] = seen ? (s[i][j] + low[i][j]) * p.scale : -INFINITY;
+        if (j < 2) x0 = fmaxf(x0, s[i][j]);
+        else x1 = fmaxf(x1, s[i][j]);
+      }
+#pragma unroll
+    for (int w = 1; w < 4; w <<= 1) {
+      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, w));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, w));
+    }
+    const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+    const float u0 = n0 == -INFINITY ? 0.f : n0, u1 = n1 == -INFINITY ? 0.f : n1;
+    const float f0 = expf(m0 - u0), f1 = expf(m1 - u1);          // (-inf: nothing so far, 0)
+    m0 = n0;
+    m1 = n1;
+    float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s[i][0] = expf(s[i][0] - u0);
+      s[i][1] = expf(s[i][1] - u0);
+      s[i][2] = expf(s[i][2] - u1);
+      s[i][3] = expf(s[i][3] - u1);
+      t0 += s[i][0] + s[i][1];
+      t1 += s[i][2] + s[i][3];
+    }
+    l0 = l0 * f0 + t0;
+    l1 = l1 * f1 + t1;
+    put(vs);
+    unsigned a[2][3][4];
+#pragma unroll
+    for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        ms_split(s[2 * kt + q][0], s[2 * kt + q][1], a[kt][0][2 * q], a[kt][1][2 * q], a[kt][2][2 * q]);
+        ms_split(s[2 * kt + q][2], s[2 * kt + q][3], a[kt][0][2 * q + 1], a[kt][1][2 * q + 1], a[kt][2][2 * q + 1]);
+      }
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+#pragma unroll
+    for (int nt = 0; nt < NO; nt += 4) {
+      if (nt == NO - 4 && tile + 2 < tiles) ask(p.k_cache, tile + 2);
+      float d[4][4], small[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[i][j] = small[i][j] = 0.f;
+#pragma unroll
+      for (int kt = 0; kt < 2; ++kt) {
+        unsigned b[4][3][2];
+        const unsigned at = vs_b + 2 * ((kt * 16 + (m8 & 1) * 8 + r8) * P + nt * 8 + (m8 >> 1) * 8);
+        ms_load_b<3, true>(b, at, 2 * AF_TK * P);
+        ms_load_b<3, true>(b + 2, at + 32, 2 * AF_TK * P);
+        ms_terms<4, 3, 3>(d, small, a[kt], b);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[nt + i][j] = fmaf(o[nt + i][j], j < 2 ? f0 : f1, d[i][j] + small[i][j]);
+    }
+  }
+  // sums over the four lanes of a row, then the second group's rows join the first's
+#pragma unroll
+  for (int w = 1; w < 4; w <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, w);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+  }
+  __syncthreads();                                             // nobody's tile or query is needed any more
+  float* meet = reinterpret_cast<float*>(af_smem);             // [64][HD + 8]: O, then maximum and sum at HD, HD + 1
+  if (half == 1) {
+    float* d0 = meet + (row + g) * P;
+    float* d1 = d0 + 8 * P;
+#pragma unroll
+    for (int i = 0; i < NO; ++i) {
+      *reinterpret_cast<float2*>(d0 + i * 8 + 2 * c) = make_float2(o[i][0], o[i][1]);
+      *reinterpret_cast<float2*>(d1 + i * 8 + 2 * c) = make_float2(o[i][2], o[i][3]);
+    }
+    if (c == 0) {
+      d0[HD] = m0; d0[HD + 1] = l0;
+      d1[HD] = m1; d1[HD + 1] = l1;
+    }
+  }
+  __syncthreads();
+  if (half == 0) {
+    const float* s0 = meet + (row + g) * P;
+    const float* s1 = s0 + 8 * P;
+    auto weights = [](float m, float l, float mq, float lq, float& w, float& wq) {
+      const float top = fmaxf(m, mq), u = top == -INFINITY ? 0.f : top;
+      w = expf(m - u);
+      wq = expf(mq - u);
+      const float sum = l * w + lq * wq, inv = sum > 0.f ? 1.0f / sum : 0.f;
+      w *= inv;
+      wq *= inv;
+    };
+    float w0, q0, w1, q1;
+    weights(m0, l0, s0[HD], s0[HD + 1], w0, q0);
+    weights(m1, l1, s1[HD], s1[HD + 1], w1, q1);
+    float* oa = p.out + (size_t)(tok0 + ra / p.group) * p.out_stride + (size_t)(head0 + ra % p.group) * HD + 2 * c;
+    float* ob = p.out + (size_t)(tok0 + rb8 / p.group) * p.out_stride + (size_t)(head0 + rb8 % p.group) * HD + 2 * c;
+#pragma unroll
+    for (int i = 0; i < NO; ++i) {
+      const float2 x = *reinterpret_cast<const float2*>(s0 + i * 8 + 2 * c), y = *reinterpret_cast<const float2*>(s1 + i * 8 + 2 * c);
+      if (ra <= rl) *reinterpret_cast<float2*>(oa + i * 8) = make_float2(o[i][0] * w0 + x.x * q0, o[i][1] * w0 + x.y * q0);
+      if (rb8 <= rl) *reinterpret_cast<float2*>(ob + i * 8) = make_float2(o[i][2] * w1 + y.x * q1, o[i][3] * w1 + y.y * q1);
+    }
+  }
+}
+
+// q: float32, head h of token t at q + t * q_stride + h * hd; out float32 [tokens, nh * hd].  cu_q, ctx_len, req_slot: the
+// entries' arrays (cu_q[e] counts the step's tokens); row_blocks: sum over the entries of ceil(new tokens * group / 64).
+extern "C" int ll_attn_f32(float* out, long out_stride, const float* q, long q_stride, const float* k_cache,
+                           const float* v_cache, const int* block_table, int bt_stride, const int* cu_q, const int* ctx_len,
+                           const int* req_slot, int n_entries, int row_blocks, int nh, int nkv, int hd, int page_size,
+                           int num_pages, int window, float scale, int* status, cudaStream_t stream) {
+  if (row_blocks <= 0 || n_entries <= 0) return 0;
+  if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv != 0 || nkv > 65535 || page_size <= 0 || (q_stride % 4) != 0 ||
+      (out_stride % 2) != 0 || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16) != 0 || ((uintptr_t)out % 8) != 0)
+    return (int)cudaErrorInvalidValue;
+  AttnF32Params p{out, out_stride, q, q_stride, k_cache, v_cache, block_table, bt_stride, cu_q, ctx_len, req_slot, n_entries,
+                  nkv, nh / nkv, page_size, num_pages, window, row_blocks, scale, status};
+  const size_t smem = 2 * (size_t)(hd + 8) * 3 * (AF_ROWS + 4 * AF_TK);
+  if (hd == 128) {
+    const cudaError_t rc = cudaFuncSetAttribute(attn_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (rc != cudaSuccess) return (int)rc;
+    ll_launch(attn_f32_kernel<128>, dim3(row_blocks, nkv), dim3(AF_THREADS), smem, stream, p);
+  } else {
+    const cudaError_t rc = cudaFuncSetAttribute(attn_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (rc != cudaSuccess) return (int)rc;
+    ll_launch(attn_f32_kernel<64>, dim3(row_blocks, nkv), dim3(AF_THREADS), smem, stream, p);
+  }
+  return LL_LAUNCH_RESULT();
+}

@@ -218,6 +218,38 @@ def paged_attention_generic(out: torch.Tensor, q: torch.Tensor, q_stride: int, k
                 c_int(window or 0), c_float(scale), _ptr(status), _stream())
 
 
+def attn_f32_supported(q: torch.Tensor, k_cache: torch.Tensor, head_dim: int, value_head_dim: int) -> bool:
+    """Whether ``attn_f32`` takes this shape."""
+    return (q.dtype == torch.float32 and head_dim in (64, 128) and value_head_dim == head_dim and q.stride(0) % 4 == 0
+            and q.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0)
+
+
+def attn_f32(out: torch.Tensor, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
+             cu_q: torch.Tensor, ctx_len: torch.Tensor, req_slot: torch.Tensor, q_lens, num_heads: int, num_kv_heads: int,
+             head_dim: int, page_size: int, window: Optional[int], scale: float, status: Optional[torch.Tensor]) -> None:
+    """Attention of entries over their requests' cached keys in true float32 on tensor cores (csrc/attention_f32.cu).
+    ``cu_q``, ``ctx_len``, ``req_slot``: the arrays from the first of these entries on (``q`` and ``out`` hold all of the step's
+    tokens); ``q_lens``: new tokens of each entry (host)."""
+    _need_cuda(out, q, k_cache, v_cache, block_table, cu_q, ctx_len, req_slot)
+    for t, nm in ((block_table, "block_table"), (cu_q, "cu_q"), (ctx_len, "ctx_len"), (req_slot, "req_slot")):
+        _i32(t, nm)
+    _need(attn_f32_supported(q, k_cache, head_dim, head_dim) and out.dtype == torch.float32 and q.stride(1) == 1,
+          "attn_f32: float32, heads of 64 or 128")
+    _need(num_heads % num_kv_heads == 0 and out.stride(1) == 1 and out.shape[1] == num_heads * head_dim and out.stride(0) % 2 == 0
+          and out.data_ptr() % 8 == 0, "attn_f32: out shape")
+    _need(k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.dtype == v_cache.dtype == torch.float32
+          and tuple(k_cache.shape[1:]) == (num_kv_heads, page_size, head_dim) and v_cache.shape == k_cache.shape
+          and v_cache.data_ptr() % 16 == 0, "attn_f32: cache plane")
+    n, group = len(q_lens), num_heads // num_kv_heads
+    _need(cu_q.numel() >= n + 1 and ctx_len.numel() >= n and req_slot.numel() >= n, "attn_f32: entry arrays too short")
+    blocks = sum((int(x) * group + 63) // 64 for x in q_lens)
+    load_library("attn_f32").call(
+        "ll_attn_f32", _ptr(out), c_long(out.stride(0)), _ptr(q), c_long(q.stride(0)), _ptr(k_cache), _ptr(v_cache),
+        _ptr(block_table), c_int(block_table.stride(0)), _ptr(cu_q), _ptr(ctx_len), _ptr(req_slot), c_int(n), c_int(blocks),
+        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(page_size), c_int(k_cache.shape[0]), c_int(window or 0),
+        c_float(scale), _ptr(status), _stream())
+
+
 def bias_rotate_store(qkv: torch.Tensor, bias: Optional[torch.Tensor], positions: Optional[torch.Tensor],
                       freq: Optional[torch.Tensor], interleaved: bool, num_heads: int, num_kv_heads: int,
                       head_dim: int, value_head_dim: int, slot_map: Optional[torch.Tensor],
@@ -1045,6 +1077,66 @@ def gemm_pair_qkv_rope(q_out: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor
 ACCUMULATE_MIN_M = 129   # more tokens than any of the hand-written plain products takes: library territory
 
 
+# Rows, and multiply-adds, from which on a float32 product goes to the tensor cores (``gemm_f32``).  Measured on a B200
+# (library / here): 64 x 17,920 x 1,536 72 / 81 us, 64 x 2,048 x 1,536 31 / 39, 64 x 1,536 x 8,960 134 / 52;
+# 128 x 37,888 x 3,584 535 / 326; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395;
+# 300 x 132 x 72 11 / 24 (its launches).
+F32_MIN_M = 96
+F32_MIN_WORK = 1 << 28
+
+
+def f32_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``gemm_f32`` takes this float32 product and is meant for it."""
+    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and TC_ENABLED and x.is_cuda and x.dim() == 2
+            and weight.dim() == 2 and x.shape[0] >= F32_MIN_M and x.shape[1] % 8 == 0 and weight.shape[0] % 4 == 0
+            and weight.shape[0] >= 64 and x.stride(1) == 1 and weight.stride(1) == 1 and x.stride(0) % 4 == 0
+            and x.shape[0] * x.shape[1] * weight.shape[0] >= F32_MIN_WORK
+            and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def f32_splits(m: int, n: int, k: int, device) -> int:
+    """Parts of k: as many as let the tiles of 256 x 256 fill the pairs of SMs, none shorter than 6 steps of 64."""
+    tiles, boxes = ((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64
+    splits = max(1, min((sm_count(device) // 2) // tiles, boxes // 6))
+    per = (boxes + splits - 1) // splits
+    return (boxes + per - 1) // per
+
+
+def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
+             gated=None, partial_ok: bool = False, splits: Optional[int] = None) -> torch.Tensor:
+    """x [n, k] times weight [m, k] transposed, true float32, on tensor cores (csrc/gemm_f32.cu).  ``accumulate``: added to
+    ``out``.  ``gated`` (a ``GateAct``): weight is [2 i, k], gate rows first, act(gate) * up comes out.  ``partial_ok``: where k
+    is cut into parts, they may be returned as [parts, n, m]."""
+    _need_cuda(x, weight, out)
+    _need(x.dtype == weight.dtype == torch.float32 and x.stride(1) == weight.stride(1) == 1 and x.shape[1] % 8 == 0
+          and x.stride(0) % 4 == 0 and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0,
+          "gemm_f32: float32 rows, k a multiple of 8, 16-byte aligned")
+    M, K = x.shape
+    N = weight.shape[0] // (2 if gated is not None else 1)
+    _need(weight.shape[1] == K and N % 4 == 0, "gemm_f32: shapes")
+    if gated is not None:
+        splits = 1
+    elif splits is None:
+        splits = f32_splits(M, N, K, x.device)
+    parts = None
+    if splits > 1 or accumulate:
+        parts = torch.empty((splits, M, N), dtype=torch.float32, device=x.device)
+    hand_on = partial_ok and splits > 1 and out is None
+    if out is None and not hand_on:
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    if out is not None:
+        _need(out.dtype == torch.float32 and tuple(out.shape) == (M, N) and out.stride(1) == 1 and out.stride(0) % 4 == 0
+              and out.data_ptr() % 16 == 0, "gemm_f32: out is float32 rows")
+    terms = torch.empty((3, M, K), dtype=torch.bfloat16, device=x.device)
+    act = gated if gated is not None else GateAct("silu")
+    load_library("gemm_f32").call(
+        "ll_gemm_f32", _ptr(out), c_long(N if out is None else out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight),
+        c_long(weight.stride(0)), c_int(M), c_int(N), c_int(K), _ptr(terms), _ptr(parts), c_int(splits),
+        c_int(1 if accumulate else 0), c_int(0 if gated is None else GATE_ACT[act.kind] + 1), c_float(act.limit),
+        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(None), _stream())
+    return parts if hand_on else out
+
+
 def accumulate_preferred(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether ``linear_accumulate`` should stand for ``linear`` + a later residual sum: when the product
     is a library one anyway (portions of prompts), its epilogue adds the residual for the price of reading it."""
@@ -1057,6 +1149,9 @@ def linear_accumulate(x: torch.Tensor, weight: torch.Tensor, acc: torch.Tensor) 
     _need_cuda(x, weight, acc)
     _need(acc.dtype == x.dtype and acc.shape[0] == x.shape[0] and acc.shape[1] == weight.shape[0]
           and acc.stride(1) == 1, "linear_accumulate: acc is [tokens, out] of the operands' dtype")
+    if f32_supported(x, weight) and acc.stride(0) % 4 == 0 and acc.data_ptr() % 16 == 0:
+        gemm_f32(x, weight, acc, accumulate=True)
+        return
     if x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("TF32 is on; call ops.configure_matmul_precision() before a float32 product")
     torch.addmm(acc, x, weight.t(), out=acc)
@@ -1076,6 +1171,8 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation="silu") ->
         return gemm_smallm(x, w_gate_up, act, gated=True, act=activation)
     if TC_ENABLED and x.shape[0] >= PAIR_MIN_M and pair_supported(x, w_gate_up):
         return gemm_pair(x, w_gate_up, act, gated=True, act=activation)
+    if inter % 4 == 0 and f32_supported(x, w_gate_up):
+        return gemm_f32(x, w_gate_up, act, gated=activation)
     gu = linear(x, w_gate_up)
     if activation.kind == "silu":
         silu_mul(act, gu)
@@ -1127,6 +1224,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
             return gemm_smallm(x, weight, out)
     if x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("TF32 is on; call ops.configure_matmul_precision() before a float32 product")
+    if (out_dtype in (None, torch.float32) and f32_supported(x, weight)
+            and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0))):
+        return gemm_f32(x, weight, out, partial_ok=partial_ok)
     if out_dtype is not None and out_dtype != x.dtype:
         res = torch.mm(x, weight.t(), out_dtype=out_dtype)
         if out is not None:

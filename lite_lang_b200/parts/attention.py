@@ -110,6 +110,10 @@ class GQAttention(Mixer):
 
     def kernel_libraries(self):
         libs = ["core"]
+        if self.w_qkv is not None and self.w_qkv.dtype == torch.float32:
+            libs.append("gemm_f32")
+            if self.head_dim in (64, 128) and self.vdim == self.head_dim:
+                libs.append("attn_f32")
         if self.w_qkv is not None and self.w_qkv.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc", "gemm_pair"])
             if self.head_dim in (64, 128) and self.vdim == self.head_dim:
@@ -297,6 +301,17 @@ class GQAttention(Mixer):
                     ops.attn_prefill(out, qkv, qkv.stride(0), cache.k, cache.v, cache.block_table, *rest, blocks,
                                      *args, step.status)
             return
+        if ops.attn_f32_supported(qkv, cache.k, self.head_dim, self.vdim):
+            # true float32: 64 (token, head) rows a CTA share the keys, products of float32 terms on tensor cores
+            captured = getattr(step, "captured", False)
+            entries = None if captured else getattr(step, "entries", None)
+            lens = [1] * step.num_entries if step.num_single == step.num_entries else \
+                None if entries is None else [len(e.tokens) for e in entries]
+            if lens is not None and sum(lens) == qkv.shape[0]:
+                ops.attn_f32(out, qkv, cache.k, cache.v, cache.block_table, step.cu_q, step.ctx_len, step.req_slot, lens,
+                             self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size, self.window, self.scale,
+                             step.status)
+                return
         ops.paged_attention_generic(out, qkv, qkv.stride(0), cache.k, cache.v, cache.block_table, step.token_req,
                                     step.req_slot, step.positions, qkv.shape[0], self.num_heads, self.num_kv_heads,
                                     self.head_dim, cache.page_size, self.window, self.scale, step.status,

@@ -1,0 +1,112 @@
+"""The true float32 path on tensor cores: products and prompt attention beside float64 and beside the general kernels."""
+
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+def _rel(x, y):
+    return float((x.double() - y).norm() / y.norm())
+
+
+# rows, features and inner sizes at the edges of tiles (256 x 256), of steps (64) and of parts of k
+@gpu
+@pytest.mark.parametrize("M,N,K,splits", [(1, 4, 8, 1), (96, 260, 72, 1), (255, 256, 64, 1), (257, 300, 200, 1), (300, 132, 1000, 3),
+                                          (513, 1028, 776, 2), (700, 512, 2048, None)])
+def test_product(M, N, K, splits):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + N + K)
+    wide = torch.randn(M, K + 12, generator=g, device="cuda")
+    x = wide[:, 4:4 + K]                                             # rows with a stride of their own
+    x[0] *= 1e-20
+    w = torch.randn(N, K, generator=g, device="cuda") * torch.logspace(-3, 3, N, device="cuda")[:, None]
+    want = x.double() @ w.double().t()
+    scale = x.double().abs() @ w.double().abs().t()                  # what a sum's rounding errors are measured by
+    got = ops.gemm_f32(x, w, splits=splits)
+    # 64 numbers of k a chain of cut-off sums (4 steps of 2^-23), then rounded additions; a term's last bits are 2^-24
+    bound = (8 + (K + 63) // 64) * 2.0 ** -24
+    assert float(((got.double() - want).abs() / scale.clamp(min=1e-300)).max()) <= bound
+    lib = torch.mm(x, w.t())
+    assert _rel(got, want) <= max(1.5 * _rel(lib, want), 1.5e-7)
+    acc = torch.randn(M, N, generator=g, device="cuda")
+    both = acc.double() + want
+    ops.gemm_f32(x, w, acc, accumulate=True, splits=splits)
+    assert float(((acc.double() - both).abs() / (scale + both.abs())).max()) <= bound + 2.0 ** -23
+    parts = ops.gemm_f32(x, w, partial_ok=True, splits=splits)
+    assert torch.equal(parts if parts.dim() == 2 else parts.sum(0), got) or _rel(parts.sum(0), got.double()) <= 2e-7
+
+
+@gpu
+@pytest.mark.parametrize("act", ["silu", "relu", "gelu_tanh", "clamped_swish"])
+@pytest.mark.parametrize("M,I,K", [(100, 132, 72), (257, 384, 256)])
+def test_gated_product(M, I, K, act):
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5
+    kind = ops.GateAct(act, 2.0 if act == "clamped_swish" else 0.0, 1.702)
+    got = ops.gemm_f32(x, w, torch.empty(M, I, device="cuda"), gated=kind)
+    gu = torch.mm(x.double(), w.double().t())
+    want = torch.empty(M, I, device="cuda")
+    ops.act_mul(want, gu.float().contiguous(), kind)
+    assert float((got - want).abs().max()) <= 4e-6 * float(want.abs().max())
+
+
+def test_which_float32_products_go_to_the_tensor_cores():
+    from lite_lang_b200 import ops
+    x, w = torch.zeros(2048, 1536), torch.zeros(2048, 1536)
+    assert not ops.f32_supported(x, w)                               # (not on a CUDA device)
+
+
+@gpu
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nh,nkv,page,window", [(4, 2, 16, None), (6, 1, 5, None), (3, 3, 16, 40), (14, 2, 64, 7)])
+def test_prompt_attention(hd, nh, nkv, page, window):
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(hd + nh + page)
+    spans = [(0, 1), (0, 65), (33, 64), (100, 130), (31, 2)]          # (cached, new) tokens; the first one is not a portion
+    pages = [(c + n + page - 1) // page for c, n in spans]
+    order = torch.randperm(sum(pages) + 3, generator=torch.Generator().manual_seed(1)).tolist()
+    k = torch.full((sum(pages) + 3, nkv, page, hd), float("nan"), device="cuda")
+    v = k.clone()
+    table = torch.full((len(spans) + 1, max(pages)), -1, dtype=torch.int32)
+    slots, ref = list(range(len(spans)))[::-1], []
+    for e, (c, n) in enumerate(spans):
+        keys, vals = torch.randn(c + n, nkv, hd, generator=g, device="cuda"), torch.randn(c + n, nkv, hd, generator=g, device="cuda")
+        for lp in range(pages[e]):
+            table[slots[e], lp] = pg = order.pop()
+            rows = slice(lp * page, min((lp + 1) * page, c + n))
+            k[pg, :, :rows.stop - rows.start] = keys[rows].transpose(0, 1)
+            v[pg, :, :rows.stop - rows.start] = vals[rows].transpose(0, 1)
+        ref.append((keys.double(), vals.double()))
+    total = sum(n for _, n in spans)
+    q = torch.randn(total, nh * hd + 8, generator=g, device="cuda") * 1.5
+    ints = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + torch.cumsum(torch.tensor([n for _, n in spans]), 0).tolist(), **ints)
+    ctx, slot = torch.tensor([c for c, _ in spans], **ints), torch.tensor(slots, **ints)
+    status, table = torch.zeros(1, **ints), table.to("cuda")
+    out = torch.full((total, nh * hd), float("nan"), device="cuda")
+    ops.attn_f32(out, q, k, v, table, cu[1:], ctx[1:], slot[1:], [n for _, n in spans[1:]], nh, nkv, hd, page, window, hd ** -0.5,
+                 status)
+    general = torch.empty_like(out)
+    req = torch.cat([torch.full((n,), e, **ints) for e, (_, n) in enumerate(spans)])
+    pos = torch.cat([torch.arange(c, c + n, **ints) for c, n in spans])
+    ops.paged_attention_generic(general, q, q.stride(0), k, v, table, req, slot, pos, total, nh, nkv, hd, page, window,
+                                hd ** -0.5, status)
+    assert int(status.item()) == 0
+    assert bool(torch.isnan(out[0]).all())                            # the token in front is left alone
+    want, at = torch.zeros(total, nh, hd, dtype=torch.float64, device="cuda"), 0
+    for (c, n), (keys, vals) in zip(spans, ref):
+        p, j = torch.arange(c, c + n, device="cuda")[:, None], torch.arange(c + n, device="cuda")[None, :]
+        ok = (j <= p) & ((p - j < window) if window else True)
+        for h in range(nh):
+            s = q[at:at + n, h * hd:(h + 1) * hd].double() @ keys[:, h // (nh // nkv)].t() * hd ** -0.5
+            want[at:at + n, h] = torch.softmax(s.masked_fill(~ok, float("-inf")), dim=1) @ vals[:, h // (nh // nkv)]
+        at += n
+    want = want.view(total, nh * hd)[1:]
+    err, was = _rel(out[1:], want), _rel(general[1:], want)
+    assert err <= max(1.5 * was, 4e-7), (err, was)
