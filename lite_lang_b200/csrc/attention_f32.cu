@@ -10,8 +10,8 @@
 //   O [64 x HD] += P V       P from the accumulators' registers
 // Two groups of four warps walk the tiles of 32 keys alternately, each with its own maximum, sum and O, and meet at the end in
 // shared memory: two tiles are on their way at a time and one group's softmax lies beside the other's products.  A tile's rows
-// of V are asked for before its scores and the next tile's rows of K before its second product (registers), and become terms
-// on their way into shared memory.
+// come by cp.async as stored, a tile ahead of the group's use of them (the pages' numbers a tile ahead of that), and become
+// terms in shared memory when their turn comes: asked for where they were needed, the trips to memory were 40 % of the time.
 //
 // Scores, softmax (expf) and sums are float32.  Keys that a row may not see get probability 0 by selection and their rows
 // of V are zeros, whatever the page holds.  The order of a row's sums depends on the tiles (which start at multiples of 32
@@ -43,6 +43,7 @@ template <int HD>
 __global__ void __launch_bounds__(AF_THREADS, 1)
 attn_f32_kernel(const AttnF32Params p) {
   constexpr int P = HD + 8, NO = HD / 8, LOADS = AF_TK * HD / 4 / 128;      // 16-byte pieces of K (and of V) a thread brings
+  constexpr int TERMS = 3 * P * (AF_ROWS + 4 * AF_TK);         // bfloat16 numbers before the rows as stored
   extern __shared__ __align__(16) unsigned char af_smem[];
   bf16* qs = reinterpret_cast<bf16*>(af_smem);                 // [3][64][P]
   LL_PDL_TRIGGER();
@@ -50,6 +51,7 @@ attn_f32_kernel(const AttnF32Params p) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = warp >> 2, gt = tid & 127;
   bf16* ks = qs + 3 * AF_ROWS * P + half * (6 * AF_TK * P);    // this group's tile: K [3][32][P], V [3][32][P]
   bf16* vs = ks + 3 * AF_TK * P;
+  float* raw = reinterpret_cast<float*>(qs + TERMS) + half * (2 * AF_TK * HD);       // K [32][HD], V [32][HD] as stored
   const int kvh = blockIdx.y;
   int rb = p.row_blocks - 1 - blockIdx.x;                      // the later, heavier blocks of the step first
   int entry = -1, rows = 0;
@@ -77,20 +79,31 @@ attn_f32_kernel(const AttnF32Params p) {
   const int tile0 = lo / AF_TK, tiles = hi / AF_TK - tile0 + 1;
   const int* bt = p.block_table + (size_t)slot * p.bt_stride;
 
-  float4 in[LOADS];                                            // rows on their way
-  auto ask = [&](const float* cache, int tile) {
+  // lane l: where the row of key l of a tile starts in the planes (-1: not seen by any row of the CTA)
+  auto place = [&](int tile) -> long {
+    const int pos = (tile0 + tile) * AF_TK + lane;
+    if (pos < lo || pos > hi) return -1;
+    const int lp = pos / p.page_size, page = lp < p.bt_stride ? bt[lp] : -1;
+    if (page < 0 || page >= p.num_pages) {
+      set_status(p.status, LL_ERR_PAGE_RANGE);
+      return -1;
+    }
+    return (((long)page * p.nkv + kvh) * p.page_size + pos % p.page_size) * HD;
+  };
+  const unsigned raw_b = ms_smem(raw);
+  auto ask = [&](long base) {                                  // a tile's rows (keys that nobody sees: zeros)
 #pragma unroll
     for (int j = 0; j < LOADS; ++j) {
-      const int i = j * 128 + gt, kk = i / (HD / 4), c = (i % (HD / 4)) * 4, pos = (tile0 + tile) * AF_TK + kk;
-      in[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (pos >= lo && pos <= hi) {
-        const int lp = pos / p.page_size, page = lp < p.bt_stride ? bt[lp] : -1;
-        if (page >= 0 && page < p.num_pages)
-          in[j] = *reinterpret_cast<const float4*>(cache + (((size_t)page * p.nkv + kvh) * p.page_size + pos % p.page_size) * HD + c);
-        else
-          set_status(p.status, LL_ERR_PAGE_RANGE);
-      }
+      const int i = j * 128 + gt, kk = i / (HD / 4), c = (i % (HD / 4)) * 4;
+      const long at = __shfl_sync(0xffffffffu, base, kk);
+      const long from = (at < 0 ? 0 : at) + c;
+      const int bytes = at < 0 ? 0 : 16;
+      const unsigned dst = raw_b + 4 * (kk * HD + c);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p.k_cache + from), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 4 * AF_TK * HD), "l"(p.v_cache + from), "r"(bytes)
+                   : "memory");
     }
+    ms_commit();
   };
   auto put4 = [](bf16* d, const float4& v, int plane) {
     uint2 t0, t1, t2;
@@ -100,14 +113,16 @@ attn_f32_kernel(const AttnF32Params p) {
     *reinterpret_cast<uint2*>(d + plane) = t1;
     *reinterpret_cast<uint2*>(d + 2 * plane) = t2;
   };
-  auto put = [&](bf16* dst) {
+  auto put = [&](bf16* dst, const float* src) {
 #pragma unroll
     for (int j = 0; j < LOADS; ++j) {
       const int i = j * 128 + gt, kk = i / (HD / 4), cc = (i % (HD / 4)) * 4;
-      put4(dst + kk * P + cc, in[j], AF_TK * P);
+      put4(dst + kk * P + cc, *reinterpret_cast<const float4*>(src + kk * HD + cc), AF_TK * P);
     }
   };
-  if (half < tiles) ask(p.k_cache, half);
+  long next = -1;
+  if (half < tiles) ask(place(half));
+  if (half + 2 < tiles) next = place(half + 2);
   for (int i = tid; i < AF_ROWS * (HD / 4); i += AF_THREADS) {
     const int rr = i / (HD / 4), c = (i % (HD / 4)) * 4, r = r0 + rr;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -125,10 +140,13 @@ attn_f32_kernel(const AttnF32Params p) {
 #pragma unroll
   for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   for (int tile = half; tile < tiles; tile += 2) {
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");      // the group is done with the tile before
-    put(ks);
-    ask(p.v_cache, tile);
+    ms_wait<0>();
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");      // the rows are here, the tile before has been read
+    put(ks, raw);
+    put(vs, raw + AF_TK * HD);
     asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+    if (tile + 2 < tiles) ask(next);
+    if (tile + 4 < tiles) next = place(tile + 4);
     float s[4][4], low[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -179,7 +197,6 @@ attn_f32_kernel(const AttnF32Params p) {
     }
     l0 = l0 * f0 + t0;
     l1 = l1 * f1 + t1;
-    put(vs);
     unsigned a[2][3][4];
 #pragma unroll
     for (int kt = 0; kt < 2; ++kt)
@@ -188,10 +205,8 @@ attn_f32_kernel(const AttnF32Params p) {
         ms_split(s[2 * kt + q][0], s[2 * kt + q][1], a[kt][0][2 * q], a[kt][1][2 * q], a[kt][2][2 * q]);
         ms_split(s[2 * kt + q][2], s[2 * kt + q][3], a[kt][0][2 * q + 1], a[kt][1][2 * q + 1], a[kt][2][2 * q + 1]);
       }
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
 #pragma unroll
     for (int nt = 0; nt < NO; nt += 4) {
-      if (nt == NO - 4 && tile + 2 < tiles) ask(p.k_cache, tile + 2);
       float d[4][4], small[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -270,7 +285,7 @@ extern "C" int ll_attn_f32(float* out, long out_stride, const float* q, long q_s
     return (int)cudaErrorInvalidValue;
   AttnF32Params p{out, out_stride, q, q_stride, k_cache, v_cache, block_table, bt_stride, cu_q, ctx_len, req_slot, n_entries,
                   nkv, nh / nkv, page_size, num_pages, window, row_blocks, scale, status};
-  const size_t smem = 2 * (size_t)(hd + 8) * 3 * (AF_ROWS + 4 * AF_TK);
+  const size_t smem = 2 * (size_t)(hd + 8) * 3 * (AF_ROWS + 4 * AF_TK) + 4 * (size_t)hd * 4 * AF_TK;
   if (hd == 128) {
     const cudaError_t rc = cudaFuncSetAttribute(attn_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (rc != cudaSuccess) return (int)rc;
