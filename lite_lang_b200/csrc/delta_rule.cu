@@ -10,10 +10,10 @@
 // [(taps - 1), channels] for the last taps - 1 inputs of the convolutions (oldest first;
 // channels = q | k | v), so that a request can go on in a later step from where it stopped.
 //
-// Four kernels, all reading the step's device arrays only (so that a step of single tokens can
+// Four kernels (a portion's recurrence may go by chunks instead: chunk_scan.cu), all reading the step's device arrays only (so that a step of single tokens can
 // be captured and replayed):
 //   delta_prepare      per token: convolution + SiLU, unit vectors, beta, decay -> float32 buffers
-//   delta_conv_update  per entry: the new last taps - 1 inputs of the record
+//   delta_conv_update  per entry of several tokens: the new last taps - 1 inputs of the record
 //   delta_recurrence   per (entry, head, 16 value columns): the scan over the entry's tokens
 //   delta_out          per (token, head): o / rms(o) * weight * gate -> storage type
 // Every value column of S evolves on its own (S^T k and S^T q are per column), so the scan is
@@ -32,74 +32,172 @@ struct DeltaShape {
 
 // proj: the step's projections, row t at proj + t * proj_stride, with q at column q_off (Hk*dk wide), k at k_off
 // (Hk*dk), v at v_off (H*dv), b at b_off (H).  a_in: the decay's input, [tokens, H] or [tokens, H*dk].
-template <typename T>
-__global__ void __launch_bounds__(256)
+//
+// A warp makes one unit of one token: a q or k head (convolution, SiLU, unit vector), a v head (convolution, SiLU), the decays
+// (of a head with one a channel, else of all heads) or the betas; a block takes a unit of eight neighbouring tokens, whose
+// convolutions read nearly the same rows.  VEC channels a lane and access; four taps, the usual number, unrolled.  Bound by
+// the lanes' loads in flight: 2,047 tokens of 2,048 channels 25 us (41 with a loop over the taps).  (A block a token with its
+// channels in shared memory took 41 us too, and 14.7 us for one token, which left 147 SMs idle; now 4 us.)
+// An entry of one token moves its convolutions' last inputs up here: nobody else reads them.
+#define DP_TOKENS 8
+template <typename T, int VEC> struct DpVec;
+template <typename T> struct DpVec<T, 1> {
+  __device__ static void load(const T* p, float (&v)[1]) { v[0] = to_f32<T>(p[0]); }
+};
+template <> struct DpVec<float, 4> {
+  __device__ static void load(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+  }
+};
+template <> struct DpVec<bf16, 4> {
+  __device__ static void load(const bf16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+};
+template <int VEC> __device__ __forceinline__ void dp_store(float* p, const float (&v)[VEC]) {
+  if (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
+  else p[0] = v[0];
+}
+
+// TAPS 4: filters of four taps at 16-byte boundaries, all loads of a channel's convolution on their way at once; 0: any.
+template <typename T, int VEC, int TAPS>
+__global__ void __launch_bounds__(32 * DP_TOKENS)
 delta_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, int k_off, int v_off, int b_off,
                      const T* __restrict__ a_in, long a_stride, const float* __restrict__ conv_q,
                      const float* __restrict__ conv_k, const float* __restrict__ conv_v,
-                     const float* __restrict__ A_log, const float* __restrict__ dt_bias,
-                     const float* __restrict__ state, long state_stride, long tail_off,
-                     const int* __restrict__ token_req, const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
-                     const int* __restrict__ req_slot, const int* __restrict__ positions, float* __restrict__ qn,
-                     float* __restrict__ kn, float* __restrict__ vc, float* __restrict__ beta, float* __restrict__ g,
-                     DeltaShape s) {
-  extern __shared__ float y[];   // [Cq + Ck + Cv] convolution outputs after SiLU
+                     const float* __restrict__ A_log, const float* __restrict__ dt_bias, float* state, long state_stride,
+                     long tail_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
+                     const int* __restrict__ ctx_len, const int* __restrict__ req_slot, const int* __restrict__ positions,
+                     float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vc, float* __restrict__ beta,
+                     float* __restrict__ g, int num_tokens, DeltaShape s) {
+  constexpr int PIECES = 8 / VEC;                 // of a q or k head of up to 256 channels: kept between the sum and the output
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
-  const int t = blockIdx.x;
+  const int lane = threadIdx.x & 31, t = blockIdx.x * DP_TOKENS + (threadIdx.x >> 5);
+  if (t >= num_tokens) return;
   const int e = token_req[t];
   const int slot = e >= 0 ? req_slot[e] : -1;
   if (slot < 0) return;   // padding entry: the scan writes its (zero) output
   const int Cq = s.Hk * s.dk, Cv = s.H * s.dv, C = 2 * Cq + Cv, K = s.taps;
-  const int first = cu_q[e], ctx = ctx_len[e], p = positions[t];
-  const float* tail = state + (size_t)slot * state_stride + tail_off;
-  const int tid = threadIdx.x;
-  for (int c = tid; c < C; c += blockDim.x) {
-    const float* w;
-    int col;
-    if (c < Cq) {
-      w = conv_q + (size_t)c * K;
-      col = q_off + c;
-    } else if (c < 2 * Cq) {
-      w = conv_k + (size_t)(c - Cq) * K;
-      col = k_off + c - Cq;
-    } else {
-      w = conv_v + (size_t)(c - 2 * Cq) * K;
-      col = v_off + c - 2 * Cq;
-    }
-    float acc = 0.f;
-    for (int j = K - 1; j >= 0; --j) {   // oldest input first
-      float x = 0.f;
-      if (t - j >= first) {
-        x = to_f32<T>(proj[(size_t)(t - j) * proj_stride + col]);
-      } else if (p - j >= 0) {
-        x = tail[(size_t)(p - j - ctx + K - 1) * C + c];   // an input of an earlier step
+  const int unit = blockIdx.y;
+  const T* row = proj + (size_t)t * proj_stride;
+  if (unit >= 2 * s.Hk + s.H) {
+    if (unit == 2 * s.Hk + s.H) {                 // betas
+      for (int h = lane; h < s.H; h += 32) beta[(size_t)t * s.H + h] = dr_sigmoid(to_f32<T>(row[b_off + h]));
+    } else if (!s.per_channel) {                  // decays, one a head
+      for (int h = lane; h < s.H; h += 32) {
+        const float a = to_f32<T>(a_in[(size_t)t * a_stride + h]) + dt_bias[h];
+        g[(size_t)t * s.H + h] = expf(-expf(A_log[h]) * dr_softplus(a));
       }
-      acc = fmaf(w[K - 1 - j], x, acc);
+    } else {                                      // decays of a head's channels
+      const int h = unit - (2 * s.Hk + s.H) - 1;
+      const float rate = -expf(A_log[h]);
+      const T* ar = a_in + (size_t)t * a_stride + (size_t)h * s.dk;
+      const float* br = dt_bias + (size_t)h * s.dk;
+      float* gr = g + ((size_t)t * s.H + h) * s.dk;
+      for (int i = lane; i < s.dk; i += 32) gr[i] = expf(rate * dr_softplus(to_f32<T>(ar[i]) + br[i]));
     }
-    y[c] = dr_silu(acc);
+    return;
   }
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  for (int hh = warp; hh < 2 * s.Hk; hh += nwarps) {   // unit vectors: q heads, then k heads
-    const float* src = y + (size_t)hh * s.dk;
-    float ss = 0.f;
-    for (int i = lane; i < s.dk; i += 32) ss = fmaf(src[i], src[i], ss);
-    ss = warp_sum(ss);
-    float inv = 1.0f / sqrtf(ss + 1e-6f);
-    const bool is_q = hh < s.Hk;
-    if (is_q) inv *= 1.0f / sqrtf((float)s.dk);
-    float* dst = (is_q ? qn + (size_t)t * Cq : kn + (size_t)t * Cq - Cq) + (size_t)hh * s.dk;
-    for (int i = lane; i < s.dk; i += 32) dst[i] = src[i] * inv;
+  // a head's channels: where they lie in the projections, in the filters, among the record's inputs and in the output
+  const int kind = unit < s.Hk ? 0 : unit < 2 * s.Hk ? 1 : 2, head = unit - (kind == 0 ? 0 : kind == 1 ? s.Hk : 2 * s.Hk);
+  const int width = kind == 2 ? s.dv : s.dk, c0 = head * width;
+  const float* filt = (kind == 0 ? conv_q : kind == 1 ? conv_k : conv_v) + (size_t)c0 * K;
+  const T* col = row + (kind == 0 ? q_off : kind == 1 ? k_off : v_off) + c0;
+  const int first = cu_q[e], ctx = ctx_len[e], p = positions[t];
+  const bool alone = cu_q[e + 1] - first == 1;
+  float* tail = state + (size_t)slot * state_stride + tail_off + (kind == 0 ? 0 : kind == 1 ? Cq : 2 * Cq) + c0;
+  auto convolved = [&](int c, float (&acc)[VEC]) {
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
+    if (TAPS == 4) {
+      float x[4][VEC];
+      float4 f[VEC];
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) f[k] = *reinterpret_cast<const float4*>(filt + (size_t)(c + k) * 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) x[j][k] = 0.f;
+        if (t - j >= first) {
+          DpVec<T, VEC>::load(col - (size_t)j * proj_stride + c, x[j]);
+        } else if (p - j >= 0) {         // an input of an earlier step
+          const float* src = tail + (size_t)(p - j - ctx + 3) * C + c;
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) x[j][k] = src[k];
+        }
+      }
+      if (alone) {                       // place 2 - j of the record holds input j from now on
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) tail[(size_t)(2 - j) * C + c + k] = x[j][k];
+      }
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) {    // oldest input first
+        acc[k] = fmaf(f[k].x, x[3][k], acc[k]);
+        acc[k] = fmaf(f[k].y, x[2][k], acc[k]);
+        acc[k] = fmaf(f[k].z, x[1][k], acc[k]);
+        acc[k] = dr_silu(fmaf(f[k].w, x[0][k], acc[k]));
+      }
+      return;
+    }
+    for (int j = K - 1; j >= 0; --j) {   // oldest input first
+      float x[VEC];
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) x[k] = 0.f;
+      if (t - j >= first) {
+        DpVec<T, VEC>::load(col - (size_t)j * proj_stride + c, x);
+      } else if (p - j >= 0) {           // an input of an earlier step
+        const float* src = tail + (size_t)(p - j - ctx + K - 1) * C + c;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) x[k] = src[k];
+      }
+      if (alone && j < K - 1) {          // place K - 2 - j of the record holds this input from now on
+        float* dst = tail + (size_t)(K - 2 - j) * C + c;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) dst[k] = x[k];
+      }
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) acc[k] = fmaf(filt[(size_t)(c + k) * K + K - 1 - j], x[k], acc[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = dr_silu(acc[k]);
+  };
+  if (kind == 2) {
+    for (int c = VEC * lane; c < width; c += 32 * VEC) {
+      float y[VEC];
+      convolved(c, y);
+      dp_store<VEC>(vc + (size_t)t * Cv + c0 + c, y);
+    }
+    return;
   }
-  for (int i = tid; i < Cv; i += blockDim.x) vc[(size_t)t * Cv + i] = y[2 * Cq + i];
-  for (int h = tid; h < s.H; h += blockDim.x)
-    beta[(size_t)t * s.H + h] = dr_sigmoid(to_f32<T>(proj[(size_t)t * proj_stride + b_off + h]));
-  const int ng = s.per_channel ? s.H * s.dk : s.H;
-  for (int i = tid; i < ng; i += blockDim.x) {
-    const int h = s.per_channel ? i / s.dk : i;
-    const float a = to_f32<T>(a_in[(size_t)t * a_stride + i]) + dt_bias[i];
-    g[(size_t)t * ng + i] = expf(-expf(A_log[h]) * dr_softplus(a));
+  float y[PIECES][VEC], ss = 0.f;        // unit vectors
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int c = (i * 32 + lane) * VEC;
+    if (c < width) {
+      convolved(c, y[i]);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) ss = fmaf(y[i][k], y[i][k], ss);
+    }
+  }
+  ss = warp_sum(ss);
+  float inv = 1.0f / sqrtf(ss + 1e-6f);
+  if (kind == 0) inv *= 1.0f / sqrtf((float)s.dk);
+  float* dst = (kind == 0 ? qn : kn) + (size_t)t * Cq + c0;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int c = (i * 32 + lane) * VEC;
+    if (c < width) {
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) y[i][k] *= inv;
+      dp_store<VEC>(dst + c, y[i]);
+    }
   }
 }
 
@@ -118,6 +216,7 @@ __global__ void delta_conv_update_kernel(const T* __restrict__ proj, long proj_s
   if (slot < 0) return;
   const int Cq = s.Hk * s.dk, Cv = s.H * s.dv, C = 2 * Cq + Cv, K = s.taps;
   const int first = cu_q[e], L = cu_q[e + 1] - first, ctx = ctx_len[e];
+  if (L == 1) return;          // (delta_prepare has done it)
   float* tail = state + (size_t)slot * state_stride + tail_off;
   for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
     const int col = c < Cq ? q_off + c : c < 2 * Cq ? k_off + c - Cq : v_off + c - 2 * Cq;
@@ -291,11 +390,13 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
   }
 }
 
-// out[t, h*dv + j] = o / sqrt(mean_j(o^2) + eps) * w[j] * act(gate[t, h*dv + j]); act: 0 SiLU, 1 sigmoid.
-template <typename T>
+// out[t, h*dv + j] = o / sqrt(mean_j(o^2) + eps) * w[j] * act(gate[t, h*dv + j]); act: 0 SiLU, 1 sigmoid.  A warp a (token,
+// head), VEC numbers a lane and access; heads of up to 256 numbers stay in registers between the sum and the output.
+template <typename T, int VEC>
 __global__ void delta_out_kernel(T* __restrict__ out, const float* __restrict__ o, const float* __restrict__ w,
                                  const T* __restrict__ gate, long gate_stride, float eps, int num_pairs, int H, int dv,
                                  int gate_act) {
+  constexpr int PIECES = 8 / VEC;
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -303,16 +404,40 @@ __global__ void delta_out_kernel(T* __restrict__ out, const float* __restrict__ 
   const int lane = threadIdx.x & 31;
   const int t = pair / H, h = pair % H;
   const float* src = o + (size_t)pair * dv;
-  float ss = 0.f;
-  for (int j = lane; j < dv; j += 32) ss = fmaf(src[j], src[j], ss);
-  ss = warp_sum(ss);
-  const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
   const T* gt = gate + (size_t)t * gate_stride + (size_t)h * dv;
   T* dst = out + (size_t)pair * dv;
-  for (int j = lane; j < dv; j += 32) {
-    const float z = to_f32<T>(gt[j]);
-    const float a = gate_act == 0 ? dr_silu(z) : dr_sigmoid(z);
-    dst[j] = from_f32<T>(src[j] * inv * w[j] * a);
+  float x[PIECES][VEC];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int c = (i * 32 + lane) * VEC;
+    if (c < dv) {
+      DpVec<float, VEC>::load(src + c, x[i]);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) ss = fmaf(x[i][k], x[i][k], ss);
+    }
+  }
+  for (int c = 256 + lane; c < dv; c += 32) ss = fmaf(src[c], src[c], ss);
+  ss = warp_sum(ss);
+  const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int c = (i * 32 + lane) * VEC;
+    if (c < dv) {
+      float z[VEC];
+      T r[VEC];
+      DpVec<T, VEC>::load(gt + c, z);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k)
+        r[k] = from_f32<T>(x[i][k] * inv * w[c + k] * (gate_act == 0 ? dr_silu(z[k]) : dr_sigmoid(z[k])));
+      if (VEC == 4 && sizeof(T) == 2) *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<const uint2*>(r);
+      else if (VEC == 4) *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(r);
+      else dst[c] = r[0];
+    }
+  }
+  for (int c = 256 + lane; c < dv; c += 32) {
+    const float z = to_f32<T>(gt[c]);
+    dst[c] = from_f32<T>(src[c] * inv * w[c] * (gate_act == 0 ? dr_silu(z) : dr_sigmoid(z)));
   }
 }
 
@@ -327,20 +452,28 @@ extern "C" int ll_delta_prepare(int dtype, const void* proj, long proj_stride, i
   if (H <= 0 || Hk <= 0 || H % Hk || dk <= 0 || dv <= 0 || taps < 1) return (int)cudaErrorInvalidValue;
   DeltaShape s{H, Hk, dk, dv, taps, per_channel};
   const int C = 2 * Hk * dk + H * dv;
-  const size_t smem = sizeof(float) * (size_t)C;
+  const int units = 2 * Hk + H + 1 + (per_channel ? H : 1);
+  // four channels a lane and access: heads, columns and rows at multiples of four numbers
+  const int esz = dtype == LL_DTYPE_F32 ? 4 : 2;
+  const bool vec = dk % 4 == 0 && dv % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && proj_stride % 4 == 0 &&
+                   (uintptr_t)proj % (4 * esz) == 0 && ((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)vc) % 16 == 0;
+  const dim3 grid((num_tokens + DP_TOKENS - 1) / DP_TOKENS, units), block(32 * DP_TOKENS);
+#define DP_ARGS                                                                                                             \
+  grid, block, 0, stream, (const T*)proj, proj_stride, q_off, k_off, v_off, b_off, (const T*)a_in, a_stride, conv_q, conv_k, \
+      conv_v, A_log, dt_bias, state, state_stride, tail_off, token_req, cu_q, ctx_len, req_slot, positions, qn, kn, vc, beta, \
+      g, num_tokens, s
   LL_DISPATCH_DTYPE(dtype, {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(delta_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ll_launch(delta_prepare_kernel<T>, dim3(num_tokens), dim3(256), smem, stream, (const T*)proj, proj_stride, q_off,
-              k_off, v_off, b_off, (const T*)a_in, a_stride, conv_q, conv_k, conv_v, A_log, dt_bias,
-              (const float*)state, state_stride, tail_off, token_req, cu_q, ctx_len, req_slot, positions, qn, kn, vc,
-              beta, g, s);
-    if (taps > 1) {
+    if (vec && taps == 4 && ((uintptr_t)conv_q | (uintptr_t)conv_k | (uintptr_t)conv_v) % 16 == 0)
+      ll_launch(delta_prepare_kernel<T, 4, 4>, DP_ARGS);
+    else if (vec) ll_launch(delta_prepare_kernel<T, 4, 0>, DP_ARGS);
+    else ll_launch(delta_prepare_kernel<T, 1, 0>, DP_ARGS);
+    if (taps > 1 && num_tokens != num_entries) {      // (as many tokens as entries: one each)
       const int by = (C + 255) / 256;
       ll_launch(delta_conv_update_kernel<T>, dim3(num_entries, by < 8 ? by : 8), dim3(256), 0, stream, (const T*)proj,
                 proj_stride, q_off, k_off, v_off, state, state_stride, tail_off, cu_q, ctx_len, req_slot, s);
     }
   });
+#undef DP_ARGS
   return LL_LAUNCH_RESULT();
 }
 
@@ -377,7 +510,16 @@ extern "C" int ll_delta_out(int dtype, void* out, const float* o, const float* w
                             float eps, int num_tokens, int H, int dv, int gate_act, cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
   const int pairs = num_tokens * H;
-  LL_DISPATCH_DTYPE(dtype, ll_launch(delta_out_kernel<T>, dim3((pairs + 3) / 4), dim3(128), 0, stream, (T*)out, o, w,
-                                     (const T*)gate, gate_stride, eps, pairs, H, dv, gate_act));
+  const int esz = dtype == LL_DTYPE_F32 ? 4 : 2;
+  const bool vec = dv % 4 == 0 && gate_stride % 4 == 0 && ((uintptr_t)gate | (uintptr_t)out) % (4 * esz) == 0 &&
+                   (uintptr_t)o % 16 == 0;
+  LL_DISPATCH_DTYPE(dtype, {
+    if (vec)
+      ll_launch(delta_out_kernel<T, 4>, dim3((pairs + 3) / 4), dim3(128), 0, stream, (T*)out, o, w, (const T*)gate, gate_stride,
+                eps, pairs, H, dv, gate_act);
+    else
+      ll_launch(delta_out_kernel<T, 1>, dim3((pairs + 3) / 4), dim3(128), 0, stream, (T*)out, o, w, (const T*)gate, gate_stride,
+                eps, pairs, H, dv, gate_act);
+  });
   return LL_LAUNCH_RESULT();
 }
