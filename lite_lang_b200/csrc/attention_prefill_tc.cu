@@ -36,6 +36,14 @@
 //
 // Sink: one more key a head, of a given score and without a value: its share joins the row's sum at the end.
 //
+// Shaped scores (a variant of its own): what attention_shaped_mma.cu does to a score between product and softmax - a factor
+// by the query's position, a cap, a bias by distance, a penalty by distance, chunks, a window that keeps the first positions
+// - done by the row's thread, a gate a head or a channel and a constant on the output.  The softmax weights are two bfloat16
+// terms (hi + lo, sixteen bits) as there, so the second product is two, P takes twice the shared memory and V has one stage.
+// Bound by the row threads' instructions (the two sums of a score and its bias, the second term of the weight), at two CTAs an
+// SM.  1,500 tokens in two requests with 28 heads of 128 on 4, window 1,024, distance bias, learned sink, gate a channel:
+// 87 us, 165 us by mma.sync (whose eight warps make the scores of 128 rows as 64 products of 16 x 8 x 16 each).
+//
 // Pairs: neighbouring query heads (2a, 2a + 1) are two score maps over the same keys and values and come out as one head,
 // z = o_even - lambda o_odd, z / sqrt(mean(z^2) + eps) * post (float32, before the gate and the one rounding).  Their rows
 // are neighbouring lanes of a warp.
@@ -44,6 +52,7 @@
 #define AT_THREADS 192
 #define AT_KB 64  // keys a block
 #define AT_KS 2   // stages of K and of V
+#define AT_LOG2E 1.4426950408889634f
 
 struct AttnTcParams {
   bf16* out;
@@ -70,12 +79,33 @@ struct AttnTcParams {
   long gate_stride;
   int pairs;           // heads 2a and 2a + 1 come out as one (half as many heads in out and gate)
   float lambda, post, pair_eps;
+  // shaped scores (all in log2 units)
+  int mask, mask_size;       // 0 causal, 1 a window of mask_size, 2 chunks of mask_size (`window` is not read)
+  int keep;                  // mask 1: positions below it stay visible
+  int zero_sink;             // one more key of score 0
+  const float* rel;          // [nd, nh]: bias (natural units) of a key min(n, nd - 1) positions back, or null
+  int nd, nh;
+  const float* slope;        // [nh]: taken off n times for a key n positions back (natural units), or null
+  float cap, inv_cap;        // cap > 0: cap tanh(s / cap), here cap log2(e) and its inverse
+  float qt_coef;
+  int qt_every;              // > 0: the query's factor by position
+  int gate_channels;         // the gate is a number a channel: gate[token * gate_stride + head * HD + channel]
+  float out_scale;
   float* scratch;      // [row blocks * nkv * nsplit][HD + 2][128]
   int* counters;       // [row blocks * nkv], zero between launches
   int* status;
 };
 
-template <int HD>
+// the first position that a row at `pos` sees, but for the kept ones (a plain window without one: 0)
+__device__ __forceinline__ int at_first_visible(const AttnTcParams& p, bool shaped, int pos) {
+  if (!shaped) return p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  if (p.mask == 1) return max(0, pos - p.mask_size + 1);
+  return p.mask == 2 ? (pos / p.mask_size) * p.mask_size : 0;
+}
+// tanh from exp2 and a division: absolute error of a few 1e-7
+__device__ __forceinline__ float at_tanh(float x) { return 1.0f - __fdividef(2.0f, at_ex2(x * 2.885390081777927f) + 1.0f); }
+
+template <int HD, bool SHAPED>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap qmap,
                        const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
@@ -84,6 +114,10 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   constexpr int KV_BYTES = AT_KB * HD * 2;     // K (or V) of a block
   constexpr int STAGE_BYTES = 2 * KV_BYTES;
   constexpr int P_BYTES = 128 * AT_KB * 2;
+  // two stages of K and V, then P; shaped: two stages of K, one of V, then P's two terms
+  constexpr int VS = SHAPED ? 1 : AT_KS;
+  constexpr int K_STEP = SHAPED ? KV_BYTES : STAGE_BYTES, V_AT = SHAPED ? AT_KS * KV_BYTES : KV_BYTES;
+  constexpr int P_AT = SHAPED ? (AT_KS + 1) * KV_BYTES : AT_KS * STAGE_BYTES;
   constexpr int TMEM_COLS = 256;               // S: 2 x 64 columns, O: HD columns (half an SM's tensor memory)
   constexpr unsigned IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(AT_KB >> 3) << 17) | ((128u >> 4) << 24);
   constexpr unsigned IDESC_PV =
@@ -94,8 +128,8 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* q_s = smem;
   unsigned char* kv_s = q_s + Q_BYTES;
-  unsigned char* p_s = kv_s + AT_KS * STAGE_BYTES;
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(p_s + P_BYTES);
+  unsigned char* p_s = kv_s + P_AT;
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(p_s + (SHAPED ? 2 : 1) * P_BYTES);
   // barriers: q_full, k_full[KS], k_empty[KS], v_full[KS], v_empty[KS], s_full[2], s_empty[2], p_full, pv_done
   const unsigned q_full = at_smem(bars);
   const unsigned k_full0 = at_smem(bars + 1), k_empty0 = k_full0 + 8 * AT_KS;
@@ -138,16 +172,21 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   const int ntok = min(p.tpb, qlen - rb * p.tpb);
   const int pos0 = p.ctx_len[entry] + rb * p.tpb;           // its position (ctx_len: tokens cached before the step)
   const int hi = pos0 + ntok - 1;
-  const int lo_min = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
-  const int nblk_all = hi / AT_KB - lo_min / AT_KB + 1;      // key blocks the rows may see
+  const int lo_min = at_first_visible(p, SHAPED, pos0);
+  // key blocks the rows may see: those of kept positions before the window's first (shaped), then lo_min's to hi's
+  const int keep = SHAPED && p.mask == 1 ? p.keep : 0;
+  const int kept = min((keep + AT_KB - 1) / AT_KB, lo_min / AT_KB);
+  const int nblk_all = kept + hi / AT_KB - lo_min / AT_KB + 1;
   // splits that have work: about split_len blocks each (the host chooses that length so that the step's CTAs
   // just fit the SMs at once), none empty; the same for every CTA of the row block
   int eff = min(p.nsplit, max(1, (nblk_all + p.split_len - 1) / p.split_len));
   const int per = (nblk_all + eff - 1) / eff;
   eff = (nblk_all + per - 1) / per;
   if (split >= eff) return;
-  const int kb_lo = lo_min / AT_KB + split * per;             // this CTA's first block
+  const int b_first = split * per;                            // this CTA's first block
   const int nblk = min(per, nblk_all - split * per);
+  // the first key of this CTA's block j
+  auto block_key = [&](int j) { return (b_first + j < kept ? b_first + j : lo_min / AT_KB + b_first + j - kept) * AT_KB; };
 
   if (tid == 32) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&qmap) : "memory");
@@ -192,12 +231,12 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     const int* bt = p.block_table + (size_t)slot * p.bt_stride;
     const int boxes = AT_KB / p.box_rows;
     auto page_of = [&](int j) -> int {   // cache row of this lane's box of block j
-      const int kp = (kb_lo + j) * AT_KB + lane * p.box_rows;
+      const int kp = block_key(j) + lane * p.box_rows;
       const int lp = kp / p.page_size;
       const bool mine = lane < boxes && j < nblk;
       int page = (mine && lp < p.bt_stride) ? bt[lp] : -1;
       if (page < 0 || page >= p.num_pages) {   // given back or beyond the context: masked, and V zeroed, below
-        if (mine && (page >= p.num_pages || (kp <= hi && kp + p.box_rows - 1 >= lo_min)))
+        if (mine && (page >= p.num_pages || (kp <= hi && (kp + p.box_rows - 1 >= lo_min || kp < keep))))
           set_status(p.status, LL_ERR_PAGE_RANGE);   // a key that a row sees has no page of the pool
         page = 0;
       }
@@ -205,15 +244,15 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     };
     // order of the copies: K(0), K(1), then V(j) before K(j + 2), the order in which the MMAs want them
     auto load = [&](int j, int row, bool is_v) {
-      const int s = j % AT_KS;
+      const int stages = is_v ? VS : AT_KS, s = j % stages;
       const unsigned full = (is_v ? v_full0 : k_full0) + 8 * s;
       if (lane == 0) {
-        at_mbar_wait((is_v ? v_empty0 : k_empty0) + 8 * s, (unsigned)(((j / AT_KS) & 1) ^ 1), p.status, dead);
+        at_mbar_wait((is_v ? v_empty0 : k_empty0) + 8 * s, (unsigned)(((j / stages) & 1) ^ 1), p.status, dead);
         at_mbar_expect_tx(full, KV_BYTES);
       }
       __syncwarp();
       if (lane < boxes) {
-        const unsigned dst = at_smem(kv_s) + s * STAGE_BYTES + (is_v ? KV_BYTES : 0) + lane * p.box_rows * 128;
+        const unsigned dst = at_smem(kv_s) + s * K_STEP + (is_v ? V_AT : 0) + lane * p.box_rows * 128;
         for (int h = 0; h < HB; ++h)
           at_tma_2d(dst + h * (KV_BYTES / HB), is_v ? &vmap : &kmap, kvh * p.head_cols + h * 64, row, full);
       }
@@ -236,7 +275,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
         at_mbar_wait(k_full0 + 8 * s, (unsigned)((j / AT_KS) & 1), p.status, dead);
         at_mbar_wait(s_empty0 + 8 * b, (unsigned)(((j >> 1) & 1) ^ 1), p.status, dead);
         AT_FENCE_AFTER();
-        const unsigned k_addr = at_smem(kv_s) + s * STAGE_BYTES;
+        const unsigned k_addr = at_smem(kv_s) + s * K_STEP;
 #pragma unroll
         for (int k16 = 0; k16 < HD / 16; ++k16) {
           const unsigned off = (k16 / 4) * (Q_BYTES / HB) + (k16 % 4) * 32;
@@ -253,16 +292,22 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
       mma_s(0);
       if (nblk > 1) mma_s(1);
       for (int j = 0; j < nblk; ++j) {
-        const int s = j % AT_KS;
-        at_mbar_wait(v_full0 + 8 * s, (unsigned)((j / AT_KS) & 1), p.status, dead);
+        const int s = j % VS;
+        at_mbar_wait(v_full0 + 8 * s, (unsigned)((j / VS) & 1), p.status, dead);
         at_mbar_wait(p_full, (unsigned)(j & 1), p.status, dead);
         AT_FENCE_AFTER();
-        const unsigned v_addr = at_smem(kv_s) + s * STAGE_BYTES + KV_BYTES;
+        const unsigned v_addr = at_smem(kv_s) + s * K_STEP + V_AT;
         const unsigned p_addr = at_smem(p_s);
+        if (SHAPED) {
+#pragma unroll
+          for (int k16 = 0; k16 < AT_KB / 16; ++k16)   // the weights' low terms
+            at_mma(tmem_o, at_desc_k(p_addr + P_BYTES + k16 * 32), at_desc_mn(v_addr + k16 * 2048, KV_BYTES / HB), IDESC_PV,
+                   (j > 0 || k16 > 0) ? 1u : 0u);
+        }
 #pragma unroll
         for (int k16 = 0; k16 < AT_KB / 16; ++k16)   // 16 keys a step: 32 bytes along P's rows, 2048 bytes down V
           at_mma(tmem_o, at_desc_k(p_addr + k16 * 32), at_desc_mn(v_addr + k16 * 2048, KV_BYTES / HB), IDESC_PV,
-                 (j > 0 || k16 > 0) ? 1u : 0u);
+                 (SHAPED || j > 0 || k16 > 0) ? 1u : 0u);
         at_commit(pv_done);            // P may be written again; O holds the blocks up to j
         at_commit(v_empty0 + 8 * s);
         if (j + 2 < nblk) mma_s(j + 2);
@@ -275,13 +320,19 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     const int t = r / p.group, g = r - t * p.group;
     const bool row_ok = r < p.tpb * p.group && t < ntok;
     const int prow = row_ok ? pos0 + t : -1;                                  // position of the row's token
-    const int lo_row = (p.window > 0 && prow >= 0) ? max(0, prow - p.window + 1) : 0;
+    const int lo_row = prow >= 0 ? at_first_visible(p, SHAPED, prow) : 0;
+    float row_scale = p.scale_log2, row_slope = 0.f;
+    const int row_head = row_ok ? kvh * p.group + g : 0;
+    if (SHAPED) {
+      if (p.qt_every > 0 && row_ok) row_scale *= 1.0f + p.qt_coef * logf((float)((prow + 1) / p.qt_every) + 1.0f);
+      if (p.slope != nullptr) row_slope = p.slope[row_head] * AT_LOG2E;
+    }
     const unsigned lane_addr = (unsigned)(32 * ew) << 16;
     float m_ref = -INFINITY, l_run = 0.f;   // reference maximum (scaled, log2 units) and sum against it
 
     for (int j = 0; j < nblk; ++j) {
       const int b = j & 1;
-      const int k0 = (kb_lo + j) * AT_KB;
+      const int k0 = block_key(j);
       at_mbar_wait(s_full0 + 8 * b, (unsigned)((j >> 1) & 1), p.status, dead);
       AT_FENCE_AFTER();
       float sv[AT_KB];
@@ -299,11 +350,36 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
       AT_FENCE_BEFORE();
       __syncwarp();
       if (lane == 0) at_mbar_arrive(s_empty0 + 8 * b);
+      if (SHAPED) {
+        // to the scores themselves, in log2 units
+#pragma unroll
+        for (int i = 0; i < AT_KB; ++i) sv[i] *= row_scale;
+        if (p.cap > 0.f) {
+#pragma unroll
+          for (int i = 0; i < AT_KB; ++i) sv[i] = p.cap * at_tanh(sv[i] * p.inv_cap);
+        }
+        const int far = prow - k0;             // distance of the block's first key (rows without a token: -1 - k0, all masked)
+        if (p.rel != nullptr && far >= 0) {
+          const float* rel = p.rel + row_head;
+          if (far - (AT_KB - 1) >= p.nd - 1) { // beyond the table: its last row for all
+            const float b = rel[(size_t)(p.nd - 1) * p.nh] * AT_LOG2E;
+#pragma unroll
+            for (int i = 0; i < AT_KB; ++i) sv[i] += b;
+          } else {
+#pragma unroll
+            for (int i = 0; i < AT_KB; ++i) sv[i] = fmaf(rel[min(max(far - i, 0), p.nd - 1) * p.nh], AT_LOG2E, sv[i]);
+          }
+        }
+        if (p.slope != nullptr) {
+#pragma unroll
+          for (int i = 0; i < AT_KB; ++i) sv[i] = fmaf(-row_slope, (float)(far - i), sv[i]);
+        }
+      }
       // mask by selection; maximum of the row's part
       if ((k0 + AT_KB - 1 > prow) || (k0 < lo_row)) {
 #pragma unroll
         for (int i = 0; i < AT_KB; ++i)
-          if (k0 + i > prow || k0 + i < lo_row) sv[i] = -INFINITY;
+          if (k0 + i > prow || (k0 + i < lo_row && (!SHAPED || k0 + i >= keep))) sv[i] = -INFINITY;
       }
       // (the softmax warps are bound by instruction issue: packed float32 pairs for the scaling and the sums,
       // three-input maxima, one MUFU instruction per exponential)
@@ -315,7 +391,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
         mx4[2] = at_max3(mx4[2], sv[i + 4], sv[i + 5]);
         mx4[3] = at_max3(mx4[3], sv[i + 6], sv[i + 7]);
       }
-      const float mxs = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      const float mxs = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * (SHAPED ? 1.0f : p.scale_log2);
       const bool grow = mxs > m_ref + 8.0f;          // also the first keys a row sees (m_ref = -inf)
       const float factor = grow ? at_ex2(m_ref - mxs) : 1.0f;   // m_ref = -inf: 0 (O and the sum are 0 then)
       if (grow) m_ref = mxs;
@@ -326,11 +402,16 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
       unsigned pw[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float2 a = __ffma2_rn(make_float2(sv[2 * i], sv[2 * i + 1]), sc2, nm2);
+        const float2 x = make_float2(sv[2 * i], sv[2 * i + 1]);
+        const float2 a = SHAPED ? __fadd2_rn(x, nm2) : __ffma2_rn(x, sc2, nm2);
         const float2 e = make_float2(at_ex2(a.x), at_ex2(a.y));
         sum2[i & 1] = __fadd2_rn(sum2[i & 1], e);
         const __nv_bfloat162 h = __floats2bfloat162_rn(e.x, e.y);
         pw[i] = *reinterpret_cast<const unsigned*>(&h);
+        if (SHAPED) {          // what the high term leaves
+          sv[2 * i] = e.x - __bfloat162float(h.x);
+          sv[2 * i + 1] = e.y - __bfloat162float(h.y);
+        }
       }
       const float2 st = __fadd2_rn(sum2[0], sum2[1]);
       l_run = l_run * factor + (st.x + st.y);
@@ -352,12 +433,12 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
       // keys that no row of the CTA may see: their rows of V (128 bytes for each 64 head-size elements, whole
       // rows, so the swizzle does not matter) become zeros before the product reads them
       if (k0 + AT_KB - 1 > hi || k0 < lo_min) {
-        const int s = j % AT_KS;
-        at_mbar_wait(v_full0 + 8 * s, (unsigned)((j / AT_KS) & 1), p.status, dead);
-        unsigned char* v_s = kv_s + s * STAGE_BYTES + KV_BYTES;
+        const int s = j % VS;
+        at_mbar_wait(v_full0 + 8 * s, (unsigned)((j / VS) & 1), p.status, dead);
+        unsigned char* v_s = kv_s + s * K_STEP + V_AT;
         for (int idx = tid - 64; idx < AT_KB * HB * 8; idx += 128) {
           const int kk = idx / (HB * 8), rest = idx - kk * (HB * 8);
-          if (k0 + kk > hi || k0 + kk < lo_min)
+          if (k0 + kk > hi || (k0 + kk < lo_min && k0 + kk >= keep))
             *reinterpret_cast<uint4*>(v_s + (rest >> 3) * (KV_BYTES / HB) + kk * 128 + ((rest & 7) << 4)) =
                 make_uint4(0u, 0u, 0u, 0u);
         }
@@ -367,6 +448,18 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
       for (int c = 0; c < 8; ++c)
         *reinterpret_cast<uint4*>(prow_s + ((c ^ (r & 7)) << 4)) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
+      if (SHAPED) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          unsigned w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(sv[8 * c + 2 * i], sv[8 * c + 2 * i + 1]);
+            w[i] = *reinterpret_cast<const unsigned*>(&h);
+          }
+          *reinterpret_cast<uint4*>(prow_s + P_BYTES + ((c ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P is read by the tensor cores
       AT_FENCE_BEFORE();                                             // and so is the rescaled O
       __syncwarp();
@@ -408,7 +501,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
         // 4 x splits trips to L2.  Online merge: the running maximum and sum are rescaled as the partials come.
         __threadfence();
         float* part_s = reinterpret_cast<float*>(kv_s);
-        static_assert(PSTRIDE * 4 <= AT_KS * STAGE_BYTES + P_BYTES, "a partial fits the freed shared memory");
+        static_assert(PSTRIDE * 4 <= P_AT + (SHAPED ? 2 : 1) * P_BYTES, "a partial fits the freed shared memory");
         float m_cur = m_ref, l_cur = l_run;
         int round = 0;
         for (int q = 0; q < eff; ++q) {
@@ -442,7 +535,9 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     }
     // (the sink's share of the sum is added once, to the whole row's; a row without keys has none to show)
     if (p.sink != nullptr && row_ok && m_ref != -INFINITY) l_run += exp2f(p.sink[kvh * p.group + g] * 1.4426950408889634f - m_ref);
+    if (SHAPED && p.zero_sink && m_ref != -INFINITY) l_run += exp2f(-m_ref);
     inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+    if (SHAPED) inv *= p.out_scale;
     if (finish && p.pairs) {
       float ss = 0.f;
 #pragma unroll
@@ -461,7 +556,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
         const float gv = __bfloat162float(p.gate[(size_t)(tok0 + t) * p.gate_stride + (size_t)((kvh * p.group + g) >> 1)]);
         post *= 1.0f / (1.0f + expf(-gv));
       }
-    } else if (finish && p.gate != nullptr) {
+    } else if (finish && p.gate != nullptr && !(SHAPED && p.gate_channels)) {
       const int tt = r / p.group, gg = r - tt * p.group;
       if (r < p.tpb * p.group && tt < ntok) {
         const float gv = __bfloat162float(p.gate[(size_t)(tok0 + tt) * p.gate_stride + (size_t)(kvh * p.group + gg)]);
@@ -477,7 +572,21 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
         at_ld32(tmem_o + lane_addr + c0, v);
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] *= inv;
-        if (p.pairs) {
+        if (SHAPED && p.gate_channels && p.gate != nullptr && row_ok) {
+          const bf16* gt = p.gate + (size_t)(tok0 + t) * p.gate_stride + (size_t)row_head * HD + c0;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint4 u = *reinterpret_cast<const uint4*>(gt + 8 * q);
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float2 z = __bfloat1622float2(h2[k]);
+              v[8 * q + 2 * k] *= 1.0f / (1.0f + expf(-z.x));
+              v[8 * q + 2 * k + 1] *= 1.0f / (1.0f + expf(-z.y));
+            }
+          }
+        }
+        if (!SHAPED && p.pairs) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = (v[i] - p.lambda * __shfl_xor_sync(0xffffffffu, v[i], 1)) * post;
         }
@@ -543,7 +652,7 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
                   const int* req_slot, int n_entries, int row_blocks, int nh, int nkv, int hd, int page_size,
                   int num_pages, int window, float scale, int nsplit, int split_len, float* scratch, int* counters,
                   const void* gate, long gate_stride, int pairs, float lambda, float post, float pair_eps, int* status,
-                  cudaStream_t stream, const float* sink = nullptr, long kv_stride = 0) {
+                  cudaStream_t stream, const float* sink = nullptr, long kv_stride = 0, const AttnTcParams* shaped = nullptr) {
   if (row_blocks <= 0 || n_entries <= 0) return 0;
   if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv != 0 || nkv > 65535 || nh / nkv > 128 || (pairs && (nh / nkv) % 2 != 0))
     return (int)cudaErrorInvalidValue;
@@ -555,7 +664,8 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
     return (int)cudaErrorInvalidValue;
   at_encode_fn enc = at_encoder();
   if (enc == nullptr) return (int)cudaErrorNotSupported;
-  AttnTcParams p;
+  AttnTcParams p = {};
+  if (shaped != nullptr) p = *shaped;
   p.out = (bf16*)out;
   p.out_stride = out_stride;
   p.block_table = block_table;
@@ -577,6 +687,7 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
   p.counters = counters;
   p.gate = (const bf16*)gate;
   p.gate_stride = gate_stride;
+  p.nh = nh;
   p.pairs = pairs;
   p.lambda = lambda;
   p.post = post;
@@ -608,16 +719,22 @@ static int at_run(void* out, long out_stride, const void* q, long q_stride, int 
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return (int)cudaErrorInvalidValue;
   }
-  const size_t smem = (size_t)128 * hd * 2 + (size_t)AT_KS * 2 * AT_KB * hd * 2 + 128 * AT_KB * 2 + 256;
+  // Q, the K and V stages, P's terms (the kernel's layouts), the barriers
+  const size_t smem = (size_t)128 * hd * 2 + (size_t)(shaped != nullptr ? AT_KS + 1 : 2 * AT_KS) * AT_KB * hd * 2 +
+                      (shaped != nullptr ? 2 : 1) * 128 * AT_KB * 2 + 256;
   p.row_blocks = row_blocks;
   p.split_len = split_len;
   dim3 grid(row_blocks * nsplit * nkv);
-  if (hd == 64) {
-    cudaFuncSetAttribute(attn_prefill_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ll_launch(attn_prefill_tc_kernel<64>, grid, dim3(AT_THREADS), smem, stream, p, qmap, kmap, vmap);
+  auto launch = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ll_launch(kernel, grid, dim3(AT_THREADS), smem, stream, p, qmap, kmap, vmap);
+  };
+  if (shaped != nullptr) {
+    if (hd == 64) launch(attn_prefill_tc_kernel<64, true>);
+    else launch(attn_prefill_tc_kernel<128, true>);
   } else {
-    cudaFuncSetAttribute(attn_prefill_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ll_launch(attn_prefill_tc_kernel<128>, grid, dim3(AT_THREADS), smem, stream, p, qmap, kmap, vmap);
+    if (hd == 64) launch(attn_prefill_tc_kernel<64, false>);
+    else launch(attn_prefill_tc_kernel<128, false>);
   }
   return LL_LAUNCH_RESULT();
 }
@@ -674,4 +791,38 @@ extern "C" int ll_attn_prefill_tc_rows(void* out, long out_stride, const void* q
   return at_run(out, out_stride, q, q_stride, num_tokens, k, v, block_table, bt_stride, cu_q, ctx_len, req_slot, n_entries,
                 row_blocks, nh, nkv, hd, page_size, num_pages, window, scale, nsplit, split_len, scratch, counters, nullptr, 0,
                 0, 0.f, 0.f, 0.f, status, stream, sink, kv_stride);
+}
+
+// Shaped scores (see the head of this file): the parameters of ll_attn_shaped (attention_shaped_mma.cu) for prompt portions
+// without mixed heads and pairs.  mask 0 causal, 1 window, 2 chunks of mask_size; sink: 1 a key of score 0, or sink_val
+// (float32 [nh]); rel float32 [nd, nh], slope float32 [nh], gate bfloat16 (16-byte aligned rows where it has channels).
+extern "C" int ll_attn_prefill_tc_shaped(void* out, long out_stride, const void* q, long q_stride, int num_tokens,
+                                         const void* k_cache, const void* v_cache, const int* block_table, int bt_stride,
+                                         const int* cu_q, const int* ctx_len, const int* req_slot, int n_entries,
+                                         int row_blocks, int nh, int nkv, int hd, int page_size, int num_pages, int mask,
+                                         int mask_size, int keep, int sink, const float* sink_val, const float* rel, int nd,
+                                         const float* slope, float cap, float qt_coef, int qt_every, float scale,
+                                         float out_scale, int nsplit, int split_len, float* scratch, int* counters,
+                                         const void* gate, long gate_stride, int gate_channels, int* status,
+                                         cudaStream_t stream) {
+  if (mask < 0 || mask > 2 || (mask != 0 && mask_size <= 0) || keep < 0 || (rel != nullptr && nd <= 0) ||
+      (gate != nullptr && gate_channels && ((gate_stride % 8) != 0 || ((uintptr_t)gate % 16) != 0)))
+    return (int)cudaErrorInvalidValue;
+  AttnTcParams s = {};
+  s.mask = mask;
+  s.mask_size = mask_size;
+  s.keep = mask == 1 ? keep : 0;
+  s.zero_sink = sink != 0 && sink_val == nullptr;
+  s.rel = rel;
+  s.nd = nd;
+  s.slope = slope;
+  s.cap = cap > 0.f ? cap * AT_LOG2E : 0.f;
+  s.inv_cap = cap > 0.f ? 1.0f / (cap * AT_LOG2E) : 0.f;
+  s.qt_coef = qt_coef;
+  s.qt_every = qt_every;
+  s.gate_channels = gate_channels;
+  s.out_scale = out_scale;
+  return at_run(out, out_stride, q, q_stride, num_tokens, k_cache, v_cache, block_table, bt_stride, cu_q, ctx_len, req_slot,
+                n_entries, row_blocks, nh, nkv, hd, page_size, num_pages, 0, scale, nsplit, split_len, scratch, counters, gate,
+                gate_stride, 0, 0.f, 0.f, 0.f, status, stream, sink ? sink_val : nullptr, 0, &s);
 }

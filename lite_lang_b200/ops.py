@@ -511,7 +511,8 @@ def _attn_tc_scratch_for(device, row_blocks: int, num_kv_heads: int, nsplit: int
     return have
 
 
-def attn_prefill_tc_plan(entries, group: int, window: Optional[int], num_kv_heads: int = 1, slots: int = 0):
+def attn_prefill_tc_plan(entries, group: int, window: Optional[int], num_kv_heads: int = 1, slots: int = 0,
+                         chunk: Optional[int] = None, keep_first: int = 0):
     """(row blocks, nsplit, split_len) of a step for ``attn_prefill_tc``.  ``entries``: (cached tokens, new tokens)
     per entry; a row block takes floor(128 / group) tokens and walks n key blocks of 64.
 
@@ -521,14 +522,14 @@ def attn_prefill_tc_plan(entries, group: int, window: Optional[int], num_kv_head
     ``split_len`` for which all CTAs of the step fit the ``slots`` (two an SM) at once: a whole causal prompt of
     2,048 tokens (row blocks of 1..32 blocks, 2 kv heads) gets 16, i.e. its longer half is cut in two.  Not below
     4 blocks a split or over 8 splits (every split's partial result goes through scratch memory); when the
-    unsplit row blocks already exceed the slots, nothing is cut."""
+    unsplit row blocks already exceed the slots, nothing is cut.  ``chunk``, ``keep_first``: the masks of shaped scores."""
     tpb = 128 // group
     lengths = []
     for ctx, q in entries:
         for first in range(0, q, tpb):
             hi = ctx + min(first + tpb, q) - 1
-            lo = max(0, ctx + first - window + 1) if window else 0
-            lengths.append(hi // 64 - lo // 64 + 1)
+            lo = max(0, ctx + first - window + 1) if window else (ctx + first) // chunk * chunk if chunk else 0
+            lengths.append(hi // 64 - lo // 64 + 1 + min((keep_first + 63) // 64, lo // 64))
     blocks = len(lengths)
     if not lengths or slots <= 0 or blocks * num_kv_heads > slots:
         return blocks, 1, 1 << 20
@@ -2204,6 +2205,51 @@ def attn_shaped(out: torch.Tensor, q: torch.Tensor, q_stride: int, mixed: bool, 
         c_int(0 if distance_bias is None else distance_bias.shape[0]), c_int(int(keep_first or 0)),
         c_float(float(softcap or 0.0)), c_float(qt_coef), c_int(qt_every), c_int(1 if gate_channels else 0),
         c_float(out_scale), _ptr(distance_slope), *_pair_args(pairs), _stream())
+
+
+def attn_prefill_tc_shaped(out: torch.Tensor, q: torch.Tensor, q_stride: int, gate: Optional[torch.Tensor],
+                           k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor, cu_q: torch.Tensor,
+                           ctx_len: torch.Tensor, req_slot: torch.Tensor, num_entries: int, plan, num_heads: int,
+                           num_kv_heads: int, head_dim: int, page_size: int, mask: str, mask_size: Optional[int], sink: bool,
+                           scale: float, status: Optional[torch.Tensor], sink_values: Optional[torch.Tensor] = None,
+                           distance_bias: Optional[torch.Tensor] = None, keep_first: int = 0, softcap: Optional[float] = None,
+                           query_temperature: Optional[Tuple[float, int]] = None, gate_channels: bool = False,
+                           out_scale: float = 1.0, distance_slope: Optional[torch.Tensor] = None) -> None:
+    """``attn_shaped`` of prompt portions (no mixed heads, pairs or temperature; values as wide as keys) on the tcgen05 kernel of
+    the plain attention; ``plan`` from ``attn_prefill_tc_plan``."""
+    _need_cuda(out, q, gate, k_cache, v_cache, block_table, cu_q, ctx_len, req_slot, sink_values, distance_bias, distance_slope)
+    for t, nm in ((sink_values, "sink_values"), (distance_bias, "distance_bias"), (distance_slope, "distance_slope")):
+        _f32(t, nm)
+    for t, nm in ((block_table, "block_table"), (cu_q, "cu_q"), (ctx_len, "ctx_len"), (req_slot, "req_slot")):
+        _i32(t, nm)
+    _need(attn_prefill_tc_supported(q.dtype, head_dim, page_size, q_stride, num_heads // num_kv_heads)
+          and out.dtype == k_cache.dtype == v_cache.dtype == torch.bfloat16, "attn_prefill_tc_shaped: dtypes, head or page size")
+    _need(out.stride(1) == 1 and out.shape[1] == num_heads * head_dim and out.stride(0) % 8 == 0 and q.stride(1) == 1
+          and q.shape[1] >= num_heads * head_dim and q.stride(0) == q_stride, "attn_prefill_tc_shaped: out, q")
+    _need(k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape == v_cache.shape
+          and tuple(k_cache.shape[1:]) == (num_kv_heads, page_size, head_dim), "cache plane shape")
+    _need(cu_q.numel() >= num_entries + 1 and ctx_len.numel() >= num_entries and req_slot.numel() >= num_entries,
+          "attn_prefill_tc_shaped: entry arrays too short")
+    _need(gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1
+                           and gate.shape[1] == (num_heads * head_dim if gate_channels else num_heads)), "gate: [tokens, heads] rows "
+          "(or a number a channel)")
+    _need(distance_bias is None or (distance_bias.dim() == 2 and distance_bias.shape[1] == num_heads), "distance_bias is "
+          "[distances, heads]")
+    _need((mask == "causal" or (mask_size or 0) > 0) and all(t is None or t.numel() == num_heads
+                                                             for t in (sink_values, distance_slope)), "a number a head")
+    row_blocks, nsplit, split_len = plan
+    scratch, counters = _attn_tc_scratch_for(q.device, row_blocks, num_kv_heads, nsplit, head_dim)
+    qt_coef, qt_every = (0.0, 0) if query_temperature is None else (float(query_temperature[0]), int(query_temperature[1]))
+    load_library("attn_tc").call(
+        "ll_attn_prefill_tc_shaped", _ptr(out), c_long(out.stride(0)), _ptr(q), c_long(q_stride), c_int(q.shape[0]),
+        _ptr(k_cache), _ptr(v_cache), _ptr(block_table), c_int(block_table.stride(0)), _ptr(cu_q), _ptr(ctx_len), _ptr(req_slot),
+        c_int(num_entries), c_int(row_blocks), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(page_size),
+        c_int(k_cache.shape[0]), c_int(ATTN_MASK[mask]), c_int(int(mask_size or 0)), c_int(int(keep_first or 0)),
+        c_int(1 if sink else 0), _ptr(sink_values), _ptr(distance_bias),
+        c_int(0 if distance_bias is None else distance_bias.shape[0]), _ptr(distance_slope), c_float(float(softcap or 0.0)),
+        c_float(qt_coef), c_int(qt_every), c_float(scale), c_float(out_scale), c_int(nsplit), c_int(max(1, int(split_len))),
+        _ptr(scratch), _ptr(counters), _ptr(gate), c_long(0 if gate is None else gate.stride(0)),
+        c_int(1 if gate_channels else 0), _ptr(status), _stream())
 
 
 def attention_modulated(out: torch.Tensor, q: torch.Tensor, q_stride: int, gate: Optional[torch.Tensor],

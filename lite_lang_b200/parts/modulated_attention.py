@@ -53,8 +53,8 @@ anything is rounded.
 
 Kernels: in bfloat16 with head sizes 64 and 128, tensor cores (``attn_shaped``: prompt portions 128 rows a CTA,
 single tokens with their keys split over CTAs; mixed heads as one wider query a head, made where q is
-normalised; prompt portions of a design without mixed heads and sink: the plain attention's tcgen05 kernel, the
-temperature on the queries and the gate in its epilogue); every other size, and float32, a block a token in
+normalised; prompt portions of a design without mixed heads: the plain attention's tcgen05 kernel, the temperature on
+the queries, the scores shaped by the softmax's threads and the gate in its epilogue); every other size, and float32, a block a token in
 float32 arithmetic (``attention_modulated``).
 """
 
@@ -286,7 +286,7 @@ class ModulatedAttention(Mixer):
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
             if self.key_dim in (64, 128) and self.vdim in (64, 128):
                 libs.append("attn_shaped")
-                if not self.head_mix and not self.sink and not self.extended and self.vdim == self.key_dim and self.mask != "chunk":
+                if not self.head_mix and self.vdim == self.key_dim:
                     libs.append("attn_tc")
         return libs
 
@@ -429,6 +429,23 @@ class ModulatedAttention(Mixer):
                                 step.ctx_len[n_single:], step.req_slot[n_single:], n_rest, plan[0], self.map_heads,
                                 self.num_kv_heads, self.key_dim, cache.page_size, window, self.scale, step.status,
                                 nsplit=plan[1], split_len=plan[2], gate=gate, pairs=self.pairs)
+        elif (n_rest > 0 and mixed_q is None and temperature is None and self.vdim == self.key_dim and self.pairs is None
+                and ops.TC_ENABLED and getattr(step, "entry_ctx", None) is not None
+                and ops.attn_prefill_tc_supported(q.dtype, self.key_dim, cache.page_size, q.stride(0), group)
+                and (gate is None or not self.channel_gate or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))):
+            # shaped scores on the same kernel: the row's thread makes them between product and softmax
+            key = ("attn_prefill_tc_shaped", group, self.mask, self.mask_size, self.keep_first)
+            plan = step.scratch.get(key)
+            if plan is None:
+                plan = step.scratch[key] = ops.attn_prefill_tc_plan(
+                    [(step.entry_ctx[n_single + i], len(e.tokens)) for i, e in enumerate(step.entries[n_single:])], group,
+                    self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(proj.device),
+                    self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0)
+            del more["pairs"]
+            ops.attn_prefill_tc_shaped(out, q, q.stride(0), gate, cache.k, cache.v, cache.block_table, step.cu_q[n_single:],
+                                       step.ctx_len[n_single:], step.req_slot[n_single:], n_rest, plan, self.map_heads,
+                                       self.num_kv_heads, self.key_dim, cache.page_size, self.mask, self.mask_size, self.sink,
+                                       self.scale, step.status, **more)
         elif n_rest > 0:
             key = ("attn_shaped", group)
             blocks = step.scratch.get(key)
