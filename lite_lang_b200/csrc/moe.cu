@@ -24,9 +24,9 @@
 // is added to the scores for the choice.  With `keep` < `count`, only outputs of the `keep` groups (E / count neighbours
 // each) with the largest best choice score can be chosen.  A place that finds nothing left gets top_idx -1 and weight 0.
 //
-// A block takes TOK tokens (one, and then a warp an output; or eight in long portions: the router's matrix is then read
-// once for eight tokens); its warps share out the outputs, and then the tokens, whose scores a warp each makes and picks
-// from.  A lane sums its pieces of four numbers of a row (four sums side by side), then the lanes are added up: an order
+// A block takes TOK tokens (one, and then a warp an output; or eight in long portions, four a warp: the router's matrix is
+// then read once for four tokens); its warps share out the outputs, and then the tokens, whose scores a warp each makes and
+// picks from.  Bound by the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row (four sums side by side), then the lanes are added up: an order
 // that depends on the sizes only.
 __device__ __forceinline__ float4 moe_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 moe_load4(const bf16* p) {
@@ -43,9 +43,9 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
                   int renormalize, const float* __restrict__ choice_bias, int count, int keep, float weight_scale,
                   float* __restrict__ identity_w, int real, int pitch) {
   extern __shared__ __align__(16) float moe_smem[];      // [TOK]: logits / scores [E + 1], choice scores [E], groups' best
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tok0 = blockIdx.x * TOK, nt = min(TOK, num_tokens - tok0);
   const int zs = 2 * E + 1 + count;
   T* xrow = reinterpret_cast<T*>(moe_smem + (TOK * zs + 3) / 4 * 4);     // the tokens' rows, `pitch` apart
@@ -64,18 +64,23 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
   __syncthreads();
   const int n_rows = E + (shared_w ? 1 : 0);
   const bool vec = (hidden & 3) == 0;
-  for (int e = warp; e < n_rows; e += THREADS / 32) {
-    float a[TOK][4];
+  constexpr int PER = TOK < 4 ? TOK : 4;                  // tokens of a warp at a time
+  const int units = n_rows * (TOK / PER);
+  for (int i = warp; i < units; i += THREADS / 32) {
+    // (blocks start at different outputs: at the same ones they would all ask the same few lines of L2 at a time)
+    const int un = TOK == 1 ? i : (i + blockIdx.x * 5) % units, e = un / (TOK / PER), k0 = un % (TOK / PER) * PER;
+    const T* xs = xrow + (size_t)k0 * pitch;
+    float a[PER][4];
 #pragma unroll
-    for (int k = 0; k < TOK; ++k) a[k][0] = a[k][1] = a[k][2] = a[k][3] = 0.f;
+    for (int k = 0; k < PER; ++k) a[k][0] = a[k][1] = a[k][2] = a[k][3] = 0.f;
     const float* wrow = Wr + (size_t)e * hidden;
     if (vec) {
 #pragma unroll(TOK == 1 ? 8 : 4)
       for (int i = 4 * lane; i < hidden; i += 128) {
         const float4 w4 = *reinterpret_cast<const float4*>(wrow + i);
 #pragma unroll
-        for (int k = 0; k < TOK; ++k) {
-          const float4 x4 = moe_load4(xrow + (size_t)k * pitch + i);
+        for (int k = 0; k < PER; ++k) {
+          const float4 x4 = moe_load4(xs + (size_t)k * pitch + i);
           a[k][0] = fmaf(w4.x, x4.x, a[k][0]);
           a[k][1] = fmaf(w4.y, x4.y, a[k][1]);
           a[k][2] = fmaf(w4.z, x4.z, a[k][2]);
@@ -85,12 +90,12 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
     } else {
       for (int i = lane; i < hidden; i += 32)
 #pragma unroll
-        for (int k = 0; k < TOK; ++k) a[k][0] = fmaf(wrow[i], to_f32<T>(xrow[(size_t)k * pitch + i]), a[k][0]);
+        for (int k = 0; k < PER; ++k) a[k][0] = fmaf(wrow[i], to_f32<T>(xs[(size_t)k * pitch + i]), a[k][0]);
     }
 #pragma unroll
-    for (int k = 0; k < TOK; ++k) {
+    for (int k = 0; k < PER; ++k) {
       const float v = warp_sum((a[k][0] + a[k][1]) + (a[k][2] + a[k][3]));
-      if (lane == 0 && k < nt) moe_smem[k * zs + e] = v + ((bias && e < E) ? bias[e] : 0.f);
+      if (lane == 0 && k0 + k < nt) moe_smem[(k0 + k) * zs + e] = v + ((bias && e < E) ? bias[e] : 0.f);
     }
   }
   __syncthreads();
@@ -275,7 +280,7 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
   } while (0)
   LL_DISPATCH_DTYPE(dtype, {
     if (num_tokens >= 512 && sizeof(float) * 8 * (size_t)zs + sizeof(T) * 8 * (size_t)pitch <= 100 * 1024)
-      MOE_ROUTER_LAUNCH(8, 256);
+      MOE_ROUTER_LAUNCH(8, 512);
     else if (E > 8)
       MOE_ROUTER_LAUNCH(1, 1024);
     else
@@ -328,21 +333,32 @@ moe_sort_kernel(const int* __restrict__ top_idx, const float* __restrict__ top_w
   LL_PDL_WAIT();      // (no early release: what runs next may be a library kernel that does not wait itself)
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 1;
   __syncthreads();
+#pragma unroll 8
   for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
     const int e = top_idx[p];
     if (e >= 0 && e < E) atomicAdd(&count[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {      // a warp adds the counts up, 32 experts at a time
     int at = 0;
-    for (int e = 0; e < E; ++e) {
-      row_token[at] = 0;
-      row_w[at] = 0.f;
-      start[e] = at + 1;
-      at += count[e];
-      ends[e] = at;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x, n = e < E ? count[e] : 0;
+      int sum = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (threadIdx.x >= o) sum += v;
+      }
+      if (e < E) {
+        const int first = at + sum - n;
+        row_token[first] = 0;
+        row_w[first] = 0.f;
+        start[e] = first + 1;
+        ends[e] = at + sum;
+      }
+      at += __shfl_sync(0xffffffffu, sum, 31);
     }
-    used = at;
+    if (threadIdx.x == 0) used = at;
   }
   __syncthreads();
   // rows behind the last run (pairs that no expert has: identities): a token that exists, weight 0
@@ -350,6 +366,7 @@ moe_sort_kernel(const int* __restrict__ top_idx, const float* __restrict__ top_w
     row_token[row] = 0;
     row_w[row] = 0.f;
   }
+#pragma unroll 8
   for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
     const int e = top_idx[p];
     if (e >= 0 && e < E) {
@@ -380,6 +397,19 @@ __global__ void moe_gather_rows_kernel(T* __restrict__ dst, const T* __restrict_
   }
 }
 
+// VEC neighbouring numbers, one access
+template <typename T, int VEC> struct MoePiece {
+  alignas(sizeof(T) * VEC) T v[VEC];
+  __device__ __forceinline__ void load(const T* p) {
+    if constexpr (VEC > 1) *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(p);
+    else v[0] = p[0];
+  }
+  __device__ __forceinline__ void store(T* p) const {
+    if constexpr (VEC > 1) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(v);
+    else p[0] = v[0];
+  }
+};
+
 // h[row, :] = act(h[row, :]) * row_w[row], in place; VEC neighbouring numbers of a row a thread
 template <typename T, int VEC>
 __global__ void moe_row_act_kernel(T* __restrict__ h, const float* __restrict__ row_w, long total_vec, int ff, int act) {
@@ -398,20 +428,44 @@ __global__ void moe_row_act_kernel(T* __restrict__ h, const float* __restrict__ 
 }
 
 // out[t, :] = base[t, :] + sum over k (in the order of k) of y[pair_row[t, k], :]; float32 sums, one rounding.
-template <typename T>
+// A thread takes VEC neighbouring columns of one token (16-byte accesses where the width allows it), four rows' loads on
+// their way at once: bound by memory.
+template <typename T, int VEC>
 __global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ base, const T* __restrict__ y,
                                    const int* __restrict__ pair_row, int top, int hidden) {
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int t = blockIdx.x;
-  for (int c = threadIdx.x; c < hidden; c += blockDim.x) {
-    float a = 0.f;
-    for (int k = 0; k < top; ++k) {
-      const int row = pair_row[(size_t)t * top + k];
-      if (row >= 0) a += to_f32<T>(y[(size_t)row * hidden + c]);
+  const int* rows = pair_row + (size_t)t * top;
+  for (int c = threadIdx.x * VEC; c < hidden; c += blockDim.x * VEC) {
+    float a[VEC];
+#pragma unroll
+    for (int u = 0; u < VEC; ++u) a[u] = 0.f;
+    for (int k0 = 0; k0 < top; k0 += 4) {
+      MoePiece<T, VEC> v[4];
+      bool on[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = k0 + i < top ? rows[k0 + i] : -1;
+        on[i] = row >= 0;
+        if (on[i]) v[i].load(y + (size_t)row * hidden + c);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (on[i]) {
+#pragma unroll
+          for (int u = 0; u < VEC; ++u) a[u] += to_f32<T>(v[i].v[u]);
+        }
     }
-    if (base) a += to_f32<T>(base[(size_t)t * hidden + c]);
-    out[(size_t)t * hidden + c] = from_f32<T>(a);
+    MoePiece<T, VEC> o;
+    if (base) {
+      o.load(base + (size_t)t * hidden + c);
+#pragma unroll
+      for (int u = 0; u < VEC; ++u) a[u] += to_f32<T>(o.v[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < VEC; ++u) o.v[u] = from_f32<T>(a[u]);
+    o.store(out + (size_t)t * hidden + c);
   }
 }
 
@@ -451,8 +505,17 @@ extern "C" int ll_moe_row_act(int dtype, void* h, const float* row_w, int rows, 
 extern "C" int ll_moe_combine(int dtype, void* out, const void* base, const void* y, const int* pair_row,
                               int num_tokens, int top, int hidden, cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
-  LL_DISPATCH_DTYPE(dtype, ll_launch(moe_combine_kernel<T>, dim3(num_tokens), dim3(256), 0, stream, (T*)out,
-                                     (const T*)base, (const T*)y, pair_row, top, hidden));
+  LL_DISPATCH_DTYPE(dtype, {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    const bool wide = (hidden % VEC) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)base % 16) == 0 && ((uintptr_t)y % 16) == 0;
+    const int threads = wide && hidden < 256 * VEC ? (hidden / VEC + 31) / 32 * 32 : 256;
+    if (wide)
+      ll_launch(moe_combine_kernel<T, VEC>, dim3(num_tokens), dim3(threads), 0, stream, (T*)out, (const T*)base, (const T*)y,
+                pair_row, top, hidden);
+    else
+      ll_launch(moe_combine_kernel<T, 1>, dim3(num_tokens), dim3(256), 0, stream, (T*)out, (const T*)base, (const T*)y,
+                pair_row, top, hidden);
+  });
   return LL_LAUNCH_RESULT();
 }
 
@@ -527,7 +590,8 @@ __global__ void moe_row_gated_act_kernel(T* __restrict__ out, const T* __restric
   const long step = (long)gridDim.x * blockDim.x;
   const int per_row = ff / VEC;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total_vec; idx += step) {
-    const long r = idx / per_row;
+    // (a 64-bit division is a subroutine)
+    const long r = total_vec <= 0xffffffffl ? (long)((unsigned)idx / (unsigned)per_row) : idx / per_row;
     const int j = (int)(idx - r * per_row) * VEC;
     const float w = row_w ? row_w[r] : 1.f;
     const T* p = in + (size_t)r * 2 * ff + j;
