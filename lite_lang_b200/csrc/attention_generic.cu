@@ -2,8 +2,8 @@
 // size up to 256 and value head size up to 512 (the two may differ), any page
 // size, any group size, float32 or bfloat16 storage.
 //
-// It is the kernel of the true 32-bit path and the fallback of the bfloat16
-// path for shapes the tensor-core kernels do not take.  Every new token t of
+// It is the fallback of both paths for shapes the tensor-core kernels
+// (attention_f32.cu for float32) do not take.  Every new token t of
 // the step is a query at position p = positions[t] of the request in entry
 // token_req[t]; it looks at the cached keys lo..p of that request, where
 // lo = max(0, p - window + 1) with a window and 0 without.  The new tokens'

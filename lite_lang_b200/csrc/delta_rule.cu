@@ -10,15 +10,15 @@
 // [(taps - 1), channels] for the last taps - 1 inputs of the convolutions (oldest first;
 // channels = q | k | v), so that a request can go on in a later step from where it stopped.
 //
-// Four kernels (a portion's recurrence may go by chunks instead: chunk_scan.cu), all reading the step's device arrays only (so that a step of single tokens can
-// be captured and replayed):
+// Four kernels (a long portion's recurrence with one decay a head goes by chunks instead: chunk_scan.cu), all reading the
+// step's device arrays only (so that a step of single tokens can be captured and replayed):
 //   delta_prepare      per token: convolution + SiLU, unit vectors, beta, decay -> float32 buffers
 //   delta_conv_update  per entry of several tokens: the new last taps - 1 inputs of the record
 //   delta_recurrence   per (entry, head, 16 value columns): the scan over the entry's tokens
 //   delta_out          per (token, head): o / rms(o) * weight * gate -> storage type
 // Every value column of S evolves on its own (S^T k and S^T q are per column), so the scan is
 // spread over value columns as well as over requests and heads; the order of every sum depends
-// on the sizes only, never on how tokens were cut into steps or batched.
+// on the sizes only; in the scan by tokens never on how they were cut into steps or batched.
 #include "common.cuh"
 
 __device__ __forceinline__ float dr_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }

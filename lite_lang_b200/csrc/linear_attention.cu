@@ -13,7 +13,8 @@
 // multiply-add a channel; the read-outs' sums over the lanes are taken for 16 tokens together (a halving
 // exchange: 15 shuffles instead of 64).  A token's arithmetic does not depend on where a step's portion began
 // (the exchange adds the same pairs whatever the token's place among the 16), so a position's result is the
-// same bits however the tokens were cut into steps.
+// same bits however the tokens were cut into steps.  (Long portions go by chunks instead: chunk_scan.cu; their sums
+// depend on where the portion began, in the last bits of float32.)
 //
 // The same scan serves a state-space layer whose decay and step size differ from token to token
 // (S_t = a_t,h S_(t-1) + dt_t,h k_t v_t^T, o_t = S_t^T q_t + D_h v_t, q and k shared by the `hpg` heads of a

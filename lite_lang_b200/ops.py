@@ -1187,8 +1187,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     """x [n, in] times weight [out, in] transposed.
 
     Up to 32 bfloat16 tokens (decode) go to the hand-written TMA weight-streaming kernel
-    (``gemm_stream``), or to ``gemm_smallm`` for shapes that one does not take.  Everything
-    else is a library (cuBLAS) product, as in the reference: float32 operands give a true
+    (``gemm_stream``), or to ``gemm_smallm`` for shapes that one does not take; large float32 products go to
+    ``gemm_f32``.  Everything else is a library (cuBLAS) product, as in the reference: float32 operands give a true
     float32 product (TF32 is off); bfloat16 operands accumulate in float32.
     ``out_dtype=torch.float32`` with bfloat16 operands keeps the float32 accumulator as the
     result (the logits).  ``partial_ok``: the caller's consumer (the fused residual-and-norm
