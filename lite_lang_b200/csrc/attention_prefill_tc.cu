@@ -151,6 +151,9 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   const int rb_step = p.row_blocks - 1 - l2 % p.row_blocks;   // row block within the step (names its scratch and counter)
   int rb = rb_step;
   int entry = -1, qlen = 0;
+  // Slots and context lengths of a cache plane's requests were uploaded before the step's first kernel.  With rows of a
+  // product they were made by a kernel of this step (latent_unpage), like the block table, and are there after the wait only.
+  if (p.head_cols > 0) LL_PDL_WAIT();
   for (int e = 0; e < p.n_entries; ++e) {
     const int ql = p.cu_q[e + 1] - p.cu_q[e];
     const int nb = (ql + p.tpb - 1) / p.tpb;
@@ -161,13 +164,13 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     }
     rb -= nb;
   }
-  if (entry < 0) return;
-  if ((at_smem(smem) & 1023u) != 0) {
-    if (threadIdx.x == 0) set_status(p.status, LL_ERR_SMEM_ALIGN);
+  const bool aligned = (at_smem(smem) & 1023u) == 0;
+  const int slot = entry >= 0 && aligned ? p.req_slot[entry] : -1;
+  if (slot < 0) {
+    if (!aligned && tid == 0) set_status(p.status, LL_ERR_SMEM_ALIGN);
+    LL_PDL_WAIT();   // (no CTA leaves before the wait: a grid of such CTAs would end before the kernels in front of it)
     return;
   }
-  const int slot = p.req_slot[entry];
-  if (slot < 0) return;
   const int tok0 = p.cu_q[entry] + rb * p.tpb;              // first token (row of q and out) of this CTA
   const int ntok = min(p.tpb, qlen - rb * p.tpb);
   const int pos0 = p.ctx_len[entry] + rb * p.tpb;           // its position (ctx_len: tokens cached before the step)
@@ -182,7 +185,10 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   int eff = min(p.nsplit, max(1, (nblk_all + p.split_len - 1) / p.split_len));
   const int per = (nblk_all + eff - 1) / eff;
   eff = (nblk_all + per - 1) / per;
-  if (split >= eff) return;
+  if (split >= eff) {
+    LL_PDL_WAIT();
+    return;
+  }
   const int b_first = split * per;                            // this CTA's first block
   const int nblk = min(per, nblk_all - split * per);
   // the first key of this CTA's block j

@@ -87,3 +87,97 @@ def test_expanded_portions_equal_the_latent_space(params, page, steps, monkeypat
         # both round their operands to bfloat16 (8 bits) in different places: a few roundings of the row's largest number
         assert float((a - b).abs().max()) <= 1.6e-2 * float(b.abs().max())
         assert float((a - b).norm()) <= 1e-2 * float(b.norm())
+
+
+def _exact(part, x):
+    """The part's output for one request's tokens, float64, from the same stored weights."""
+    H, d, r, R, n = part.H, part.d, part.r, part.R, x.shape[0]
+
+    def f(t):
+        return t.double()
+
+    proj = f(x) @ f(part.w_in).t()
+    q = proj[:, :H * (d + r)]
+    if part.q_rank is not None:
+        c = proj[:, :part.q_rank]
+        q = (c / (c.pow(2).mean(1, keepdim=True) + part.eps).sqrt() * f(part.q_norm_w)) @ f(part.w_uq).t()
+    q = q.reshape(n, H, d + r)
+    c, kr = proj[:, part.kv_off:part.kv_off + R], proj[:, part.kv_off + R:part.kv_off + R + r]
+    c = c / (c.pow(2).mean(1, keepdim=True) + part.eps).sqrt() * f(part.norm_w)
+    half = part.rot_dims // 2
+    angle = torch.arange(n, device=x.device, dtype=torch.float64)[:, None] * f(part.freq)[None, :half]
+    cs, sn = angle.cos() * part.amplitude, angle.sin() * part.amplitude
+
+    def turned(t):                       # [n, ..., r]
+        t = t.clone()
+        u = slice(0, half) if part.half_split else slice(0, 2 * half, 2)
+        v = slice(half, 2 * half) if part.half_split else slice(1, 2 * half, 2)
+        shape = (n,) + (1,) * (t.dim() - 2) + (half,)
+        a, b, co, si = t[..., u].clone(), t[..., v].clone(), cs.view(shape), sn.view(shape)
+        t[..., u], t[..., v] = a * co - b * si, b * co + a * si
+        return t
+
+    k = torch.cat([torch.einsum("nr,hdr->nhd", c, f(part.w_uk)), turned(kr)[:, None, :].expand(n, H, r)], dim=2)
+    q = torch.cat([q[..., :d], turned(q[..., d:])], dim=2)
+    s = torch.einsum("ihd,jhd->hij", q, k) * part.scale
+    i, j = torch.arange(n, device=x.device)[:, None], torch.arange(n, device=x.device)[None, :]
+    seen = (j <= i) & ((i - j < part.window) if part.window else True)
+    s = s.masked_fill(~seen, float("-inf"))
+    if part.sink:
+        s = torch.cat([s, f(part.sink_w)[:, None, None].expand(H, n, 1)], dim=2)
+    p = torch.softmax(s, dim=2)[:, :, :n]
+    o = torch.einsum("hij,jhe->ihe", p, torch.einsum("nr,hre->nhe", c, f(part.w_uv_t))).reshape(n, -1)
+    if part.channel_gate:
+        o = o * torch.sigmoid(proj[:, part.gate_off:part.gate_off + o.shape[1]])
+    return o @ f(part.w_o).t()
+
+
+def _rel(x, y):
+    return float((x.double() - y).norm() / y.norm())
+
+
+# 64 expanded rows (one page): their product with the expanded weights is this package's own (tcgen05 from 8,192 weight rows
+# on, streaming where the inner size is a multiple of 256), which lets the attention start before the rows' table is made
+@gpu
+@pytest.mark.parametrize("params", [
+    dict(hidden_size=256, heads=32, dim=64, rot_dim=64, vdim=128, kv_rank=512, rot_dims=64, eps=1e-6),
+    dict(hidden_size=256, heads=2, dim=128, rot_dim=0, vdim=128, kv_rank=256, sink=True, eps=1e-6)])
+@pytest.mark.parametrize("tokens", [64, 37])
+def test_expanded_portions_behind_the_packages_own_products(params, tokens, monkeypatch):
+    """Several layers queued behind a busy device, so that every kernel starts as early as it may."""
+    from lite_lang_b200 import ops
+    from lite_lang_b200.cache.manager import CacheManager, PagedGroupSpec
+    from lite_lang_b200.cache.storage import CacheStorage
+    from lite_lang_b200.engine.batch import BatchBuilder, StepEntry
+    device, layers, calls = torch.device("cuda", 0), 6, []
+    for name in ("gemm_tc", "gemm_stream"):
+        real = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, _real=real, **k: (calls.append(tuple(a[1].shape)), _real(*a, **k))[1])
+    parts = [_part(params, 20 + i) for i in range(layers)]
+    need = parts[0].cache_need()
+    manager = CacheManager([PagedGroupSpec(1, need.head_dim, need.window, layers, 0)], [8], 16, 1, tokens)
+    storage = CacheStorage(manager, torch.bfloat16, device)
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    builder = BatchBuilder(manager, tokens, 1, device, status)
+    slot = manager.open()
+    assert manager.reserve(slot, tokens)
+    storage.sync()
+    batch = builder.build([StepEntry(slot, [0] * tokens)])
+    x = torch.randn(tokens, 256, device=device, generator=torch.Generator(device="cuda").manual_seed(3)).to(torch.bfloat16)
+    busy = torch.randn(8192, 8192, device=device, dtype=torch.bfloat16)
+
+    def run():
+        torch.cuda.synchronize()
+        for _ in range(8):
+            torch.mm(busy, busy)                                     # milliseconds: the launches below pile up behind it
+        return [p.forward(x, batch, storage.paged_view(0, i, batch.slot_maps[0], True)) for i, p in enumerate(parts)]
+
+    outs = run()
+    assert sum(shape == tuple(p.w_kv.shape) for p in parts for shape in calls) >= layers, calls
+    again = run()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for p, a, b in zip(parts, outs, again):
+        assert torch.equal(a, b)
+        # bfloat16 at each of five products and twice in the attention: a few 2^-9 of the result
+        assert _rel(a.float().sum(0) if a.dim() == 3 else a, _exact(p, x)) <= 1.2e-2
