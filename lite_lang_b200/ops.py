@@ -1183,7 +1183,7 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation="silu") ->
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
-           out_dtype: Optional[torch.dtype] = None, partial_ok: bool = False) -> torch.Tensor:
+           out_dtype: Optional[torch.dtype] = None, partial_ok: bool = False, weight_made: bool = False) -> torch.Tensor:
     """x [n, in] times weight [out, in] transposed.
 
     Up to 32 bfloat16 tokens (decode) go to the hand-written TMA weight-streaming kernel
@@ -1193,16 +1193,19 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     ``out_dtype=torch.float32`` with bfloat16 operands keeps the float32 accumulator as the
     result (the logits).  ``partial_ok``: the caller's consumer (the fused residual-and-norm
     kernel) accepts float32 partial sums [parts, n, out] of a product split over k.
+    ``weight_made``: ``weight`` was written by a kernel of the same step (rows gathered from the cache); the weight-streaming
+    kernels, which fetch their weights before they wait for the kernels in front of them, do not take such a product.
     """
     _need_cuda(x, weight)
-    if out is None and partial_ok and out_dtype in (None, x.dtype) and tc_preferred(x, weight):
+    early = not weight_made
+    if early and out is None and partial_ok and out_dtype in (None, x.dtype) and tc_preferred(x, weight):
         parts = tc_ksplit(weight.shape[0], x.shape[1], x.device)
         out = torch.empty((parts, x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
         return gemm_tc(x, weight, out)
-    if out is None and weight.shape[0] >= 8192 and tc_preferred(x, weight, wide=True):
+    if early and out is None and weight.shape[0] >= 8192 and tc_preferred(x, weight, wide=True):
         out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
         return gemm_tc(x, weight, out)
-    mode = stream_mode(x, weight) if (out is None or out.stride(1) == 1) else None
+    mode = stream_mode(x, weight) if early and (out is None or out.stride(1) == 1) else None
     many = x.shape[0] > STREAM_M       # 33 to 64 tokens: bfloat16 out, k whole
     if mode is not None and many and ((out_dtype or x.dtype) != torch.bfloat16 or (out is not None and out.dtype != torch.bfloat16)):
         mode = None

@@ -273,7 +273,7 @@ class LatentAttention(Mixer):
             ops.latent_gather(keys, cache.k, cache.block_table, slot, lo, cache.page_size, step.status,
                               first=first, last=p0 + nb - 1)
             qb = q_full[t0 + b0:t0 + b0 + nb].view(nb * H, KD)
-            scores = ops.linear(qb, keys, out_dtype=torch.float32)                       # [nb * H, keys]
+            scores = ops.linear(qb, keys, out_dtype=torch.float32, weight_made=True)     # [nb * H, keys]
             weights = torch.empty(scores.shape, dtype=lat.dtype, device=lat.device)
             ops.latent_masked_softmax(weights, scores, H, p0, lo, self.window, self.scale, sink=self.sink_w)
             ops.product(weights, keys[:, :R], out=lat[t0 + b0:t0 + b0 + nb].view(nb * H, R))

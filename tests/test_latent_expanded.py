@@ -181,3 +181,26 @@ def test_expanded_portions_behind_the_packages_own_products(params, tokens, monk
         assert torch.equal(a, b)
         # bfloat16 at each of five products and twice in the attention: a few 2^-9 of the result
         assert _rel(a.float().sum(0) if a.dim() == 3 else a, _exact(p, x)) <= 1.2e-2
+
+
+# the last block of queries of these portions is short enough for the products that stream their weights, which here are
+# rows that a kernel of the same step gathers: those must not be asked for before that kernel has written them
+@gpu
+@pytest.mark.parametrize("params", [
+    dict(hidden_size=256, heads=2, dim=96, rot_dim=128, vdim=64, kv_rank=384, rot_dims=128, eps=1e-6),
+    dict(hidden_size=256, heads=3, dim=64, rot_dim=0, vdim=128, kv_rank=256, window=100, eps=1e-6)])
+@pytest.mark.parametrize("tokens", [258, 276])
+def test_gathered_rows_are_not_streamed_as_weights(params, tokens, monkeypatch):
+    from lite_lang_b200 import ops
+    streamed, scored = [], []
+    for name in ("gemm_tc", "gemm_stream"):
+        real = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, _real=real, **k: (streamed.append(a[1].data_ptr()), _real(*a, **k))[1])
+    gather = ops.latent_gather
+    monkeypatch.setattr(ops, "latent_gather", lambda dst, *a, **k: (scored.append(dst.data_ptr()), gather(dst, *a, **k))[1])
+    part = _part(params, 5)
+    monkeypatch.setattr(type(part), "EXPAND_MIN_TOKENS", 1 << 30)
+    got = _run(part, [[tokens]], 16, 9)[0]
+    assert len(scored) == 2 and not set(scored) & set(streamed)
+    x = torch.randn(tokens, part.hidden_size, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda")
+    assert _rel(got, _exact(part, x.to(torch.bfloat16))) <= 1.2e-2
