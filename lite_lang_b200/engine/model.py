@@ -20,6 +20,7 @@ from typing import Callable, Dict, List, Optional, Tuple
 
 import torch
 
+from .. import ops
 from ..cache.manager import PagedGroupSpec, StateGroupSpec
 from ..config.spec import ModelSpec
 from ..parts import base as parts_base
@@ -201,6 +202,10 @@ class CausalLM:
     # ------------------------------------------------------------------
     def forward(self, step, storage) -> Optional[torch.Tensor]:
         """Run the step's tokens through every run-step; float32 logits [wanted rows, vocab]."""
+        with ops.reporting_to(step.status):
+            return self._forward(step, storage)
+
+    def _forward(self, step, storage) -> Optional[torch.Tensor]:
         n = step.num_tokens
         h = self.embedding.forward(step.token_ids, n, step.status)
         delta = None

@@ -13,8 +13,10 @@ float32 path TF32 is switched off so that it is a true 32-bit product.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_long, c_void_p
 from typing import NamedTuple, Optional, Tuple
 
@@ -1103,12 +1105,30 @@ def f32_splits(m: int, n: int, k: int, device) -> int:
     return (boxes + per - 1) // per
 
 
+_reporting = threading.local()
+
+
+@contextlib.contextmanager
+def reporting_to(status: Optional[torch.Tensor]):
+    """Inside the block, products of this thread that are given no status word report to ``status``: a model's parts call
+    ``linear`` without one."""
+    before = getattr(_reporting, "status", None)
+    _reporting.status = status
+    try:
+        yield
+    finally:
+        _reporting.status = before
+
+
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
-             gated=None, partial_ok: bool = False, splits: Optional[int] = None) -> torch.Tensor:
+             gated=None, partial_ok: bool = False, splits: Optional[int] = None,
+             status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x [n, k] times weight [m, k] transposed, true float32, on tensor cores (csrc/gemm_f32.cu).  ``accumulate``: added to
     ``out``.  ``gated`` (a ``GateAct``): weight is [2 i, k], gate rows first, act(gate) * up comes out.  ``partial_ok``: where k
-    is cut into parts, they may be returned as [parts, n, m]."""
-    _need_cuda(x, weight, out)
+    is cut into parts, they may be returned as [parts, n, m].  ``status``: where the kernel reports a wait that ran out (the
+    word of ``reporting_to`` where none is given); the output is wrong then."""
+    _need_cuda(x, weight, out, status)
+    status = getattr(_reporting, "status", None) if status is None else status
     _need(x.dtype == weight.dtype == torch.float32 and x.stride(1) == weight.stride(1) == 1 and x.shape[1] % 8 == 0
           and x.stride(0) % 4 == 0 and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0,
           "gemm_f32: float32 rows, k a multiple of 8, 16-byte aligned")
@@ -1134,7 +1154,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         "ll_gemm_f32", _ptr(out), c_long(N if out is None else out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight),
         c_long(weight.stride(0)), c_int(M), c_int(N), c_int(K), _ptr(terms), _ptr(parts), c_int(splits),
         c_int(1 if accumulate else 0), c_int(0 if gated is None else GATE_ACT[act.kind] + 1), c_float(act.limit),
-        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(None), _stream())
+        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(status), _stream())
     return parts if hand_on else out
 
 

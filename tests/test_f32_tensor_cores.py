@@ -110,3 +110,60 @@ def test_prompt_attention(hd, nh, nkv, page, window):
     want = want.view(total, nh * hd)[1:]
     err, was = _rel(out[1:], want), _rel(general[1:], want)
     assert err <= max(1.5 * was, 4e-7), (err, was)
+
+
+class _Spy:
+    """Stands in for the kernel library: what it is called with, and nothing runs."""
+
+    def __init__(self):
+        self.status = []
+
+    def call(self, name, *args):
+        assert name == "ll_gemm_f32"
+        self.status.append(args[-2].value)
+
+
+def test_products_report_to_the_steps_status_word(monkeypatch):
+    """A wait that runs out leaves a wrong output: the kernel has to be handed a word to say so."""
+    import threading
+    import types
+
+    from lite_lang_b200 import ops
+    from lite_lang_b200.engine.model import CausalLM
+    spy, word = _Spy(), torch.zeros(1, dtype=torch.int32)
+    monkeypatch.setattr(ops, "_need_cuda", lambda *ts: None)
+    monkeypatch.setattr(ops, "load_library", lambda name: spy)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "f32_supported", lambda x, w: x.dtype == torch.float32)
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", False)
+    x, w = torch.zeros(96, 64), torch.zeros(64, 64)
+    ops.gemm_f32(x, w, status=word)
+    assert spy.status.pop() == word.data_ptr()
+
+    def products():
+        ops.linear(x, w)
+        ops.gated_linear(x, w)
+        ops.linear_accumulate(x, w, torch.zeros(96, 64))
+        got, spy.status[:] = list(spy.status), []
+        return got
+
+    other = []
+
+    def forward(ids, n, status):                       # the model's first part
+        other.clear()
+        t = threading.Thread(target=lambda: other.extend(products()))
+        t.start()
+        t.join()
+        assert other == [None] * 3                     # (another thread has a step of its own)
+        assert products() == [word.data_ptr()] * 3
+        return torch.zeros(n, 64)
+
+    model = CausalLM.__new__(CausalLM)
+    model.embedding = types.SimpleNamespace(forward=forward)
+    model.plan = []
+    model.forward(types.SimpleNamespace(num_tokens=96, token_ids=None, status=word, num_logits=0), None)
+    assert products() == [None] * 3
+    with pytest.raises(RuntimeError), ops.reporting_to(word):
+        raise RuntimeError
+    assert products() == [None] * 3
