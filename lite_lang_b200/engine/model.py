@@ -178,7 +178,8 @@ class CausalLM:
                 mixer.prepare(device, dtype)      # (a composite mixer prepares its members)
 
     def kernel_libraries(self) -> List[str]:
-        libs: List[str] = []
+        # (any part's product of many float32 rows goes to this one)
+        libs: List[str] = ["gemm_f32"] if self.dtype == torch.float32 else []
         for part in self._all_parts():
             for name in part.kernel_libraries():
                 if name not in libs:

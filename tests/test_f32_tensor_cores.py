@@ -61,6 +61,19 @@ def test_which_float32_products_go_to_the_tensor_cores():
     assert not ops.f32_supported(x, w)                               # (not on a CUDA device)
 
 
+def test_every_float32_model_loads_the_products_kernel_at_its_start():
+    """Whatever its parts are: the first large prompt would build or load it in the middle of a step otherwise."""
+    from lite_lang_b200.config import config_from_dict
+    from lite_lang_b200.engine.model import CausalLM
+    from nevurax_cases import CASES
+    for case in CASES.values():
+        model = CausalLM(config_from_dict(case["config"]).model_spec())
+        model.dtype = torch.float32
+        assert "gemm_f32" in model.kernel_libraries()
+        model.dtype = torch.bfloat16
+        assert "gemm_f32" not in model.kernel_libraries()
+
+
 @gpu
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("nh,nkv,page,window", [(4, 2, 16, None), (6, 1, 5, None), (3, 3, 16, 40), (14, 2, 64, 7)])
