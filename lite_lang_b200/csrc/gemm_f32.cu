@@ -9,8 +9,12 @@
 // the terms' last bits.  So a chain is 64 numbers of k long: the five small products first, while the sum is small, then
 // the leading product's four steps; then the eight epilogue warps of each CTA take the sum out of tensor memory and add it to
 // their registers with rounded additions (128 a thread), while the next chain runs in the other half of tensor memory.
-// Measured against float64 the result is nearer than the library's (see the tests).  Numbers above 3.38e38 and
-// infinities give NaN.
+// Measured against float64 the result is nearer than the library's (see the tests).
+//
+// Infinities and numbers above 3.39e38 have no such terms (the first one rounds to infinity, the second is NaN), so every
+// sum that one of them is in comes out as NaN.  A thread that finds NaN among its sums makes the outputs again by
+// multiply-adds of the numbers as stored (`gf_plain`): an infinity stays one, as in a float32 product.  (Numbers below
+// 2^-109 lose their last bits: a bfloat16 number ends at 2^-133.)
 //
 // x comes as its three terms (`f32_terms_kernel`, [3][M][K]: x is small and read by every column tile).  W stays float32 in
 // memory: its rows come by TMA into two buffers of 128 x 32, and their terms are written into the stage in the layout that
@@ -174,6 +178,9 @@ f32_join_kernel(float* __restrict__ out, long out_stride, const float* __restric
 }
 
 struct GfParams {
+  const float* x;                    // the operands as stored (and their row strides), for sums that are NaN
+  const float* w;
+  long x_stride, w_stride;
   float* out;
   long out_stride, part_stride;      // numbers from a row, and from a part, to the next
   int M, N, K;                       // rows, output features (gated: W has 2 N rows), inner size
@@ -213,6 +220,19 @@ __device__ __forceinline__ void gf_terms(unsigned char* smem, const unsigned cha
     gf_mbar_arrive(raw_empty0 + 8 * q);
     gf_mbar_arrive_cluster(b_full_lead + 8 * s);
   }
+}
+
+// a sum over numbers k0 .. k1 - 1 of k in float32
+__device__ __noinline__ float gf_plain(const float* x, const float* w, int k0, int k1) {
+  float s = 0.f;
+  for (int k = k0; k < k1 && s == s; k += 4) {       // (K is a multiple of 8; NaN stays NaN)
+    const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+    s = fmaf(a.x, b.x, s);
+    s = fmaf(a.y, b.y, s);
+    s = fmaf(a.z, b.z, s);
+    s = fmaf(a.w, b.w, s);
+  }
+  return s;
 }
 
 template <bool GATED>
@@ -379,6 +399,9 @@ gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, cons
         const int row = mt * 256 + (int)rank * 128 + 32 * ew + lane;
         if (row < p.M) {
           float* dst = p.out + part * p.part_stride + (size_t)row * p.out_stride;
+          bool nan = false;
+#pragma unroll
+          for (int i = 0; i < 128; ++i) nan |= sum[i] != sum[i];
           if (GATED) {
             const int f0 = nt * 128 + 64 * eh;
 #pragma unroll
@@ -397,7 +420,23 @@ gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, cons
               if (f < p.N) *reinterpret_cast<float4*>(dst + f) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
             }
           }
+          if (nan) {
+            const float* xr = p.x + (size_t)row * p.x_stride;
+            const int last = min(p.K, k1 * 64);
+#pragma unroll 1
+            for (int i = 0; i < (GATED ? 64 : 128); ++i) {
+              const int f = nt * COLS + 64 * eh + (GATED ? i : (i >> 6) * 128 + (i & 63));
+              if (f >= p.N) continue;
+              if (GATED) {      // (an activation may have made a number of NaN)
+                const float g = gf_plain(xr, p.w + (size_t)f * p.w_stride, k0 * 64, last);
+                dst[f] = ll_gated(g, gf_plain(xr, p.w + (size_t)(p.N + f) * p.w_stride, k0 * 64, last), p.gate);
+              } else if (dst[f] != dst[f]) {
+                dst[f] = gf_plain(xr, p.w + (size_t)f * p.w_stride, k0 * 64, last);
+              }
+            }
+          }
         }
+        __syncwarp();
       }
     }
   }
@@ -487,6 +526,10 @@ extern "C" int ll_gemm_f32(float* out, long out_stride, const float* x, long x_s
   ll_launch(f32_terms_kernel, dim3((unsigned)((pieces + 255) / 256 < most ? (pieces + 255) / 256 : most)), dim3(256), 0, stream,
             (bf16*)terms, x, x_stride, (long)M, K);
   GfParams p;
+  p.x = x;
+  p.w = w;
+  p.x_stride = x_stride;
+  p.w_stride = w_stride;
   p.out = join ? parts : out;
   p.out_stride = join ? N : out_stride;
   p.part_stride = (long)M * N;

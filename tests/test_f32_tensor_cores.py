@@ -180,3 +180,49 @@ def test_products_report_to_the_steps_status_word(monkeypatch):
     with pytest.raises(RuntimeError), ops.reporting_to(word):
         raise RuntimeError
     assert products() == [None] * 3
+
+
+def _same_kind(got, want):
+    """Finite numbers, NaN and infinities (with their sign) in the same places."""
+    return (torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want))
+            and torch.equal(torch.isneginf(got), torch.isneginf(want)))
+
+
+@gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_product_of_numbers_without_bfloat16_terms(gated, splits):
+    """Infinities and numbers above bfloat16's largest: a float32 product keeps them, and every other number stays what it is."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    M, N, K, inf = 300, 264, 520, float("inf")
+    x, w = torch.rand(M, K, generator=g, device="cuda") - 0.5, torch.rand(N, K, generator=g, device="cuda") - 0.5
+    plain = x.double() @ w.double().t()
+    x[3, 500], x[70, 9], x[70, 400], x[290, 1], x[128, 77] = inf, -inf, -inf, 3.4e38, float("nan")
+    w[5, 3], w[255, 519], w[130, 64] = -inf, 3.4e38, float("nan")
+    w[255] *= 1e-3                                                  # (3.4e35: its sums stay in range, and one term is 3.4e38 x 0)
+    x[:, 519], w[255, 519] = x[:, 519] * 1e-3, 3.4e38
+    x[290], w[:, 1] = x[290] * 1e-3, w[:, 1] * 1e-3
+    x[290, 1] = 3.4e38
+    want = (x.double() @ w.double().t()).float()
+    bad = torch.zeros(M, N, dtype=torch.bool, device="cuda")
+    bad[[3, 70, 290, 128]] = True
+    bad[:, [5, 255, 130]] = True
+    assert bool(torch.isfinite(want[290]).any()) and bool(torch.isinf(want[3]).any()) and bool(torch.isfinite(want[:, 255]).any())
+    if not gated:
+        got = ops.gemm_f32(x, w, splits=splits)
+        assert _same_kind(got, want)
+        fin = torch.isfinite(want)
+        scale = x.double().abs() @ w.double().abs().t()
+        assert float(((got.double() - want.double()).abs() / scale)[fin].max()) <= (8 + K) * 2.0 ** -24
+        return
+    if splits != 1:
+        return
+    for act in ("silu", "relu"):
+        got = ops.gemm_f32(x, w, torch.empty(M, N // 2, device="cuda"), gated=ops.GateAct(act))
+        ref = torch.empty(M, N // 2, device="cuda")
+        ops.act_mul(ref, want.contiguous(), ops.GateAct(act))
+        assert _same_kind(got, ref)
+        fin = torch.isfinite(ref) & ~bad[:, :N // 2] & ~bad[:, N // 2:]
+        assert float((got - ref)[fin].abs().max()) <= 4e-6 * float(ref[fin].abs().max())
