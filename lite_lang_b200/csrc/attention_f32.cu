@@ -2,8 +2,8 @@
 // tokens.
 //
 // The float32 path's general kernel (attention_generic.cu) gives a block a (token, kv head) pair and reads the keys once for
-// its group of heads only: 337 us for two prompts of 262 and 439 tokens with 12 heads of 128 on 2 kv heads (71 us here), and
-// 704 us for 64 single tokens at contexts of 500 to 1,000, whose blocks walk their keys alone.  Here a CTA takes 64 rows
+// its group of heads only: 337 us for two prompts of 262 and 439 tokens with 12 heads of 128 on 2 kv heads (50 us here), and
+// 704 us for 64 single tokens at contexts of 500 to 1,000 (106 here), whose blocks walk their keys alone.  Here a CTA takes 64 rows
 // (a row = a (token, query head of the kv head's group) pair, token-major), so the keys are read once for 64 rows, and both
 // products run on mma.sync with every float32 operand as three bfloat16 terms that hold its 24 bits (mma_split.cuh):
 //   S [64 x 32]  = Q K^T     a warp 16 rows, 6 products a step of 16 channels
@@ -78,6 +78,7 @@ attn_f32_kernel(const AttnF32Params p) {
   const int hi = ctx + rl / p.group, lo = p.window > 0 ? max(0, ctx + r0 / p.group - p.window + 1) : 0;
   const int tile0 = lo / AF_TK, tiles = hi / AF_TK - tile0 + 1;
   const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+  const int own = half ^ (tile0 & 1);                          // this group's first tile: the even or the odd ones of the context
 
   // lane l: where the row of key l of a tile starts in the planes (-1: not seen by any row of the CTA)
   auto place = [&](int tile) -> long {
@@ -121,8 +122,8 @@ attn_f32_kernel(const AttnF32Params p) {
     }
   };
   long next = -1;
-  if (half < tiles) ask(place(half));
-  if (half + 2 < tiles) next = place(half + 2);
+  if (own < tiles) ask(place(own));
+  if (own + 2 < tiles) next = place(own + 2);
   for (int i = tid; i < AF_ROWS * (HD / 4); i += AF_THREADS) {
     const int rr = i / (HD / 4), c = (i % (HD / 4)) * 4, r = r0 + rr;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -139,7 +140,7 @@ attn_f32_kernel(const AttnF32Params p) {
   float o[NO][4], m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 #pragma unroll
   for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  for (int tile = half; tile < tiles; tile += 2) {
+  for (int tile = own; tile < tiles; tile += 2) {
     ms_wait<0>();
     asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");      // the rows are here, the tile before has been read
     put(ks, raw);

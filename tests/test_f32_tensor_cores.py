@@ -226,3 +226,26 @@ def test_product_of_numbers_without_bfloat16_terms(gated, splits):
         assert _same_kind(got, ref)
         fin = torch.isfinite(ref) & ~bad[:, :N // 2] & ~bad[:, N // 2:]
         assert float((got - ref)[fin].abs().max()) <= 4e-6 * float(ref[fin].abs().max())
+
+
+@gpu
+@pytest.mark.parametrize("window", [None, 40])
+def test_attention_is_the_same_bits_however_a_prompt_is_cut(window):
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    nh, nkv, page, n, hd = 6, 2, 16, 200, 64
+    pages = (n + page - 1) // page
+    k, v = (torch.randn(pages, nkv, page, hd, generator=g, device="cuda") for _ in range(2))
+    q = torch.randn(n, nh * hd, generator=g, device="cuda")
+    ints = dict(dtype=torch.int32, device="cuda")
+    table, slot, status = torch.arange(pages, **ints)[None], torch.zeros(1, **ints), torch.zeros(1, **ints)
+    outs = []
+    for cuts in ([0, 200], [0, 33, 70, 71, 137, 200]):
+        out = torch.empty_like(q)
+        for a, b in zip(cuts, cuts[1:]):
+            ops.attn_f32(out[a:b], q[a:b], k, v, table, torch.tensor([0, b - a], **ints), torch.tensor([a], **ints), slot, [b - a], nh,
+                         nkv, hd, page, window, hd ** -0.5, status)
+        outs.append(out)
+    assert int(status.item()) == 0
+    assert torch.equal(*outs)
