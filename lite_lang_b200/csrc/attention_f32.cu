@@ -13,9 +13,13 @@
 // come by cp.async as stored, a tile ahead of the group's use of them (the pages' numbers a tile ahead of that), and become
 // terms in shared memory when their turn comes: asked for where they were needed, the trips to memory were 40 % of the time.
 //
-// Scores, softmax (expf) and sums are float32.  Keys that a row may not see get probability 0 by selection and their rows
-// of V are zeros, whatever the page holds.  The order of a row's sums depends on the tiles (which start at multiples of 32
-// positions) and, through the two groups, on the first tile that its row block sees.
+// Scores, softmax (expf) and sums are float32.  Keys that a row may not see get probability 0 by selection; the V of keys that
+// no row of the CTA sees are zeros, whatever the page holds.  Tiles start at multiples of 32 positions and a group takes every
+// other one of the context's, so the order of a row's sums depends on its position only.
+//
+// Infinities and numbers above 3.39e38 have no bfloat16 terms, and a probability of 0 makes NaN of an infinity in V that other
+// rows of the CTA see: a row that comes out with NaN is made again by a warp in multiply-adds (`af_plain_row`), as
+// attention_generic.cu would.
 #include "mma_split.cuh"
 
 #define AF_THREADS 256
@@ -38,6 +42,32 @@ struct AttnF32Params {
   float scale;
   int* status;
 };
+
+// one row by one warp: keys lo .. pos of the table `bt`, HD / 32 channels a lane
+template <int HD>
+__device__ __forceinline__ void af_plain_row(const AttnF32Params& p, const int* bt, int kvh, int lo, int pos, const float* q, float* out) {
+  constexpr int N = HD / 32;
+  const int lane = threadIdx.x & 31;
+  float x[N], o[N] = {}, m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = q[lane + 32 * i];
+  for (int j = lo; j <= pos && l == l; ++j) {        // (a sum that is NaN stays NaN)
+    const int lp = j / p.page_size, page = lp < p.bt_stride ? bt[lp] : -1;
+    if (page < 0 || page >= p.num_pages) continue;   // (has been reported)
+    const size_t at = (((size_t)page * p.nkv + kvh) * p.page_size + j % p.page_size) * HD;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) s = fmaf(x[i], p.k_cache[at + lane + 32 * i], s);
+    s = warp_sum(s) * p.scale;
+    const float n = fmaxf(m, s), u = n == -INFINITY ? 0.f : n, f = expf(m - u), w = expf(s - u);
+    m = n;
+    l = fmaf(l, f, w);
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = fmaf(o[i], f, w * p.v_cache[at + lane + 32 * i]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) out[lane + 32 * i] = l != l ? l : l > 0.f ? o[i] / l : 0.f;
+}
 
 template <int HD>
 __global__ void __launch_bounds__(AF_THREADS, 1)
@@ -246,12 +276,14 @@ attn_f32_kernel(const AttnF32Params p) {
     if (c == 0) {
       d0[HD] = m0; d0[HD + 1] = l0;
       d1[HD] = m1; d1[HD + 1] = l1;
+      d0[HD + 2] = d1[HD + 2] = 0.f;      // not zero: the row has NaN
     }
   }
   __syncthreads();
   if (half == 0) {
-    const float* s0 = meet + (row + g) * P;
-    const float* s1 = s0 + 8 * P;
+    float* s0 = meet + (row + g) * P;
+    float* s1 = s0 + 8 * P;
+    bool nan0 = false, nan1 = false;
     auto weights = [](float m, float l, float mq, float lq, float& w, float& wq) {
       const float top = fmaxf(m, mq), u = top == -INFINITY ? 0.f : top;
       w = expf(m - u);
@@ -268,10 +300,23 @@ attn_f32_kernel(const AttnF32Params p) {
 #pragma unroll
     for (int i = 0; i < NO; ++i) {
       const float2 x = *reinterpret_cast<const float2*>(s0 + i * 8 + 2 * c), y = *reinterpret_cast<const float2*>(s1 + i * 8 + 2 * c);
-      if (ra <= rl) *reinterpret_cast<float2*>(oa + i * 8) = make_float2(o[i][0] * w0 + x.x * q0, o[i][1] * w0 + x.y * q0);
-      if (rb8 <= rl) *reinterpret_cast<float2*>(ob + i * 8) = make_float2(o[i][2] * w1 + y.x * q1, o[i][3] * w1 + y.y * q1);
+      const float2 a = make_float2(o[i][0] * w0 + x.x * q0, o[i][1] * w0 + x.y * q0);
+      const float2 b = make_float2(o[i][2] * w1 + y.x * q1, o[i][3] * w1 + y.y * q1);
+      nan0 |= a.x != a.x || a.y != a.y;
+      nan1 |= b.x != b.x || b.y != b.y;
+      if (ra <= rl) *reinterpret_cast<float2*>(oa + i * 8) = a;
+      if (rb8 <= rl) *reinterpret_cast<float2*>(ob + i * 8) = b;
     }
+    if (nan0) s0[HD + 2] = 1.f;
+    if (nan1) s1[HD + 2] = 1.f;
   }
+  __syncthreads();
+  for (int rr = warp; rr <= rl - r0; rr += AF_THREADS / 32)
+    if (meet[rr * P + HD + 2] != 0.f) {
+      const int r = r0 + rr, pos = ctx + r / p.group;
+      const size_t t = tok0 + r / p.group, h = (size_t)(head0 + r % p.group) * HD;
+      af_plain_row<HD>(p, bt, kvh, p.window > 0 ? max(0, pos - p.window + 1) : 0, pos, p.q + t * p.q_stride + h, p.out + t * p.out_stride + h);
+    }
 }
 
 // q: float32, head h of token t at q + t * q_stride + h * hd; out float32 [tokens, nh * hd].  cu_q, ctx_len, req_slot: the

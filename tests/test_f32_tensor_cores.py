@@ -229,6 +229,44 @@ def test_product_of_numbers_without_bfloat16_terms(gated, splits):
 
 
 @gpu
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_of_numbers_without_bfloat16_terms(hd):
+    """A key or value that is not finite shows in the rows that see it, as on the general kernel, and in no other."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(hd)
+    nh, nkv, page, n, inf = 6, 2, 16, 150, float("inf")
+    pages = (n + page - 1) // page
+    k, v = (torch.randn(pages, nkv, page, hd, generator=g, device="cuda") for _ in range(2))
+    q = torch.randn(n, nh * hd, generator=g, device="cuda")
+    ints = dict(dtype=torch.int32, device="cuda")
+    table, cu = torch.arange(pages, **ints)[None], torch.tensor([0, n], **ints)
+    ctx, slot, status = torch.zeros(1, **ints), torch.zeros(1, **ints), torch.zeros(1, **ints)
+
+    def put(plane, pos, head, channel, value):
+        plane[pos // page, head, pos % page, channel] = value
+
+    put(v, 50, 0, 3, inf)
+    put(v, 90, 0, 4, 3.4e38)
+    put(v, 120, 0, 5, float("nan"))
+    put(k, 100, 1, 7, inf)
+    put(k, 140, 1, 9, float("nan"))
+    q[30, 2] = inf
+    for window in (None, 33):
+        out, general = torch.empty_like(q), torch.empty_like(q)
+        ops.attn_f32(out, q, k, v, table, cu, ctx, slot, [n], nh, nkv, hd, page, window, hd ** -0.5, status)
+        ops.paged_attention_generic(general, q, nh * hd, k, v, table, torch.zeros(n, **ints), slot, torch.arange(n, **ints), n, nh,
+                                    nkv, hd, page, window, hd ** -0.5, status)
+        assert int(status.item()) == 0
+        assert _same_kind(out, general)
+        assert not bool(torch.isnan(out[:30]).any()) and bool(torch.isinf(out[50]).any())
+        fin = torch.isfinite(general) & (general.abs() < 1e30)
+        assert float((out - general)[fin].abs().max()) <= 1e-5
+        big = torch.isfinite(general) & ~fin
+        assert float(((out - general)[big] / general[big]).abs().max()) <= 1e-5
+
+
+@gpu
 @pytest.mark.parametrize("window", [None, 40])
 def test_attention_is_the_same_bits_however_a_prompt_is_cut(window):
     from lite_lang_b200 import ops
