@@ -20,8 +20,10 @@
 // Everything is float32 as in the walk by tokens: decays are running products (a decay that underflows to 0 stays 0,
 // nothing is divided), products of float32 numbers are made of bfloat16 terms that hold all 24 bits (mma_split.cuh), and
 // operands that are stored as bfloat16 are taken as they are.  A chunk starts where the step's portion does, so the order
-// of the sums depends on how a prompt was cut into portions, within rounding.  A value that is not finite makes
-// NaN of its whole chunk (its own request's) instead of the tokens from it on.
+// of the sums depends on how a prompt was cut into portions, within rounding.  Infinities have no bfloat16 terms and a
+// product with 0 makes NaN of them, so a number that is not finite would show in the chunk's tokens before it, too: a thread
+// that finds a state or a read-out not finite makes that number again token by token (`cs_again`), as the walk does.  (The
+// delta rule's walk over chunks has NaN in a state where the walk by tokens may still have an infinity.)
 //
 // Taken for longer portions, key heads of 64 or 128 channels and value heads of a multiple of 64 (delta rule: 64 or 128,
 // one decay a head): see `ops.chunked_scan`.
@@ -185,6 +187,62 @@ template <> __device__ __forceinline__ float4 cs_load4<bf16>(const bf16* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// One number of the state behind token `last` of a chunk: S <- a S + k (w v) over the tokens 0 .. last, from S (`from` null: 0,
+// without the first decay).  k and v point at the number's channel and column in the chunk's first row.
+template <typename T, typename A, typename W>
+__device__ __forceinline__ float cs_again(const float* from, const T* k, long k_stride, const T* v, long v_stride, int last, A decay,
+                                          W scale) {
+  float s = 0.f;
+  for (int t = 0; t <= last && s == s; ++t) {
+    const float x = to_f32<T>(k[(size_t)t * k_stride]) * (to_f32<T>(v[(size_t)t * v_stride]) * scale(t));
+    s = t > 0 ? fmaf(decay(t), s, x) : from != nullptr ? fmaf(decay(0), *from, x) : x;
+  }
+  return s;
+}
+
+// The numbers of a thread's that are not finite, again.  (Where operands are float32 as calls of their own: inlined, they took
+// the registers of chunk_read from 176 to 255 and 3 us of a delta rule's 277; bfloat16 operands: called, 6 of 125 us.)
+// chunk_write: the thread's part of the states, from channel `ch0` and value column `v0` (of all heads') on.
+template <typename T, int DK>
+__device__ __forceinline__ void cs_write_again(const CsRows<T>& in, float* dst, int base, int n, int h, int H, int ch0, size_t v0) {
+  const T* row = in.proj + (size_t)base * in.stride;
+  auto decay = [&](int t) { return in.tok_decay ? in.tok_decay[(size_t)(base + t) * H + h] : in.decay[h]; };
+  auto scale = [&](int t) { return in.tok_scale ? in.tok_scale[(size_t)(base + t) * H + h] : 1.f; };
+#pragma unroll 1
+  for (int i = 0; i < DK / 4; ++i) {
+    const int col = 8 * ((i >> 1) & 1), ch = (i >> 2) * 8 + (i & 1);
+    float* d = dst + col * DK + ch;
+    if (!(fabsf(*d) < INFINITY))
+      *d = cs_again<T>(nullptr, row + in.k_off + (h / in.hpg) * DK + ch0 + ch, in.stride, row + in.v_off + v0 + col, in.stride, n - 1,
+                       decay, scale);
+  }
+}
+// chunk_read: rows t0 and t0 + 8, 16 of every 64 columns
+template <typename T, int DK>
+__device__ __forceinline__ void cs_read_again(float* out, long out_stride, const T* q, const T* k, long stride, const T* v, long v_stride,
+                                           const float* state, const float* av, const float* sc, bool skipped, float skip, int n,
+                                           int dv, int t0, int col0) {
+  auto decay = [&](int t) { return av[t]; };
+  auto scale = [&](int t) { return sc[t]; };
+#pragma unroll 1
+  for (int i = 0; i < dv / 4; ++i) {
+    const int t = t0 + 8 * ((i >> 3) & 1), col = (i >> 4) * 64 + col0 + ((i >> 1) & 3) * 8 + (i & 1);
+    if (t >= n) continue;
+    float* d = out + (size_t)t * out_stride + col;
+    if (fabsf(*d) < INFINITY) continue;
+    float a = 0.f;
+    for (int ch = 0; ch < DK && a == a; ++ch)
+      a = fmaf(cs_again<T>(state + (size_t)col * DK + ch, k + ch, stride, v + col, v_stride, t, decay, scale),
+               to_f32<T>(q[(size_t)t * stride + ch]), a);
+    *d = skipped ? fmaf(skip, to_f32<T>(v[(size_t)t * v_stride + col]), a) : a;
+  }
+}
+
+template <int DK, typename... A>
+__device__ __noinline__ void cs_write_again_f32(A... a) { cs_write_again<float, DK>(a...); }
+template <int DK, typename... A>
+__device__ __noinline__ void cs_read_again_f32(A... a) { cs_read_again<float, DK>(a...); }
+
 // ---------------------------------------------------------------------------------------------------------------
 // ds[item][h][dv][dk] = sum over the chunk's tokens of (G(C, s) scale_s v_s) k_s^T; gam[item][h] = G(C, -).
 // Value columns are the M side (16 of the CTA's 64 a warp, half of the key channels each), tokens the inner dimension.
@@ -275,10 +333,21 @@ chunk_write_kernel(CsRows<T> in, const int* __restrict__ cu_q, const int* __rest
   }
   const int g = lane >> 2, c = lane & 3;
   float* dst = ds + (((size_t)item * H + h) * dv + c0 + rt + g) * DK + kc + 2 * c;
+  bool odd = false;
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
-    *reinterpret_cast<float2*>(dst + nt * 8) = make_float2(acc[nt][0] + low[nt][0], acc[nt][1] + low[nt][1]);
-    *reinterpret_cast<float2*>(dst + 8 * DK + nt * 8) = make_float2(acc[nt][2] + low[nt][2], acc[nt][3] + low[nt][3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[nt][j] += low[nt][j];
+      odd |= !(fabsf(acc[nt][j]) < INFINITY);
+    }
+    *reinterpret_cast<float2*>(dst + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
+    *reinterpret_cast<float2*>(dst + 8 * DK + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
+  }
+  if (odd) {
+    const size_t v0 = (size_t)h * dv + c0 + rt + g;
+    if constexpr (sizeof(T) == 4) cs_write_again_f32<DK>(in, dst, base, n, h, H, kc + 2 * c, v0);
+    else cs_write_again<T, DK>(in, dst, base, n, h, H, kc + 2 * c, v0);
   }
 }
 
@@ -436,6 +505,7 @@ chunk_read_kernel(CsRows<T> in, const int* __restrict__ cu_q, const int* __restr
   }
   const float f0 = pre[row + g], f1 = pre[row + g + 8];
   const float skip = in.skip ? in.skip[h] : 0.f;
+  bool odd = false;
   for (int c0 = 0; c0 < dv; c0 += 64) {
     const bool more = c0 + 64 < dv;
     __syncthreads();                                    // the scores, this pass's state and values are there
@@ -491,6 +561,7 @@ chunk_read_kernel(CsRows<T> in, const int* __restrict__ cu_q, const int* __restr
           w = fmaf(skip, to_f32<T>(vrow[(size_t)t * vstride + col + i * 8 + 1]), w);
         }
         *reinterpret_cast<float2*>(orow + (size_t)t * H * dv + col + i * 8) = make_float2(u, w);
+        odd |= !(fabsf(u) < INFINITY && fabsf(w) < INFINITY);
       }
     }
     if (more) {
@@ -498,6 +569,16 @@ chunk_read_kernel(CsRows<T> in, const int* __restrict__ cu_q, const int* __restr
       st.put(ss);
       vt.put(vs);
     }
+  }
+  if (odd) {
+    const T *qh = prow + in.q_off + (h / in.hpg) * DK, *kh = krow + (h / in.hpg) * DK;
+    const float *a = av, *w = sc;
+    if constexpr (sizeof(T) == 4)
+      cs_read_again_f32<DK>(orow, (long)H * dv, qh, kh, in.stride, vrow, vstride, srow, a, w, in.skip != nullptr, skip, n, dv, row + g,
+                            half * 32 + 2 * c);
+    else
+      cs_read_again<T, DK>(orow, (long)H * dv, qh, kh, in.stride, vrow, vstride, srow, a, w, in.skip != nullptr, skip, n, dv, row + g,
+                           half * 32 + 2 * c);
   }
 }
 

@@ -134,3 +134,63 @@ def test_delta_rule_by_chunks(lens, single, H, Hk, dk, dv, monkeypatch):
             assert bool((o == 0).all()) and torch.equal(st, state0)
     if err:
         assert err["chunks"][0] <= max(2 * err["walk"][0], 3e-7) and err["chunks"][1] <= max(2 * err["walk"][1], 3e-7), err
+
+
+def _same_kind(got, want):
+    return (torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want))
+            and torch.equal(torch.isneginf(got), torch.isneginf(want)))
+
+
+@gpu
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.bfloat16, 128, 128), (torch.float32, 128, 64), (torch.float32, 64, 192)])
+def test_decay_scan_of_numbers_that_are_not_finite(dtype, dk, dv, monkeypatch):
+    """They show from their own token on, in the numbers that the walk by tokens shows them in."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk + dv)
+    H, lens, rnd, inf = 3, [200, 70], dict(generator=g, device="cuda"), float("inf")
+    n = sum(lens)
+    proj = torch.randn(n, H * (2 * dk + dv), **rnd).to(dtype)
+    q, k, v = (proj[:, a:b].view(n, H, -1) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, H * (2 * dk + dv))))
+    k[100, 0, 5] = inf                      # one channel of a key: every column's read-out
+    v[130, 1, 7], v[20, 1, 60] = -inf, float("nan")
+    q[40, 2, 3] = inf
+    v[235, 2, 1] = 3.4e38 if dtype == torch.float32 else inf
+    if dtype == torch.float32:
+        k[235, 2] *= 1e-3
+    decay, skip = torch.tensor([0.9, 0.99, 1.0], device="cuda"), torch.randn(H, **rnd)
+    state0, step, res = torch.randn(2, H * dk * dv, **rnd), _step(lens, [1, 0]), {}
+    for way, least in (("walk", 1 << 30), ("chunks", 1)):
+        monkeypatch.setattr(ops, "DECAY_CHUNKED_MIN", least)
+        st, o = state0.clone(), torch.empty(n, H * dv, device="cuda")
+        ops.decay_scan(proj, 0, H * dk, 2 * H * dk, decay, st, step, o, H, dk, dv, True, 1, None, None, skip)
+        res[way] = (o, st)
+    for got, want in zip(res["chunks"], res["walk"]):
+        assert bool(torch.isinf(want).any()) and _same_kind(got, want)
+        fin = torch.isfinite(want) & (want.abs() < 1e30)
+        assert float((got - want)[fin].norm()) <= 1e-5 * float(want[fin].norm())
+    assert int(step.status.item()) == 0
+
+
+@gpu
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64)])
+def test_delta_rule_of_numbers_that_are_not_finite(dk, dv, monkeypatch):
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk + dv)
+    H, lens, rnd = 3, [200, 70], dict(generator=g, device="cuda")
+    n = sum(lens)
+    qn, kn = (torch.nn.functional.normalize(torch.randn(n, H, dk, **rnd), dim=-1) for _ in range(2))
+    vc, beta = torch.randn(n, H, dv, **rnd), torch.rand(n, H, **rnd)
+    decay = torch.exp(-torch.rand(n, H, **rnd))
+    vc[100, 0, 5], kn[150, 1, 3], vc[30, 2, 40], vc[69 + 200, 2, 0] = float("inf"), float("nan"), float("nan"), -float("inf")
+    state0, step, res = torch.randn(2, H * dk * dv, **rnd), _step(lens, [1, 0]), {}
+    for way, least in (("walk", 1 << 30), ("chunks", 1)):
+        monkeypatch.setattr(ops, "DELTA_CHUNKED_MIN", least)
+        st, o = state0.clone(), torch.empty(n, H * dv, device="cuda")
+        ops.delta_recurrence(qn.view(n, -1), kn.view(n, -1), vc.view(n, -1), beta, decay, st, step, o, H, H, dk, dv, False)
+        res[way] = (o, st)
+    for got, want in zip(res["chunks"], res["walk"]):
+        assert bool(torch.isnan(want).any()) and torch.equal(torch.isfinite(got), torch.isfinite(want))
+        fin = torch.isfinite(want)
+        assert float((got - want)[fin].norm()) <= 1e-5 * float(want[fin].norm())
