@@ -30,6 +30,7 @@ Further parameters, for designs that differ:
 
 from __future__ import annotations
 
+import itertools
 from typing import Dict
 
 import torch
@@ -161,38 +162,67 @@ class LatentAttention(Mixer):
     PRODUCT_MIN_TOKENS = 32
     QUERY_BLOCK = 256
     # Portions of at least this many tokens are served with expanded keys and values, as long as the rows to expand are at
-    # most so many times the step's tokens in them (a row costs (kv_rank + rot_dim) * 2 vdim multiply-adds a head to expand
+    # most so many times the tokens in them (a row costs (kv_rank + rot_dim) * 2 vdim multiply-adds a head to expand
     # and saves kv_rank * 2 a head and query; below the line the step's time is its launches, which are fewer this way).
-    # Measured on a B200, 12 heads of 128, a latent of 512: 2,048 tokens in three requests with a window of 512, 237 us of
-    # kernels in 41 launches by the products over the latents, 76 us in 6 launches this way (690 and 131 us with the host).
-    EXPAND_MIN_TOKENS = 16
+    # Measured on a B200, heads of 128, a latent of 512 (in the latent space / this way; us of kernels, us with the host):
+    # 12 heads, 2,048 tokens in three requests with a window of 512 237 / 76, 690 / 131; 28 heads, four times 256 behind
+    # 2,000 with the window 217 / 85, 361 / 140; one portion of 12 heads: 32 behind 480 33 / 36, 192 / 161, 128 behind 1,920
+    # 51 / 54, 187 / 143; 28 heads: 32 behind 480 36 / 42, 186 / 149, 32 behind 1,280 (40 rows a token) 42 / 55, 189 / 152;
+    # 2 heads: 128 behind 1,920 35 / 42, 184 / 148.  Where the kernels take a little longer this way, the host decides.
+    # Shorter ones stay with the kernel over the latents, which carries the softmax weights in sixteen bits (two terms): the
+    # tcgen05 attention has one term of eight, as the products over the latents have.
+    EXPAND_MIN_TOKENS = PRODUCT_MIN_TOKENS
     EXPAND_MAX_ROWS = 16
 
-    def _expanded(self, step, qrows):
-        """(cached, new) tokens of the step's portions if they are to be served with expanded keys and values, else None."""
+    def _runs(self, step, qrows):
+        """How the step's entries are served: (tokens that meet the latents themselves, as runs [(first, behind the last)];
+        groups of entries with expanded keys and values [(first entry, their (cached, new) tokens, plan)]).  Layers alike
+        share it."""
+        key = ("latent_runs", self.H, self.dv, self.R + self.r, self.window)
+        if self.w_kv is None or not ops.TC_ENABLED or qrows.stride(0) % 8:
+            return [(0, qrows.shape[0])], ()
+        got = step.scratch.get(key)
+        if got is None:
+            got = step.scratch[key] = self._plan_runs(step, qrows)
+        return got
+
+    def _plan_runs(self, step, qrows):
         entries = None if getattr(step, "captured", False) else getattr(step, "entries", None)
         ctxs = getattr(step, "entry_ctx", None)
-        if self.w_kv is None or not ops.TC_ENABLED or entries is None or ctxs is None or qrows.stride(0) % 8:
-            return None
-        single = step.num_single
-        spans = [(c, len(e.tokens)) for e, c in zip(entries[single:], ctxs[single:])]
-        if not spans or min(q for _, q in spans) < self.EXPAND_MIN_TOKENS:
-            return None
-        rows = sum(q + (min(c, self.window - 1) if self.window else c) for c, q in spans)
-        return spans if rows <= self.EXPAND_MAX_ROWS * sum(q for _, q in spans) else None
+        whole = [(0, qrows.shape[0])], ()
+        if entries is None or ctxs is None:
+            return whole
+        spans = [(c, len(e.tokens)) for c, e in zip(ctxs, entries)]
+        long = [(self._seen(c), q) for c, q in spans if q >= self.EXPAND_MIN_TOKENS]
+        if not long or sum(c + q for c, q in long) > self.EXPAND_MAX_ROWS * sum(q for _, q in long):
+            return whole
+        latent, groups, at, e0 = [], [], 0, 0
+        for expanded, run in itertools.groupby(spans, lambda span: span[1] >= self.EXPAND_MIN_TOKENS):
+            run = list(run)
+            if expanded:
+                for a, b in self._groups(run):
+                    groups.append((e0 + a, run[a:b], ops.attn_prefill_tc_plan(
+                        [(self._seen(c), q) for c, q in run[a:b]], 1, self.window, self.H, 2 * ops.sm_count(qrows.device))))
+            else:
+                latent.append((at, at + sum(q for _, q in run)))
+            at += sum(q for _, q in run)
+            e0 += len(run)
+        return latent, groups
 
-    def _attend_expanded(self, heads, qrows, step, cache, spans) -> None:
-        """The portions behind the step's single tokens: ``heads`` rows = attention over expanded keys and values."""
-        n1, H, hd = step.num_single, self.H, self.dv
-        rows, table, rel, own = ops.latent_unpage(cache.k, cache.block_table, step.cu_q[n1:], step.ctx_len[n1:],
-                                                  step.req_slot[n1:], spans, self.window, step.status)
+    def _seen(self, ctx: int) -> int:
+        """Cached tokens that a portion behind ``ctx`` of them may see."""
+        return min(ctx, self.window - 1) if self.window else ctx
+
+    def _groups(self, spans):
+        yield 0, len(spans)
+
+    def _attend_expanded(self, heads, qrows, step, cache, e0, spans, plan) -> None:
+        """Entries ``e0`` ... of the step: their ``heads`` rows = attention over expanded keys and values."""
+        width, cu_q = self.H * self.dv, step.cu_q[e0:]
+        rows, table, rel, own = ops.latent_unpage(cache.k, cache.block_table, cu_q, step.ctx_len[e0:], step.req_slot[e0:], spans,
+                                                  self.window, step.status)
         kv = ops.linear(rows, self.w_kv)
-        key = ("latent_expanded", H, self.window)
-        plan = step.scratch.get(key)
-        if plan is None:
-            seen = [(min(c, self.window - 1) if self.window else c, q) for c, q in spans]
-            plan = step.scratch[key] = ops.attn_prefill_tc_plan(seen, 1, self.window, H, 2 * ops.sm_count(heads.device))
-        ops.attn_prefill_tc_rows(heads, qrows, kv[:, :H * hd], kv[:, H * hd:], table, step.cu_q[n1:], rel, own, plan, H, hd,
+        ops.attn_prefill_tc_rows(heads, qrows, kv[:, :width], kv[:, width:], table, cu_q, rel, own, plan, self.H, self.dv,
                                  self.window, self.scale, self.sink_w, step.status)
 
     def forward(self, x, step, cache):
@@ -203,22 +233,27 @@ class LatentAttention(Mixer):
             cq = torch.empty((n, self.q_rank), dtype=x.dtype, device=dev)
             ops.rmsnorm(cq, proj[:, :self.q_rank], self.q_norm_w, self.eps)
             qrows = ops.linear(cq, self.w_uq)
-        spans = self._expanded(step, qrows)
-        na = n if spans is None else step.num_single        # tokens that meet the latents themselves
+        latent, groups = self._runs(step, qrows)
+        # (tokens in front of the first expanded portion, the step's single tokens among them, have their rotated parts put
+        # where the products over heads write; everybody else's are turned where they lie)
+        na, front = (latent[-1][1], latent[0][1] if latent[0][0] == 0 else 0) if latent else (0, 0)
         q_full = torch.empty((na, H, R + r), dtype=x.dtype, device=dev)
         ops.latent_prepare(proj, 0, self.kv_off, self.norm_w, self.eps, self.freq, self.rot_dims, step.positions,
                            cache.slot_map if cache.writable else None, cache.k, q_full, H, d, r, R, step.status,
-                           amplitude=self.amplitude, q=qrows, half_split=self.half_split, inplace_from=na)
+                           amplitude=self.amplitude, q=qrows, half_split=self.half_split, inplace_from=front)
         heads = torch.empty((n, H * self.dv), dtype=x.dtype, device=dev)
-        if na:
-            # queries into the latent space: a_h = Uk_h^T q_h, written in front of the rotated parts
-            q_plain = qrows[:na, :H * (d + r)].view(na, H, d + r)[:, :, :d].permute(1, 0, 2)         # [H, na, d]
-            ops.batched_heads(q_plain, self.w_uk, out=q_full[:, :, :R].permute(1, 0, 2))            # [H, na, R]
+        if latent:
             lat = torch.empty((na, H, R), dtype=x.dtype, device=dev)
-            self.attend(lat, q_full, step, cache, spans is not None)
-            ops.batched_heads(lat.permute(1, 0, 2), self.w_uv_t, out=heads[:na].view(na, H, self.dv).permute(1, 0, 2))
-        if spans is not None:
-            self._attend_expanded(heads, qrows, step, cache, spans)
+        for t0, t1 in latent:
+            q_head = qrows[t0:t1, :H * (d + r)].view(t1 - t0, H, d + r)
+            if t0 >= front and r:
+                q_full[t0:t1, :, R:].copy_(q_head[:, :, d:])
+            # queries into the latent space: a_h = Uk_h^T q_h, written in front of the rotated parts
+            ops.batched_heads(q_head[:, :, :d].permute(1, 0, 2), self.w_uk, out=q_full[t0:t1, :, :R].permute(1, 0, 2))  # [H, tokens, R]
+            self.attend(lat, q_full, step, cache, (t0, t1) if groups else None)
+            ops.batched_heads(lat[t0:t1].permute(1, 0, 2), self.w_uv_t, out=heads[t0:t1].view(t1 - t0, H, self.dv).permute(1, 0, 2))
+        for e0, spans, plan in groups:
+            self._attend_expanded(heads, qrows, step, cache, e0, spans, plan)
         if self.channel_gate:
             ops.gate_rows(heads, proj[:, self.gate_off:self.gate_off + H * self.dv])
         return ops.linear(heads, self.w_o, partial_ok=self.partial_ok)
@@ -237,13 +272,15 @@ class LatentAttention(Mixer):
         nsplit = max(1, min(tiles, (2 * ops.sm_count(device)) // max(1, ctas), 16))
         return nsplit, (tiles + nsplit - 1) // nsplit
 
-    def attend(self, lat, q_full, step, cache, single_only: bool = False) -> None:
+    def attend(self, lat, q_full, step, cache, tokens=None) -> None:
+        """All of the step's tokens, or (``tokens``) a run of single tokens and short portions."""
         n, H, R, r = q_full.shape[0], self.H, self.R, self.r
         args = (H, R, r, cache.page_size, self.window, self.scale)
         entries = None if getattr(step, "captured", False) else getattr(step, "entries", None)
-        if single_only or entries is None or all(len(e.tokens) < self.PRODUCT_MIN_TOKENS for e in entries):
-            ops.latent_attention(lat, q_full, cache.k, cache.block_table, step, 0, n, *args,
-                                 *self._splits(n, step, lat.device), sink=self.sink_w)
+        if tokens is not None or entries is None or all(len(e.tokens) < self.PRODUCT_MIN_TOKENS for e in entries):
+            t0, t1 = tokens or (0, n)
+            ops.latent_attention(lat, q_full, cache.k, cache.block_table, step, t0, t1 - t0, *args,
+                                 *self._splits(t1 - t0, step, lat.device), sink=self.sink_w)
             return
         t, run0 = 0, 0          # run0: first token of the current run of entries that go to the kernel
         for e, ctx in zip(entries, step.entry_ctx):

@@ -27,8 +27,9 @@ def _part(params, seed):
     return part
 
 
-def _run(part, steps, page, seed):
-    """Outputs of the steps (lists of new tokens a request, 0: the request is not in the step) through one cache."""
+def _run(part, steps, page, seed, seen=None):
+    """Outputs of the steps (lists of new tokens a request, 0: the request is not in the step) through one cache.  ``seen``:
+    gets each step's input and the requests of its rows."""
     from lite_lang_b200.cache.manager import CacheManager, PagedGroupSpec
     from lite_lang_b200.cache.storage import CacheStorage
     from lite_lang_b200.engine.batch import BatchBuilder, StepEntry
@@ -52,6 +53,8 @@ def _run(part, steps, page, seed):
         batch = builder.build(entries)
         x = torch.randn(batch.num_tokens, part.hidden_size, generator=g, device="cuda").to(torch.bfloat16)
         outs.append(part.forward(x, batch, storage.paged_view(0, 0, batch.slot_maps[0], True)))
+        if seen is not None:
+            seen.append((x, torch.tensor([slots.index(e.slot) for e in batch.entries for _ in e.tokens], device="cuda")))
         for e in entries:
             manager.advance(e.slot, manager.length(e.slot) + len(e.tokens))
         torch.cuda.synchronize()
@@ -204,3 +207,38 @@ def test_gathered_rows_are_not_streamed_as_weights(params, tokens, monkeypatch):
     assert len(scored) == 2 and not set(scored) & set(streamed)
     x = torch.randn(tokens, part.hidden_size, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda")
     assert _rel(got, _exact(part, x.to(torch.bfloat16))) <= 1.2e-2
+
+
+# single tokens, portions too short to be expanded in front of, between and behind long ones; then portions that go on
+_MIXED = [[[1, 8, 100, 20, 300, 5, 31, 32], [40, 1, 33, 64, 2, 90, 1, 1]], [[0, 17, 17, 64], [64, 1, 200, 16]], [[16, 31], [31, 2]]]
+
+
+@gpu
+@pytest.mark.parametrize("steps", _MIXED)
+@pytest.mark.parametrize("params", [
+    dict(hidden_size=256, heads=3, dim=96, rot_dim=32, vdim=128, kv_rank=64, window=100, rot_dims=32, eps=1e-6),
+    dict(hidden_size=256, heads=2, dim=64, rot_dim=0, vdim=64, kv_rank=128, q_rank=64, sink=True, eps=1e-6),
+    dict(hidden_size=192, heads=5, dim=48, rot_dim=16, vdim=64, kv_rank=96, rot_dims=8, rot_layout="half_split",
+         channel_gate=True, eps=1e-6)])
+def test_portions_of_all_lengths_beside_float64(params, steps, monkeypatch):
+    """No further off than the same portions in the latent space, with the long ones expanded; those below 32 tokens never are."""
+    from lite_lang_b200 import ops
+    lens, real = [], ops.latent_unpage
+    monkeypatch.setattr(ops, "latent_unpage", lambda *a, **k: (lens.append([n for _, n in a[5]]), real(*a, **k))[1])
+    part, err = _part(params, 5), {}
+    for way in ("latent", "expanded"):
+        monkeypatch.setattr(type(part), "EXPAND_MIN_TOKENS", 1 << 30 if way == "latent" else part.PRODUCT_MIN_TOKENS)
+        lens.clear()
+        seen = []
+        outs = _run(part, steps, 16, 9, seen)
+        long = sorted(n for s in steps for n in s if n >= 32)
+        assert sorted(n for span in lens for n in span) == ([] if way == "latent" else long)
+        got, want = [], []
+        for i in range(len(steps[0])):
+            x = torch.cat([x[who == i] for x, who in seen])
+            got.append(torch.cat([o[who == i] for o, (_, who) in zip(outs, seen)]))
+            want.append(_exact(part, x))
+            # bfloat16 at each of five products and twice in the attention: a few 2^-9 of the result
+            assert _rel(got[-1], want[-1]) <= 1.2e-2
+        err[way] = _rel(torch.cat(got), torch.cat(want))
+    assert err["expanded"] <= 1.15 * err["latent"], err
