@@ -173,6 +173,9 @@ class LatentAttention(Mixer):
     # tcgen05 attention has one term of eight, as the products over the latents have.
     EXPAND_MIN_TOKENS = PRODUCT_MIN_TOKENS
     EXPAND_MAX_ROWS = 16
+    # Memory that the expanded rows of a call may take at a time: entries are served in groups that stay below it.  (One
+    # entry may be more; the products' scores and weights, 6 bytes a head, key and query of a block of 256, are more then.)
+    EXPAND_BYTES = 256 << 20
 
     def _runs(self, step, qrows):
         """How the step's entries are served: (tokens that meet the latents themselves, as runs [(first, behind the last)];
@@ -214,7 +217,16 @@ class LatentAttention(Mixer):
         return min(ctx, self.window - 1) if self.window else ctx
 
     def _groups(self, spans):
-        yield 0, len(spans)
+        """(first, behind the last) of neighbouring entries whose expanded rows fit ``EXPAND_BYTES`` together."""
+        row = 2 * (2 * self.H * self.dv + self.R + self.r)
+        first, used = 0, 0
+        for i, (c, q) in enumerate(spans):
+            need = (self._seen(c) + q + ops.CHUNK - 1) // ops.CHUNK * ops.CHUNK * row
+            if i > first and used + need > self.EXPAND_BYTES:
+                yield first, i
+                first, used = i, 0
+            used += need
+        yield first, len(spans)
 
     def _attend_expanded(self, heads, qrows, step, cache, e0, spans, plan) -> None:
         """Entries ``e0`` ... of the step: their ``heads`` rows = attention over expanded keys and values."""
