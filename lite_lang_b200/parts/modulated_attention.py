@@ -53,8 +53,8 @@ anything is rounded.
 
 Kernels: in bfloat16 with head sizes 64 and 128, tensor cores (``attn_shaped``: prompt portions 128 rows a CTA,
 single tokens with their keys split over CTAs; mixed heads as one wider query a head, made where q is
-normalised; prompt portions of a design without mixed heads: the plain attention's tcgen05 kernel, the temperature on
-the queries, the scores shaped by the softmax's threads and the gate in its epilogue); every other size, and float32, a block a token in
+normalised; prompt portions of a design without mixed heads, but for short ones: the plain attention's tcgen05 kernel, the
+temperature on the queries, the scores shaped by the softmax's threads and the gate in its epilogue); every other size, and float32, a block a token in
 float32 arithmetic (``attention_modulated``).
 """
 
@@ -374,6 +374,41 @@ class ModulatedAttention(Mixer):
                                 query_temperature=self.query_temperature, gate_channels=self.channel_gate,
                                 out_scale=out_scale, distance_slope=self.slopes, pairs=self.pairs)
 
+    # Shaped portions whose rows see at least this many keys go to the tcgen05 kernel, shorter ones to the mma.sync kernel.
+    # With a distance bias a block of 64 keys costs its row threads 64 reads of the table at the start of a chain of that one
+    # block.  Measured on a B200 (mma.sync / tcgen05, us; heads on kv heads of 128; one portion without cached tokens):
+    # bias, sink and gate, 28 on 4: 16 tokens 15.6 / 21.0, 64 18.7 / 21.0, 128 24.7 / 23.4, 256 36.8 / 26.8, 16 behind 1,024
+    # (window 512) 69 / 32; 2 on 2: 64 17.5 / 19.3, 128 23.2 / 22.3; four portions of 128, 28 on 4 25.2 / 26.0, 12 on 2
+    # 25.0 / 24.0.  Cap, 12 on 2: 64 12.1 / 9.6; 8 on 8: 2 tokens 7.9 / 8.7; 4 on 1 of 64: 16 6.3 / 6.8, 64 8.3 / 6.9.
+    TC_MIN_KEYS = 32
+    TC_MIN_KEYS_BIAS = 128
+
+    def _shaped_plan(self, step, n_single: int, group: int, device):
+        """The plan of the step's portions for the tcgen05 kernel; None where it is not meant for them."""
+        key = ("attn_prefill_tc_shaped", group, self.num_kv_heads, self.mask, self.mask_size, self.keep_first,
+               self.bias_by_distance is None)
+        plan = step.scratch.get(key, 0)
+        if plan == 0:
+            spans = [(c, len(e.tokens)) for c, e in zip(step.entry_ctx[n_single:], step.entries[n_single:])]
+            plan = step.scratch[key] = ops.attn_prefill_tc_plan(
+                spans, group, self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(device),
+                self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0
+            ) if self._tc_preferred(spans, group) else None
+        return plan
+
+    def _tc_preferred(self, spans, group: int) -> bool:
+        """Whether the tcgen05 kernel is meant for the shaped scores of portions ``spans`` ((cached, new) tokens)."""
+        most = 0
+        for c, q in spans:
+            if self.mask == "window":
+                seen = min(c + q, self.mask_size - 1 + 128 // group + self.keep_first)
+            elif self.mask == "chunk":
+                seen = min(c % self.mask_size + q, self.mask_size)
+            else:
+                seen = c + q
+            most = max(most, seen)
+        return most >= (self.TC_MIN_KEYS if self.bias_by_distance is None else self.TC_MIN_KEYS_BIAS)
+
     def attend_shaped(self, out, proj, mixed_q, gate, step, cache, temperature, out_scale: float = 1.0) -> None:
         """Tensor cores.  Single-token entries come first in a step: their keys are cut into parts of one or more
         stages of 64 keys, a CTA each (as many parts as the step's single tokens leave SMs for, so the order of a
@@ -432,15 +467,9 @@ class ModulatedAttention(Mixer):
         elif (n_rest > 0 and mixed_q is None and temperature is None and self.vdim == self.key_dim and self.pairs is None
                 and ops.TC_ENABLED and getattr(step, "entry_ctx", None) is not None
                 and ops.attn_prefill_tc_supported(q.dtype, self.key_dim, cache.page_size, q.stride(0), group)
-                and (gate is None or not self.channel_gate or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))):
+                and (gate is None or not self.channel_gate or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))
+                and (plan := self._shaped_plan(step, n_single, group, proj.device))):
             # shaped scores on the same kernel: the row's thread makes them between product and softmax
-            key = ("attn_prefill_tc_shaped", group, self.mask, self.mask_size, self.keep_first)
-            plan = step.scratch.get(key)
-            if plan is None:
-                plan = step.scratch[key] = ops.attn_prefill_tc_plan(
-                    [(step.entry_ctx[n_single + i], len(e.tokens)) for i, e in enumerate(step.entries[n_single:])], group,
-                    self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(proj.device),
-                    self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0)
             del more["pairs"]
             ops.attn_prefill_tc_shaped(out, q, q.stride(0), gate, cache.k, cache.v, cache.block_table, step.cu_q[n_single:],
                                        step.ctx_len[n_single:], step.req_slot[n_single:], n_rest, plan, self.map_heads,

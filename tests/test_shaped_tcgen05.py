@@ -75,3 +75,62 @@ def test_shaped_scores_equal_the_other_kernels(shape, hd, nh, nkv, splits):
     # the same scores and sixteen-bit weights: what remains is the order of the sums and the one rounding to bfloat16
     assert float((outs[1] - outs[0]).abs().max()) <= 2.0 ** -7 * float(outs[0].abs().max())
     assert float((outs[1] - outs[0]).norm()) <= 2e-3 * float(outs[0].norm())
+
+
+@pytest.mark.parametrize("params,spans,taken", [
+    (dict(mask="window", mask_size=512, bias=True), [(0, 127)], False),
+    (dict(mask="window", mask_size=512, bias=True), [(0, 128)], True),
+    (dict(mask="window", mask_size=512, bias=True), [(0, 16), (120, 8), (0, 64)], True),
+    (dict(mask="window", mask_size=20, bias=True), [(4000, 2000)], False),      # (a row block sees 19 keys and its own tokens)
+    (dict(mask="window", mask_size=20, keep_first=100, bias=True), [(4000, 2000)], True),
+    (dict(mask="causal", mask_size=None), [(0, 31), (0, 2)], False),
+    (dict(mask="causal", mask_size=None), [(30, 2)], True),
+    (dict(mask="chunk", mask_size=256), [(256, 20)], False),
+    (dict(mask="chunk", mask_size=256), [(255, 20)], True)])
+def test_which_shaped_portions_go_to_tcgen05(params, spans, taken):
+    from lite_lang_b200.parts.modulated_attention import ModulatedAttention
+    part = ModulatedAttention.__new__(ModulatedAttention)
+    part.mask, part.mask_size, part.keep_first = params["mask"], params["mask_size"], params.get("keep_first", 0)
+    part.bias_by_distance = torch.zeros(1) if params.get("bias") else None
+    assert part._tc_preferred(spans, 7) is taken
+
+
+# on both sides of the lines: which kernel a part's portion takes, and that a layer with other kv heads plans for itself
+@gpu
+@pytest.mark.parametrize("bias,tokens,taken", [(True, 127, False), (True, 128, True), (False, 31, False), (False, 32, True)])
+def test_parts_take_the_kernel_that_is_meant(bias, tokens, taken, monkeypatch):
+    from lite_lang_b200 import ops
+    from lite_lang_b200.cache.manager import CacheManager, PagedGroupSpec
+    from lite_lang_b200.cache.storage import CacheStorage
+    from lite_lang_b200.config.spec import PartSpec
+    from lite_lang_b200.engine.batch import BatchBuilder, StepEntry
+    from lite_lang_b200.parts.base import build_part
+    import lite_lang_b200.parts  # noqa: F401
+    ops.configure_matmul_precision()
+    device, names = torch.device("cuda", 0), []
+    for name in ("attn_prefill_tc_shaped", "attn_shaped"):
+        real = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, _real=real, _name=name, **k: (names.append(_name), _real(*a, **k))[1])
+    g = torch.Generator(device="cuda").manual_seed(4)
+    part = build_part("mixer", PartSpec("modulated_attention", dict(
+        hidden_size=128, num_heads=4, num_kv_heads=2, head_dim=64, scale=0.125, mask="window", mask_size=200, sink="learned",
+        distance_bias=dict(max=400.0, buckets=32) if bias else None)))
+    part.load(lambda n: (torch.randn([32 if d is None else d for d in part.tensors()[n].shape], generator=g, device="cuda") * 0.1)
+              .to(torch.bfloat16), torch.bfloat16, device)
+    part.prepare(device, torch.bfloat16)
+    manager = CacheManager([PagedGroupSpec(2, 64, 200, 1, 64)], [64], 16, 1, tokens)
+    storage, status = CacheStorage(manager, torch.bfloat16, device), torch.zeros(1, dtype=torch.int32, device=device)
+    slot = manager.open()
+    assert manager.reserve(slot, tokens)
+    storage.sync()
+    x, outs = torch.randn(tokens, 128, generator=g, device="cuda").to(torch.bfloat16), []
+    for least in (None, 1 << 30):                       # as meant, and by the other kernel
+        if least:
+            monkeypatch.setattr(type(part), "TC_MIN_KEYS", least)
+            monkeypatch.setattr(type(part), "TC_MIN_KEYS_BIAS", least)
+        batch = BatchBuilder(manager, tokens, 1, device, status).build([StepEntry(slot, [0] * tokens)])
+        out = part.forward(x, batch, storage.paged_view(0, 0, batch.slot_maps[0], True))
+        outs.append(out.float().sum(0) if out.dim() == 3 else out.float())
+    assert names == ["attn_prefill_tc_shaped" if taken else "attn_shaped", "attn_shaped"]
+    assert int(status.item()) == 0
+    assert float((outs[0] - outs[1]).norm()) <= 1e-2 * float(outs[1].norm())
