@@ -1080,29 +1080,47 @@ def gemm_pair_qkv_rope(q_out: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor
 ACCUMULATE_MIN_M = 129   # more tokens than any of the hand-written plain products takes: library territory
 
 
-# Rows, and multiply-adds, from which on a float32 product goes to the tensor cores (``gemm_f32``).  Measured on a B200
-# (library / here): 64 x 17,920 x 1,536 72 / 81 us, 64 x 2,048 x 1,536 31 / 39, 64 x 1,536 x 8,960 134 / 52;
-# 128 x 37,888 x 3,584 535 / 326; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395;
-# 300 x 132 x 72 11 / 24 (its launches).
+# Rows, and multiply-adds, from which on a float32 product may go to the tensor cores (``gemm_f32``): below them its launches
+# count.  Measured on a B200 (library / here): 64 x 17,920 x 1,536 72 / 81 us, 64 x 2,048 x 1,536 31 / 39, 300 x 132 x 72
+# 11 / 24.  Above them `f32_preferred` says which is the faster.
 F32_MIN_M = 96
 F32_MIN_WORK = 1 << 28
 
 
-def f32_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+def f32_supported(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
     """Whether ``gemm_f32`` takes this float32 product and is meant for it."""
     return (x.dtype == torch.float32 and weight.dtype == torch.float32 and TC_ENABLED and x.is_cuda and x.dim() == 2
             and weight.dim() == 2 and x.shape[0] >= F32_MIN_M and x.shape[1] % 8 == 0 and weight.shape[0] % 4 == 0
             and weight.shape[0] >= 64 and x.stride(1) == 1 and weight.stride(1) == 1 and x.stride(0) % 4 == 0
             and x.shape[0] * x.shape[1] * weight.shape[0] >= F32_MIN_WORK
-            and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+            and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and f32_preferred(x.shape[0], weight.shape[0], x.shape[1], sm_count(x.device), gated))
+
+
+def f32_preferred(m: int, n: int, k: int, sms: int, gated: bool = False) -> bool:
+    """Whether ``gemm_f32`` is expected to be faster than the library.  A step of 64 numbers of k takes a pair of SMs 3.1 us
+    and a tile's end 4, however many of the tile's 256 rows and columns are there, and tiles are handed out in rounds; the
+    library takes 12 us, 0.009 for a number of k and its operations at 68 TFLOP/s (measured on a B200 over 96 to 1,024 rows,
+    64 to 65,536 features and 72 to 18,944 numbers of k).  Few tiles with a gate (its k is not cut; library / here):
+    128 x 4,096 x 1,024 34 / 58 us, 1,024 x 4,096 x 1,024 173 / 63; a short k: 128 x 40,000 x 72 28 / 47, 512 x 40,000 x 72
+    90 / 75, 96 x 8,192 x 512 26 / 31, 192 x 8,192 x 512 41 / 32.  Else: 96 x 2,048 x 1,536 32 / 28, 128 x 37,888 x 3,584
+    568 / 342; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395."""
+    tiles, boxes = ((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64
+    splits = 1 if gated else _f32_parts(tiles, boxes, sms)
+    rounds = -(-tiles * splits // (sms // 2))
+    here = 8 + rounds * (-(-boxes // splits) * 3.1 + 4)
+    return here < 12 + 0.009 * k + 2 * m * n * k / 68e6
+
+
+def _f32_parts(tiles: int, boxes: int, sms: int) -> int:
+    splits = max(1, min((sms // 2) // tiles, boxes // 6))
+    per = (boxes + splits - 1) // splits
+    return (boxes + per - 1) // per
 
 
 def f32_splits(m: int, n: int, k: int, device) -> int:
     """Parts of k: as many as let the tiles of 256 x 256 fill the pairs of SMs, none shorter than 6 steps of 64."""
-    tiles, boxes = ((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64
-    splits = max(1, min((sm_count(device) // 2) // tiles, boxes // 6))
-    per = (boxes + splits - 1) // splits
-    return (boxes + per - 1) // per
+    return _f32_parts(((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64, sm_count(device))
 
 
 _reporting = threading.local()
@@ -1192,7 +1210,7 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation="silu") ->
         return gemm_smallm(x, w_gate_up, act, gated=True, act=activation)
     if TC_ENABLED and x.shape[0] >= PAIR_MIN_M and pair_supported(x, w_gate_up):
         return gemm_pair(x, w_gate_up, act, gated=True, act=activation)
-    if inter % 4 == 0 and f32_supported(x, w_gate_up):
+    if inter % 4 == 0 and f32_supported(x, w_gate_up, gated=True):
         return gemm_f32(x, w_gate_up, act, gated=activation)
     gu = linear(x, w_gate_up)
     if activation.kind == "silu":

@@ -61,6 +61,55 @@ def test_which_float32_products_go_to_the_tensor_cores():
     assert not ops.f32_supported(x, w)                               # (not on a CUDA device)
 
 
+@gpu
+@pytest.mark.parametrize("M,N,K,shift,out_pad,taken", [
+    (96, 1536, 2048, 0, 0, True), (95, 1536, 2048, 0, 0, False),                # rows
+    (256, 512, 2048, 0, 0, True), (256, 508, 2048, 0, 0, False),                # multiply-adds: 2^28
+    (96, 64, 65536, 0, 0, True), (96, 60, 65536, 0, 0, False),                  # features
+    (300, 1536, 2056, 0, 0, True), (300, 1536, 2052, 0, 0, False),              # numbers of k: a multiple of 8
+    (300, 1538, 2048, 0, 0, False),                                             # features: of 4
+    (300, 1536, 2048, 1, 0, False), (300, 1536, 2048, 4, 0, True),              # rows that start off 16 bytes
+    (300, 1536, 2048, 0, 2, False), (300, 1536, 2048, 0, 4, True),              # outputs of another stride
+    (192, 8192, 512, 0, 0, True), (128, 8192, 512, 0, 0, False)])               # few steps of k a tile: the library is faster
+def test_dispatch_of_float32_products(M, N, K, shift, out_pad, taken, monkeypatch):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    calls, real = [], ops.gemm_f32
+    monkeypatch.setattr(ops, "gemm_f32", lambda *a, **k: (calls.append(k.get("gated")), real(*a, **k))[1])
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K + 8, generator=g, device="cuda")[:, shift:shift + K]
+    w = torch.randn(N, K, generator=g, device="cuda")
+    want = x.double() @ w.double().t()
+    if not out_pad:
+        assert _rel(ops.linear(x, w), want) <= 2e-6
+        assert bool(calls) == taken
+        calls.clear()
+    out = torch.empty(M, N + out_pad, device="cuda")[:, :N]
+    assert ops.linear(x, w, out) is out and _rel(out, want) <= 2e-6
+    assert bool(calls) == taken
+    calls.clear()
+    acc = torch.randn(M, N + out_pad, generator=g, device="cuda")[:, :N]
+    both = acc.double() + want
+    ops.linear_accumulate(x, w, acc)
+    assert _rel(acc, both) <= 2e-6
+    assert bool(calls) == taken
+
+
+@gpu
+@pytest.mark.parametrize("M,I,K,gated", [(1024, 2048, 1024, True), (128, 2048, 1024, False), (300, 1538, 2048, False)])
+def test_dispatch_of_gated_float32_products(M, I, K, gated, monkeypatch):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    calls, real = [], ops.gemm_f32
+    monkeypatch.setattr(ops, "gemm_f32", lambda *a, **k: (calls.append(k.get("gated")), real(*a, **k))[1])
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5
+    gu = x.double() @ w.double().t()
+    want = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+    assert _rel(ops.gated_linear(x, w), want) <= 2e-6
+    assert any(c is not None for c in calls) is gated
+
+
 def test_every_float32_model_loads_the_products_kernel_at_its_start():
     """Whatever its parts are: the first large prompt would build or load it in the middle of a step otherwise."""
     from lite_lang_b200.config import config_from_dict
@@ -148,7 +197,7 @@ def test_products_report_to_the_steps_status_word(monkeypatch):
     monkeypatch.setattr(ops, "load_library", lambda name: spy)
     monkeypatch.setattr(ops, "_stream", lambda: None)
     monkeypatch.setattr(ops, "sm_count", lambda device: 148)
-    monkeypatch.setattr(ops, "f32_supported", lambda x, w: x.dtype == torch.float32)
+    monkeypatch.setattr(ops, "f32_supported", lambda x, w, **k: x.dtype == torch.float32)
     monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", False)
     x, w = torch.zeros(96, 64), torch.zeros(64, 64)
     ops.gemm_f32(x, w, status=word)
