@@ -226,6 +226,15 @@ def attn_f32_supported(q: torch.Tensor, k_cache: torch.Tensor, head_dim: int, va
             and q.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0)
 
 
+def attn_f32_preferred(tokens: int, num_kv_heads: int, longest: int, sms: int) -> bool:
+    """Whether a step of single tokens is meant for ``attn_f32``: 64 rows a CTA of which a token fills its group of heads, one
+    CTA an SM.  Measured on a B200 (general kernel / here, us; heads of 128): one token 64 keys 42 / 14, 8,192 keys 3,717 /
+    781; 64 tokens on 2 kv heads 64 keys 43 / 19, 8,192 keys 5,548 / 807; on 8 kv heads (four CTAs an SM in turn) 64 keys
+    35 / 62, 512 keys 312 / 232, 2,048 keys 1,198 / 818.  Short contexts of many (token, kv head) pairs stay with the
+    general kernel."""
+    return tokens * num_kv_heads <= 2 * sms or longest > 192
+
+
 def attn_f32(out: torch.Tensor, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
              cu_q: torch.Tensor, ctx_len: torch.Tensor, req_slot: torch.Tensor, q_lens, num_heads: int, num_kv_heads: int,
              head_dim: int, page_size: int, window: Optional[int], scale: float, status: Optional[torch.Tensor]) -> None:

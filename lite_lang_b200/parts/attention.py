@@ -307,7 +307,10 @@ class GQAttention(Mixer):
             entries = None if captured else getattr(step, "entries", None)
             lens = [1] * step.num_entries if step.num_single == step.num_entries else \
                 None if entries is None else [len(e.tokens) for e in entries]
-            if lens is not None and sum(lens) == qkv.shape[0]:
+            if lens is not None and sum(lens) == qkv.shape[0] and (
+                    len(lens) != sum(lens) or ops.attn_f32_preferred(
+                        len(lens), self.num_kv_heads, min(step.max_kv_len, self.window or step.max_kv_len),
+                        ops.sm_count(qkv.device))):
                 ops.attn_f32(out, qkv, cache.k, cache.v, cache.block_table, step.cu_q, step.ctx_len, step.req_slot, lens,
                              self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size, self.window, self.scale,
                              step.status)

@@ -110,6 +110,16 @@ def test_dispatch_of_gated_float32_products(M, I, K, gated, monkeypatch):
     assert any(c is not None for c in calls) is gated
 
 
+def test_rules_of_float32_products_and_attention():
+    """The lines that were measured, both sides (see ops.py)."""
+    from lite_lang_b200 import ops
+    assert ops.f32_preferred(96, 2048, 1536, 148) and ops.f32_preferred(701, 17920, 1536, 148, True)
+    assert ops.f32_preferred(1024, 4096, 1024, 148, True) and not ops.f32_preferred(128, 4096, 1024, 148, True)
+    assert not ops.f32_preferred(128, 40000, 72, 148) and ops.f32_preferred(192, 65536, 128, 148)
+    assert ops.attn_f32_preferred(64, 2, 64, 148) and ops.attn_f32_preferred(1, 8, 8192, 148)
+    assert not ops.attn_f32_preferred(64, 8, 192, 148) and ops.attn_f32_preferred(64, 8, 193, 148)
+
+
 def test_every_float32_model_loads_the_products_kernel_at_its_start():
     """Whatever its parts are: the first large prompt would build or load it in the middle of a step otherwise."""
     from lite_lang_b200.config import config_from_dict
