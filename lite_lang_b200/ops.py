@@ -1363,15 +1363,31 @@ def delta_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b_off:
 
 
 CHUNK = 64                 # tokens of a chunk (csrc/chunk_scan.cu)
-# Tokens of a portion, on average, from which on it is scanned by chunks.  Measured on a B200, 12 heads of 128 x 128, one
-# portion (the walk's time grows with the tokens, the chunks' three launches take 28 us down to the smallest):
-#   decay scan, bfloat16: 64 tokens 14 us by the walk, 29 by chunks; 128 tokens 27 and 28; 2,048 tokens 320 and 53
-#   delta rule:           64 tokens 31 us by the walk, 37 by chunks; 128 tokens 58 and 47; 2,048 tokens 872 and 185
+# Tokens of a portion, on average, from which on it is scanned by chunks, for one portion with 12 heads of 128 x 128; for
+# other steps `decay_chunked_min` and `delta_chunked_min`.  The walk's time is its tokens times what a token takes, which
+# grows with the heads of all entries once they outnumber the SMs; the chunks' three launches take as long as the host
+# needs for them (26 us; the kernels 17) or, as a delta rule, 42 us and more.  Measured on a B200 with the launches (us, walk / chunks):
+#   decay scan, heads of 128: 2 heads x 160 tokens 23 / 27, x 192 28 / 26; 12 x 128 26 / 26; 28 x 96 26 / 26; 64 x 64 31 / 27;
+#     4 portions: 8 heads x 96 28 / 27; 2,048 tokens of 12 heads 320 / 53
+#   delta rule:  2 heads x 128 41 / 43, x 160 51 / 46; 8 x 96 43 / 45; 12 x 96 44 / 41; 28 x 64 54 / 48; heads of 64, 12 x 64
+#     22 / 30, x 128 40 / 33; 2,048 tokens of 12 heads of 128 872 / 185
 DECAY_CHUNKED_MIN = 128
 DELTA_CHUNKED_MIN = 96
 
 
-def chunked_scan(step, tokens: int, dk: int, dv: int, least: int) -> Optional[Tuple[int, int, int]]:
+def decay_chunked_min(heads: int, dk: int, dv: int) -> float:
+    """``heads``: of all entries together.  A token's time in the walk: 0.11 us and 0.006 for each state of 128 x 128."""
+    states = heads * dk * dv / 16384
+    return DECAY_CHUNKED_MIN * (0.11 + 0.006 * 12) / (0.11 + 0.006 * states)
+
+
+def delta_chunked_min(heads: int, dk: int, dv: int) -> float:
+    """As above: 0.33 us a token and 0.012 for each state of 128 x 128 against 30 us and 15.5 for states of that size."""
+    size = dk * dv / 16384
+    return DELTA_CHUNKED_MIN * (30 + 15.5 * size) / 45.5 * (0.33 + 0.012 * 12) / (0.33 + 0.012 * heads * size)
+
+
+def chunked_scan(step, tokens: int, dk: int, dv: int, least: float) -> Optional[Tuple[int, int, int]]:
     """How a step's recurrences are cut: None (all entries token by token), or (entries at the front that stay with the
     walk by tokens, entries behind them that go by chunks, an upper bound of their chunks).
 
@@ -1384,6 +1400,10 @@ def chunked_scan(step, tokens: int, dk: int, dv: int, least: int) -> Optional[Tu
     if rest <= 0 or tokens - single < least * rest:
         return None
     return single, rest, (tokens - single) // CHUNK + rest
+
+
+def _portions(step) -> int:
+    return int(step.num_entries) - int(getattr(step, "num_single", 0) or 0)
 
 
 def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, cut) -> None:
@@ -1408,7 +1428,7 @@ def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta:
     _need(dk <= 256, f"delta rule: key heads of {dk} channels are wider than the scan kernel takes (256)")
     entries = step.num_entries
     if not per_channel and dv <= 128 and state.stride(0) % 4 == 0 and all(t.data_ptr() % 16 == 0 for t in (qn, kn, vc, state, o)):
-        cut = chunked_scan(step, qn.shape[0], dk, dv, DELTA_CHUNKED_MIN)
+        cut = chunked_scan(step, qn.shape[0], dk, dv, delta_chunked_min(H * _portions(step), dk, dv))
         if cut is not None:
             _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H, Hk, dk, dv, cut)
             entries = cut[0]
@@ -1841,7 +1861,7 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay: Op
     entries, size = step.num_entries, proj.element_size()
     if (proj.stride(0) * size % 16 == 0 and all(x * size % 16 == 0 for x in (q_off, k_off, v_off))
             and all(t_.data_ptr() % 16 == 0 for t_ in (proj, o))):
-        cut = chunked_scan(step, proj.shape[0], dk, dv, DECAY_CHUNKED_MIN)
+        cut = chunked_scan(step, proj.shape[0], dk, dv, decay_chunked_min(H * _portions(step), dk, dv))
         if cut is not None:
             single, rest, items = cut
             ds = torch.empty(items * H * dv * dk, dtype=torch.float32, device=proj.device)

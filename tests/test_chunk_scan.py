@@ -29,6 +29,16 @@ def test_which_portions_go_by_chunks():
     assert items >= sum((n + 63) // 64 for n in (100, 156))
 
 
+def test_the_lines_move_with_the_heads():
+    """Tokens a portion from which on the chunks were measured ahead (see ops.py): more for few heads, fewer for many."""
+    from lite_lang_b200 import ops
+    for heads, low, high in ((2, 160, 224), (8, 128, 192), (12, 127, 129), (28, 64, 112), (64, 32, 64)):
+        assert low <= ops.decay_chunked_min(heads, 128, 128) <= high
+    for heads, low, high in ((2, 112, 160), (8, 96, 128), (12, 95, 97), (28, 48, 96), (64, 32, 64)):
+        assert low <= ops.delta_chunked_min(heads, 128, 128) <= high
+    assert 64 < ops.delta_chunked_min(12, 64, 64) < 128
+
+
 # lengths at the edges of a chunk, several entries, and single tokens in front that stay with the walk
 _LENS = [([64], 0), ([65, 63, 1, 128], 0), ([1, 1, 200], 2), ([129, 300], 0)]
 
