@@ -39,8 +39,27 @@ def test_the_lines_move_with_the_heads():
     assert 64 < ops.delta_chunked_min(12, 64, 64) < 128
 
 
-# lengths at the edges of a chunk, several entries, and single tokens in front that stay with the walk
-_LENS = [([64], 0), ([65, 63, 1, 128], 0), ([1, 1, 200], 2), ([129, 300], 0)]
+# lengths at the edges of a chunk, several entries, single tokens in front that stay with the walk, many chunks with a ragged
+# end, and (third number) an entry of padding, whose read-outs are zeros
+_LENS = [([64], 0, None), ([65, 63, 1, 128], 0, None), ([1, 1, 200], 2, None), ([129, 300], 0, None), ([411], 0, None),
+         ([1, 100, 90, 70], 1, 2), ([64], 0, 0)]
+
+
+def _entry_points(monkeypatch):
+    """The names of the kernel libraries' entry points, as they are called."""
+    from lite_lang_b200 import ops
+    names, real = [], ops.load_library
+
+    class Spy:
+        def __init__(self, lib):
+            self.lib = lib
+
+        def call(self, name, *args):
+            names.append(name)
+            return self.lib.call(name, *args)
+
+    monkeypatch.setattr(ops, "load_library", lambda lib: Spy(real(lib)))
+    return names
 
 
 def _rel(x, y):
@@ -48,11 +67,11 @@ def _rel(x, y):
 
 
 @gpu
-@pytest.mark.parametrize("lens,single", _LENS)
+@pytest.mark.parametrize("lens,single,pad", _LENS)
 @pytest.mark.parametrize("dtype,H,hpg,dk,dv,token_decay", [
     (torch.bfloat16, 3, 1, 128, 128, False), (torch.float32, 4, 2, 128, 64, True), (torch.float32, 2, 1, 64, 192, False),
     (torch.bfloat16, 2, 2, 64, 64, True)])
-def test_decay_scan_by_chunks(lens, single, dtype, H, hpg, dk, dv, token_decay, monkeypatch):
+def test_decay_scan_by_chunks(lens, single, pad, dtype, H, hpg, dk, dv, token_decay, monkeypatch):
     """Both ways beside float64: the chunks are no further off than twice the walk's error (float32 sums in another order)."""
     from lite_lang_b200 import ops
     g = torch.Generator(device="cuda")
@@ -66,10 +85,14 @@ def test_decay_scan_by_chunks(lens, single, dtype, H, hpg, dk, dv, token_decay, 
         td, ts, skip = torch.exp(-2 * torch.rand(n, H, **rnd)), torch.rand(n, H, **rnd), torch.randn(H, **rnd)
         td[::7] = 0.0                                           # a decay that forgets everything
     slots = list(range(len(lens)))[::-1]
+    if pad is not None:
+        slots[pad] = -1
     state0 = torch.randn(len(lens) + 1, H * dk * dv, **rnd)
-    step = _step(lens, slots, single)
+    step, names = _step(lens, slots, single), _entry_points(monkeypatch)
     want, state = torch.zeros(n, H, dv, dtype=torch.float64, device="cuda"), state0.double().clone()
     for e, length in enumerate(lens):
+        if slots[e] < 0:
+            continue
         a, S = int(step.cu_q[e]), state[slots[e]].view(H, dv, dk).clone()
         rows = proj[a:a + length].double()
         q = rows[:, :G * dk].view(length, G, dk).repeat_interleave(hpg, 1)
@@ -89,19 +112,27 @@ def test_decay_scan_by_chunks(lens, single, dtype, H, hpg, dk, dv, token_decay, 
         st, o = state0.clone(), torch.full((n, H * dv), float("nan"), device="cuda")
         ops.decay_scan(proj, *off, None if token_decay else decay, st, step, o, H, dk, dv, True, hpg, td, ts, skip)
         assert int(step.status.item()) == 0
+        assert names == ["ll_chunk_decay_scan"] * (way == "chunks") + ["ll_decay_scan"] * (way == "walk" or single > 0)
         assert torch.equal(st[len(lens)], state0[len(lens)])          # a record that no entry names
+        if pad == 0:
+            assert bool((o == 0).all()) and torch.equal(st, state0)
+            names.clear()
+            continue
         err[way] = (_rel(o.view(n, H, dv), want), _rel(st, state))
         if way == "chunks":
             kept = st.clone()
             ops.decay_scan(proj, *off, None if token_decay else decay, kept, step, o, H, dk, dv, False, hpg, td, ts, skip)
             assert torch.equal(kept, st)                              # not writable: the record stays
+        names.clear()
+    if pad == 0:
+        return
     assert err["chunks"][0] <= max(2 * err["walk"][0], 3e-7) and err["chunks"][1] <= max(2 * err["walk"][1], 3e-7), err
 
 
 @gpu
-@pytest.mark.parametrize("lens,single", _LENS)
+@pytest.mark.parametrize("lens,single,pad", _LENS)
 @pytest.mark.parametrize("H,Hk,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 128), (2, 1, 128, 64), (2, 2, 64, 64)])
-def test_delta_rule_by_chunks(lens, single, H, Hk, dk, dv, monkeypatch):
+def test_delta_rule_by_chunks(lens, single, pad, H, Hk, dk, dv, monkeypatch):
     from lite_lang_b200 import ops
     g = torch.Generator(device="cuda")
     g.manual_seed(dk + dv + len(lens))
@@ -116,9 +147,10 @@ def test_delta_rule_by_chunks(lens, single, H, Hk, dk, dv, monkeypatch):
     decay = torch.exp(-torch.rand(n, H, **rnd) * torch.linspace(0.01, 3.0, H, device="cuda"))
     decay[::11] = 0.0
     slots = list(range(len(lens)))[::-1]
-    slots[-1] = -1                                              # a padding entry: zeros
+    if pad is not None:
+        slots[pad] = -1
     state0 = torch.randn(len(lens) + 1, H * dk * dv + 12, **rnd)
-    step = _step(lens, slots, single)
+    step, names = _step(lens, slots, single), _entry_points(monkeypatch)
     want, state = torch.zeros(n, H, dv, dtype=torch.float64, device="cuda"), state0.double().clone()
     for e, length in enumerate(lens):
         if slots[e] < 0:
@@ -138,10 +170,13 @@ def test_delta_rule_by_chunks(lens, single, H, Hk, dk, dv, monkeypatch):
         monkeypatch.setattr(ops, "DELTA_CHUNKED_MIN", least)
         st, o = state0.clone(), torch.full((n, H * dv), float("nan"), device="cuda")
         ops.delta_recurrence(qn, kn, vc, beta, decay, st, step, o, H, Hk, dk, dv, False)
-        if len(lens) > 1:
-            err[way] = (_rel(o.view(n, H, dv), want), _rel(st, state))
-        else:
+        assert int(step.status.item()) == 0
+        assert names == ["ll_chunk_delta_scan"] * (way == "chunks") + ["ll_delta_recurrence"] * (way == "walk" or single > 0)
+        names.clear()
+        if pad == 0:
             assert bool((o == 0).all()) and torch.equal(st, state0)
+        else:
+            err[way] = (_rel(o.view(n, H, dv), want), _rel(st, state))
     if err:
         assert err["chunks"][0] <= max(2 * err["walk"][0], 3e-7) and err["chunks"][1] <= max(2 * err["walk"][1], 3e-7), err
 
