@@ -15,6 +15,43 @@ _SHAPES = [
 ]
 
 
+def _exact(q, k, v, table, spans, nh, hd, mask, size, keep, sink, more, gates, page):
+    """The portions' outputs in float64 (the first span is no portion)."""
+    outs, at, nkv = [], spans[0][1], k.shape[1]
+    for e, (c, n) in enumerate(spans[1:], 1):
+        p, j = torch.arange(c, c + n, device="cuda")[:, None], torch.arange(c + n, device="cuda")[None, :]
+        seen = j <= p
+        if mask == "window":
+            seen &= (p - j < size) | (j < keep)
+        elif mask == "chunk":
+            seen &= j // size == p // size
+        pg = table[e][j[0] // page].long()
+        keys, vals = (torch.where((pg < 0)[:, None, None], 0.0, t[pg.clamp(min=0), :, j[0] % page].double()) for t in (k, v))
+        rows = torch.empty(n, nh, hd, dtype=torch.float64, device="cuda")
+        for h in range(nh):
+            s = q[at:at + n, h * hd:(h + 1) * hd].double() @ keys[:, h // (nh // nkv)].t() * hd ** -0.5
+            if more["query_temperature"] is not None:
+                coef, every = more["query_temperature"]
+                s = s * (1 + coef * torch.log(((p + 1) // every + 1).double()))
+            if more["softcap"]:
+                s = more["softcap"] * torch.tanh(s / more["softcap"])
+            if more["distance_bias"] is not None:
+                s = s + more["distance_bias"].double()[(p - j).clamp(0, more["distance_bias"].shape[0] - 1), h]
+            if more["distance_slope"] is not None:
+                s = s - more["distance_slope"].double()[h] * (p - j)
+            s = s.masked_fill(~seen, float("-inf"))
+            if sink:
+                extra = torch.zeros((), device="cuda") if more["sink_values"] is None else more["sink_values"][h]
+                s = torch.cat([s, extra.double().expand(n, 1)], dim=1)
+            rows[:, h] = torch.softmax(s, dim=1)[:, :c + n] @ vals[:, h // (nh // nkv)]
+        if gates is not None:
+            g = torch.sigmoid(gates[at:at + n].double())
+            rows = rows * (g.view(n, nh, hd) if more["gate_channels"] else g[:, :, None])
+        outs.append(rows.view(n, nh * hd) * more["out_scale"])
+        at += n
+    return torch.cat(outs)
+
+
 @gpu
 @pytest.mark.parametrize("shape", _SHAPES)
 @pytest.mark.parametrize("hd,nh,nkv", [(128, 14, 2), (64, 3, 3)])
@@ -72,6 +109,10 @@ def test_shaped_scores_equal_the_other_kernels(shape, hd, nh, nkv, splits):
         assert int(status.item()) == 0
         assert bool((out[0] == 7.0).all())
         outs.append(out[1:].float())
+    want = _exact(q, k, v, table, spans, nh, hd, mask, size, keep, sink, more, gates, page)
+    was, err = (float((o.double() - want).norm() / want.norm()) for o in outs)
+    # one rounding to bfloat16 (2^-9 at most, a third of that in the mean) on top of both, and sixteen-bit weights
+    assert err <= max(1.1 * was, 2.0 ** -9), (err, was)
     # the same scores and sixteen-bit weights: what remains is the order of the sums and the one rounding to bfloat16
     assert float((outs[1] - outs[0]).abs().max()) <= 2.0 ** -7 * float(outs[0].abs().max())
     assert float((outs[1] - outs[0]).norm()) <= 2e-3 * float(outs[0].norm())
