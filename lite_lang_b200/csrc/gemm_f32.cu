@@ -30,7 +30,8 @@
 // Gated: the even CTA's rows of W are gate rows and the odd one's the up rows of the same features (act(gate) * up
 // leaves; one part).
 //
-// Every mbarrier wait is bounded and records LL_ERR_WAIT_TIMEOUT; the kernel then runs to its end and frees its memory.
+// Every mbarrier wait is bounded and records LL_ERR_WAIT_TIMEOUT in the status word that the call was given (a model's step
+// gives its own); the kernel then runs to its end with a wrong output and frees its memory.
 #include <cuda.h>
 
 #include "mma_split.cuh"
