@@ -27,6 +27,8 @@
 //
 // Taken for longer portions, key heads of 64 or 128 channels and value heads of a multiple of 64 (delta rule: 64 or 128,
 // one decay a head): see `ops.chunked_scan`.
+#include <atomic>
+
 #include "mma_split.cuh"
 
 #define CS_C 64
@@ -843,13 +845,24 @@ delta_walk_kernel(float* __restrict__ u, const float* __restrict__ w, const floa
   }
 }
 
+// lets KERNEL have `bytes` of dynamic shared memory: asked for once a device (the call takes the host about as long as a launch)
+template <auto KERNEL> static cudaError_t cs_room(size_t bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int device = 0;
+  cudaError_t rc = cudaGetDevice(&device);
+  if (rc != cudaSuccess || (device < 64 && ((done.load() >> device) & 1))) return rc;
+  rc = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (rc == cudaSuccess && device < 64) done.fetch_or(1ull << device);
+  return rc;
+}
+
 template <typename T, int DK>
 static int cs_read(const CsRows<T>& in, const int* cu_q, const int* req_slot, int E, int num_slots, const float* s0,
                    float* o, int H, int dv, int items, cudaStream_t stream) {
   constexpr int NPL = sizeof(T) == 2 ? 1 : 3;
   constexpr int KROWS = NPL * (DK + 8) > 3 * 72 ? NPL * (DK + 8) : 3 * 72;
   const size_t smem = 2 * (size_t)CS_C * ((NPL + 3) * (DK + 8) + KROWS + NPL * 72);
-  const cudaError_t rc = cudaFuncSetAttribute(chunk_read_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t rc = cs_room<chunk_read_kernel<T, DK>>(smem);
   if (rc != cudaSuccess) return (int)rc;
   ll_launch(chunk_read_kernel<T, DK>, dim3(items, H), dim3(CS_THREADS), smem, stream, in, cu_q, req_slot, E, num_slots, s0, o,
             H, dv);
@@ -862,7 +875,7 @@ static int cs_decay(const CsRows<T>& in, float* state, long slot_stride, int num
                     int items, cudaStream_t stream) {
   constexpr int NPL = sizeof(T) == 2 ? 1 : 3;
   const size_t smem = 2 * (size_t)CS_C * (NPL * (DK + 8) + 3 * 72);
-  const cudaError_t rc = cudaFuncSetAttribute(chunk_write_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t rc = cs_room<chunk_write_kernel<T, DK>>(smem);
   if (rc != cudaSuccess) return (int)rc;
   ll_launch(chunk_write_kernel<T, DK>, dim3(items, H, dv / 64), dim3(CS_THREADS), smem, stream, in, cu_q, req_slot, E,
             num_slots, ds, gam, H, dv);
@@ -902,9 +915,9 @@ static int cs_delta(const float* qn, const float* kn, const float* vc, const flo
                     float* s0, float* u, float* w, float* suf, float* gam, int items, cudaStream_t stream) {
   const size_t solve = 2 * (size_t)3 * CS_C * (DK + 8) + 4 * CS_C * CS_C;
   const size_t walk = 4 * (size_t)(4 * CS_C * (DK + 4) + 8 * 16 * (CS_C + 4)) + 2 * 3 * 16 * (CS_C + 8);
-  cudaError_t rc = cudaFuncSetAttribute(delta_solve_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve);
+  cudaError_t rc = cs_room<delta_solve_kernel<DK, DV>>(solve);
   if (rc != cudaSuccess) return (int)rc;
-  rc = cudaFuncSetAttribute(delta_walk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
+  rc = cs_room<delta_walk_kernel<DK>>(walk);
   if (rc != cudaSuccess) return (int)rc;
   ll_launch(delta_solve_kernel<DK, DV>, dim3(items, H), dim3(DK + DV), solve, stream, kn, vc, beta, g, cu_q, req_slot, E, u,
             w, suf, gam, H, Hk);
