@@ -1369,27 +1369,29 @@ def delta_prepare(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b_off:
 
 CHUNK = 64                 # tokens of a chunk (csrc/chunk_scan.cu)
 # Tokens of a portion, on average, from which on it is scanned by chunks, for one portion with 12 heads of 128 x 128; for
-# other steps `decay_chunked_min` and `delta_chunked_min`.  The walk's time is its tokens times what a token takes, which
-# grows with the heads of all entries once they outnumber the SMs; the chunks' three launches take as long as the host
-# needs for them (26 us; the kernels 17) or, as a delta rule, 42 us and more.  Measured on a B200 with the launches (us, walk / chunks):
-#   decay scan, heads of 128: 2 heads x 160 tokens 23 / 27, x 192 28 / 26; 12 x 128 26 / 26; 28 x 96 26 / 26; 64 x 64 31 / 27;
-#     4 portions: 8 heads x 96 28 / 27; 2,048 tokens of 12 heads 320 / 53
-#   delta rule:  2 heads x 128 41 / 43, x 160 51 / 46; 8 x 96 43 / 45; 12 x 96 44 / 41; 28 x 64 54 / 48; heads of 64, 12 x 64
-#     22 / 30, x 128 40 / 33; 2,048 tokens of 12 heads of 128 872 / 185
-DECAY_CHUNKED_MIN = 128
-DELTA_CHUNKED_MIN = 96
+# other steps `decay_chunked_min` and `delta_chunked_min`.  The kernels alone are ahead sooner (one portion of 12 heads,
+# walk / chunks, us: decay scan 128 tokens 23 / 19, 512 82 / 21; delta rule 96 43 / 40, 512 216 / 64), but three launches
+# take the host 9 us longer than one (13 with a delta rule), and while a layer's kernels take less than its launches the walk's
+# time does not show.  So the lines lie where whole calls of a layer with its products are equal.  Measured on a B200 (walk /
+# chunks, us; portions x heads):
+#   linear attention  12 heads: 1 x 256 tokens 80 / 89, x 384 90 / 89, x 512 114 / 90; 2 x 192 81 / 90, x 256 92 / 90; 4 x 128
+#     87 / 95, x 160 105 / 91; 28 heads: 1 x 128 85 / 94, x 160 92 / 92, x 192 101 / 91; 4 x 48 99 / 91
+#   delta rule        12 heads: 1 x 192 105 / 117, x 256 140 / 117; 2 x 96 105 / 117, x 128 130 / 118; 4 x 48 105 / 117, x 64
+#     124 / 118; 28 heads: 1 x 96 116 / 120, x 128 143 / 119; 2 x 48 118 / 120, x 64 143 / 120; 4 x 48 193 / 135
+#   2,048 tokens of 12 heads, the kernels alone: decay scan 320 / 53, delta rule 872 / 185
+DECAY_CHUNKED_MIN = 275
+DELTA_CHUNKED_MIN = 178
 
 
 def decay_chunked_min(heads: int, dk: int, dv: int) -> float:
     """``heads``: of all entries together.  A token's time in the walk: 0.11 us and 0.006 for each state of 128 x 128."""
-    states = heads * dk * dv / 16384
-    return DECAY_CHUNKED_MIN * (0.11 + 0.006 * 12) / (0.11 + 0.006 * states)
+    return DECAY_CHUNKED_MIN * 0.182 / (0.11 + 0.006 / 16384 * heads * dk * dv)
 
 
 def delta_chunked_min(heads: int, dk: int, dv: int) -> float:
-    """As above: 0.33 us a token and 0.012 for each state of 128 x 128 against 30 us and 15.5 for states of that size."""
-    size = dk * dv / 16384
-    return DELTA_CHUNKED_MIN * (30 + 15.5 * size) / 45.5 * (0.33 + 0.012 * 12) / (0.33 + 0.012 * heads * size)
+    """As above; a token's time: 0.32 us and 0.012 a state, from as many as there are SMs for on 0.2 and 0.0235."""
+    states = heads * dk * dv / 16384
+    return DELTA_CHUNKED_MIN * 0.482 / max(0.32 + 0.012 * states, 0.2 + 0.0235 * states)
 
 
 def chunked_scan(step, tokens: int, dk: int, dv: int, least: float) -> Optional[Tuple[int, int, int]]:

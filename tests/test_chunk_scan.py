@@ -32,11 +32,11 @@ def test_which_portions_go_by_chunks():
 def test_the_lines_move_with_the_heads():
     """Tokens a portion from which on the chunks were measured ahead (see ops.py): more for few heads, fewer for many."""
     from lite_lang_b200 import ops
-    for heads, low, high in ((2, 160, 224), (8, 128, 192), (12, 127, 129), (28, 64, 112), (64, 32, 64)):
+    for heads, low, high in ((2, 350, 450), (12, 256, 384), (24, 192, 256), (28, 160, 192), (48, 120, 160), (112, 32, 80)):
         assert low <= ops.decay_chunked_min(heads, 128, 128) <= high
-    for heads, low, high in ((2, 112, 160), (8, 96, 128), (12, 95, 97), (28, 48, 96), (64, 32, 64)):
+    for heads, low, high in ((2, 200, 260), (12, 160, 256), (24, 96, 128), (28, 96, 128), (48, 56, 80), (112, 16, 48)):
         assert low <= ops.delta_chunked_min(heads, 128, 128) <= high
-    assert 64 < ops.delta_chunked_min(12, 64, 64) < 128
+    assert ops.decay_chunked_min(12, 128, 128) == ops.decay_chunked_min(48, 64, 64)
 
 
 # lengths at the edges of a chunk, several entries, single tokens in front that stay with the walk, many chunks with a ragged
