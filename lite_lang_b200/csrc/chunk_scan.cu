@@ -408,8 +408,9 @@ chunk_prefix_kernel(float* __restrict__ ds, const float* __restrict__ gam, float
 // The read-outs: o_t = G(t, -) S0^T q_t + sum over s <= t of G(t, s) (q_t . k_s) scale_s v_s (+ skip_h v_t).
 // Tokens are the M side (16 of the chunk's 64 a warp).  The scores of a row are made by two warps, half of the keys each,
 // and go through shared memory (in k's place) as the second product's operand, so they are made once for all value
-// columns; the columns come 64 at a time, 32 a warp, the next 64's state and values on their way meanwhile.  Bound by
-// the tensor cores' rate for mma.sync where q is float32 (six products a term of S0^T q_t), by loads otherwise.
+// columns; the columns come 64 at a time, 32 a warp, the next 64's state and values on their way meanwhile.  One CTA an
+// SM (registers, shared memory): two warps a scheduler, bound by the latencies of their own instructions (tensor pipe 30 % active where
+// q is float32, with six products a term of S0^T q_t, 18 % otherwise).
 // ---------------------------------------------------------------------------------------------------------------
 template <typename T, int DK>
 __global__ void __launch_bounds__(CS_THREADS)
