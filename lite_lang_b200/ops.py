@@ -13,8 +13,8 @@ float32 path TF32 is switched off so that it is a true 32-bit product.
 
 from __future__ import annotations
 
-import contextlib
 import ctypes
+import functools
 import os
 import threading
 from ctypes import c_float, c_int, c_long, c_void_p
@@ -1103,14 +1103,17 @@ F32_MIN_WORK = 1 << 28
 
 def f32_supported(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
     """Whether ``gemm_f32`` takes this float32 product and is meant for it."""
-    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and TC_ENABLED and x.is_cuda and x.dim() == 2
-            and weight.dim() == 2 and x.shape[0] >= F32_MIN_M and x.shape[1] % 8 == 0 and weight.shape[0] % 4 == 0
-            and weight.shape[0] >= 64 and x.stride(1) == 1 and weight.stride(1) == 1 and x.stride(0) % 4 == 0
-            and x.shape[0] * x.shape[1] * weight.shape[0] >= F32_MIN_WORK
-            and weight.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-            and f32_preferred(x.shape[0], weight.shape[0], x.shape[1], sm_count(x.device), gated))
+    if x.dtype != torch.float32 or x.dim() != 2 or weight.dim() != 2:
+        return False
+    (m, k), n = x.shape, weight.shape[0]      # (first what most products of a decode step or a small model fail)
+    if m < F32_MIN_M or m * k * n < F32_MIN_WORK or k % 8 or n % 4 or n < 64 or not (TC_ENABLED and x.is_cuda):
+        return False
+    return (f32_preferred(m, n, k, sm_count(x.device), gated) and weight.dtype == torch.float32 and x.stride(1) == 1
+            and weight.stride(1) == 1 and x.stride(0) % 4 == 0 and weight.stride(0) % 4 == 0
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
+@functools.lru_cache(maxsize=1024)
 def f32_preferred(m: int, n: int, k: int, sms: int, gated: bool = False) -> bool:
     """Whether ``gemm_f32`` is expected to be faster than the library.  A step of 64 numbers of k takes a pair of SMs 3.1 us
     and a tile's end 4, however many of the tile's 256 rows and columns are there, and tiles are handed out in rounds; the
@@ -1140,16 +1143,21 @@ def f32_splits(m: int, n: int, k: int, device) -> int:
 _reporting = threading.local()
 
 
-@contextlib.contextmanager
-def reporting_to(status: Optional[torch.Tensor]):
+class reporting_to:
     """Inside the block, products of this thread that are given no status word report to ``status``: a model's parts call
     ``linear`` without one."""
-    before = getattr(_reporting, "status", None)
-    _reporting.status = status
-    try:
-        yield
-    finally:
-        _reporting.status = before
+
+    __slots__ = ("status", "before")
+
+    def __init__(self, status: Optional[torch.Tensor]):
+        self.status = status
+
+    def __enter__(self):
+        self.before = getattr(_reporting, "status", None)
+        _reporting.status = self.status
+
+    def __exit__(self, *exc):
+        _reporting.status = self.before
 
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
@@ -1278,11 +1286,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
             out = torch.empty((x.shape[0], weight.shape[0]), dtype=dt, device=x.device)
         if out.dtype == dt:
             return gemm_smallm(x, weight, out)
-    if x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
-        raise RuntimeError("TF32 is on; call ops.configure_matmul_precision() before a float32 product")
-    if (out_dtype in (None, torch.float32) and f32_supported(x, weight)
-            and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0))):
-        return gemm_f32(x, weight, out, partial_ok=partial_ok)
+    if x.dtype == torch.float32:
+        if torch.backends.cuda.matmul.allow_tf32:
+            raise RuntimeError("TF32 is on; call ops.configure_matmul_precision() before a float32 product")
+        if (out_dtype in (None, torch.float32) and f32_supported(x, weight)
+                and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0
+                                     and out.data_ptr() % 16 == 0))):
+            return gemm_f32(x, weight, out, partial_ok=partial_ok)
     if out_dtype is not None and out_dtype != x.dtype:
         res = torch.mm(x, weight.t(), out_dtype=out_dtype)
         if out is not None:
@@ -1409,8 +1419,9 @@ def chunked_scan(step, tokens: int, dk: int, dv: int, least: float) -> Optional[
     return single, rest, (tokens - single) // CHUNK + rest
 
 
-def _portions(step) -> int:
-    return int(step.num_entries) - int(getattr(step, "num_single", 0) or 0)
+def _cut(step, tokens: int, heads: int, dk: int, dv: int, minimum) -> Optional[Tuple[int, int, int]]:
+    rest = step.num_entries - (getattr(step, "num_single", 0) or 0)
+    return chunked_scan(step, tokens, dk, dv, minimum(heads * rest, dk, dv)) if rest > 0 else None
 
 
 def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, cut) -> None:
@@ -1435,9 +1446,10 @@ def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta:
     _need_cuda(qn, kn, vc, beta, g, state, o)
     _need(dk <= 256, f"delta rule: key heads of {dk} channels are wider than the scan kernel takes (256)")
     entries = step.num_entries
-    if not per_channel and dv <= 128 and state.stride(0) % 4 == 0 and all(t.data_ptr() % 16 == 0 for t in (qn, kn, vc, state, o)):
-        cut = chunked_scan(step, qn.shape[0], dk, dv, delta_chunked_min(H * _portions(step), dk, dv))
-        if cut is not None:
+    if not per_channel and dv <= 128:
+        cut = _cut(step, qn.shape[0], H, dk, dv, delta_chunked_min)
+        if cut is not None and state.stride(0) % 4 == 0 and (
+                qn.data_ptr() | kn.data_ptr() | vc.data_ptr() | state.data_ptr() | o.data_ptr()) % 16 == 0:
             _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H, Hk, dk, dv, cut)
             entries = cut[0]
     if entries == 0:
@@ -1867,10 +1879,9 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay: Op
           and o.shape[1] == H * dv and o.is_contiguous() and H % heads_per_group == 0,
           "decay_scan: shapes (key heads of at most 256 channels)")
     entries, size = step.num_entries, proj.element_size()
-    if (proj.stride(0) * size % 16 == 0 and all(x * size % 16 == 0 for x in (q_off, k_off, v_off))
-            and all(t_.data_ptr() % 16 == 0 for t_ in (proj, o))):
-        cut = chunked_scan(step, proj.shape[0], dk, dv, decay_chunked_min(H * _portions(step), dk, dv))
-        if cut is not None:
+    cut = _cut(step, proj.shape[0], H, dk, dv, decay_chunked_min)
+    if cut is not None:
+        if (proj.stride(0) | q_off | k_off | v_off) * size % 16 == 0 and (proj.data_ptr() | o.data_ptr()) % 16 == 0:
             single, rest, items = cut
             ds = torch.empty(items * H * (dv * dk + 1), dtype=torch.float32, device=proj.device)     # states, chunks' decays
             load_library("chunk_scan").call(

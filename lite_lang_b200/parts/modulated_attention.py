@@ -383,17 +383,18 @@ class ModulatedAttention(Mixer):
     TC_MIN_KEYS = 32
     TC_MIN_KEYS_BIAS = 128
 
-    def _shaped_plan(self, step, n_single: int, group: int, device):
-        """The plan of the step's portions for the tcgen05 kernel; None where it is not meant for them."""
+    def _shaped_plan(self, step, n_single: int, q, page_size: int, group: int):
+        """The plan of the step's portions for the tcgen05 kernel; None where it does not take them or is not meant for them."""
         key = ("attn_prefill_tc_shaped", group, self.num_kv_heads, self.mask, self.mask_size, self.keep_first,
-               self.bias_by_distance is None)
+               self.bias_by_distance is None, self.key_dim, q.stride(0))
         plan = step.scratch.get(key, 0)
         if plan == 0:
             spans = [(c, len(e.tokens)) for c, e in zip(step.entry_ctx[n_single:], step.entries[n_single:])]
             plan = step.scratch[key] = ops.attn_prefill_tc_plan(
-                spans, group, self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(device),
+                spans, group, self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(q.device),
                 self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0
-            ) if self._tc_preferred(spans, group) else None
+            ) if (ops.attn_prefill_tc_supported(q.dtype, self.key_dim, page_size, q.stride(0), group)
+                  and self._tc_preferred(spans, group)) else None
         return plan
 
     def _tc_preferred(self, spans, group: int) -> bool:
@@ -466,9 +467,8 @@ class ModulatedAttention(Mixer):
                                 nsplit=plan[1], split_len=plan[2], gate=gate, pairs=self.pairs)
         elif (n_rest > 0 and mixed_q is None and temperature is None and self.vdim == self.key_dim and self.pairs is None
                 and ops.TC_ENABLED and getattr(step, "entry_ctx", None) is not None
-                and ops.attn_prefill_tc_supported(q.dtype, self.key_dim, cache.page_size, q.stride(0), group)
-                and (gate is None or not self.channel_gate or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))
-                and (plan := self._shaped_plan(step, n_single, group, proj.device))):
+                and (plan := self._shaped_plan(step, n_single, q, cache.page_size, group))
+                and (gate is None or not self.channel_gate or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))):
             # shaped scores on the same kernel: the row's thread makes them between product and softmax
             del more["pairs"]
             ops.attn_prefill_tc_shaped(out, q, q.stride(0), gate, cache.k, cache.v, cache.block_table, step.cu_q[n_single:],
