@@ -21,8 +21,8 @@
 //                     where all (token, head) rows of a block of queries meet the same run of cached rows:
 //                     the run is copied out of its pages, scores = Q K^T and sum = P C are products, and the
 //                     masked softmax between them is the kernel here
-// In latent_attention keys are walked in tiles of 32 positions that start at multiples of 32, so the order of
-// every sum depends on the position only, not on how the tokens were cut into steps or batched.
+// In latent_attention keys are walked in tiles of 32 positions (64 on tensor cores) that start at multiples of it, so the order of
+// every sum depends on the position (and on how many CTAs share a query's keys), not on how the tokens were cut into steps.
 #include "common.cuh"
 
 #define LA_LATENT_PIECES 4        // latents of up to 512 numbers: 4 a thread
@@ -588,8 +588,7 @@ extern "C" int ll_latent_attention_mma_ok(int R, int r);
 extern "C" int ll_latent_attention_mma(void* out, const void* q, const void* cache, const int* block_table, int bt_stride,
                                        const int* token_req, const int* req_slot, const int* positions, int first,
                                        int num_tokens, int H, int R, int r, int page_size, int num_pages, int window,
-                                       float scale, int* status, int nsplit, int tiles_per_split, float* part_acc,
-                                       float* part_ml, const float* sink, cudaStream_t stream);
+                                       float scale, int* status, int nsplit, const float* sink, cudaStream_t stream);
 static bool la_mma_enabled() {
   static int v = -1;
   if (v < 0) {
@@ -610,19 +609,14 @@ extern "C" int ll_latent_attention(int dtype, void* out, const void* q, const vo
                                    float* part_acc, float* part_ml, const float* sink, cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || R <= 0 || R > LA_MAX_R || r < 0 || page_size <= 0 || nsplit < 1) return (int)cudaErrorInvalidValue;
-  if (nsplit > 32 || (nsplit > 1 && (tiles_per_split < 1 || part_acc == nullptr || part_ml == nullptr)))
-    return (int)cudaErrorInvalidValue;
+  if (nsplit > 32 || (nsplit > 1 && tiles_per_split < 1)) return (int)cudaErrorInvalidValue;
   const int KD = R + r;
-  if (ll_latent_attention_heads(dtype, R, r) == 16 && ((uintptr_t)cache % 16) == 0 && ((uintptr_t)q % 16) == 0) {
-    const int rc = ll_latent_attention_mma(out, q, cache, block_table, bt_stride, token_req, req_slot, positions, first,
-                                           num_tokens, H, R, r, page_size, num_pages, window, scale, status, nsplit,
-                                           tiles_per_split, part_acc, part_ml, sink, stream);
-    if (rc != 0 || nsplit == 1) return rc;
-    const int pairs = num_tokens * H;
-    ll_launch(latent_merge_kernel<bf16>, dim3(pairs), dim3(128), 0, stream, (bf16*)out + (size_t)first * H * R,
-              (const float*)part_acc, (const float*)part_ml, pairs, R, nsplit, sink, H);
-    return LL_LAUNCH_RESULT();
-  }
+  // (its parts meet in a cluster's shared memory, without the buffers for them)
+  if (ll_latent_attention_heads(dtype, R, r) == 16 && ((uintptr_t)cache % 16) == 0 && ((uintptr_t)q % 16) == 0 &&
+      ((uintptr_t)out % 8) == 0)
+    return ll_latent_attention_mma(out, q, cache, block_table, bt_stride, token_req, req_slot, positions, first, num_tokens, H,
+                                   R, r, page_size, num_pages, window, scale, status, nsplit, sink, stream);
+  if (nsplit > 1 && (part_acc == nullptr || part_ml == nullptr)) return (int)cudaErrorInvalidValue;
   const size_t smem = sizeof(float) * ((size_t)LA_GH * KD + (size_t)LA_TK * la_pitch(KD) + LA_GH * LA_TK + 2 * LA_GH);
   dim3 grid(num_tokens, (H + LA_GH - 1) / LA_GH, nsplit);
   LL_DISPATCH_DTYPE(dtype, {

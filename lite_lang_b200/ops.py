@@ -1537,9 +1537,10 @@ def latent_attention(out: torch.Tensor, q_full: torch.Tensor, cache: torch.Tenso
                      sink: Optional[torch.Tensor] = None) -> None:
     """Attention in the latent space for tokens ``first .. first + count - 1`` of the step.  ``q_full``
     [tokens, H, R + r] and ``out`` [tokens, H, R] (sum_j p_j c_j per head) have the cache's dtype.
-    ``nsplit`` > 1: every query's keys are shared out over that many CTAs, ``tiles_per_split`` tiles of 32
-    positions each (counted from the query's first visible tile; together they must cover the longest run of
-    keys a query of the step sees), and merged by a second kernel.  ``sink`` float32 [H]: every head's softmax
+    ``nsplit`` > 1: every query's keys are shared out over that many CTAs.  On tensor cores (``latent_attention_heads`` 16)
+    these are a cluster of at most 16, each with an equal part of the query's own tiles of 64 positions; else each has
+    ``tiles_per_split`` tiles (counted from the query's first visible tile; together they must cover the longest run of
+    keys a query of the step sees), merged by a second kernel.  ``sink`` float32 [H]: every head's softmax
     has one more key of that score, which carries no value."""
     _need_cuda(out, q_full, cache, block_table, sink)
     _f32(sink, "sink")
@@ -1549,8 +1550,9 @@ def latent_attention(out: torch.Tensor, q_full: torch.Tensor, cache: torch.Tenso
     _need(R <= 512, f"latent_attention: a latent of {R} numbers is wider than the kernel takes (512)")
     _need(0 <= first and first + count <= q_full.shape[0], "latent_attention: token range")
     part_acc = part_ml = None
-    if nsplit > 1:
-        _need(tiles_per_split >= 1, "latent_attention: splits need tiles_per_split")
+    _need(nsplit == 1 or tiles_per_split >= 1, "latent_attention: splits need tiles_per_split")
+    if nsplit > 1 and (latent_attention_heads(out.dtype, R, r) != 16 or q_full.data_ptr() % 16 or cache.data_ptr() % 16
+                       or out.data_ptr() % 8):
         part_acc = torch.empty((count, H, nsplit, R), dtype=torch.float32, device=out.device)
         part_ml = torch.empty((count, H, nsplit, 2), dtype=torch.float32, device=out.device)
     load_library("latent_attn").call(
@@ -1561,12 +1563,23 @@ def latent_attention(out: torch.Tensor, q_full: torch.Tensor, cache: torch.Tenso
         _ptr(sink), _stream())
 
 
+@functools.lru_cache(maxsize=256)
 def latent_attention_heads(dtype: torch.dtype, R: int, r: int) -> int:
     """Heads a CTA of ``latent_attention`` takes for these sizes (16 on tensor cores: bfloat16, R + r a multiple of
     16, R a multiple of 32; else 8): what a plan of the parts counts its CTAs with."""
     if dtype not in _DT:
         return 8
     return int(load_library("latent_attn").fn("ll_latent_attention_heads")(c_int(_DT[dtype]), c_int(R), c_int(r)))
+
+
+@functools.lru_cache(maxsize=4096)
+def latent_attention_splits(pairs: int, longest: int) -> int:
+    """CTAs that share the keys of each of ``pairs`` (query, group of 16 heads) on tensor cores, for runs of up to ``longest``
+    keys: the largest cluster (16 at most) that lets all of them run at once, since a CTA takes an SM and a second round
+    of clusters doubles the time.  Measured on a B200 (12 heads, a latent of 512, context 2,048; us):
+    16 tokens with 4, 6 and 8 CTAs 21.6, 17.0 and 25.2, 64 tokens with 1, 2 and 4 60.0, 37.1 and 43.0; one token with 8, 10
+    and 16 14.2, 12.6 and 13.6."""
+    return int(load_library("latent_attn").fn("ll_latent_attention_mma_splits")(c_int(pairs), c_int((longest + 63) // 64 + 1)))
 
 
 def latent_gather(dst: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, slot: int, lo: int, page_size: int,
