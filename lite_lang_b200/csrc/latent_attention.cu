@@ -26,6 +26,7 @@
 #include "common.cuh"
 
 #define LA_LATENT_PIECES 4        // latents of up to 512 numbers: 4 a thread
+#define LA_CQ_PIECES 12           // the queries' latents: 1,536 numbers in registers, the rest read twice
 
 // the r numbers at src turned into dst (dst may be src): pairs below `half` by their angle (cs, sn), the rest as they are.
 // Called with consecutive `first` of a group of `step` threads.
@@ -46,19 +47,44 @@ __device__ __forceinline__ void la_turn(T* dst, const T* src, int first, int ste
 // through a latent of their own): q heads at q_off, head h's rotated part at q_off + h * (d + r) + d; proj row t:
 // the latent at kv_off (R wide), then the rotated key part (r wide).  Both cos and sin are multiplied by
 // `amplitude` (a scaled rotation's factor; 1 otherwise).  Tokens from `inplace_from` on have their rotated query parts
-// turned where they lie instead of into q_full.
+// turned where they lie instead of into q_full; turn_q = 0: nobody's are.  With cq a second block a token makes the norm of the
+// row's first cq_width numbers, the latent that the queries come from: both norms wait for the same product, and a norm alone
+// was a launch of 2.8 us in a chain of nine (16 tokens).
 template <typename T>
 __global__ void __launch_bounds__(128)
 latent_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, int kv_off, const float* __restrict__ norm_w,
                       float eps, const float* __restrict__ freq, int rot_dims, const int* __restrict__ positions,
                       const int* __restrict__ slot_map, T* __restrict__ cache, long num_slots,
                       T* __restrict__ q_full, int H, int d, int r, int R, int* status, float amplitude,
-                      T* qsrc, long q_stride, int half_split, int inplace_from) {
+                      T* qsrc, long q_stride, int half_split, int inplace_from, int turn_q, T* __restrict__ cq,
+                      const float* __restrict__ cq_w, int cq_width) {
   extern __shared__ float la_cs[];      // cos [half], sin [half]
   __shared__ float scratch[32];
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int t = blockIdx.x, tid = threadIdx.x;
+  if (blockIdx.y == 1) {      // the queries' own latent
+    const T* src = proj + (size_t)t * proj_stride;
+    T* dst = cq + (size_t)t * cq_width;
+    float x[LA_CQ_PIECES];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < LA_CQ_PIECES; ++k) {
+      const int i = tid + 128 * k;
+      x[k] = i < cq_width ? to_f32<T>(src[i]) : 0.f;
+      ss = fmaf(x[k], x[k], ss);
+    }
+    for (int i = tid + 128 * LA_CQ_PIECES; i < cq_width; i += 128) ss = fmaf(to_f32<T>(src[i]), to_f32<T>(src[i]), ss);
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)cq_width + eps);
+#pragma unroll
+    for (int k = 0; k < LA_CQ_PIECES; ++k) {
+      const int i = tid + 128 * k;
+      if (i < cq_width) dst[i] = from_f32<T>(x[k] * inv * cq_w[i]);
+    }
+    for (int i = tid + 128 * LA_CQ_PIECES; i < cq_width; i += 128) dst[i] = from_f32<T>(to_f32<T>(src[i]) * inv * cq_w[i]);
+    return;
+  }
   const float p = (float)positions[t];
   const int half = rot_dims / 2;
   float* la_sn = la_cs + half;
@@ -85,7 +111,7 @@ latent_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, i
   }
   __syncthreads();
   // every head's rotated query part: a group of 16 threads a head
-  if (r > 0) {
+  if (r > 0 && turn_q) {
     T* qrow = qsrc + (size_t)t * q_stride + q_off + d;
     for (int h = tid >> 4; h < H; h += 8) {
       T* src = qrow + (size_t)h * (d + r);
@@ -515,13 +541,15 @@ extern "C" int ll_latent_prepare(int dtype, const void* proj, long proj_stride, 
                                  const float* norm_w, float eps, const float* freq, int rot_dims, const int* positions,
                                  const int* slot_map, void* cache, long num_slots, void* q_full, int num_tokens, int H,
                                  int d, int r, int R, int* status, float amplitude, void* qsrc, long q_stride,
-                                 int half_split, int inplace_from, cudaStream_t stream) {
+                                 int half_split, int inplace_from, int turn_q, void* cq, const float* cq_w, int cq_width,
+                                 cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
-  if (H <= 0 || d < 0 || r < 0 || R <= 0 || rot_dims < 0 || rot_dims > r) return (int)cudaErrorInvalidValue;
-  LL_DISPATCH_DTYPE(dtype, ll_launch(latent_prepare_kernel<T>, dim3(num_tokens), dim3(128), (size_t)(rot_dims / 2) * 8, stream, (const T*)proj,
+  if (H <= 0 || d < 0 || r < 0 || R <= 0 || rot_dims < 0 || rot_dims > r || (cq != nullptr && (cq_w == nullptr || cq_width <= 0)))
+    return (int)cudaErrorInvalidValue;
+  LL_DISPATCH_DTYPE(dtype, ll_launch(latent_prepare_kernel<T>, dim3(num_tokens, cq != nullptr ? 2 : 1), dim3(128), (size_t)(rot_dims / 2) * 8, stream, (const T*)proj,
                                      proj_stride, q_off, kv_off, norm_w, eps, freq, rot_dims, positions, slot_map,
                                      (T*)cache, num_slots, (T*)q_full, H, d, r, R, status, amplitude,
-                                     (T*)qsrc, q_stride, half_split, inplace_from));
+                                     (T*)qsrc, q_stride, half_split, inplace_from, turn_q, (T*)cq, cq_w, cq_width));
   return LL_LAUNCH_RESULT();
 }
 

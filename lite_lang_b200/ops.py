@@ -1479,17 +1479,22 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Te
                    rot_dims: int, positions: torch.Tensor, slot_map: Optional[torch.Tensor], cache: torch.Tensor,
                    q_full: torch.Tensor, H: int, d: int, r: int, R: int, status: Optional[torch.Tensor],
                    amplitude: float = 1.0, q: Optional[torch.Tensor] = None, half_split: bool = False,
-                   inplace_from: Optional[int] = None) -> None:
+                   inplace_from: Optional[int] = None, turn_q: bool = True, cq: Optional[torch.Tensor] = None,
+                   cq_norm: Optional[torch.Tensor] = None) -> None:
     """Per token: the latent's RMS norm and the rotated key part into the cache row, and every head's rotated
     query part into ``q_full`` [tokens, H, R + r] behind the R latent-space numbers (which a product fills).
     ``q``: the rows that hold the query heads at ``q_off`` when they are not rows of ``proj`` (queries made by a
     second product); ``amplitude``: a factor on cos and sin; ``half_split``: pairs (i, i + rot_dims / 2) instead of
     neighbours.  ``inplace_from``: tokens from there on have their rotated query parts turned where they lie (``q_full``
-    holds the tokens before)."""
+    holds the tokens before).  ``turn_q=False``: the queries are left alone.  ``cq`` [tokens, width] with ``cq_norm``: the RMS
+    norm of the first ``width`` numbers of ``proj``'s rows (the queries' own latent), beside the rest."""
     n = proj.shape[0]
     first = n if inplace_from is None else int(inplace_from)
-    _need_cuda(proj, norm_w, freq, positions, slot_map, cache, q_full, q)
+    _need_cuda(proj, norm_w, freq, positions, slot_map, cache, q_full, q, cq, cq_norm)
     q = proj if q is None else q
+    _f32(cq_norm, "cq_norm")
+    _need(cq is None or (cq_norm is not None and cq.is_contiguous() and cq.dtype == proj.dtype and cq.shape[0] == n
+                         and cq_norm.numel() == cq.shape[1] <= proj.shape[1]), "latent_prepare: cq")
     _need(q.dtype == proj.dtype and q.stride(1) == 1 and q.shape[0] == proj.shape[0], "latent_prepare: q rows")
     _f32(norm_w, "norm_w")
     _f32(freq, "freq")
@@ -1504,7 +1509,7 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Te
         _ptr(norm_w), c_float(eps), _ptr(freq), c_int(rot_dims), _ptr(positions), _ptr(slot_map), _ptr(cache),
         c_long(cache.shape[0] * cache.shape[2]), _ptr(q_full), c_int(proj.shape[0]), c_int(H), c_int(d), c_int(r),
         c_int(R), _ptr(status), c_float(amplitude), _ptr(q), c_long(q.stride(0)), c_int(1 if half_split else 0),
-        c_int(first), _stream())
+        c_int(first), c_int(1 if turn_q else 0), _ptr(cq), _ptr(cq_norm), c_int(0 if cq is None else cq.shape[1]), _stream())
 
 
 def latent_unpage(cache: torch.Tensor, block_table: torch.Tensor, cu_q: torch.Tensor, ctx_len: torch.Tensor,

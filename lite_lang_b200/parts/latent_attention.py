@@ -237,22 +237,32 @@ class LatentAttention(Mixer):
         ops.attn_prefill_tc_rows(heads, qrows, kv[:, :width], kv[:, width:], table, cu_q, rel, own, plan, self.H, self.dv,
                                  self.window, self.scale, self.sink_w, step.status)
 
+    def _prepare(self, proj, qrows, step, cache, q_full, front, cq=None) -> None:
+        """The new tokens' cache rows and the rotated parts of their queries (``q_full``, in place from token ``front`` on).
+        Queries with a latent of their own: the cache rows and that latent's norm ``cq`` first, the rotated parts in a call
+        after the second product."""
+        second = self.q_rank is not None and cq is None
+        ops.latent_prepare(proj, 0, self.kv_off, self.norm_w, self.eps, self.freq, self.rot_dims, step.positions,
+                           cache.slot_map if cache.writable and not second else None, cache.k, q_full, self.H, self.d, self.r,
+                           self.R, step.status, amplitude=self.amplitude, q=qrows, half_split=self.half_split,
+                           inplace_from=0 if cq is not None else front, turn_q=cq is None, cq=cq,
+                           cq_norm=None if cq is None else self.q_norm_w)
+
     def forward(self, x, step, cache):
         n, dev, H, d, r, R = x.shape[0], x.device, self.H, self.d, self.r, self.R
         proj = ops.linear(x, self.w_in)
         qrows = proj
-        if self.q_rank is not None:          # the queries' own latent: norm, then the second product
+        if self.q_rank is not None:          # the queries' own latent: norm (with the cache rows), then the second product
             cq = torch.empty((n, self.q_rank), dtype=x.dtype, device=dev)
-            ops.rmsnorm(cq, proj[:, :self.q_rank], self.q_norm_w, self.eps)
+            self._prepare(proj, proj, step, cache, proj.new_empty((0, H, R + r)), 0, cq)
             qrows = ops.linear(cq, self.w_uq)
         latent, groups = self._runs(step, qrows)
         # (tokens in front of the first expanded portion, the step's single tokens among them, have their rotated parts put
         # where the products over heads write; everybody else's are turned where they lie)
         na, front = (latent[-1][1], latent[0][1] if latent[0][0] == 0 else 0) if latent else (0, 0)
         q_full = torch.empty((na, H, R + r), dtype=x.dtype, device=dev)
-        ops.latent_prepare(proj, 0, self.kv_off, self.norm_w, self.eps, self.freq, self.rot_dims, step.positions,
-                           cache.slot_map if cache.writable else None, cache.k, q_full, H, d, r, R, step.status,
-                           amplitude=self.amplitude, q=qrows, half_split=self.half_split, inplace_from=front)
+        if self.q_rank is None or r:
+            self._prepare(proj, qrows, step, cache, q_full, front)
         heads = torch.empty((n, H * self.dv), dtype=x.dtype, device=dev)
         if latent:
             lat = torch.empty((na, H, R), dtype=x.dtype, device=dev)
