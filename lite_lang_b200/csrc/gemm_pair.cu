@@ -30,6 +30,12 @@
 //             (q|k|v mode: -> shared memory, then rows finished by consecutive threads); a warp reads the 32
 //             lanes that its number modulo 4 gives, so two warps share a token row and each takes half of the
 //             tile's columns (a pair with one tile has nothing to hide its epilogue behind).
+// The loops of warps 0 and 1 are run by the whole warp with one elected lane at the copies and MMAs, and count stages and
+// phases instead of dividing: see gp_elect.  Gated product of 2,048 tokens, 1,536 -> 2 x 8,960, back to back: 85.1 us (1,325
+// TFLOP/s) as one lane's loops with an exponential and division of their own an element in the epilogue, 83.0 with counted
+// stages, 75.0 with the activation chosen once a tile (it had made the epilogue longer than a tile's MMAs: 15,000 clocks
+// against 12,300), 70.5 (1,600) with whole warps: 519 clocks a stage, whose MMAs are 512.
+//
 // Tiles go to the pairs round-robin, tokens fastest, so the pairs that run together share weight rows in L2.
 //
 // Every mbarrier wait is bounded (about two seconds of clock): a wait that runs out records
@@ -38,12 +44,8 @@
 // LL_ERR_TMEM_PAIR and computes nothing.
 //
 // Needs K % 8 == 0 and 16-byte aligned rows; rows beyond M or N and k beyond K are zero-filled by TMA.
-#include <cuda.h>
+#include "tc05_pair.cuh"
 
-#include "common.cuh"
-
-#define LL_ERR_WAIT_TIMEOUT 5
-#define LL_ERR_TMEM_PAIR 7
 #define GP_THREADS 320
 #define GP_STAGES 6
 #define GP_A_BYTES (128 * 128)
@@ -52,119 +54,6 @@
 #define GP_MODE_GATED 1
 #define GP_MODE_QKV 2
 #define GP_SMEM (1024 + GP_STAGES * GP_STAGE_BYTES + (2 * GP_STAGES + 4) * 8 + 16)
-
-__device__ __forceinline__ unsigned gp_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void gp_mbar_init(unsigned bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void gp_mbar_expect_tx(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// arrive on a barrier of a CTA of the cluster (the address comes from gp_mapa)
-__device__ __forceinline__ void gp_mbar_arrive_cluster(unsigned bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-__device__ __forceinline__ bool gp_mbar_try(unsigned bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// `dead` is the calling thread's memory of a wait that ran out: after the first one it waits no more.
-__device__ __forceinline__ void gp_mbar_wait(unsigned bar, unsigned parity, int* status, bool& dead) {
-  if (dead || gp_mbar_try(bar, parity)) return;
-  const long long t0 = clock64();
-  while (!gp_mbar_try(bar, parity)) {
-    if (clock64() - t0 > 4000000000ll) {
-      set_status(status, LL_ERR_WAIT_TIMEOUT);
-      dead = true;
-      return;
-    }
-  }
-}
-__device__ __forceinline__ unsigned gp_cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void gp_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the address of this CTA's shared-memory location `addr` in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned gp_mapa(unsigned addr, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ unsigned gp_ld_cluster(unsigned addr_cluster) {
-  unsigned v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr_cluster) : "memory");
-  return v;
-}
-// TMA box into this CTA's shared memory; its bytes complete on a barrier that may be the pair's other CTA's
-__device__ __forceinline__ void gp_tma_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar_cluster) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(bar_cluster)
-      : "memory");
-}
-// Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with the 128-byte
-// swizzle (what TMA writes): groups of 8 rows are 1024 bytes apart; 16 elements of k are 32 bytes.
-__device__ __forceinline__ unsigned long long gp_desc(unsigned smem_addr) {
-  return (unsigned long long)((smem_addr >> 4) & 0x3FFF) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void gp_mma(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
-                                       unsigned idesc, unsigned accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrives on the barrier at this shared-memory offset in both CTAs of the pair when the MMAs issued so far are done
-__device__ __forceinline__ void gp_commit_pair(unsigned bar) {
-  const unsigned short mask = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-               "h"(mask)
-               : "memory");
-}
-__device__ __forceinline__ void gp_ld32_issue(unsigned taddr, unsigned (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-// (the registers are tied to the wait so that no use of them can be scheduled before it)
-__device__ __forceinline__ void gp_ld_wait(unsigned (&a)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]),
-                 "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]), "+r"(a[16]),
-                 "+r"(a[17]), "+r"(a[18]), "+r"(a[19]), "+r"(a[20]), "+r"(a[21]), "+r"(a[22]), "+r"(a[23]), "+r"(a[24]),
-                 "+r"(a[25]), "+r"(a[26]), "+r"(a[27]), "+r"(a[28]), "+r"(a[29]), "+r"(a[30]), "+r"(a[31])
-               :
-               : "memory");
-}
-__device__ __forceinline__ void gp_ld_wait2(unsigned (&a)[32], unsigned (&b)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]),
-                 "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]), "+r"(a[16]),
-                 "+r"(a[17]), "+r"(a[18]), "+r"(a[19]), "+r"(a[20]), "+r"(a[21]), "+r"(a[22]), "+r"(a[23]), "+r"(a[24]),
-                 "+r"(a[25]), "+r"(a[26]), "+r"(a[27]), "+r"(a[28]), "+r"(a[29]), "+r"(a[30]), "+r"(a[31]), "+r"(b[0]),
-                 "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]), "+r"(b[9]),
-                 "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15]), "+r"(b[16]), "+r"(b[17]),
-                 "+r"(b[18]), "+r"(b[19]), "+r"(b[20]), "+r"(b[21]), "+r"(b[22]), "+r"(b[23]), "+r"(b[24]), "+r"(b[25]),
-                 "+r"(b[26]), "+r"(b[27]), "+r"(b[28]), "+r"(b[29]), "+r"(b[30]), "+r"(b[31])
-               :
-               : "memory");
-}
 
 struct GpParams {
   bf16* out;
@@ -245,22 +134,6 @@ __device__ __forceinline__ void gp_stage32(unsigned char* stg, int row, int col0
     }
     *reinterpret_cast<uint4*>(stg + gp_stg_offset(row, (col0 >> 3) + q)) = pk;
   }
-}
-__device__ __forceinline__ void gp_unpack8(const uint4& a, float (&x)[8]) {
-  const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 f = __bfloat1622float2(a2[k]);
-    x[2 * k] = f.x;
-    x[2 * k + 1] = f.y;
-  }
-}
-__device__ __forceinline__ uint4 gp_pack8(const float (&x)[8]) {
-  uint4 o;
-  __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) o2[k] = __floats2bfloat162_rn(x[2 * k], x[2 * k + 1]);
-  return o;
 }
 // step 2 for the CTA's 128 rows.  A work item is 8 columns of the first half of a head and their 8 partners in
 // the second half; a row has 16 of them, and epilogue thread e (of 256) takes item e % 16 of the rows
@@ -385,7 +258,7 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
   const unsigned full0 = gp_smem(bars), empty0 = gp_smem(bars + GP_STAGES);
   const unsigned acc_full0 = gp_smem(bars + 2 * GP_STAGES), acc_empty0 = gp_smem(bars + 2 * GP_STAGES + 2);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const unsigned rank = gp_cluster_rank();   // 0: issues the MMAs and owns the `full` and `acc_empty` barriers
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;   // the pair is a cluster of two along x
   if (tid == 32) {
@@ -423,48 +296,60 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
   if (paired) {
     if (warp == 0) {
       // ------------------------------ producer ------------------------------
-      if (lane == 0) {
-        long it = 0;
+      {
+        const unsigned lead_full = gp_mapa(full0, 0);
+        int s = 0;
+        unsigned ph = 1;      // (a fresh barrier counts as passed in this phase)
         for (int t = pair; t < p.tiles; t += pairs) {
           const int mt = t % p.m_tiles, nt = t / p.m_tiles;
           const int x_row = mt * 256 + (int)rank * 128;
           const int w_row = (MODE == GP_MODE_GATED) ? (int)rank * p.N + nt * 128 : nt * 256 + (int)rank * 128;
-          for (int kc = 0; kc < kboxes; ++kc, ++it) {
-            const int s = (int)(it % STAGES);
-            const unsigned ph = (unsigned)((it / STAGES) & 1);
-            if (it >= STAGES) gp_mbar_wait(empty0 + 8 * s, ph ^ 1, p.status, dead);
-            if (rank == 0) gp_mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
-            const unsigned bar = gp_mapa(full0 + 8 * s, 0);
-            gp_tma_load(stage0 + s * STAGE_BYTES, &xmap, kc * 64, x_row, bar);
-            gp_tma_load(stage0 + s * STAGE_BYTES + A_BYTES, &wmap, kc * 64, w_row, bar);
+          for (int k = 0; k < 64 * kboxes; k += 64) {
+            gp_mbar_wait(empty0 + 8 * s, ph, p.status, dead);
+            if (gp_elect()) {
+              if (rank == 0) gp_mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+              gp_tma_load(stage0 + s * STAGE_BYTES, &xmap, k, x_row, lead_full + 8 * s);
+              gp_tma_load(stage0 + s * STAGE_BYTES + A_BYTES, &wmap, k, w_row, lead_full + 8 * s);
+            }
+            __syncwarp();
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1;
+            }
           }
         }
       }
     } else if (warp == 1) {
       // ------------------------------ MMA issue (even CTA) ------------------------------
-      if (lane == 0 && rank == 0) {
+      if (rank == 0) {
         // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = 256, M = 256 (the pair's)
         constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
-        long it = 0;
-        int tl = 0;
+        const unsigned long long desc0 = gp_desc(stage0);
+        int tl = 0, s = 0;
+        unsigned ph = 0;
         for (int t = pair; t < p.tiles; t += pairs, ++tl) {
           const int b = tl & 1;
           // both CTAs' epilogues of the tile before last must have read this accumulator
           gp_mbar_wait(acc_empty0 + 8 * b, (unsigned)(((tl >> 1) & 1) ^ 1), p.status, dead);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const unsigned acc = tmem + (unsigned)(b * 256);
-          for (int kc = 0; kc < kboxes; ++kc, ++it) {
-            const int s = (int)(it % STAGES);
-            const unsigned ph = (unsigned)((it / STAGES) & 1);
+          for (int kc = 0; kc < kboxes; ++kc) {
             gp_mbar_wait(full0 + 8 * s, ph, p.status, dead);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned a_addr = stage0 + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
+            const unsigned long long a_desc = desc0 + (unsigned)(s * (STAGE_BYTES >> 4)), b_desc = a_desc + (A_BYTES >> 4);
+            if (gp_elect()) {
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16)
-              gp_mma(acc, gp_desc(a_addr + 32 * k16), gp_desc(b_addr + 32 * k16), IDESC, (kc > 0 || k16 > 0) ? 1u : 0u);
-            gp_commit_pair(empty0 + 8 * s);   // the stage is free in both CTAs once these MMAs have read it
+              for (int k16 = 0; k16 < 4; ++k16)      // (16 of k are 32 bytes further)
+                gp_mma(acc, a_desc + 2 * k16, b_desc + 2 * k16, IDESC, (kc > 0 || k16 > 0) ? 1u : 0u);
+              gp_commit_pair(empty0 + 8 * s);   // the stage is free in both CTAs once these MMAs have read it
+            }
+            __syncwarp();
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1;
+            }
           }
-          gp_commit_pair(acc_full0 + 8 * b);  // the tile's accumulator is complete once all its MMAs are done
+          if (gp_elect()) gp_commit_pair(acc_full0 + 8 * b);  // the tile's accumulator is complete once all its MMAs are done
         }
       }
     } else {
@@ -501,15 +386,11 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
             gp_ld32_issue(taddr + 32 * c, g);
             gp_ld32_issue(taddr + 128 + 32 * c, u);
             gp_ld_wait2(g, u);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              // gate and up rounded to bfloat16 first, as the unfused path does between product and activation
-              const float gt = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[i])));
-              const float uv = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[i])));
-              // (x * rcp(y) instead of the IEEE division: that one's chain of dependent instructions with a
-              //  branch an element, on the one warp a scheduler has here, made the epilogue twice as long as the MMAs)
-              v[i] = ll_gated_fast(gt, uv, p.gate);
-            }
+            // gate and up rounded to bfloat16 first, as the unfused path does between product and activation
+            float uv[32];
+            ll_round_bf16<32>(v, g);
+            ll_round_bf16<32>(uv, u);
+            ll_gated_any<32>(v, uv, p.gate);
           } else {
             unsigned a[32];
             gp_ld32_issue(taddr + 32 * c, a);
@@ -556,22 +437,6 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
-}
-
-typedef CUresult (*gp_encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static gp_encode_fn gp_encoder() {
-  static gp_encode_fn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (gp_encode_fn)ptr;
-  }
-  return fn;
 }
 
 // Tensor map of a bfloat16 matrix [rows, K] with row stride `stride` elements: boxes of 128 rows x 64 k.
