@@ -41,6 +41,7 @@ LIBRARIES: Dict[str, Tuple[Tuple[str, ...], Tuple[str, ...]]] = {
     "gemm_stream": (("gemm_stream.cu",), ()),
     "gemm_tc": (("gemm_tc.cu",), ()),
     "gemm_pair": (("gemm_pair.cu",), ()),
+    "gemm_group": (("gemm_group.cu",), ()),
     "gemm_f32": (("gemm_f32.cu",), ()),
     "attn_f32": (("attention_f32.cu",), ()),
     "attn_tc": (("attention_prefill_tc.cu",), ()),

@@ -11,7 +11,7 @@
 // `moe_act` then applies the activation and multiplies every hidden unit by the weight of its expert for that
 // token (1 for the always-on rows, 0 for experts not chosen), so that one second product over all hidden units
 // gives the weighted sum of the chosen experts' outputs plus the always-on expert's.
-#include "common.cuh"
+#include "moe_act.cuh"
 
 #define MOE_MAX_E 256
 
@@ -198,23 +198,6 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
     for (int e = lane; e < real; e += 32) gr[e] = gr[e] / total;
     for (int k = lane; k < top; k += 32) top_w[(size_t)t * top + k] /= total;
   }
-}
-
-// act: 0 relu(z)^2, 1 silu(z), 2 gelu_tanh(z), 3 gelu(z) (the erf form).
-__device__ __forceinline__ float moe_activation(float z, int act) {
-  if (act == 0) {
-    const float r = fmaxf(z, 0.f);
-    return r * r;
-  }
-  if (act == 1) return z / (1.0f + expf(-z));
-  if (act == 3) return 0.5f * z * (1.0f + erff(z * 0.7071067811865476f));
-  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
-// The expert's weight w for the token goes onto the activation's output, act(z) w, or (MOE_ACT_WEIGHT_IN set in
-// `act`) onto its input, act(w z): the expert then works on w times the token's row, since U (w x) = w (U x).
-#define MOE_ACT_WEIGHT_IN 16
-__device__ __forceinline__ float moe_weighted_activation(float z, float w, int act) {
-  return (act & MOE_ACT_WEIGHT_IN) ? moe_activation(z * w, act & 15) : moe_activation(z, act) * w;
 }
 
 // h: T [tokens, shared_ff + E * ff] in place: h = act(h) * weight, weight 1 for the first shared_ff columns,

@@ -1785,18 +1785,46 @@ def moe_combine(base: Optional[torch.Tensor], y: torch.Tensor, pair_row: torch.T
     return out
 
 
-def grouped_product(rows: torch.Tensor, weights: torch.Tensor, ends: torch.Tensor) -> torch.Tensor:
-    """Library grouped product: rows [total, k] cut into runs that end at ``ends`` [groups] (int32, on the
-    device), run g times weights[g] [n, k] transposed; bfloat16 with float32 accumulation."""
-    _need_cuda(rows, weights, ends)
+def expert_products(rows: torch.Tensor, weights: torch.Tensor, ends: torch.Tensor, gated: bool = False, act=None,
+                    row_w: Optional[torch.Tensor] = None, weight_in: bool = False, x: Optional[torch.Tensor] = None,
+                    shared: Optional[torch.Tensor] = None, shared_w: Optional[torch.Tensor] = None,
+                    shared_limit: float = 0.0, status: Optional[torch.Tensor] = None):
+    """The routed experts' products on the tensor cores (csrc/gemm_group.cu): rows [total, k] cut into runs that end at ``ends``
+    [groups] (int32, on the device), run g times weights[g] transposed, and, in the same launch, an expert's for every token:
+    ``x`` [tokens, k'] times ``shared`` transposed.  Returns (runs' result [total, n], ``x``'s [tokens, n'] or None).
+
+    ``gated``: weights [groups, 2 n, k] (gate rows, then up rows; contiguous) and the result is the gated activation ``act``
+    (``GateAct``; ``shared_limit``: its limit for ``x``) times ``row_w`` [total] (``shared_w`` [tokens]); else weights [groups, n, k]
+    of any row and group stride and the result is the product, or with ``act`` (of ``MOE_ACT``) the activation times the
+    weights (``weight_in``: of the weights times the product)."""
+    _need_cuda(rows, weights, ends, row_w, x, shared, shared_w, status)
     _i32(ends, "ends")
-    _need(rows.dtype == torch.bfloat16 and weights.dtype == torch.bfloat16 and weights.dim() == 3,
-          "grouped_product: bfloat16 rows and weights [groups, n, k]")
-    return torch.nn.functional.grouped_mm(rows, weights.transpose(1, 2), offs=ends)
-
-
-def grouped_product_available() -> bool:
-    return hasattr(torch.nn.functional, "grouped_mm")
+    _f32(row_w, "row_w")
+    _f32(shared_w, "shared_w")
+    total, k = rows.shape
+    groups, n = weights.shape[0], weights.shape[1] // 2 if gated else weights.shape[1]
+    _need(rows.dtype == weights.dtype == torch.bfloat16 and rows.is_contiguous() and weights.shape[2] == k
+          and weights.stride(2) == 1 and (not gated or weights.is_contiguous()) and ends.numel() == groups
+          and (row_w is None or row_w.numel() == total), "expert_products: bfloat16 rows [total, k], weights [groups, n, k]")
+    out = torch.empty((total, n), dtype=torch.bfloat16, device=rows.device)
+    out_s, tokens, n_s, k_s = None, 0, 0, 0
+    if x is not None:
+        tokens, k_s = x.shape
+        n_s = shared.shape[0] // 2 if gated else shared.shape[0]
+        _need(x.dtype == shared.dtype == torch.bfloat16 and x.stride(1) == 1 and shared.shape[1] == k_s
+              and shared.stride(1) == 1 and (not gated or shared.is_contiguous())
+              and (shared_w is None or shared_w.numel() == tokens), "expert_products: x [tokens, k'], shared [n', k']")
+        out_s = torch.empty((tokens, n_s), dtype=torch.bfloat16, device=rows.device)
+    g = _gate_act(act) if gated else GateAct("silu")
+    code = -1 if gated or act is None else MOE_ACT[act] + (16 if weight_in else 0)
+    load_library("gemm_group").call(
+        "ll_gemm_group", _ptr(out), _ptr(rows), _ptr(weights), c_int(total), c_int(n), c_int(k), c_long(weights.stride(1)),
+        c_long(weights.stride(0)), c_int(groups), _ptr(ends), _ptr(row_w), _ptr(out_s), _ptr(x),
+        c_long(0 if x is None else x.stride(0)), _ptr(shared), c_int(tokens), c_int(n_s), c_int(k_s),
+        c_long(0 if x is None else shared.stride(0)), _ptr(shared_w), c_int(1 + GATE_ACT[g.kind] if gated else 0),
+        c_float(g.limit), c_float(shared_limit), c_float(g.alpha), c_int(code), c_int(sm_count(rows.device)), _ptr(status),
+        _stream())
+    return out, out_s
 
 
 # --------------------------------------------------------------------------

@@ -14,8 +14,9 @@ Two ways through the experts, both without the host ever knowing who chose whom:
   chosen), and one product with the stacked down matrices gives the weighted sum.  With few tokens a step reads
   every expert's weights anyway, and that is what bounds it.
 * many tokens (``GROUPED_MIN_TOKENS``; bfloat16; widths that are multiples of 8): the (token, expert) pairs are
-  put in the order of the experts on the device, the chosen tokens' rows gathered, and two grouped library
-  products (a group an expert, the groups' ends a device array) do only the chosen experts' arithmetic; the
+  put in the order of the experts on the device, the chosen tokens' rows gathered, and two grouped products
+  (``ops.expert_products``: a group an expert, the groups' ends a device array, the shared expert's product in the
+  same launch, the activation in the first one's epilogue) do only the chosen experts' arithmetic; the
   pairs' results are added per token in the order of the pairs, onto the shared expert's output.
 
 A token's result does not depend on which other tokens are in the step (beyond which of the two ways it takes).
@@ -140,8 +141,7 @@ class RoutedExperts(FeedForward):
         self.w_up_experts = self.w_up[sff:].view(E, ff, h)
         sff, ff = self.shared_ff, self.ff
         self.w_down_experts = self.w_down[:, sff:].unflatten(1, (E, ff)).permute(1, 0, 2)
-        self.grouped = (dtype == torch.bfloat16 and h % 8 == 0 and ff % 8 == 0 and sff % 8 == 0
-                        and ops.grouped_product_available())
+        self.grouped = dtype == torch.bfloat16 and h % 8 == 0 and ff % 8 == 0 and sff % 8 == 0
 
     def weight_bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.w_up, self.w_down, self.w_router))
@@ -152,6 +152,8 @@ class RoutedExperts(FeedForward):
         libs = ["core", "moe"]
         if self.w_up is not None and self.w_up.dtype == torch.bfloat16:
             libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
+            if self.grouped and ops.TC_ENABLED:
+                libs.append("gemm_group")
         return libs
 
     def route(self, x):
@@ -174,14 +176,9 @@ class RoutedExperts(FeedForward):
 
     def _experts(self, x, step):
         gates, idx, wts = self.route(x)
-        if self.grouped and x.shape[0] >= self.GROUPED_MIN_TOKENS and not getattr(step, "captured", False):
-            try:
-                return self._forward_grouped(x, idx, wts)
-            except (RuntimeError, NotImplementedError) as exc:      # a shape the library's grouped product refuses
-                import sys
-                print(f"[lite_lang_b200] routed_experts {self.prefix}: grouped product refused ({str(exc)[:120]}); "
-                      "the stacked way is used instead", file=sys.stderr)
-                self.grouped = False
+        if (self.grouped and x.shape[0] >= self.GROUPED_MIN_TOKENS and ops.TC_ENABLED and not getattr(step, "captured", False)
+                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+            return self._forward_grouped(x, idx, wts, getattr(step, "status", None))
         hidden = ops.linear(x, self.w_up)
         if self.gated:
             hidden = ops.moe_gated_act(hidden, gates, self._shared_w, self.shared_ff, self.ff, self.E, self.limit,
@@ -192,25 +189,20 @@ class RoutedExperts(FeedForward):
         return ops.linear(hidden, self.w_down, partial_ok=True)
 
 
-    def _forward_grouped(self, x, idx, wts):
+    def _forward_grouped(self, x, idx, wts, status):
         sff = self.shared_ff
-        base = None
-        if sff and self.gated:
-            hs = ops.linear(x, self.w_up[:2 * sff])
-            hs = ops.moe_row_gated_act(hs, self._shared_w, self.shared_limit, self.swish_alpha)
-            base = ops.linear(hs, self.w_down[:, :sff])
-        elif sff:
-            hs = ops.linear(x, self.w_up[:sff])
-            ops.moe_act(hs, wts, sff, self.ff, 0, self.activation)      # (no routed columns: every weight is 1)
-            base = ops.linear(hs, self.w_down[:, :sff])
         ends, row_token, row_w, pair_row = ops.moe_sort(idx, wts, self.E)
         rows = ops.moe_gather_rows(x, row_token)
-        hidden = ops.grouped_product(rows, self.w_up_experts, ends)
+        up = dict(x=x, shared=self.w_up[:2 * sff if self.gated else sff]) if sff else {}
         if self.gated:
-            hidden = ops.moe_row_gated_act(hidden, row_w, self.limit, self.swish_alpha)
+            act = ops.GateAct("clamped_swish", self.limit, self.swish_alpha) if self.limit > 0 else ops.GateAct("silu")
+            hidden, hs = ops.expert_products(rows, self.w_up_experts, ends, True, act, row_w, shared_w=self._shared_w if sff else None,
+                                             shared_limit=self.shared_limit, status=status, **up)
         else:
-            ops.moe_row_act(hidden, row_w, self.activation, self.weight_in)
-        y = ops.grouped_product(hidden, self.w_down_experts, ends)
+            hidden, hs = ops.expert_products(rows, self.w_up_experts, ends, False, self.activation, row_w, self.weight_in,
+                                             status=status, **up)
+        down = dict(x=hs, shared=self.w_down[:, :sff]) if sff else {}
+        y, base = ops.expert_products(hidden, self.w_down_experts, ends, status=status, **down)
         return ops.moe_combine(base, y, pair_row)
 
 
