@@ -17,13 +17,17 @@
 // 2^-109 lose their last bits: a bfloat16 number ends at 2^-133.)
 //
 // x comes as its three terms (`f32_terms_kernel`, [3][M][K]: x is small and read by every column tile).  W stays float32 in
-// memory: its rows come by TMA into two buffers of 128 x 32, and their terms are written into the stage in the layout that
-// the MMAs read (the MMAs of 64 numbers of k take 3,072 cycles at the tensor cores' full rate).
+// memory: its rows come by TMA into two buffers of 128 x 32, and four warps write their terms into the stage in the layout
+// that the MMAs read (the MMAs of 64 numbers of k take 3,072 clocks at the tensor cores' full rate, and shared memory, which the
+// MMAs read 196 KB of meanwhile, nine tenths of that).
 //
-// Roles in a CTA (384 threads): warp 0 loads (one thread); warp 1 issues the MMAs (one thread of the even CTA); warps 2-9
-// make the terms of W's second buffer a step ahead and add a step's sum to theirs; warps 10 and 11 make the terms of W's first
-// buffer (all of them by the adding warps, or all by those two: 3.2 us a step either way).  A stage is 64 numbers of k: three terms of 128 rows of x and
-// three of 128 rows of W, 96 KB; two stages.
+// Roles in a CTA (512 threads, registers shared out between the warpgroups): warp 0 loads x's terms, warp 2 W; warp 1 of the even
+// CTA issues the MMAs; warps 4-11 add a step's sum to theirs; warps 12-15 make W's terms.  A stage is 64 numbers of k: three terms of
+// 128 rows of x and three of 128 rows of W, 96 KB; two stages.
+// Measured on a B200, 701 x 17,920 x 1,536 gated (two thirds of a wave's last round are work): 241 us with the loads and MMAs issued by
+// one lane, W's terms made by two warps and, between their sums, by the adding ones, and IEEE divisions in the epilogue (a step
+// of 64 numbers 5,600 clocks; a tile's end 26,000); 170 us now (3,790 and 8,500).  What is left above the MMAs' 3,072 is the way
+// from a stage that is free to its terms: 3,000 clocks, a third of them the fence before the MMAs may read.
 //
 // Where the tiles do not fill the chip, k is cut into `splits` parts of a work item each, whose results are
 // [splits][M][N] and added up in the order of the parts (`f32_join_kernel`, or the norm that reads them).
@@ -38,10 +42,14 @@
 
 #define LL_ERR_WAIT_TIMEOUT 5
 #define LL_ERR_TMEM_PAIR 7
-#define GF_THREADS 384
+#define GF_THREADS 512
+// registers a thread of the warpgroups {loads and MMAs, sums, sums, terms}: together the 4 x 128 of the launch
+#define GF_REGS_ISSUE 56
+#define GF_REGS_SUMS 176
+#define GF_REGS_TERMS 104
 #define GF_TERM_BYTES (128 * 128)                 // one term of 128 rows x 64
 #define GF_STAGE_BYTES (6 * GF_TERM_BYTES)
-#define GF_RAW_BYTES (128 * 32 * 4)
+#define GF_RAW_BYTES (128 * 32 * 4)               // W as stored: 128 rows x 32, two of them
 #define GF_SMEM (1024 + 2 * GF_STAGE_BYTES + 2 * GF_RAW_BYTES + 256)
 
 __device__ __forceinline__ void gf_mbar_init(unsigned bar, unsigned count) {
@@ -75,6 +83,13 @@ __device__ __forceinline__ void gf_mbar_wait(unsigned bar, unsigned parity, int*
       return;
     }
   }
+}
+// One lane of a converged warp, always the same (whole warps run the loops that issue copies and MMAs, so that their operands
+// stay in uniform registers; in a branch of one lane an MMA took 145 clocks to issue).
+__device__ __forceinline__ bool gf_elect() {
+  unsigned p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ unsigned gf_cluster_rank() {
   unsigned r;
@@ -119,17 +134,21 @@ __device__ __forceinline__ void gf_commit_pair(unsigned bar) {
                "h"(mask)
                : "memory");
 }
-__device__ __forceinline__ void gf_ld16(unsigned taddr, float (&v)[16]) {
-  unsigned r[16];
+// 16 columns of the thread's lane of tensor memory: asked for, and there (the registers are tied to the wait)
+__device__ __forceinline__ void gf_ld16_issue(unsigned taddr, unsigned (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      " tcgen05.wait::ld.sync.aligned;"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void gf_ld16_wait(unsigned (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
 }
 
 // terms[p][i] of x[M][K] (row stride x_stride): four numbers a thread
@@ -190,39 +209,6 @@ struct GfParams {
   int* status;
 };
 
-// the terms of buffer q (32 numbers of k) of step `it`'s rows of W into its stage, by THREADS threads (e: this one's number)
-template <int THREADS>
-__device__ __forceinline__ void gf_terms(unsigned char* smem, const unsigned char* raw, int q, int e, long it, unsigned free0,
-                                         unsigned raw_full0, unsigned raw_empty0, unsigned b_full_lead, int* status, bool& dead) {
-  const int s = (int)(it & 1);
-  if (it >= 2) gf_mbar_wait(free0 + 8 * s, (unsigned)(((it >> 1) & 1) ^ 1), status, dead);
-  unsigned char* dst = smem + s * GF_STAGE_BYTES + 3 * GF_TERM_BYTES;
-  const unsigned char* src = raw + q * GF_RAW_BYTES;
-  gf_mbar_wait(raw_full0 + 8 * q, (unsigned)(it & 1), status, dead);
-#pragma unroll 4
-  for (int i = e; i < 512; i += THREADS) {
-    const int row = i >> 2, c = i & 3;      // 8 numbers: 32 bytes as stored, 16 a term (the halves in an order that spares banks)
-    const float4 u = *reinterpret_cast<const float4*>(src + row * 128 + c * 32 + ((row & 1) << 4));
-    const float4 v = *reinterpret_cast<const float4*>(src + row * 128 + c * 32 + ((~row & 1) << 4));
-    const float4 lo = (row & 1) ? v : u, hi = (row & 1) ? u : v;
-    uint4 t0, t1, t2;
-    ms_split(lo.x, lo.y, t0.x, t1.x, t2.x);
-    ms_split(lo.z, lo.w, t0.y, t1.y, t2.y);
-    ms_split(hi.x, hi.y, t0.z, t1.z, t2.z);
-    ms_split(hi.z, hi.w, t0.w, t1.w, t2.w);
-    unsigned char* d = dst + row * 128 + (((q * 4 + c) ^ (row & 7)) << 4);
-    *reinterpret_cast<uint4*>(d) = t0;
-    *reinterpret_cast<uint4*>(d + GF_TERM_BYTES) = t1;
-    *reinterpret_cast<uint4*>(d + 2 * GF_TERM_BYTES) = t2;
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) {
-    gf_mbar_arrive(raw_empty0 + 8 * q);
-    gf_mbar_arrive_cluster(b_full_lead + 8 * s);
-  }
-}
-
 // a sum over numbers k0 .. k1 - 1 of k in float32
 __device__ __noinline__ float gf_plain(const float* x, const float* w, int k0, int k1) {
   float s = 0.f;
@@ -236,8 +222,43 @@ __device__ __noinline__ float gf_plain(const float* x, const float* w, int k0, i
   return s;
 }
 
+// x / d for d of 1 to 2^126, rounded to within a unit of the last place: the reciprocal instruction, Newton's iteration on it and
+// the quotient corrected by its remainder (Markstein's scheme), without the branch of the compiler's division
+__device__ __forceinline__ float gf_divide(float x, float d) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.f), r, r);
+  const float y = x * r;
+  return fmaf(fmaf(-d, y, x), r, y);
+}
+// The activation of 64 pairs (gate numbers, then up numbers) to dst[0 .. left - 1].  (The divisions of ll_gated, with a branch
+// each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some divisor was above 2^126, or NaN.
+template <int ACT>
+__device__ __forceinline__ bool gf_gate_row(float* dst, const float (&v)[128], int left, const GateAct& k) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < 64; i += 4) {
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float g = v[i + j], u = v[64 + i + j];
+      if (ACT == 1) {
+        o[j] = fmaxf(g, 0.f) * u;
+      } else {
+        const float a = ACT == 2 ? fminf(g, k.limit) : g;
+        const float z = ACT == 2 ? k.alpha * a : ACT == 3 ? 1.5957691216057308f * (a + 0.044715f * a * a * a) : a;
+        const float d = 1.0f + expf(-z);
+        odd |= !(d < 8.507059e37f);
+        o[j] = gf_divide(a, d) * (ACT == 2 ? fminf(fmaxf(u, -k.limit), k.limit) + 1.0f : u);
+      }
+    }
+    if (i < left) *reinterpret_cast<float4*>(dst + i) = make_float4(o[0], o[1], o[2], o[3]);      // (N is a multiple of 4)
+  }
+  return odd;
+}
+
 template <bool GATED>
-__global__ void __launch_bounds__(GF_THREADS)
+__global__ void __launch_bounds__(GF_THREADS, 1)
 gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap) {
   constexpr int COLS = GATED ? 128 : 256;
   extern __shared__ unsigned char smem_raw[];
@@ -245,24 +266,24 @@ gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, cons
   unsigned char* raw = smem + 2 * GF_STAGE_BYTES;
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(raw + 2 * GF_RAW_BYTES);
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 14);
-  const unsigned stage0 = ms_smem(smem), raw0 = ms_smem(raw);
+  const unsigned stage0 = ms_smem(smem);
   const unsigned a_full0 = ms_smem(bars), b_full0 = a_full0 + 16;          // even CTA: x's terms, W's terms of a stage are there
   const unsigned free0 = a_full0 + 32;                                     // both: the MMAs have read the stage
   const unsigned acc_full0 = a_full0 + 48, acc_empty0 = a_full0 + 64;      // both; even CTA
   const unsigned raw_full0 = a_full0 + 80, raw_empty0 = a_full0 + 96;      // this CTA's buffers of W as stored
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const unsigned rank = gf_cluster_rank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) {
       gf_mbar_init(a_full0 + 8 * s, 1);        // the even CTA announces both CTAs' bytes
-      gf_mbar_init(b_full0 + 8 * s, 20);       // the two and the eight warps that make terms, of both CTAs
+      gf_mbar_init(b_full0 + 8 * s, 8);        // the four warps that make terms, of both CTAs
       gf_mbar_init(free0 + 8 * s, 1);
       gf_mbar_init(acc_full0 + 8 * s, 1);
       gf_mbar_init(acc_empty0 + 8 * s, 16);
       gf_mbar_init(raw_full0 + 8 * s, 1);
-      gf_mbar_init(raw_empty0 + 8 * s, s == 0 ? 2 : 8);
+      gf_mbar_init(raw_empty0 + 8 * s, 4);     // the warps that make terms
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -294,108 +315,165 @@ gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, cons
     k1 = min(kboxes, k0 + per);
   };
   if (paired) {
-    if (warp == 0) {
-      // ------------------------------ loads ------------------------------
-      if (lane == 0) {
-        long it = 0;
+    if (warp < 4) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(GF_REGS_ISSUE));
+      if (warp == 0) {
+        // ------------------------------ loads of x's terms ------------------------------
+        const unsigned lead_a_full = gf_mapa(a_full0, 0);
+        int s = 0;
+        unsigned ph = 1;      // (a fresh barrier counts as passed in this phase)
         for (int item = pair; item < items; item += pairs) {
           int mt, nt, part, k0, k1;
           work(item, mt, nt, part, k0, k1);
           const int x_row = mt * 256 + (int)rank * 128;
-          const int w_row = GATED ? (int)rank * p.N + nt * 128 : nt * 256 + (int)rank * 128;
-          for (int kc = k0; kc < k1; ++kc, ++it) {
-            const int s = (int)(it & 1);
-            const unsigned ph = (unsigned)((it >> 1) & 1);
-            // W first: it has to pass through the epilogue warps' hands
-            for (int q = 0; q < 2; ++q) {
-              const unsigned rf = raw_full0 + 8 * q;
-              if (it >= 1) gf_mbar_wait(raw_empty0 + 8 * q, (unsigned)((it - 1) & 1), p.status, dead);
-              gf_mbar_expect_tx(rf, GF_RAW_BYTES);
-              gf_tma_load(raw0 + q * GF_RAW_BYTES, &wmap, kc * 64 + q * 32, w_row, gf_mapa(rf, rank));
+          for (int kc = k0; kc < k1; ++kc) {
+            gf_mbar_wait(free0 + 8 * s, ph, p.status, dead);
+            if (gf_elect()) {
+              if (rank == 0) gf_mbar_expect_tx(a_full0 + 8 * s, 2 * 3 * GF_TERM_BYTES);
+#pragma unroll
+              for (int q = 0; q < 3; ++q)
+                gf_tma_load(stage0 + s * GF_STAGE_BYTES + q * GF_TERM_BYTES, &xmap, kc * 64, q * p.M + x_row, lead_a_full + 8 * s);
             }
-            if (it >= 2) gf_mbar_wait(free0 + 8 * s, ph ^ 1, p.status, dead);
-            if (rank == 0) gf_mbar_expect_tx(a_full0 + 8 * s, 2 * 3 * GF_TERM_BYTES);
-            const unsigned bar = gf_mapa(a_full0 + 8 * s, 0);
-            for (int q = 0; q < 3; ++q)
-              gf_tma_load(stage0 + s * GF_STAGE_BYTES + q * GF_TERM_BYTES, &xmap, kc * 64, q * p.M + x_row, bar);
+            __syncwarp();
+            s ^= 1;
+            if (s == 0) ph ^= 1;
           }
         }
-      }
-    } else if (warp == 1) {
-      // ------------------------------ MMA issue (even CTA) ------------------------------
-      if (lane == 0 && rank == 0) {
-        constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
-        long it = 0;
+      } else if (warp == 2) {
+        // ------------------------------ loads of W as stored ------------------------------
+        const unsigned own_full = gf_mapa(raw_full0, rank);
+        unsigned ph = 1;
         for (int item = pair; item < items; item += pairs) {
           int mt, nt, part, k0, k1;
           work(item, mt, nt, part, k0, k1);
-          for (int kc = k0; kc < k1; ++kc, ++it) {
-            const int s = (int)(it & 1);
-            const unsigned ph = (unsigned)((it >> 1) & 1);
-            if (it >= 2) gf_mbar_wait(acc_empty0 + 8 * s, ph ^ 1, p.status, dead);
+          const int w_row = GATED ? (int)rank * p.N + nt * 128 : nt * 256 + (int)rank * 128;
+          for (int kc = k0; kc < k1; ++kc, ph ^= 1) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              gf_mbar_wait(raw_empty0 + 8 * q, ph, p.status, dead);
+              if (gf_elect()) {
+                gf_mbar_expect_tx(raw_full0 + 8 * q, GF_RAW_BYTES);
+                gf_tma_load(ms_smem(raw) + q * GF_RAW_BYTES, &wmap, kc * 64 + q * 32, w_row, own_full + 8 * q);
+              }
+              __syncwarp();
+            }
+          }
+        }
+      } else if (warp == 1 && rank == 0) {
+        // ------------------------------ MMA issue (even CTA) ------------------------------
+        constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+        const unsigned long long desc0 = gf_desc(stage0);
+        int s = 0;
+        unsigned ph = 0;
+        for (int item = pair; item < items; item += pairs) {
+          int mt, nt, part, k0, k1;
+          work(item, mt, nt, part, k0, k1);
+          for (int kc = k0; kc < k1; ++kc) {
+            gf_mbar_wait(acc_empty0 + 8 * s, ph ^ 1, p.status, dead);
             gf_mbar_wait(a_full0 + 8 * s, ph, p.status, dead);
             gf_mbar_wait(b_full0 + 8 * s, ph, p.status, dead);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned acc = tmem + (unsigned)(s * 256);
-            const unsigned a = stage0 + s * GF_STAGE_BYTES, b = a + 3 * GF_TERM_BYTES;
-            // (term of x, term of W): the small products first, the leading one last
+            const unsigned long long a = desc0 + (unsigned)(s * (GF_STAGE_BYTES >> 4)), b = a + (3 * GF_TERM_BYTES >> 4);
+            // (term of x, term of W): the small products first, the leading one last; 16 of k are 32 bytes further
             constexpr int TA[6] = {2, 1, 0, 1, 0, 0}, TB[6] = {0, 1, 2, 0, 1, 0};
+            if (gf_elect()) {
 #pragma unroll
-            for (int q = 0; q < 6; ++q)
+              for (int q = 0; q < 6; ++q)
 #pragma unroll
-              for (int k16 = 0; k16 < 4; ++k16)
-                gf_mma(acc, gf_desc(a + TA[q] * GF_TERM_BYTES + 32 * k16), gf_desc(b + TB[q] * GF_TERM_BYTES + 32 * k16), IDESC,
-                       (q > 0 || k16 > 0) ? 1u : 0u);
-            gf_commit_pair(free0 + 8 * s);
-            gf_commit_pair(acc_full0 + 8 * s);
+                for (int k16 = 0; k16 < 4; ++k16)
+                  gf_mma(acc, a + TA[q] * (GF_TERM_BYTES >> 4) + 2 * k16, b + TB[q] * (GF_TERM_BYTES >> 4) + 2 * k16, IDESC,
+                         (q > 0 || k16 > 0) ? 1u : 0u);
+              gf_commit_pair(free0 + 8 * s);
+              gf_commit_pair(acc_full0 + 8 * s);
+            }
+            __syncwarp();
+            s ^= 1;
+            if (s == 0) ph ^= 1;
           }
         }
       }
-    } else if (warp >= 10) {
-      // ------------------------------ terms of W's first buffer (warps 10 and 11) ------------------------------
+    } else if (warp >= 12) {
+      // ------------------------------ W's terms ------------------------------
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(GF_REGS_TERMS));
       const unsigned b_full_lead = gf_mapa(b_full0, 0);
-      long it = 0;
+      // thread e has numbers 8 c .. 8 c + 7 of a buffer in rows r, r + 32, ... r + 96: 32 bytes as stored, 16 a term.  Of eight
+      // threads half have rows 4 further, and read the halves of their 32 bytes in the other order: all meet different banks
+      const int e = tid - 384, c = e & 3, t = e >> 2, odd = t & 1, r = odd * 4 + ((t >> 1) & 3) + (t & 24);
+      const unsigned char* src = raw + r * 128 + c * 32;
+      int s = 0;
+      unsigned ph = 1, rph = 0;
       for (int item = pair; item < items; item += pairs) {
         int mt, nt, part, k0, k1;
         work(item, mt, nt, part, k0, k1);
-        for (int kc = k0; kc < k1; ++kc, ++it) gf_terms<64>(smem, raw, 0, tid - 320, it, free0, raw_full0, raw_empty0, b_full_lead, p.status, dead);
+        for (int kc = k0; kc < k1; ++kc, rph ^= 1) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            float4 v[4][2];
+            gf_mbar_wait(raw_full0 + 8 * q, rph, p.status, dead);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              v[j][0] = *reinterpret_cast<const float4*>(src + q * GF_RAW_BYTES + 4096 * j + 16 * odd);
+              v[j][1] = *reinterpret_cast<const float4*>(src + q * GF_RAW_BYTES + 4096 * j + 16 - 16 * odd);
+            }
+            if (q == 0) gf_mbar_wait(free0 + 8 * s, ph, p.status, dead);
+            unsigned char* dst = smem + s * GF_STAGE_BYTES + 3 * GF_TERM_BYTES + r * 128 + (((q * 4 + c) ^ (r & 7)) << 4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {      // (32 rows further: 4,096 bytes, the same swizzle)
+              const float4 lo = odd ? v[j][1] : v[j][0], hi = odd ? v[j][0] : v[j][1];
+              uint4 t0, t1, t2;
+              ms_split(lo.x, lo.y, t0.x, t1.x, t2.x);
+              ms_split(lo.z, lo.w, t0.y, t1.y, t2.y);
+              ms_split(hi.x, hi.y, t0.z, t1.z, t2.z);
+              ms_split(hi.z, hi.w, t0.w, t1.w, t2.w);
+              *reinterpret_cast<uint4*>(dst + 4096 * j) = t0;
+              *reinterpret_cast<uint4*>(dst + 4096 * j + GF_TERM_BYTES) = t1;
+              *reinterpret_cast<uint4*>(dst + 4096 * j + 2 * GF_TERM_BYTES) = t2;
+            }
+            // (the buffer is given back behind the last use of what was read from it: an arrival right behind the loads
+            // overtook them, and the next copy was in their place)
+            __syncwarp();
+            if (lane == 0) gf_mbar_arrive(raw_empty0 + 8 * q);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) gf_mbar_arrive_cluster(b_full_lead + 8 * s);
+          s ^= 1;
+          if (s == 0) ph ^= 1;
+        }
       }
     } else {
-      // ------------------------------ terms of W's second buffer, sums (warps 2..9) ------------------------------
+      // ------------------------------ sums (warps 4..11) ------------------------------
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(GF_REGS_SUMS));
       const int ew = warp & 3;              // the 32 tensor-memory lanes this warp may read
-      const int eh = (warp - 2) >> 2;       // its columns: 64 eh .. + 63 and 128 + 64 eh .. + 63
-      const unsigned b_full_lead = gf_mapa(b_full0, 0), acc_empty_lead = gf_mapa(acc_empty0, 0);
+      const int eh = (warp - 4) >> 2;       // its columns: 64 eh .. + 63 and 128 + 64 eh .. + 63
+      const unsigned acc_empty_lead = gf_mapa(acc_empty0, 0);
       float sum[128];
-      long total = 0;                       // steps of all items
-      for (int item = pair; item < items; item += pairs) {
-        int mt, nt, part, k0, k1;
-        work(item, mt, nt, part, k0, k1);
-        total += k1 - k0;
-      }
-      long it = 0;
-      if (total > 0) gf_terms<256>(smem, raw, 1, tid - 64, 0, free0, raw_full0, raw_empty0, b_full_lead, p.status, dead);
+      int s = 0;
+      unsigned ph = 0;
       for (int item = pair; item < items; item += pairs) {
         int mt, nt, part, k0, k1;
         work(item, mt, nt, part, k0, k1);
 #pragma unroll
         for (int i = 0; i < 128; ++i) sum[i] = 0.f;
-        for (int kc = k0; kc < k1; ++kc, ++it) {
-          if (it + 1 < total)
-            gf_terms<256>(smem, raw, 1, tid - 64, it + 1, free0, raw_full0, raw_empty0, b_full_lead, p.status, dead);
-          const int s = (int)(it & 1);
-          gf_mbar_wait(acc_full0 + 8 * s, (unsigned)((it >> 1) & 1), p.status, dead);
+        for (int kc = k0; kc < k1; ++kc) {
+          gf_mbar_wait(acc_full0 + 8 * s, ph, p.status, dead);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const unsigned taddr = tmem + ((unsigned)(32 * ew) << 16) + (unsigned)(s * 256 + 64 * eh);
+          unsigned v[2][16];      // (the next 16 columns are on their way while these are added)
+          gf_ld16_issue(taddr, v[0]);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            float v[16];
-            gf_ld16(taddr + (c >> 2) * 128 + (c & 3) * 16, v);
+            gf_ld16_wait(v[c & 1]);
+            if (c < 7) gf_ld16_issue(taddr + ((c + 1) >> 2) * 128 + ((c + 1) & 3) * 16, v[(c + 1) & 1]);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) sum[16 * c + i] += v[i];
+            for (int i = 0; i < 16; ++i) sum[16 * c + i] += __uint_as_float(v[c & 1][i]);
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) gf_mbar_arrive_cluster(acc_empty_lead + 8 * s);
+          s ^= 1;
+          if (s == 0) ph ^= 1;
         }
         const int row = mt * 256 + (int)rank * 128 + 32 * ew + lane;
         if (row < p.M) {
@@ -404,15 +482,16 @@ gemm_f32_kernel(const GfParams p, const __grid_constant__ CUtensorMap xmap, cons
 #pragma unroll
           for (int i = 0; i < 128; ++i) nan |= sum[i] != sum[i];
           if (GATED) {
-            const int f0 = nt * 128 + 64 * eh;
+            const int f0 = nt * 128 + 64 * eh, left = p.N - f0;
+            bool odd = false;
+            if (p.gate.act == 0) odd = gf_gate_row<0>(dst + f0, sum, left, p.gate);
+            else if (p.gate.act == 2) odd = gf_gate_row<2>(dst + f0, sum, left, p.gate);
+            else if (p.gate.act == 3) odd = gf_gate_row<3>(dst + f0, sum, left, p.gate);
+            else gf_gate_row<1>(dst + f0, sum, left, p.gate);
+            if (odd) {
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
-              float4 v;
-              v.x = ll_gated(sum[i], sum[64 + i], p.gate);
-              v.y = ll_gated(sum[i + 1], sum[65 + i], p.gate);
-              v.z = ll_gated(sum[i + 2], sum[66 + i], p.gate);
-              v.w = ll_gated(sum[i + 3], sum[67 + i], p.gate);
-              if (f0 + i < p.N) *reinterpret_cast<float4*>(dst + f0 + i) = v;      // (N is a multiple of 4)
+              for (int i = 0; i < 64; ++i)
+                if (i < left) dst[f0 + i] = ll_gated(sum[i], sum[64 + i], p.gate);
             }
           } else {
 #pragma unroll
@@ -481,10 +560,10 @@ static int gf_make_map(CUtensorMap* map, const void* base, long rows, long K, lo
 }
 
 template <bool GATED>
-static int gf_launch(GfParams& p, const void* terms, const float* w, long w_stride, int sm_count, cudaStream_t stream) {
+static int gf_launch(GfParams& p, const void* terms, int sm_count, cudaStream_t stream) {
   CUtensorMap xmap, wmap;
   int rc = gf_make_map(&xmap, terms, 3l * p.M, p.K, p.K, true);
-  if (rc == 0) rc = gf_make_map(&wmap, w, GATED ? 2l * p.N : (long)p.N, p.K, w_stride, false);
+  if (rc == 0) rc = gf_make_map(&wmap, p.w, GATED ? 2l * p.N : (long)p.N, p.K, p.w_stride, false);
   if (rc != 0) return rc;
   const cudaError_t ac = cudaFuncSetAttribute(gemm_f32_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GF_SMEM);
   if (ac != cudaSuccess) return (int)ac;
@@ -542,8 +621,8 @@ extern "C" int ll_gemm_f32(float* out, long out_stride, const float* x, long x_s
   p.splits = splits;
   p.gate = {gated > 0 ? gated - 1 : 0, limit, alpha};
   p.status = status;
-  const int rc = gated ? gf_launch<true>(p, terms, w, w_stride, sm_count, stream)
-                       : gf_launch<false>(p, terms, w, w_stride, sm_count, stream);
+  const int rc = gated ? gf_launch<true>(p, terms, sm_count, stream)
+                       : gf_launch<false>(p, terms, sm_count, stream);
   if (rc != 0 || !join || out == nullptr) return rc;
   const long out_pieces = (long)M * (N / 4);
   ll_launch(f32_join_kernel, dim3((unsigned)((out_pieces + 255) / 256 < most ? (out_pieces + 255) / 256 : most)), dim3(256), 0,
