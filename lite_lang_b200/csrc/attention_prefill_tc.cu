@@ -139,7 +139,7 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 1 + 4 * AT_KS + 6);
   unsigned* merge_flag = tmem_slot + 1;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // ---- which rows: row block rb of the step.  Order of the CTAs (the hardware starts them in the order of
   // their number, and one that has to wait holds back all after it): first split 0 of every row block, the
   // heavier, later blocks of an entry first, the kv heads side by side; then split 1 of every row block, and
@@ -275,49 +275,60 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issue ------------------------------
-    if (lane == 0) {
-      auto mma_s = [&](int j) {   // S[j % 2] = Q K(j)^T
-        const int s = j % AT_KS, b = j & 1;
-        at_mbar_wait(k_full0 + 8 * s, (unsigned)((j / AT_KS) & 1), p.status, dead);
-        at_mbar_wait(s_empty0 + 8 * b, (unsigned)(((j >> 1) & 1) ^ 1), p.status, dead);
-        AT_FENCE_AFTER();
-        const unsigned k_addr = at_smem(kv_s) + s * K_STEP;
+    // (descriptors of the first step: 16 of k further are 32 bytes along a row, or 2,048 down V)
+    const unsigned long long q_desc = at_desc_k(at_smem(q_s)), p_desc = at_desc_k(at_smem(p_s)), k_desc0 = at_desc_k(at_smem(kv_s)),
+                             v_desc0 = at_desc_mn(at_smem(kv_s) + V_AT, KV_BYTES / HB);
+    unsigned ks = 0, kph = 0;             // K's stage and its phase, counted
+    auto mma_s = [&](int j) {   // S[j % 2] = Q K(j)^T
+      const int b = j & 1;
+      at_mbar_wait(k_full0 + 8 * ks, kph, p.status, dead);
+      at_mbar_wait(s_empty0 + 8 * b, (unsigned)(((j >> 1) & 1) ^ 1), p.status, dead);
+      AT_FENCE_AFTER();
+      if (at_elect()) {
+        const unsigned long long k_desc = k_desc0 + ks * (K_STEP >> 4);
 #pragma unroll
-        for (int k16 = 0; k16 < HD / 16; ++k16) {
-          const unsigned off = (k16 / 4) * (Q_BYTES / HB) + (k16 % 4) * 32;
-          const unsigned koff = (k16 / 4) * (KV_BYTES / HB) + (k16 % 4) * 32;
-          at_mma(tmem_s + b * AT_KB, at_desc_k(at_smem(q_s) + off), at_desc_k(k_addr + koff), IDESC_S, k16 > 0 ? 1u : 0u);
-        }
+        for (int k16 = 0; k16 < HD / 16; ++k16)
+          at_mma(tmem_s + b * AT_KB, q_desc + (k16 / 4) * (Q_BYTES / HB >> 4) + (k16 % 4) * 2,
+                 k_desc + (k16 / 4) * (KV_BYTES / HB >> 4) + (k16 % 4) * 2, IDESC_S, k16 > 0 ? 1u : 0u);
         at_commit(s_full0 + 8 * b);
-        at_commit(k_empty0 + 8 * s);   // the K stage is free once these MMAs have read it
-      };
-      at_mbar_wait(q_full, 0, p.status, dead);
-      // S runs a whole block ahead of the softmax: S(j + 2) is issued as soon as P(j) has gone into O, into
-      // the buffer whose S(j) the softmax warps read long ago, so S(j + 1) is complete when they want it
-      // however far apart the four warps have drifted
-      mma_s(0);
-      if (nblk > 1) mma_s(1);
-      for (int j = 0; j < nblk; ++j) {
-        const int s = j % VS;
-        at_mbar_wait(v_full0 + 8 * s, (unsigned)((j / VS) & 1), p.status, dead);
-        at_mbar_wait(p_full, (unsigned)(j & 1), p.status, dead);
-        AT_FENCE_AFTER();
-        const unsigned v_addr = at_smem(kv_s) + s * K_STEP + V_AT;
-        const unsigned p_addr = at_smem(p_s);
+        at_commit(k_empty0 + 8 * ks);   // the K stage is free once these MMAs have read it
+      }
+      __syncwarp();
+      if (++ks == AT_KS) {
+        ks = 0;
+        kph ^= 1;
+      }
+    };
+    at_mbar_wait(q_full, 0, p.status, dead);
+    // S runs a whole block ahead of the softmax: S(j + 2) is issued as soon as P(j) has gone into O, into
+    // the buffer whose S(j) the softmax warps read long ago, so S(j + 1) is complete when they want it
+    // however far apart the four warps have drifted
+    mma_s(0);
+    if (nblk > 1) mma_s(1);
+    unsigned vs = 0, vph = 0;
+    for (int j = 0; j < nblk; ++j) {
+      at_mbar_wait(v_full0 + 8 * vs, vph, p.status, dead);
+      at_mbar_wait(p_full, (unsigned)(j & 1), p.status, dead);
+      AT_FENCE_AFTER();
+      if (at_elect()) {
+        const unsigned long long v_desc = v_desc0 + vs * (K_STEP >> 4);
         if (SHAPED) {
 #pragma unroll
           for (int k16 = 0; k16 < AT_KB / 16; ++k16)   // the weights' low terms
-            at_mma(tmem_o, at_desc_k(p_addr + P_BYTES + k16 * 32), at_desc_mn(v_addr + k16 * 2048, KV_BYTES / HB), IDESC_PV,
-                   (j > 0 || k16 > 0) ? 1u : 0u);
+            at_mma(tmem_o, p_desc + (P_BYTES >> 4) + k16 * 2, v_desc + k16 * 128, IDESC_PV, (j > 0 || k16 > 0) ? 1u : 0u);
         }
 #pragma unroll
-        for (int k16 = 0; k16 < AT_KB / 16; ++k16)   // 16 keys a step: 32 bytes along P's rows, 2048 bytes down V
-          at_mma(tmem_o, at_desc_k(p_addr + k16 * 32), at_desc_mn(v_addr + k16 * 2048, KV_BYTES / HB), IDESC_PV,
-                 (SHAPED || j > 0 || k16 > 0) ? 1u : 0u);
+        for (int k16 = 0; k16 < AT_KB / 16; ++k16)
+          at_mma(tmem_o, p_desc + k16 * 2, v_desc + k16 * 128, IDESC_PV, (SHAPED || j > 0 || k16 > 0) ? 1u : 0u);
         at_commit(pv_done);            // P may be written again; O holds the blocks up to j
-        at_commit(v_empty0 + 8 * s);
-        if (j + 2 < nblk) mma_s(j + 2);
+        at_commit(v_empty0 + 8 * vs);
       }
+      __syncwarp();
+      if (++vs == VS) {
+        vs = 0;
+        vph ^= 1;
+      }
+      if (j + 2 < nblk) mma_s(j + 2);
     }
   } else {
     // ------------------------------ softmax rows (warps 2..5) ------------------------------

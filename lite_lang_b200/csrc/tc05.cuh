@@ -42,6 +42,14 @@ __device__ __forceinline__ void at_mbar_wait(unsigned bar, unsigned parity, int*
     }
   }
 }
+// One lane of a converged warp, always the same.  (The loops that issue copies and MMAs are run by whole warps: what they compute
+// then stays in uniform registers, where the instructions want it; in a branch of one lane every operand is moved there
+// anew, about 145 clocks an MMA.)
+__device__ __forceinline__ bool at_elect() {
+  unsigned p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void at_tma_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
