@@ -109,13 +109,28 @@ __device__ __forceinline__ void gt_mbar_wait(unsigned bar, unsigned parity, int*
     }
   }
 }
-// One TMA box: rows [y, y + box rows) x k [x, x + 64) of W into shared memory (x is a multiple of 64
-// elements, i.e. of 128 bytes, as TMA's 16-byte rule on the innermost coordinate demands).
-__device__ __forceinline__ void gt_tma_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+// One TMA box a stage and operand: k is a dimension of blocks of 64 (the innermost coordinate is 0), so a box brings all of a
+// stage's blocks: [block][row][64 k].  (A box a block, four of 2 KB and four of 1 KB a stage of 16 rows, took the producer 60
+// to 150 clocks each, more than their bytes.)
+// W: blocks kb .. of rows y .. and, where a unit has two runs of rows (gate and up, a head's halves), of the run `far` beyond.
+__device__ __forceinline__ void gt_tma_w(unsigned dst, const CUtensorMap* map, int y, int kb, unsigned bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(bar)
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(map), "r"(0), "r"(y), "r"(0), "r"(kb), "r"(bar)
       : "memory");
+}
+__device__ __forceinline__ void gt_tma_x(unsigned dst, const CUtensorMap* map, int y, int kb, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(0), "r"(y), "r"(kb), "r"(bar)
+      : "memory");
+}
+// One lane of a converged warp, always the same (the producer's loops are run by its whole warp, so that what the copies take
+// stays in uniform registers).
+__device__ __forceinline__ bool gt_elect() {
+  unsigned p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ uint4 gt_lds16(unsigned addr) {
   uint4 v;
@@ -221,7 +236,7 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
   const unsigned scale_bar = gt_smem(bars + 2 * STAGES);                                   //  row factors' barrier)
   const unsigned stage0 = gt_smem(smem);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if (tid == GT_CONSUMERS * 32) {   // the producer's maps
     asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
@@ -279,65 +294,64 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
     // ------------------------------ producer ------------------------------
     // The weights do not depend on the kernel before this one, so streaming starts at once.  The token
     // rows do: their boxes follow after griddepcontrol.wait, first for the stages already under way.
-    if (lane == 0) {
-      int uu = blockIdx.x, kc = 0, kc_end = 0, y[RBOXES];
-      auto open_unit = [&]() {   // rows and k range of work unit uu
-        if (uu >= p.units) return;
-        const int u = uu / p.ksplit, kp = uu - u * p.ksplit;
-        if (MODE == GT_MODE_WIDE) {
-          y[0] = u * 64;
-        } else if (MODE == GT_MODE_GATED) {
-          y[0] = u * 32;                 // gate rows of the unit's 32 features
-          y[RBOXES - 1] = p.N + u * 32;  // their up rows
-        } else if (MODE == GT_MODE_QKV_ROPE) {
-          const int upr = p.hd / 16;                  // units per head
-          const int head = u / upr, i0 = (u - head * upr) * 8;
-          y[0] = head * p.hd + i0;                    // 8 features of the first half of the head
-          y[RBOXES - 1] = y[0] + p.hd / 2;            // their partners in the second half
-        } else {
-          y[0] = u * 16;
-        }
-        kc = kp * p.cpp;
-        kc_end = min(kchunks, (kp + 1) * p.cpp);
-      };
-      auto advance = [&]() {
-        if (++kc >= kc_end) {
-          uu += gridDim.x;
-          open_unit();
-        }
-      };
-      auto issue_w = [&](int s) {
-#pragma unroll
-        for (int kb = 0; kb < KBOXES; ++kb)
-#pragma unroll
-          for (int rb = 0; rb < RBOXES; ++rb)
-            gt_tma_load(stage0 + s * STAGE_BYTES + (kb * RBOXES + rb) * BOX_BYTES, &wmap, kc * S::KC + kb * 64, y[rb],
-                        full0 + 8 * s);
-      };
-      auto issue_x = [&](int s, int k) {
-#pragma unroll
-        for (int kb = 0; kb < KBOXES; ++kb)
-          gt_tma_load(stage0 + s * STAGE_BYTES + W_BYTES + kb * XBOX_BYTES, &xmap, k * S::KC + kb * 64, tok0, full0 + 8 * s);
-      };
-      open_unit();
-      int early_kc[STAGES];
-      int early = 0;
-      for (; early < STAGES && uu < p.units; ++early) {   // the ring's first round: weights now
-        gt_mbar_expect_tx(full0 + 8 * early, STAGE_BYTES);
-        issue_w(early);
-        early_kc[early] = kc;
-        advance();
+    struct Walk {
+      int uu, kc, kc_end, y;      // unit, k chunk, the unit's last, its first row
+    };
+    auto open_unit = [&](Walk& w) {
+      if (w.uu >= p.units) return;
+      const int u = w.uu / p.ksplit, kp = w.uu - u * p.ksplit;
+      if (MODE == GT_MODE_WIDE) {
+        w.y = u * 64;
+      } else if (MODE == GT_MODE_GATED) {
+        w.y = u * 32;                               // gate rows of the unit's 32 features (their up rows: the second run)
+      } else if (MODE == GT_MODE_QKV_ROPE) {
+        const int upr = p.hd / 16;                  // units per head
+        const int head = u / upr, i0 = (u - head * upr) * 8;
+        w.y = head * p.hd + i0;                     // 8 features of the first half of the head (the second: their partners)
+      } else {
+        w.y = u * 16;
       }
-      LL_PDL_WAIT();
-      for (int s = 0; s < early; ++s) issue_x(s, early_kc[s]);   // their token rows once those exist
-      for (long it = early; uu < p.units; ++it) {
-        const int s = (int)(it % STAGES);
-        const unsigned ph = (unsigned)((it / STAGES) & 1);
-        gt_mbar_wait(empty0 + 8 * s, ph ^ 1, p.status);
+      w.kc = kp * p.cpp;
+      w.kc_end = min(kchunks, (kp + 1) * p.cpp);
+    };
+    auto advance = [&](Walk& w) {
+      if (++w.kc >= w.kc_end) {
+        w.uu += gridDim.x;
+        open_unit(w);
+      }
+    };
+    Walk w = {(int)blockIdx.x, 0, 0, 0};
+    open_unit(w);
+    Walk x = w;                 // the stages whose token rows are still to come
+    int early = 0;
+    for (; early < STAGES && w.uu < p.units; ++early) {   // the ring's first round: weights now
+      if (gt_elect()) {
+        gt_mbar_expect_tx(full0 + 8 * early, STAGE_BYTES);
+        gt_tma_w(stage0 + early * STAGE_BYTES, &wmap, w.y, w.kc * KBOXES, full0 + 8 * early);
+      }
+      __syncwarp();
+      advance(w);
+    }
+    LL_PDL_WAIT();
+    for (int s = 0; s < early; ++s) {      // their token rows once those exist
+      if (gt_elect()) gt_tma_x(stage0 + s * STAGE_BYTES + W_BYTES, &xmap, tok0, x.kc * KBOXES, full0 + 8 * s);
+      __syncwarp();
+      advance(x);
+    }
+    int s = 0;
+    unsigned ph = 0;            // (early < STAGES: nothing is left)
+    while (w.uu < p.units) {
+      gt_mbar_wait(empty0 + 8 * s, ph, p.status);
+      if (gt_elect()) {
         gt_mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
-        issue_w(s);
-        issue_x(s, kc);
-        advance();
+        gt_tma_w(stage0 + s * STAGE_BYTES, &wmap, w.y, w.kc * KBOXES, full0 + 8 * s);
+        gt_tma_x(stage0 + s * STAGE_BYTES + W_BYTES, &xmap, tok0, w.kc * KBOXES, full0 + 8 * s);
+      }
+      __syncwarp();
+      advance(w);
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
       }
     }
     return;
@@ -367,7 +381,8 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
   // 16-byte chunk q of a 128-byte row r sits at chunk q ^ (r & 7); all rows used here have r & 7 == g
   const unsigned sw = (unsigned)g;
 
-  long it = 0;
+  int s = 0;
+  unsigned ph = 0;
   for (int uu = blockIdx.x; uu < p.units; uu += gridDim.x) {
     const int u = uu / p.ksplit, kp = uu - u * p.ksplit;
     float acc[MT][4];
@@ -423,9 +438,7 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
       }
     }
     const int kc_end = min(kchunks, (kp + 1) * p.cpp);
-    for (int kc = kp * p.cpp; kc < kc_end; ++kc, ++it) {
-      const int s = (int)(it % STAGES);
-      const unsigned ph = (unsigned)((it / STAGES) & 1);
+    for (int kc = kp * p.cpp; kc < kc_end; ++kc) {
       uint4 xv[MYBOXES][2][MT];
       gt_mbar_wait(full0 + 8 * s, ph, p.status);
       // token row 8 j + g of the stage's x box: its 16-byte chunk 4 i + c sits at chunk (4 i + c) ^ g
@@ -454,6 +467,10 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
       }
       __syncwarp();
       if (lane == 0) gt_mbar_arrive(empty0 + 8 * s);
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
+      }
     }
     // ---- the unit's results ----
     OutT* out = reinterpret_cast<OutT*>(p.out) + (size_t)kp * p.M * p.out_stride;  // this part's [M, N] block
@@ -611,18 +628,28 @@ static gt_encode_fn gt_encoder() {
   return fn;
 }
 
-// Tensor map of a bfloat16 matrix [rows, K] (rows row_stride elements apart; 0: K) with boxes of box_rows rows
-// x 64 k, 128-byte swizzle.  Rows beyond the matrix read as zeros.
-static int gt_make_map(CUtensorMap* map, const void* w, long rows, long K, int box_rows, long row_stride = 0) {
+// Tensor map of a bfloat16 matrix as blocks of 64 k, 128-byte swizzle: [K / 64][runs][rows][64], `runs` 1 or 2 runs of rows `far`
+// rows apart (0 runs: no such dimension), rows row_stride elements apart; boxes of kboxes blocks, all runs, box_rows rows.
+// Rows beyond the matrix read as zeros.
+static int gt_make_map(CUtensorMap* map, const void* w, long rows, long K, long row_stride, int box_rows, int kboxes, int runs, long far) {
   gt_encode_fn enc = gt_encoder();
   if (enc == nullptr) return (int)cudaErrorNotSupported;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)(row_stride > 0 ? row_stride : K) * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint64_t row = (cuuint64_t)row_stride * 2;
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r;
+  if (runs == 0) {
+    const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(K / 64)};
+    const cuuint64_t strides[2] = {row, 128};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)kboxes};
+    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  } else {
+    const cuuint64_t dims[4] = {64, (cuuint64_t)rows, (cuuint64_t)runs, (cuuint64_t)(K / 64)};
+    const cuuint64_t strides[3] = {row, (cuuint64_t)(runs > 1 ? far : 1) * row, 128};
+    const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, (cuuint32_t)runs, (cuuint32_t)kboxes};
+    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
@@ -631,10 +658,12 @@ static int gt_launch(const GtParams& p, const void* w, int sm_count, cudaStream_
   using S = GtShape<MODE>;
   using G = GtStage<MODE, MT>;
   CUtensorMap map, xmap;
-  const long w_rows = (MODE == GT_MODE_GATED) ? 2l * p.N : p.N;
-  int rc = gt_make_map(&map, w, w_rows, p.K, S::BOX_ROWS);
+  // (gated: N gate rows, N up rows behind them; q|k|v: a head's second half hd / 2 rows beyond its first)
+  constexpr int RUNS = S::ROWS / S::BOX_ROWS;
+  const long far = MODE == GT_MODE_GATED ? p.N : MODE == GT_MODE_QKV_ROPE ? p.hd / 2 : 0;
+  int rc = gt_make_map(&map, w, MODE == GT_MODE_QKV_ROPE ? p.N - far : (long)p.N, p.K, p.K, S::BOX_ROWS, G::KBOXES, RUNS, far);
   if (rc != 0) return rc;
-  rc = gt_make_map(&xmap, p.x, p.M, p.K, 8 * MT, p.x_stride);   // token rows: boxes of 8 MT rows, zeros beyond M
+  rc = gt_make_map(&xmap, p.x, p.M, p.K, p.x_stride, 8 * MT, G::KBOXES, 0, 0);   // token rows: 8 MT of them, zeros beyond M
   if (rc != 0) return rc;
   const size_t smem = 1024 + (size_t)G::STAGES * G::STAGE_BYTES + 2 * G::STAGES * 8 + 8 +   // (+ the row factors' barrier)
                       ((MODE == GT_MODE_NARROW || MODE == GT_MODE_QKV_ROPE) ? sizeof(float) * GT_CONSUMERS * 16 * 8 * MT : 0);

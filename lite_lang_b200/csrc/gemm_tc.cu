@@ -68,6 +68,20 @@ __device__ __forceinline__ void tc_tma_load(unsigned dst, const CUtensorMap* map
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// The weights' 128 rows of a stage, one box: 128 features' rows, or 64 gate rows and the 64 up rows of the same features
+__device__ __forceinline__ void tc_tma_w(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(0), "r"(bar)
+      : "memory");
+}
+// One lane of a converged warp, always the same (whole warps run the loops that issue copies and MMAs, so that their operands
+// stay in uniform registers; in a branch of one lane an MMA took 145 clocks to issue).
+__device__ __forceinline__ bool tc_elect() {
+  unsigned p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
+}
 // Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with the 128-byte
 // swizzle (what TMA writes): groups of 8 rows are 1024 bytes apart; 16 elements of k are 32 bytes.
 __device__ __forceinline__ unsigned long long tc_desc(unsigned smem_addr) {
@@ -141,7 +155,7 @@ gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap wmap, const
   const unsigned full0 = tc_smem(bars), empty0 = tc_smem(bars + STAGES);
   const unsigned acc_full = tc_smem(bars + 2 * STAGES), acc_empty = tc_smem(bars + 2 * STAGES + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if (tid == 32) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
@@ -171,93 +185,96 @@ gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap wmap, const
 
   bool dead = false;
   const int kboxes = p.K / 64;
-  long total = 0;  // stages this CTA goes through
-  for (int uu = blockIdx.x; uu < p.units; uu += gridDim.x) {
-    const int kp = uu % p.ksplit;
-    total += min(kboxes, (kp + 1) * p.cpp) - kp * p.cpp;
-  }
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      // weights first (they do not depend on the kernel before), up to a ring's worth; then wait for
-      // the kernel before and send the tokens' boxes after them
-      int uu = blockIdx.x, kc = 0, kc_end = 0;
-      auto open_unit = [&]() {  // the k boxes of unit uu
-        if (uu < p.units) {
-          const int kp = uu % p.ksplit;
-          kc = kp * p.cpp;
-          kc_end = min(kboxes, (kp + 1) * p.cpp);
-        }
-      };
-      auto advance = [&]() {
-        if (++kc >= kc_end) {
-          uu += gridDim.x;
-          open_unit();
-        }
-      };
-      auto issue_a = [&](int s) {
-        const int u = uu / p.ksplit;
-        if (MODE == TC_MODE_GATED) {  // two boxes of 64 rows: gate rows, then the up rows of the same features
-          tc_tma_load(stage0 + s * STAGE_BYTES, &wmap, kc * 64, u * 64, full0 + 8 * s);
-          tc_tma_load(stage0 + s * STAGE_BYTES + A_BYTES / 2, &wmap, kc * 64, p.N + u * 64, full0 + 8 * s);
-        } else {
-          tc_tma_load(stage0 + s * STAGE_BYTES, &wmap, kc * 64, u * 128, full0 + 8 * s);
-        }
-      };
-      auto issue_b = [&](int s, int k) {
-        tc_tma_load(stage0 + s * STAGE_BYTES + A_BYTES, &xmap, k * 64, 0, full0 + 8 * s);
-      };
-      const int early = (int)(total < STAGES ? total : STAGES);
-      int early_kc[STAGES];
-      open_unit();
-      for (int s = 0; s < early; ++s) {
-        tc_mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
-        issue_a(s);
-        early_kc[s] = kc;
-        advance();
+    // weights first (they do not depend on the kernel before), up to a ring's worth; then wait for
+    // the kernel before and send the tokens' boxes after them
+    struct Walk {
+      int uu, kc, kc_end;      // unit, k box, the unit's last
+    };
+    auto open_unit = [&](Walk& w) {
+      if (w.uu < p.units) {
+        const int kp = w.uu % p.ksplit;
+        w.kc = kp * p.cpp;
+        w.kc_end = min(kboxes, (kp + 1) * p.cpp);
       }
-      LL_PDL_WAIT();
-      for (int s = 0; s < early; ++s) issue_b(s, early_kc[s]);
-      for (long it = early; it < total; ++it) {
-        const int s = (int)(it % STAGES);
-        const unsigned ph = (unsigned)((it / STAGES) & 1);
-        tc_mbar_wait(empty0 + 8 * s, ph ^ 1, p.status, dead);
-        tc_mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
-        issue_a(s);
-        issue_b(s, kc);
-        advance();
+    };
+    auto advance = [&](Walk& w) {
+      if (++w.kc >= w.kc_end) {
+        w.uu += gridDim.x;
+        open_unit(w);
       }
-    } else {
-      LL_PDL_WAIT();
+    };
+    auto issue_w = [&](int s, const Walk& w) {
+      tc_mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+      tc_tma_w(stage0 + s * STAGE_BYTES, &wmap, w.kc * 64, (w.uu / p.ksplit) * S::FEATS, full0 + 8 * s);
+    };
+    auto issue_x = [&](int s, const Walk& w) {
+      tc_tma_load(stage0 + s * STAGE_BYTES + A_BYTES, &xmap, w.kc * 64, 0, full0 + 8 * s);
+    };
+    Walk w = {(int)blockIdx.x, 0, 0};
+    open_unit(w);
+    Walk x = w;               // the stages whose token rows are still to come
+    int early = 0;
+    for (; early < STAGES && w.uu < p.units; ++early) {
+      if (tc_elect()) issue_w(early, w);
+      __syncwarp();
+      advance(w);
+    }
+    LL_PDL_WAIT();
+    for (int s = 0; s < early; ++s) {
+      if (tc_elect()) issue_x(s, x);
+      __syncwarp();
+      advance(x);
+    }
+    int s = 0;
+    unsigned ph = 0;          // (early < STAGES: nothing is left)
+    while (w.uu < p.units) {
+      tc_mbar_wait(empty0 + 8 * s, ph, p.status, dead);
+      if (tc_elect()) {
+        issue_w(s, w);
+        issue_x(s, w);
+      }
+      __syncwarp();
+      advance(w);
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
+      }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issue ------------------------------
     LL_PDL_WAIT();
-    if (lane == 0) {
-      // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = NT, M = 128
-      constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) | ((128u >> 4) << 24);
-      long it = 0;
-      int unit_no = 0;
-      for (int uu = blockIdx.x; uu < p.units; uu += gridDim.x, ++unit_no) {
-        const int kp = uu % p.ksplit;
-        const int kc0 = kp * p.cpp, kc1 = min(kboxes, (kp + 1) * p.cpp);
-        // the epilogue of the unit before must have read the accumulator
-        tc_mbar_wait(acc_empty, (unsigned)((unit_no & 1) ^ 1), p.status, dead);
+    // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = NT, M = 128
+    constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) | ((128u >> 4) << 24);
+    const unsigned long long desc0 = tc_desc(stage0);
+    int unit_no = 0, s = 0;
+    unsigned ph = 0;
+    for (int uu = blockIdx.x; uu < p.units; uu += gridDim.x, ++unit_no) {
+      const int kp = uu % p.ksplit;
+      const int kc0 = kp * p.cpp, kc1 = min(kboxes, (kp + 1) * p.cpp);
+      // the epilogue of the unit before must have read the accumulator
+      tc_mbar_wait(acc_empty, (unsigned)((unit_no & 1) ^ 1), p.status, dead);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int kc = kc0; kc < kc1; ++kc) {
+        tc_mbar_wait(full0 + 8 * s, ph, p.status, dead);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kc = kc0; kc < kc1; ++kc, ++it) {
-          const int s = (int)(it % STAGES);
-          const unsigned ph = (unsigned)((it / STAGES) & 1);
-          tc_mbar_wait(full0 + 8 * s, ph, p.status, dead);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const unsigned a_addr = stage0 + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
+        if (tc_elect()) {
+          const unsigned long long a_desc = desc0 + (unsigned)(s * (STAGE_BYTES >> 4)), b_desc = a_desc + (A_BYTES >> 4);
 #pragma unroll
-          for (int k16 = 0; k16 < 4; ++k16)
-            tc_mma(tmem, tc_desc(a_addr + 32 * k16), tc_desc(b_addr + 32 * k16), IDESC, (kc > kc0 || k16 > 0) ? 1u : 0u);
+          for (int k16 = 0; k16 < 4; ++k16)      // (16 of k are 32 bytes further)
+            tc_mma(tmem, a_desc + 2 * k16, b_desc + 2 * k16, IDESC, (kc > kc0 || k16 > 0) ? 1u : 0u);
           tc_commit(empty0 + 8 * s);  // the stage is free once these MMAs have read it
         }
-        tc_commit(acc_full);          // the unit's accumulator is complete once all its MMAs are done
+        __syncwarp();
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
       }
+      if (tc_elect()) tc_commit(acc_full);          // the unit's accumulator is complete once all its MMAs are done
+      __syncwarp();
     }
   } else {
     // ------------------------------ epilogue (warps 2..5) ------------------------------
@@ -409,11 +426,25 @@ static int tc_make_map(CUtensorMap* map, const void* base, long rows, long K, lo
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
+// The weights as [runs][rows][K], two runs (gate rows, then up rows) or one: boxes of 128 rows of all runs together
+static int tc_make_w_map(CUtensorMap* map, const void* base, long rows, long K, int runs) {
+  tc_encode_fn enc = tc_encoder();
+  if (enc == nullptr) return (int)cudaErrorNotSupported;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)runs};
+  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)rows * K * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)(128 / runs), (cuuint32_t)runs};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
 template <int MODE, int NT, int OUT, bool SCALED = false>
 static int tc_launch(const TcParams& p, const void* w, const void* x, long x_stride, int sm_count, cudaStream_t stream) {
   constexpr bool GATED = MODE == TC_MODE_GATED;
   CUtensorMap wmap, xmap;
-  int rc = tc_make_map(&wmap, w, GATED ? 2l * p.N : (long)p.N, p.K, p.K, GATED ? 64 : 128);
+  int rc = tc_make_w_map(&wmap, w, p.N, p.K, GATED ? 2 : 1);
   if (rc == 0) rc = tc_make_map(&xmap, x, p.M, p.K, x_stride, NT);
   if (rc != 0) return rc;
   const size_t smem = TcShape<MODE, NT>::SMEM;
