@@ -7,7 +7,7 @@
 // The tokens are the M side of the MMA here (a token is a lane of tensor memory, its features are columns),
 // so a thread of the epilogue holds gate and up of the same token and feature side by side.
 //
-// A tile is 256 tokens x 256 columns, made by a pair of CTAs on two SMs (a thread-block cluster of two,
+// A tile is 256 tokens x 256 columns (plain products also 128 or 192), made by a pair of CTAs on two SMs (a thread-block cluster of two,
 // tcgen05 with cta_group::2): each CTA brings 128 token rows (A) and 128 weight rows (B) of every 64-wide
 // k block into its own shared memory by TMA (no multicast: the pair's two halves of B are different rows)
 // and holds the accumulator rows of its own 128 tokens in its own tensor memory; the even CTA of the pair
@@ -53,7 +53,14 @@
 #define GP_MODE_PLAIN 0
 #define GP_MODE_GATED 1
 #define GP_MODE_QKV 2
-#define GP_SMEM (1024 + GP_STAGES * GP_STAGE_BYTES + (2 * GP_STAGES + 4) * 8 + 16)
+// Shared-memory plan: BN columns a tile (plain: 128, 192 or 256, so that the tiles fill the pairs better; else 256), half of
+// whose weight rows each CTA brings; q|k|v gives two stages' room to its epilogue's staging tile.
+template <int MODE, int BN> struct GpShape {
+  static constexpr int STAGE_BYTES = GP_A_BYTES + BN / 2 * 128;
+  static constexpr int STAGES = MODE == GP_MODE_QKV ? 4 : BN == 128 ? 8 : BN == 192 ? 7 : GP_STAGES;
+  static constexpr int STG_BYTES = MODE == GP_MODE_QKV ? 128 * 512 : 0;
+  static constexpr int SMEM = 1024 + STAGES * STAGE_BYTES + STG_BYTES + (2 * STAGES + 4) * 8 + 16;
+};
 
 struct GpParams {
   bf16* out;
@@ -64,6 +71,7 @@ struct GpParams {
   int vec_ok;       // the output takes 16-byte pieces (aligned base and stride, N a multiple of 8)
   GateAct gate;     // gated: the activation
   int act;          // plain: 0 none, 1 gelu (tanh form), 2 ReLU, 3 SiLU, 4 ReLU squared
+  int act_cols;     // plain: the columns the activation is for, the first ones
   int* status;
   // q|k|v mode only: what follows the projection (N = (nh + 2 nkv) hd; out is q [M, nh hd])
   const float* bias;      // float32 [N] or null
@@ -242,21 +250,20 @@ __device__ __forceinline__ void gp_qkv_finish(const GpParams& p, const unsigned 
   }
 }
 
-template <int MODE>
+template <int MODE, int BN>
 __global__ void __launch_bounds__(GP_THREADS)
 gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap) {
-  // (q|k|v mode gives two of the six stages' room to its epilogue's staging tile)
-  constexpr int STAGES = (MODE == GP_MODE_QKV) ? GP_STAGES - GP_STG_BYTES / GP_STAGE_BYTES : GP_STAGES;
-  constexpr int STAGE_BYTES = GP_STAGE_BYTES, A_BYTES = GP_A_BYTES;
-  constexpr int COLS = (MODE == GP_MODE_GATED) ? 128 : 256;   // output features a tile
+  using S = GpShape<MODE, BN>;
+  constexpr int STAGES = S::STAGES, STAGE_BYTES = S::STAGE_BYTES, A_BYTES = GP_A_BYTES;
+  constexpr int COLS = (MODE == GP_MODE_GATED) ? 128 : BN;   // output features a tile
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + GP_STAGES * STAGE_BYTES);
   unsigned char* stg = smem + STAGES * STAGE_BYTES;   // q|k|v mode only
-  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * GP_STAGES + 4);
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(stg + S::STG_BYTES);
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * STAGES + 4);
   const unsigned stage0 = gp_smem(smem);
-  const unsigned full0 = gp_smem(bars), empty0 = gp_smem(bars + GP_STAGES);
-  const unsigned acc_full0 = gp_smem(bars + 2 * GP_STAGES), acc_empty0 = gp_smem(bars + 2 * GP_STAGES + 2);
+  const unsigned full0 = gp_smem(bars), empty0 = gp_smem(bars + STAGES);
+  const unsigned acc_full0 = gp_smem(bars + 2 * STAGES), acc_empty0 = gp_smem(bars + 2 * STAGES + 2);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const unsigned rank = gp_cluster_rank();   // 0: issues the MMAs and owns the `full` and `acc_empty` barriers
@@ -303,7 +310,7 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
         for (int t = pair; t < p.tiles; t += pairs) {
           const int mt = t % p.m_tiles, nt = t / p.m_tiles;
           const int x_row = mt * 256 + (int)rank * 128;
-          const int w_row = (MODE == GP_MODE_GATED) ? (int)rank * p.N + nt * 128 : nt * 256 + (int)rank * 128;
+          const int w_row = (MODE == GP_MODE_GATED) ? (int)rank * p.N + nt * 128 : nt * BN + (int)rank * (BN / 2);
           for (int k = 0; k < 64 * kboxes; k += 64) {
             gp_mbar_wait(empty0 + 8 * s, ph, p.status, dead);
             if (gp_elect()) {
@@ -322,8 +329,8 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
     } else if (warp == 1) {
       // ------------------------------ MMA issue (even CTA) ------------------------------
       if (rank == 0) {
-        // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = 256, M = 256 (the pair's)
-        constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+        // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 256 (the pair's)
+        constexpr unsigned IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((256u >> 4) << 24);
         const unsigned long long desc0 = gp_desc(stage0);
         int tl = 0, s = 0;
         unsigned ph = 0;
@@ -397,21 +404,27 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
             gp_ld_wait(a);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(a[i]);
-            if (MODE == GP_MODE_PLAIN && p.act != 0) {
-              // the activation of a feed-forward without a gate, on the product rounded to bfloat16 first (as a
-              // product followed by an activation kernel has it); gelu in its tanh form is z * sigmoid(2 u),
-              // u = sqrt(2/pi) (z + 0.044715 z^3); x * rcp(y) for the division, as in the gated mode
+            if (MODE == GP_MODE_PLAIN) {
+              const int f0 = nt * COLS + 32 * c;
+              if (p.act != 0 && f0 < p.act_cols) {
+                // the activation of a feed-forward without a gate, on the product rounded to bfloat16 first (as a
+                // product followed by an activation kernel has it); gelu in its tanh form is z * sigmoid(2 u),
+                // u = sqrt(2/pi) (z + 0.044715 z^3)
+                float z[32];
+                ll_round_bf16<32>(z, a);
+                if (p.act == 3) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const float z = __bfloat162float(__float2bfloat16_rn(v[i]));
-                if (p.act == 2) {
-                  v[i] = fmaxf(z, 0.f);
-                } else if (p.act == 4) {
-                  v[i] = fmaxf(z, 0.f) * fmaxf(z, 0.f);
+                  for (int i = 0; i < 32; ++i) z[i] *= ll_sigmoid_fast(z[i]);
+                } else if (p.act == 1) {
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) z[i] *= ll_sigmoid_fast(1.5957691216057308f * (z[i] + 0.044715f * z[i] * z[i] * z[i]));
                 } else {
-                  const float u = p.act == 3 ? z : 1.5957691216057308f * (z + 0.044715f * z * z * z);
-                  v[i] = __fdividef(z, 1.0f + __expf(-u));
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) z[i] = p.act == 4 ? fmaxf(z[i], 0.f) * fmaxf(z[i], 0.f) : fmaxf(z[i], 0.f);
                 }
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (f0 + i < p.act_cols) v[i] = z[i];
               }
             }
           }
@@ -439,13 +452,13 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
   }
 }
 
-// Tensor map of a bfloat16 matrix [rows, K] with row stride `stride` elements: boxes of 128 rows x 64 k.
-static int gp_make_map(CUtensorMap* map, const void* base, long rows, long K, long stride) {
+// Tensor map of a bfloat16 matrix [rows, K] with row stride `stride` elements: boxes of box_rows rows x 64 k.
+static int gp_make_map(CUtensorMap* map, const void* base, long rows, long K, long stride, int box_rows) {
   gp_encode_fn enc = gp_encoder();
   if (enc == nullptr) return (int)cudaErrorNotSupported;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
-  const cuuint32_t box[2] = {64, 128};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -454,14 +467,14 @@ static int gp_make_map(CUtensorMap* map, const void* base, long rows, long K, lo
 }
 
 // Pairs of CTAs that can be resident at once (a pair needs two SMs of one GPU processing cluster)
-template <int MODE>
+template <int MODE, int BN>
 static int gp_max_pairs(int sm_count) {
   static int cached = -1;
   if (cached < 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count & ~1, 1, 1);
     cfg.blockDim = dim3(GP_THREADS);
-    cfg.dynamicSmemBytes = GP_SMEM;
+    cfg.dynamicSmemBytes = GpShape<MODE, BN>::SMEM;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -470,7 +483,7 @@ static int gp_max_pairs(int sm_count) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<MODE>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<MODE, BN>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = sm_count / 2;
     }
@@ -479,24 +492,24 @@ static int gp_max_pairs(int sm_count) {
   return cached;
 }
 
-template <int MODE>
+template <int MODE, int BN = 256>
 static int gp_launch(GpParams& p, const void* w, const void* x, long x_stride, int sm_count, cudaStream_t stream) {
   constexpr bool GATED = MODE == GP_MODE_GATED;
   CUtensorMap wmap, xmap;
-  int rc = gp_make_map(&wmap, w, GATED ? 2l * p.N : (long)p.N, p.K, p.K);
-  if (rc == 0) rc = gp_make_map(&xmap, x, p.M, p.K, x_stride);
+  int rc = gp_make_map(&wmap, w, GATED ? 2l * p.N : (long)p.N, p.K, p.K, BN / 2);
+  if (rc == 0) rc = gp_make_map(&xmap, x, p.M, p.K, x_stride, 128);
   if (rc != 0) return rc;
-  cudaFuncSetAttribute(gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-  const int cols = GATED ? 128 : 256;
+  cudaFuncSetAttribute(gemm_pair_kernel<MODE, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GpShape<MODE, BN>::SMEM);
+  const int cols = GATED ? 128 : BN;
   p.m_tiles = (p.M + 255) / 256;
   p.tiles = p.m_tiles * ((p.N + cols - 1) / cols);
-  const int most = gp_max_pairs<MODE>(sm_count);
+  const int most = gp_max_pairs<MODE, BN>(sm_count);
   const int pairs = p.tiles < most ? p.tiles : most;
   // a pair is a cluster of two CTAs along x (what a kernel with cta_group::2 instructions is launched as)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(GP_THREADS);
-  cfg.dynamicSmemBytes = GP_SMEM;
+  cfg.dynamicSmemBytes = GpShape<MODE, BN>::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -507,63 +520,46 @@ static int gp_launch(GpParams& p, const void* w, const void* x, long x_stride, i
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, gemm_pair_kernel<MODE>, p, wmap, xmap);
+  cudaLaunchKernelEx(&cfg, gemm_pair_kernel<MODE, BN>, p, wmap, xmap);
   return LL_LAUNCH_RESULT();
 }
 
-// x: bfloat16 [M, K] (row stride x_stride, a multiple of 8); w: bfloat16 [N, K] contiguous (gated: [2 N, K],
-// gate rows first); out: bfloat16 [M, N] (gated: silu(gate) * up).  Any M; meant for hundreds of tokens and more.
-extern "C" int ll_gemm_pair(void* out, long out_stride, const void* x, long x_stride, const void* w, int M, int N,
-                            int K, int gated, int sm_count, float limit, float alpha, int* status, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || (K % 8) != 0 || (x_stride % 8) != 0 || sm_count < 2) return (int)cudaErrorInvalidValue;
-  GpParams p;
+static GpParams gp_params(void* out, long out_stride, int M, int N, int K, int* status) {
+  GpParams p = {};
   p.out = reinterpret_cast<bf16*>(out);
   p.out_stride = out_stride;
   p.M = M;
   p.N = N;
   p.K = K;
   p.status = status;
-  if (gated < 0 || gated > 4) return (int)cudaErrorInvalidValue;
-  p.gate = {gated > 0 ? gated - 1 : 0, limit, alpha};      // (gated: 1 SiLU, 2 ReLU, 3 clamped swish, 4 gelu)
-  p.act = 0;
   p.vec_ok = ((uintptr_t)out % 16 == 0 && out_stride % 8 == 0 && N % 8 == 0) ? 1 : 0;
-  p.bias = nullptr;
-  p.positions = nullptr;
-  p.cos_sin = nullptr;
-  p.slot_map = nullptr;
-  p.k_cache = p.v_cache = nullptr;
-  p.max_pos = p.nh = p.nkv = p.hd = p.page_size = 0;
-  p.num_slots = 0;
-  return gated ? gp_launch<GP_MODE_GATED>(p, w, x, x_stride, sm_count, stream)
-               : gp_launch<GP_MODE_PLAIN>(p, w, x, x_stride, sm_count, stream);
+  return p;
 }
 
-// out = act(x W^T) for a feed-forward without a gate: act 1 gelu (tanh form), 2 ReLU, 3 SiLU (0: none), applied to
-// the product as bfloat16 holds it.  Operands as in ll_gemm_pair.
-extern "C" int ll_gemm_pair_act(void* out, long out_stride, const void* x, long x_stride, const void* w, int M, int N,
-                                int K, int act, int sm_count, int* status, cudaStream_t stream) {
+// x: bfloat16 [M, K] (row stride x_stride, a multiple of 8); w: bfloat16 [2 N, K] contiguous, gate rows first; out: bfloat16
+// [M, N] = act(gate) * up, `act`: see GateAct.  Any M; meant for hundreds of tokens and more.
+extern "C" int ll_gemm_pair_gated(void* out, long out_stride, const void* x, long x_stride, const void* w, int M, int N,
+                                  int K, int act, int sm_count, float limit, float alpha, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || (K % 8) != 0 || (x_stride % 8) != 0 || sm_count < 2 || act < 0 || act > 4)
-    return (int)cudaErrorInvalidValue;
-  GpParams p;
-  p.out = reinterpret_cast<bf16*>(out);
-  p.out_stride = out_stride;
-  p.M = M;
-  p.N = N;
-  p.K = K;
-  p.status = status;
-  p.gate = {0, 0.f, 0.f};
+  if (K <= 0 || (K % 8) != 0 || (x_stride % 8) != 0 || sm_count < 2 || act < 0 || act > 3) return (int)cudaErrorInvalidValue;
+  GpParams p = gp_params(out, out_stride, M, N, K, status);
+  p.gate = {act, limit, alpha};
+  return gp_launch<GP_MODE_GATED>(p, w, x, x_stride, sm_count, stream);
+}
+
+// out = act(x W^T) for w [N, K]: act 1 gelu (tanh form), 2 ReLU, 3 SiLU, 4 ReLU squared (0: none) on the first act_cols columns,
+// applied to the product as bfloat16 holds it.  `cols`: columns a tile, 128, 192 or 256.
+extern "C" int ll_gemm_pair(void* out, long out_stride, const void* x, long x_stride, const void* w, int M, int N, int K, int act,
+                            int act_cols, int cols, int sm_count, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (K % 8) != 0 || (x_stride % 8) != 0 || sm_count < 2 || act < 0 || act > 4) return (int)cudaErrorInvalidValue;
+  GpParams p = gp_params(out, out_stride, M, N, K, status);
   p.act = act;
-  p.vec_ok = ((uintptr_t)out % 16 == 0 && out_stride % 8 == 0 && N % 8 == 0) ? 1 : 0;
-  p.bias = nullptr;
-  p.positions = nullptr;
-  p.cos_sin = nullptr;
-  p.slot_map = nullptr;
-  p.k_cache = p.v_cache = nullptr;
-  p.max_pos = p.nh = p.nkv = p.hd = p.page_size = 0;
-  p.num_slots = 0;
-  return gp_launch<GP_MODE_PLAIN>(p, w, x, x_stride, sm_count, stream);
+  p.act_cols = act_cols;
+  if (cols == 128) return gp_launch<GP_MODE_PLAIN, 128>(p, w, x, x_stride, sm_count, stream);
+  if (cols == 192) return gp_launch<GP_MODE_PLAIN, 192>(p, w, x, x_stride, sm_count, stream);
+  if (cols == 256) return gp_launch<GP_MODE_PLAIN, 256>(p, w, x, x_stride, sm_count, stream);
+  return (int)cudaErrorInvalidValue;
 }
 
 // The q|k|v projection of an attention layer with what follows it: qkv = x W^T (+ bias), q and k rotated by
@@ -581,15 +577,7 @@ extern "C" int ll_gemm_pair_qkv_rope(void* q_out, long q_stride, const void* x, 
       (slot_map != nullptr && (k_cache == nullptr || v_cache == nullptr || page_size <= 0 || (uintptr_t)k_cache % 16 != 0 ||
                                (uintptr_t)v_cache % 16 != 0)))
     return (int)cudaErrorInvalidValue;
-  GpParams p;
-  p.out = reinterpret_cast<bf16*>(q_out);
-  p.out_stride = q_stride;
-  p.M = M;
-  p.N = (nh + 2 * nkv) * hd;
-  p.K = K;
-  p.status = status;
-  p.gate = {0, 0.f, 0.f};
-  p.act = 0;
+  GpParams p = gp_params(q_out, q_stride, M, (nh + 2 * nkv) * hd, K, status);
   p.vec_ok = 1;
   p.bias = bias;
   p.positions = positions;

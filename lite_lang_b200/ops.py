@@ -1020,28 +1020,46 @@ def pair_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
+# clocks that a stage of 64 numbers of k takes a pair of SMs, by the columns of a tile (the MMAs alone: twice the columns)
+PAIR_STAGE_CLOCKS = ((256, 520), (192, 420), (128, 320))
+
+
+@functools.lru_cache(maxsize=4096)
+def pair_columns(m: int, n: int, sms: int) -> int:
+    """Columns of a tile of ``gemm_pair``'s plain product: the width whose rounds of tiles over the pairs of SMs take least.
+    Measured on a B200 (128 / 192 / 256 columns, us): 2,048 x 6,144 x 1,536 34.5 / 31.6 / 30.7, 2,048 x 1,536 x 8,960 49.4 /
+    41.2 / 51.9, 512 x 6,144 x 1,536 14.7 / 13.5 / 16.1, 300 x 3,584 x 3,584 15.0 / 19.8 / 24.2."""
+    rows = (m + 255) // 256
+    return min((-(-rows * (-(-n // w)) // (sms // 2)) * clocks, -w) for w, clocks in PAIR_STAGE_CLOCKS)[1] * -1
+
+
 def gemm_pair(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gated: bool = False,
-              status: Optional[torch.Tensor] = None, act="silu", row_act: Optional[str] = None) -> torch.Tensor:
+              status: Optional[torch.Tensor] = None, act="silu", row_act: Optional[str] = None,
+              act_cols: Optional[int] = None, cols: int = 0) -> torch.Tensor:
     """out = x @ weight.T for many bfloat16 tokens on the tcgen05 tensor cores, a pair of SMs a tile of
     256 tokens x 256 columns.  ``gated``: weight is [2 I, K] and out = silu(gate) * up, the activation done
-    on the accumulator, so gate and up never go to memory."""
+    on the accumulator, so gate and up never go to memory.  ``row_act``: a feed-forward without a gate, out = act(x @ weight.T),
+    act of ``ROW_ACT``, on the first ``act_cols`` columns (None: all).  ``cols``: the columns of a tile (128, 192 or 256; 0:
+    ``pair_columns``)."""
     _need_cuda(x, weight, out, status)
-    act = _gate_act(act)
     _need(pair_supported(x, weight), "gemm_pair: bfloat16, K % 8 == 0, 16-byte aligned rows")
     m, k = x.shape
     n = weight.shape[0] // 2 if gated else weight.shape[0]
     _need(out.dtype == torch.bfloat16 and out.dim() == 2 and out.shape[0] == m and out.shape[1] == n
           and out.stride(1) == 1, "gemm_pair: out is bfloat16 [M, N] with unit column stride")
-    if row_act is not None:      # a feed-forward without a gate: out = act(x @ weight.T), act of ``ROW_ACT``
-        _need(not gated, "gemm_pair: row_act goes with the plain product")
+    sms = sm_count(x.device)
+    if gated:
+        _need(row_act is None, "gemm_pair: row_act goes with the plain product")
+        act = _gate_act(act)
         load_library("gemm_pair").call(
-            "ll_gemm_pair_act", _ptr(out), c_long(out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight), c_int(m),
-            c_int(n), c_int(k), c_int(ROW_ACT[row_act] + 1), c_int(sm_count(x.device)), _ptr(status), _stream())
+            "ll_gemm_pair_gated", _ptr(out), c_long(out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight), c_int(m),
+            c_int(n), c_int(k), c_int(GATE_ACT[act.kind]), c_int(sms), c_float(act.limit), c_float(act.alpha), _ptr(status),
+            _stream())
         return out
     load_library("gemm_pair").call(
-        "ll_gemm_pair", _ptr(out), c_long(out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight), c_int(m),
-        c_int(n), c_int(k), c_int(1 + GATE_ACT[act.kind] if gated else 0), c_int(sm_count(x.device)), c_float(act.limit),
-        c_float(act.alpha), _ptr(status), _stream())
+        "ll_gemm_pair", _ptr(out), c_long(out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight), c_int(m), c_int(n), c_int(k),
+        c_int(0 if row_act is None else ROW_ACT[row_act] + 1), c_int(n if act_cols is None else act_cols),
+        c_int(cols or pair_columns(m, n, sms)), c_int(sms), _ptr(status), _stream())
     return out
 
 
@@ -1240,6 +1258,18 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation="silu") ->
     else:
         act_mul(act, gu, activation)
     return act
+
+
+def linear_silu(x: torch.Tensor, weight: torch.Tensor, cols: int) -> torch.Tensor:
+    """x @ weight.T with SiLU on the first ``cols`` columns, applied to the product as its dtype holds it: in the product's
+    epilogue for portions of prompts in bfloat16 (``gemm_pair``; measured on a B200, 6,144 columns of which 4,608, k 1,536,
+    product and kernel / here: 2,048 tokens 30.2 + 11.7 / 31 us, 128 tokens 6.3 + 3 / 9.7), else by a kernel behind it."""
+    if TC_ENABLED and x.shape[0] >= PAIR_MIN_M and pair_supported(x, weight):
+        out = torch.empty((x.shape[0], weight.shape[0]), dtype=x.dtype, device=x.device)
+        return gemm_pair(x, weight, out, row_act="silu", act_cols=cols)
+    out = linear(x, weight)
+    silu_rows(out[:, :cols])
+    return out
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,

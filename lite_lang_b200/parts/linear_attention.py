@@ -79,13 +79,12 @@ class DecayLinearAttention(Mixer):
     def kernel_libraries(self):
         libs = ["core", "linear_attn", "chunk_scan"]
         if self.w_in is not None and self.w_in.dtype == torch.bfloat16:
-            libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc"])
+            libs.extend(["gemm_smallm", "gemm_stream", "gemm_tc", "gemm_pair"])
         return libs
 
     def forward(self, x, step, cache):
         n, dev = x.shape[0], x.device
-        proj = ops.linear(x, self.w_in)
-        ops.silu_rows(proj[:, :self.off["g"]])        # q | k | v (and the zero columns that pad them)
+        proj = ops.linear_silu(x, self.w_in, self.off["g"])        # q | k | v (and the zero columns that pad them)
         o = torch.empty((n, self.Cv), dtype=torch.float32, device=dev)
         ops.decay_scan(proj, self.off["q"], self.off["k"], self.off["v"], self.decay, cache.state, step, o,
                        self.H, self.dk, self.dv, cache.writable)

@@ -1,0 +1,52 @@
+"""Plain products of two SMs a tile: every tile width at the edges of rows, columns and k, and SiLU on the first columns."""
+
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+@gpu
+@pytest.mark.parametrize("cols", [0, 128, 192, 256])
+@pytest.mark.parametrize("m,n,k", [(65, 8, 8), (256, 192, 64), (257, 193, 72), (300, 520, 136), (1030, 1544, 200)])
+def test_tile_widths_and_activated_columns(m, n, k, cols):
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=g, device="cuda") * 2 * k ** -0.5).to(torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    wide = torch.full((m + 1, n + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    product = x.double() @ w.double().T
+    rounded = product.to(torch.bfloat16).double()
+    for act_cols in (0, n // 2 + 1, None):
+        ops.gemm_pair(x, w, wide[:m, :n], status=status, row_act=None if act_cols == 0 else "silu", act_cols=act_cols, cols=cols)
+        first = n if act_cols is None else act_cols
+        # (a float32 sum in another order rounds elsewhere now and then: 2^-8 of a number, twice where SiLU follows)
+        want = torch.cat([torch.nn.functional.silu(rounded[:, :first]), rounded[:, first:]], dim=1)
+        assert float(((wide[:m, :n].double() - want).abs() / (want.abs() + 0.05)).max()) <= 2 ** -6
+        assert float((wide[:m, :n].double() - want).norm() / want.norm()) <= 2 ** -8
+        assert bool((wide[m:] == 7).all()) and bool((wide[:, n:] == 7).all())
+    assert int(status.item()) == 0
+
+
+def test_columns_of_a_tile():
+    from lite_lang_b200 import ops
+    for m in (65, 256, 300, 2048, 5000):
+        for n in (8, 1536, 6144, 18944):
+            assert ops.pair_columns(m, n, 148) in (128, 192, 256)
+    assert ops.pair_columns(2048, 6144, 148) == 256 and ops.pair_columns(2048, 1536, 148) == 192
+
+
+@gpu
+@pytest.mark.parametrize("dtype,m", [(torch.bfloat16, 300), (torch.bfloat16, 40), (torch.float32, 70)])
+def test_product_with_silu_on_its_first_columns(dtype, m):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    x, w = torch.randn(m, 256, generator=g, device="cuda").to(dtype), (torch.randn(200, 256, generator=g, device="cuda") / 8).to(dtype)
+    want = (x.double() @ w.double().T).to(dtype).double()
+    want[:, :136] = torch.nn.functional.silu(want[:, :136])
+    got = ops.linear_silu(x, w, 136).double()
+    assert float((got - want).norm() / want.norm()) <= (1e-5 if dtype == torch.float32 else 2 ** -7)
