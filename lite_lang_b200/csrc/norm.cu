@@ -309,3 +309,36 @@ extern "C" int ll_add_rmsnorm(int dtype, void* out, void* residual, const void* 
   });
   return LL_LAUNCH_RESULT();
 }
+
+// out[i] = the parts' numbers i added up in their order, rounded once.  Four numbers a thread, all parts' loads on their way at
+// once.  (The library's sum over a dimension and a conversion behind it: 4.0 + 1.9 us for 4 parts of 8 x 1,536, two launches.)
+template <typename T>
+__global__ void __launch_bounds__(128)
+sum_parts_kernel(T* __restrict__ out, const float* __restrict__ parts, int n_parts, long numbers) {
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const long i = 4 * ((long)blockIdx.x * 128 + threadIdx.x);
+  if (i >= numbers) return;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int p = 0; p < n_parts; ++p) {
+    const float4 v = *reinterpret_cast<const float4*>(parts + p * numbers + i);
+    a.x += v.x;
+    a.y += v.y;
+    a.z += v.z;
+    a.w += v.w;
+  }
+  out[i] = from_f32<T>(a.x);
+  out[i + 1] = from_f32<T>(a.y);
+  out[i + 2] = from_f32<T>(a.z);
+  out[i + 3] = from_f32<T>(a.w);
+}
+
+// numbers: a multiple of 4
+extern "C" int ll_sum_parts(int dtype, void* out, const float* parts, int n_parts, long numbers, cudaStream_t stream) {
+  if (numbers <= 0) return 0;
+  if (n_parts <= 0 || (numbers % 4) != 0 || ((uintptr_t)parts % 16) != 0) return (int)cudaErrorInvalidValue;
+  LL_DISPATCH_DTYPE(dtype, ll_launch(sum_parts_kernel<T>, dim3((unsigned)((numbers / 4 + 127) / 128)), dim3(128), 0, stream, (T*)out, parts,
+                                     n_parts, numbers));
+  return LL_LAUNCH_RESULT();
+}

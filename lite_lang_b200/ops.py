@@ -148,6 +148,16 @@ def add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: Optional[torch
                 c_int(hidden), _ptr(rows), c_int(wr), _stream())
 
 
+def sum_parts(parts: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """[tokens, n] of ``dtype`` from float32 partial sums [parts, tokens, n], added up in their order and rounded once."""
+    _need_cuda(parts)
+    _f32(parts, "partial sums")
+    out = torch.empty(parts.shape[1:], dtype=dtype, device=parts.device)
+    core().call("ll_sum_parts", c_int(_dtype_code(out)), _ptr(out), _ptr(parts), c_int(parts.shape[0]), c_long(out.numel()),
+                _stream())
+    return out
+
+
 def bias_rope_store(qkv: torch.Tensor, bias: Optional[torch.Tensor], positions: Optional[torch.Tensor],
                     cos_sin: Optional[torch.Tensor], num_heads: int, num_kv_heads: int, head_dim: int,
                     slot_map: Optional[torch.Tensor], k_cache: Optional[torch.Tensor],
