@@ -11,6 +11,7 @@
 // `moe_act` then applies the activation and multiplies every hidden unit by the weight of its expert for that
 // token (1 for the always-on rows, 0 for experts not chosen), so that one second product over all hidden units
 // gives the weighted sum of the chosen experts' outputs plus the always-on expert's.
+#include "mma_split.cuh"
 #include "moe_act.cuh"
 
 #define MOE_MAX_E 256
@@ -24,10 +25,15 @@
 // is added to the scores for the choice.  With `keep` < `count`, only outputs of the `keep` groups (E / count neighbours
 // each) with the largest best choice score can be chosen.  A place that finds nothing left gets top_idx -1 and weight 0.
 //
-// A block takes TOK tokens (one, and then a warp an output; or eight in long portions, four a warp: the router's matrix is
-// then read once for four tokens); its warps share out the outputs, and then the tokens, whose scores a warp each makes and
-// picks from.  Bound by the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row (four sums side by side), then the lanes are added up: an order
-// that depends on the sizes only.
+// Two kernels.  `moe_router_tc_kernel`: portions of bfloat16 rows and at most 32 outputs (experts and the shared one's gate), 16 tokens a
+// block on tensor cores.  `moe_router_kernel`: a block takes TOK tokens: one, with a warp an output, which has asked for the first
+// pieces of its row before the token's was there; or eight in long portions, four a warp: the router's matrix is then read
+// once for four tokens.  Its warps share out the outputs, and then the tokens, whose scores a warp each makes and picks from.  Bound by
+// the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row, then the lanes are added up: an
+// order that depends on the sizes only.  In `moe_pick` a lane has one of at most 32 outputs, and a pick is one maximum over the
+// warp and a ballot.
+// Measured on a B200, hidden 1,536, 16 outputs and a shared gate, 4 chosen (us; multiply-adds / tensor cores): 100 tokens 6.3 / 10,
+// 256 11.4 / 10.4, 512 14.1 / 10.3, 2,048 17.2 / 11.0, 4,096 31.6 / 19.5: the line is 256.
 __device__ __forceinline__ float4 moe_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 moe_load4(const bf16* p) {
   const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -35,73 +41,18 @@ __device__ __forceinline__ float4 moe_load4(const bf16* p) {
   const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
-template <typename T, int TOK, int THREADS>
-__global__ void __launch_bounds__(THREADS)
-moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restrict__ Wr, const float* __restrict__ bias,
-                  float* __restrict__ gates, int* __restrict__ top_idx, float* __restrict__ top_w,
-                  float* __restrict__ shared_w, int num_tokens, int hidden, int E, int top, int score_fn,
-                  int renormalize, const float* __restrict__ choice_bias, int count, int keep, float weight_scale,
-                  float* __restrict__ identity_w, int real, int pitch) {
-  extern __shared__ __align__(16) float moe_smem[];      // [TOK]: logits / scores [E + 1], choice scores [E], groups' best
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  LL_PDL_TRIGGER();
-  LL_PDL_WAIT();
-  const int tok0 = blockIdx.x * TOK, nt = min(TOK, num_tokens - tok0);
-  const int zs = 2 * E + 1 + count;
-  T* xrow = reinterpret_cast<T*>(moe_smem + (TOK * zs + 3) / 4 * 4);     // the tokens' rows, `pitch` apart
-  constexpr int VEC = 16 / (int)sizeof(T);
-  if ((hidden % VEC) == 0 && (x_stride % VEC) == 0 && ((uintptr_t)x % 16) == 0) {
-    const int per = hidden / VEC;
-    for (int i = threadIdx.x; i < nt * per; i += THREADS) {
-      const int k = i / per, c = (i - k * per) * VEC;
-      *reinterpret_cast<uint4*>(xrow + (size_t)k * pitch + c) =
-          *reinterpret_cast<const uint4*>(x + (size_t)(tok0 + k) * x_stride + c);
-    }
-  } else {
-    for (int k = 0; k < nt; ++k)
-      for (int i = threadIdx.x; i < hidden; i += THREADS) xrow[(size_t)k * pitch + i] = x[(size_t)(tok0 + k) * x_stride + i];
-  }
-  __syncthreads();
-  const int n_rows = E + (shared_w ? 1 : 0);
-  const bool vec = (hidden & 3) == 0;
-  constexpr int PER = TOK < 4 ? TOK : 4;                  // tokens of a warp at a time
-  const int units = n_rows * (TOK / PER);
-  for (int i = warp; i < units; i += THREADS / 32) {
-    // (blocks start at different outputs: at the same ones they would all ask the same few lines of L2 at a time)
-    const int un = TOK == 1 ? i : (i + blockIdx.x * 5) % units, e = un / (TOK / PER), k0 = un % (TOK / PER) * PER;
-    const T* xs = xrow + (size_t)k0 * pitch;
-    float a[PER][4];
-#pragma unroll
-    for (int k = 0; k < PER; ++k) a[k][0] = a[k][1] = a[k][2] = a[k][3] = 0.f;
-    const float* wrow = Wr + (size_t)e * hidden;
-    if (vec) {
-#pragma unroll(TOK == 1 ? 8 : 4)
-      for (int i = 4 * lane; i < hidden; i += 128) {
-        const float4 w4 = *reinterpret_cast<const float4*>(wrow + i);
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-          const float4 x4 = moe_load4(xs + (size_t)k * pitch + i);
-          a[k][0] = fmaf(w4.x, x4.x, a[k][0]);
-          a[k][1] = fmaf(w4.y, x4.y, a[k][1]);
-          a[k][2] = fmaf(w4.z, x4.z, a[k][2]);
-          a[k][3] = fmaf(w4.w, x4.w, a[k][3]);
-        }
-      }
-    } else {
-      for (int i = lane; i < hidden; i += 32)
-#pragma unroll
-        for (int k = 0; k < PER; ++k) a[k][0] = fmaf(wrow[i], to_f32<T>(xs[(size_t)k * pitch + i]), a[k][0]);
-    }
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const float v = warp_sum((a[k][0] + a[k][1]) + (a[k][2] + a[k][3]));
-      if (lane == 0 && k0 + k < nt) moe_smem[(k0 + k) * zs + e] = v + ((bias && e < E) ? bias[e] : 0.f);
-    }
-  }
-  __syncthreads();
-  if (warp >= nt) return;                                // (from here on a warp a token)
-  const int t = tok0 + warp;
-  float* z = moe_smem + warp * zs;
+// a float32 number as an unsigned one of the same order; NaN below all, the zeros equal
+__device__ __forceinline__ unsigned moe_order(float v) {
+  const unsigned u = __float_as_uint(v + 0.0f);
+  return v != v ? 0u : (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+// What a token's logits z [E + 1] (by one warp, in shared memory, the choice scores and the groups' best behind them) come to:
+// its scores, its choice and the weights.
+__device__ __forceinline__ void moe_pick(float* z, int t, float* __restrict__ gates, int* __restrict__ top_idx, float* __restrict__ top_w,
+                                         float* __restrict__ shared_w, int E, int top, int score_fn, int renormalize,
+                                         const float* __restrict__ choice_bias, int count, int keep, float weight_scale,
+                                         float* __restrict__ identity_w, int real) {
+  const int lane = threadIdx.x & 31;
   float* cs = z + E + 1;                                 // choice scores
   float* gb = cs + E;                                    // the groups' best
   if (shared_w && lane == 0) shared_w[t] = 1.0f / (1.0f + expf(-z[E]));
@@ -142,22 +93,27 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
   }
   float total = 0.f, ident = 0.f;
   for (int k = 0; k < top; ++k) {
-    float best = -INFINITY;
     int arg = E;
-    for (int e = lane; e < E; e += 32) {
-      const float v = cs[e];
-      if (v > best) {   // (a lane walks upwards, so it keeps its lowest index among equals)
-        best = v;
-        arg = e;
+    if (E <= 32) {
+      const unsigned mine = lane < E ? moe_order(cs[lane]) : 0u, most = __reduce_max_sync(0xffffffffu, mine);
+      if (most > 0x007fffffu) arg = __ffs(__ballot_sync(0xffffffffu, mine == most)) - 1;      // (above minus infinity: something is left)
+    } else {
+      float best = -INFINITY;
+      for (int e = lane; e < E; e += 32) {
+        const float v = cs[e];
+        if (v > best) {   // (a lane walks upwards, so it keeps its lowest index among equals)
+          best = v;
+          arg = e;
+        }
       }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
-      if (ob > best || (ob == best && oa < arg)) {
-        best = ob;
-        arg = oa;
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+        if (ob > best || (ob == best && oa < arg)) {
+          best = ob;
+          arg = oa;
+        }
       }
     }
     if (arg >= E) {       // nothing left to choose
@@ -198,6 +154,174 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
     for (int e = lane; e < real; e += 32) gr[e] = gr[e] / total;
     for (int k = lane; k < top; k += 32) top_w[(size_t)t * top + k] /= total;
   }
+}
+
+template <typename T, int TOK>
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 512)
+moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restrict__ Wr, const float* __restrict__ bias,
+                  float* __restrict__ gates, int* __restrict__ top_idx, float* __restrict__ top_w,
+                  float* __restrict__ shared_w, int num_tokens, int hidden, int E, int top, int score_fn,
+                  int renormalize, const float* __restrict__ choice_bias, int count, int keep, float weight_scale,
+                  float* __restrict__ identity_w, int real, int pitch) {
+  extern __shared__ __align__(16) float moe_smem[];      // [TOK]: logits / scores [E + 1], choice scores [E], groups' best
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int tok0 = blockIdx.x * TOK, nt = min(TOK, num_tokens - tok0);
+  const int zs = 2 * E + 1 + count;
+  T* xrow = reinterpret_cast<T*>(moe_smem + (TOK * zs + 3) / 4 * 4);     // the tokens' rows, `pitch` apart
+  const int n_rows = E + (shared_w ? 1 : 0), warps = blockDim.x >> 5;
+  const bool vec = (hidden & 3) == 0;
+  constexpr int AHEAD = TOK == 1 ? 8 : 0;                 // pieces of the warp's first row that are asked for now
+  float4 head[AHEAD > 0 ? AHEAD : 1];
+  if (AHEAD > 0 && vec && warp < n_rows) {
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (4 * lane + 128 * j < hidden) head[j] = *reinterpret_cast<const float4*>(Wr + (size_t)warp * hidden + 4 * lane + 128 * j);
+  }
+  constexpr int VEC = 16 / (int)sizeof(T);
+  if ((hidden % VEC) == 0 && (x_stride % VEC) == 0 && ((uintptr_t)x % 16) == 0) {
+    const int per = hidden / VEC;
+    for (int i = threadIdx.x; i < nt * per; i += blockDim.x) {
+      const int k = i / per, c = (i - k * per) * VEC;
+      *reinterpret_cast<uint4*>(xrow + (size_t)k * pitch + c) =
+          *reinterpret_cast<const uint4*>(x + (size_t)(tok0 + k) * x_stride + c);
+    }
+  } else {
+    for (int k = 0; k < nt; ++k)
+      for (int i = threadIdx.x; i < hidden; i += blockDim.x) xrow[(size_t)k * pitch + i] = x[(size_t)(tok0 + k) * x_stride + i];
+  }
+  __syncthreads();
+  constexpr int PER = TOK < 4 ? TOK : 4;                  // tokens of a warp at a time
+  const int units = n_rows * (TOK / PER);
+  for (int n = warp; n < units; n += warps) {
+    // (blocks start at different outputs: at the same ones they would all ask the same few lines of L2 at a time)
+    const int un = TOK == 1 ? n : (n + blockIdx.x * 5) % units, e = un / (TOK / PER), k0 = un % (TOK / PER) * PER;
+    const T* xs = xrow + (size_t)k0 * pitch;
+    float a[PER][4];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) a[k][0] = a[k][1] = a[k][2] = a[k][3] = 0.f;
+    const float* wrow = Wr + (size_t)e * hidden;
+    auto add = [&](int i, const float4& w4) {
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        const float4 x4 = moe_load4(xs + (size_t)k * pitch + i);
+        a[k][0] = fmaf(w4.x, x4.x, a[k][0]);
+        a[k][1] = fmaf(w4.y, x4.y, a[k][1]);
+        a[k][2] = fmaf(w4.z, x4.z, a[k][2]);
+        a[k][3] = fmaf(w4.w, x4.w, a[k][3]);
+      }
+    };
+    if (vec) {
+      int i = 4 * lane;
+      if (AHEAD > 0 && n == warp) {
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j, i += 128)
+          if (i < hidden) add(i, head[j]);
+      }
+#pragma unroll(TOK == 1 ? 8 : 4)
+      for (; i < hidden; i += 128) add(i, *reinterpret_cast<const float4*>(wrow + i));
+    } else {
+      for (int i = lane; i < hidden; i += 32)
+#pragma unroll
+        for (int k = 0; k < PER; ++k) a[k][0] = fmaf(wrow[i], to_f32<T>(xs[(size_t)k * pitch + i]), a[k][0]);
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const float v = warp_sum((a[k][0] + a[k][1]) + (a[k][2] + a[k][3]));
+      if (lane == 0 && k0 + k < nt) moe_smem[(k0 + k) * zs + e] = v + ((bias && e < E) ? bias[e] : 0.f);
+    }
+  }
+  __syncthreads();
+  if (warp >= nt) return;                                // (from here on a warp a token)
+  moe_pick(moe_smem + warp * zs, tok0 + warp, gates, top_idx, top_w, shared_w, E, top, score_fn, renormalize, choice_bias, count, keep,
+           weight_scale, identity_w, real);
+}
+
+// Long portions, bfloat16 rows and at most 32 outputs: 16 tokens a block, on tensor cores.  A row is bfloat16 as it is and the
+// router's numbers are three bfloat16 terms that hold all 24 bits, so a product is three of mma.sync, with the leading
+// one's steps added with rounded additions (mma_split.cuh); the block's sixteen warps share out k and meet in shared memory.  (The
+// multiply-adds of 16 tokens and 17 outputs are 29,000 warp instructions with their conversions, these 11,000.)
+#define MOE_TC_TOKENS 16
+#define MOE_TC_WARPS 16
+#define MOE_TC_STEPS 3              // steps of 16 whose numbers are on their way together
+template <int NT>
+__global__ void __launch_bounds__(32 * MOE_TC_WARPS)
+moe_router_tc_kernel(const bf16* __restrict__ x, long x_stride, const float* __restrict__ Wr, const float* __restrict__ bias,
+                     float* __restrict__ gates, int* __restrict__ top_idx, float* __restrict__ top_w, float* __restrict__ shared_w,
+                     int num_tokens, int hidden, int E, int top, int score_fn, int renormalize,
+                     const float* __restrict__ choice_bias, int count, int keep, float weight_scale, float* __restrict__ identity_w,
+                     int real) {
+  extern __shared__ __align__(16) float moe_smem[];      // [16]: logits [E + 1], choice scores [E], groups' best; then the warps' sums
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int tok0 = blockIdx.x * MOE_TC_TOKENS, nt = min(MOE_TC_TOKENS, num_tokens - tok0);
+  const int zs = 2 * E + 1 + count, n_rows = E + (shared_w ? 1 : 0);
+  float* sums = moe_smem + (MOE_TC_TOKENS * zs + 3) / 4 * 4;      // [warps][16][8 NT + 1]
+  const int steps = hidden / 16, each = (steps + MOE_TC_WARPS - 1) / MOE_TC_WARPS;
+  float acc[NT][4], low[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = low[i][j] = 0.f;
+  const bool r0 = g < nt, r1 = g + 8 < nt;
+  const bf16* x0 = x + (size_t)(tok0 + (r0 ? g : 0)) * x_stride + 2 * c;
+  const bf16* x1 = x + (size_t)(tok0 + (r1 ? g + 8 : 0)) * x_stride + 2 * c;
+  const int s1 = min(steps, (warp + 1) * each);
+  for (int s0 = warp * each; s0 < s1; s0 += MOE_TC_STEPS) {
+    unsigned a[MOE_TC_STEPS][1][4];
+    float2 w[MOE_TC_STEPS][NT][2];
+#pragma unroll
+    for (int j = 0; j < MOE_TC_STEPS; ++j) {
+      const int s = s0 + j;
+      const bool on = s < s1;
+      a[j][0][0] = on && r0 ? *reinterpret_cast<const unsigned*>(x0 + 16 * s) : 0u;
+      a[j][0][1] = on && r1 ? *reinterpret_cast<const unsigned*>(x1 + 16 * s) : 0u;
+      a[j][0][2] = on && r0 ? *reinterpret_cast<const unsigned*>(x0 + 16 * s + 8) : 0u;
+      a[j][0][3] = on && r1 ? *reinterpret_cast<const unsigned*>(x1 + 16 * s + 8) : 0u;
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const float* wr = Wr + (size_t)(8 * i + g) * hidden + 16 * s + 2 * c;
+        w[j][i][0] = w[j][i][1] = make_float2(0.f, 0.f);
+        if (on && 8 * i + g < n_rows) {
+          w[j][i][0] = *reinterpret_cast<const float2*>(wr);
+          w[j][i][1] = *reinterpret_cast<const float2*>(wr + 8);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < MOE_TC_STEPS; ++j) {
+      unsigned b[NT][3][2];
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) ms_split(w[j][i][h].x, w[j][i][h].y, b[i][0][h], b[i][1][h], b[i][2][h]);
+      ms_terms<NT, 1, 3>(acc, low, a[j], b);
+    }
+  }
+  constexpr int SP = 8 * NT + 1;
+  float* mine = sums + warp * MOE_TC_TOKENS * SP;
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mine[(g + 8 * (j >> 1)) * SP + 8 * i + 2 * c + (j & 1)] = acc[i][j] + low[i][j];
+  __syncthreads();
+  for (int i = threadIdx.x; i < MOE_TC_TOKENS * n_rows; i += 32 * MOE_TC_WARPS) {
+    const int k = i / n_rows, e = i - k * n_rows;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < MOE_TC_WARPS; ++w) v += sums[(w * MOE_TC_TOKENS + k) * SP + e];
+    if (!(fabsf(v) < INFINITY) && k < nt) {      // (an infinity has no terms: the sum again by multiply-adds)
+      v = 0.f;
+      for (int j = 0; j < hidden; ++j) v = fmaf(Wr[(size_t)e * hidden + j], __bfloat162float(x[(size_t)(tok0 + k) * x_stride + j]), v);
+    }
+    moe_smem[k * zs + e] = v + ((bias && e < E) ? bias[e] : 0.f);
+  }
+  __syncthreads();
+  for (int k = warp; k < nt; k += MOE_TC_WARPS)
+    moe_pick(moe_smem + k * zs, tok0 + k, gates, top_idx, top_w, shared_w, E, top, score_fn, renormalize, choice_bias, count, keep,
+             weight_scale, identity_w, real);
 }
 
 // h: T [tokens, shared_ff + E * ff] in place: h = act(h) * weight, weight 1 for the first shared_ff columns,
@@ -251,23 +375,43 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
     return (int)cudaErrorInvalidValue;
   if (E <= 0 || E > MOE_MAX_E || top <= 0 || top > E || hidden <= 0) return (int)cudaErrorInvalidValue;
   const int zs = 2 * E + 1 + count, pitch = (hidden + 7) / 8 * 8;
-#define MOE_ROUTER_LAUNCH(TOK, THREADS)                                                                                  \
+  const int rows = E + (shared_w != nullptr ? 1 : 0);
+#define MOE_ROUTER_LAUNCH(TOK)                                                                                           \
   do {                                                                                                                   \
     const size_t smem = sizeof(float) * (size_t)((TOK * zs + 3) / 4 * 4) + sizeof(T) * (size_t)TOK * pitch;              \
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;                                                            \
     if (smem > 48 * 1024)                                                                                                \
-      cudaFuncSetAttribute(moe_router_kernel<T, TOK, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-    ll_launch(moe_router_kernel<T, TOK, THREADS>, dim3((num_tokens + TOK - 1) / TOK), dim3(THREADS), smem,               \
-              stream, (const T*)x, x_stride, Wr, bias, gates, top_idx, top_w, shared_w, num_tokens, hidden, E, top,      \
-              score_fn, renormalize, choice_bias, count, keep, weight_scale, identity_w, real, pitch);                   \
+      cudaFuncSetAttribute(moe_router_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+    const int warps = TOK > 1 ? 16 : rows < 32 ? (rows > 8 ? rows : 8) : 32;                                              \
+    ll_launch(moe_router_kernel<T, TOK>, dim3((num_tokens + TOK - 1) / TOK), dim3(32 * warps), smem, stream, (const T*)x, x_stride, \
+              Wr, bias, gates, top_idx, top_w, shared_w, num_tokens, hidden, E, top, score_fn, renormalize, choice_bias, count, \
+              keep, weight_scale, identity_w, real, pitch);                                                              \
   } while (0)
+  if (dtype == LL_DTYPE_BF16 && num_tokens >= 256 && rows <= 32 && hidden % 16 == 0 && x_stride % 2 == 0 && ((uintptr_t)x % 4) == 0 &&
+      ((uintptr_t)Wr % 8) == 0) {
+    const int tiles = (rows + 7) / 8;
+    const size_t smem = sizeof(float) * ((size_t)(MOE_TC_TOKENS * zs + 3) / 4 * 4 + (size_t)MOE_TC_WARPS * MOE_TC_TOKENS * (8 * tiles + 1));
+    const dim3 grid((num_tokens + MOE_TC_TOKENS - 1) / MOE_TC_TOKENS);
+#define MOE_ROUTER_TC(NT)                                                                                                       \
+  case NT:                                                                                                                      \
+    ll_launch(moe_router_tc_kernel<NT>, grid, dim3(32 * MOE_TC_WARPS), smem, stream, (const bf16*)x, x_stride, Wr, bias, gates, top_idx, \
+              top_w, shared_w, num_tokens, hidden, E, top, score_fn, renormalize, choice_bias, count, keep, weight_scale, identity_w, \
+              real);                                                                                                            \
+    break
+    switch (tiles) {
+      MOE_ROUTER_TC(1);
+      MOE_ROUTER_TC(2);
+      MOE_ROUTER_TC(3);
+      MOE_ROUTER_TC(4);
+    }
+#undef MOE_ROUTER_TC
+    return LL_LAUNCH_RESULT();
+  }
   LL_DISPATCH_DTYPE(dtype, {
     if (num_tokens >= 512 && sizeof(float) * 8 * (size_t)zs + sizeof(T) * 8 * (size_t)pitch <= 100 * 1024)
-      MOE_ROUTER_LAUNCH(8, 512);
-    else if (E > 8)
-      MOE_ROUTER_LAUNCH(1, 1024);
+      MOE_ROUTER_LAUNCH(8);
     else
-      MOE_ROUTER_LAUNCH(1, 256);
+      MOE_ROUTER_LAUNCH(1);
   });
 #undef MOE_ROUTER_LAUNCH
   return LL_LAUNCH_RESULT();
