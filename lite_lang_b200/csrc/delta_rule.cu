@@ -63,27 +63,40 @@ template <int VEC> __device__ __forceinline__ void dp_store(float* p, const floa
   else p[0] = v[0];
 }
 
-// TAPS 4: filters of four taps at 16-byte boundaries, all loads of a channel's convolution on their way at once; 0: any.
+// silu of N numbers, to a unit of the last place, without the branch of the compiler's division: the reciprocal instruction with
+// Newton's iteration and the quotient corrected by its remainder (Markstein's scheme); numbers below -87, whose divisor has no
+// reciprocal in range, and infinities, whose remainder is no number, again by the division
+template <int N> __device__ __forceinline__ void dp_silu(float (&v)[N]) {
+  float y[N];
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const float d = 1.0f + expf(-v[k]);
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(fmaf(-d, r, 1.f), r, r);
+    const float q = v[k] * r;
+    y[k] = fmaf(fmaf(-d, q, v[k]), r, q);
+    odd |= !(d < 8.507059e37f && v[k] < INFINITY);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = odd ? dr_silu(v[k]) : y[k];
+}
+
+// What one token's projections of a unit (a q, k or v head, the betas, or decays) come to, by one warp.
 template <typename T, int VEC, int TAPS>
-__global__ void __launch_bounds__(32 * DP_TOKENS)
-delta_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, int k_off, int v_off, int b_off,
-                     const T* __restrict__ a_in, long a_stride, const float* __restrict__ conv_q,
-                     const float* __restrict__ conv_k, const float* __restrict__ conv_v,
-                     const float* __restrict__ A_log, const float* __restrict__ dt_bias, float* state, long state_stride,
-                     long tail_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
-                     const int* __restrict__ ctx_len, const int* __restrict__ req_slot, const int* __restrict__ positions,
-                     float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vc, float* __restrict__ beta,
-                     float* __restrict__ g, int num_tokens, DeltaShape s) {
+__device__ __forceinline__ void delta_prepare_token(
+    int t, int unit, int lane, const T* __restrict__ proj, long proj_stride, int q_off, int k_off, int v_off, int b_off,
+    const T* __restrict__ a_in, long a_stride, const float* __restrict__ conv_q, const float* __restrict__ conv_k,
+    const float* __restrict__ conv_v, const float* __restrict__ A_log, const float* __restrict__ dt_bias, float* state,
+    long state_stride, long tail_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
+    const int* __restrict__ ctx_len, const int* __restrict__ req_slot, const int* __restrict__ positions, float* __restrict__ qn,
+    float* __restrict__ kn, float* __restrict__ vc, float* __restrict__ beta, float* __restrict__ g, const DeltaShape& s) {
   constexpr int PIECES = 8 / VEC;                 // of a q or k head of up to 256 channels: kept between the sum and the output
-  LL_PDL_TRIGGER();
-  LL_PDL_WAIT();
-  const int lane = threadIdx.x & 31, t = blockIdx.x * DP_TOKENS + (threadIdx.x >> 5);
-  if (t >= num_tokens) return;
   const int e = token_req[t];
   const int slot = e >= 0 ? req_slot[e] : -1;
   if (slot < 0) return;   // padding entry: the scan writes its (zero) output
   const int Cq = s.Hk * s.dk, Cv = s.H * s.dv, C = 2 * Cq + Cv, K = s.taps;
-  const int unit = blockIdx.y;
   const T* row = proj + (size_t)t * proj_stride;
   if (unit >= 2 * s.Hk + s.H) {
     if (unit == 2 * s.Hk + s.H) {                 // betas
@@ -199,6 +212,85 @@ delta_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, in
       dp_store<VEC>(dst + c, y[i]);
     }
   }
+}
+
+// TAPS 4: filters of four taps at 16-byte boundaries, all loads of a channel's convolution on their way at once; 0: any.
+// RUN: neighbouring tokens a warp takes of a head.  With more than one (long portions, four taps) the filter's numbers, twice as many
+// bytes as a token's inputs, are read once for them and the inputs once and not four times, all of them on their way
+// together; tokens at an entry's start are served one by one.  2,047 tokens of two entries, 12 heads on 2 of 128: 25 us a token
+// at a time, 18 with eight.
+template <typename T, int VEC, int TAPS, int RUN>
+__global__ void __launch_bounds__(32 * DP_TOKENS)
+delta_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, int k_off, int v_off, int b_off,
+                     const T* __restrict__ a_in, long a_stride, const float* __restrict__ conv_q,
+                     const float* __restrict__ conv_k, const float* __restrict__ conv_v,
+                     const float* __restrict__ A_log, const float* __restrict__ dt_bias, float* state, long state_stride,
+                     long tail_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
+                     const int* __restrict__ ctx_len, const int* __restrict__ req_slot, const int* __restrict__ positions,
+                     float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vc, float* __restrict__ beta,
+                     float* __restrict__ g, int num_tokens, DeltaShape s) {
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int lane = threadIdx.x & 31, t_first = (blockIdx.x * DP_TOKENS + (threadIdx.x >> 5)) * RUN;
+  const int Cq = s.Hk * s.dk, Cv = s.H * s.dv, C = 2 * Cq + Cv, K = s.taps;
+  const int unit = blockIdx.y;
+  if (RUN > 1 && unit < 2 * s.Hk + s.H && t_first + RUN <= num_tokens) {
+    const int e = token_req[t_first], slot = e >= 0 ? req_slot[e] : -1;
+    const int kind = unit < s.Hk ? 0 : unit < 2 * s.Hk ? 1 : 2, head = unit - (kind == 0 ? 0 : kind == 1 ? s.Hk : 2 * s.Hk);
+    const int width = kind == 2 ? s.dv : s.dk, c0 = head * width;
+    // all of one live entry, and so are the three inputs before them; heads of at most 32 accesses of a warp
+    if (slot >= 0 && token_req[t_first + RUN - 1] == e && t_first - 3 >= cu_q[e] && width <= 32 * VEC) {
+      const float* filt = (kind == 0 ? conv_q : kind == 1 ? conv_k : conv_v) + (size_t)c0 * 4;
+      const int c = VEC * lane;
+      const bool on = c < width;
+      const T* col = proj + (size_t)(t_first - 3) * proj_stride + (kind == 0 ? q_off : kind == 1 ? k_off : v_off) + c0 + c;
+      float x[RUN + 3][VEC], f[VEC][4];
+#pragma unroll
+      for (int j = 0; j < RUN + 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) x[j][k] = 0.f;
+        if (on) DpVec<T, VEC>::load(col + (size_t)j * proj_stride, x[j]);
+      }
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) {
+        const float4 w = on ? *reinterpret_cast<const float4*>(filt + (size_t)(c + k) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f[k][0] = w.x;
+        f[k][1] = w.y;
+        f[k][2] = w.z;
+        f[k][3] = w.w;
+      }
+#pragma unroll
+      for (int i = 0; i < RUN; ++i) {
+        float y[VEC];
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {      // oldest input first
+          y[k] = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) y[k] = fmaf(f[k][j], x[i + j][k], y[k]);
+        }
+        dp_silu<VEC>(y);
+        if (kind == 2) {
+          if (on) dp_store<VEC>(vc + (size_t)(t_first + i) * Cv + c0 + c, y);
+          continue;
+        }
+        float ss = 0.f;                      // unit vectors
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) ss = fmaf(y[k], y[k], ss);
+        ss = warp_sum(ss);
+        float inv = 1.0f / sqrtf(ss + 1e-6f);
+        if (kind == 0) inv *= 1.0f / sqrtf((float)s.dk);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) y[k] *= inv;
+        if (on) dp_store<VEC>((kind == 0 ? qn : kn) + (size_t)(t_first + i) * Cq + c0 + c, y);
+      }
+      return;
+    }
+  }
+#pragma unroll 1
+  for (int t = t_first; t < min(t_first + RUN, num_tokens); ++t)
+    delta_prepare_token<T, VEC, TAPS>(t, unit, lane, proj, proj_stride, q_off, k_off, v_off, b_off, a_in, a_stride, conv_q, conv_k,
+                                      conv_v, A_log, dt_bias, state, state_stride, tail_off, token_req, cu_q, ctx_len, req_slot,
+                                      positions, qn, kn, vc, beta, g, s);
 }
 
 // The record's last taps - 1 inputs after the step: inputs of this step where it brought enough tokens,
@@ -457,16 +549,20 @@ extern "C" int ll_delta_prepare(int dtype, const void* proj, long proj_stride, i
   const int esz = dtype == LL_DTYPE_F32 ? 4 : 2;
   const bool vec = dk % 4 == 0 && dv % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && proj_stride % 4 == 0 &&
                    (uintptr_t)proj % (4 * esz) == 0 && ((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)vc) % 16 == 0;
-  const dim3 grid((num_tokens + DP_TOKENS - 1) / DP_TOKENS, units), block(32 * DP_TOKENS);
+  const bool four = vec && taps == 4 && ((uintptr_t)conv_q | (uintptr_t)conv_k | (uintptr_t)conv_v) % 16 == 0;
+  // eight tokens a warp where the portions are long enough for most warps to have a run and there are enough of them (2,047 tokens
+  // of two entries 18 us and 25 one by one; a step of many single tokens would walk through eight of them in turn)
+  const int run = four && num_tokens >= 512 && num_tokens >= 32 * (long)num_entries ? 8 : 1;
+  const dim3 grid((num_tokens + DP_TOKENS * run - 1) / (DP_TOKENS * run), units), block(32 * DP_TOKENS);
 #define DP_ARGS                                                                                                             \
   grid, block, 0, stream, (const T*)proj, proj_stride, q_off, k_off, v_off, b_off, (const T*)a_in, a_stride, conv_q, conv_k, \
       conv_v, A_log, dt_bias, state, state_stride, tail_off, token_req, cu_q, ctx_len, req_slot, positions, qn, kn, vc, beta, \
       g, num_tokens, s
   LL_DISPATCH_DTYPE(dtype, {
-    if (vec && taps == 4 && ((uintptr_t)conv_q | (uintptr_t)conv_k | (uintptr_t)conv_v) % 16 == 0)
-      ll_launch(delta_prepare_kernel<T, 4, 4>, DP_ARGS);
-    else if (vec) ll_launch(delta_prepare_kernel<T, 4, 0>, DP_ARGS);
-    else ll_launch(delta_prepare_kernel<T, 1, 0>, DP_ARGS);
+    if (run > 1) ll_launch(delta_prepare_kernel<T, 4, 4, 8>, DP_ARGS);
+    else if (four) ll_launch(delta_prepare_kernel<T, 4, 4, 1>, DP_ARGS);
+    else if (vec) ll_launch(delta_prepare_kernel<T, 4, 0, 1>, DP_ARGS);
+    else ll_launch(delta_prepare_kernel<T, 1, 0, 1>, DP_ARGS);
     if (taps > 1 && num_tokens != num_entries) {      // (as many tokens as entries: one each)
       const int by = (C + 255) / 256;
       ll_launch(delta_conv_update_kernel<T>, dim3(num_entries, by < 8 ? by : 8), dim3(256), 0, stream, (const T*)proj,
