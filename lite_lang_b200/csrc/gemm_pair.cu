@@ -146,21 +146,37 @@ __device__ __forceinline__ void gp_stage32(unsigned char* stg, int row, int col0
 // step 2 for the CTA's 128 rows.  A work item is 8 columns of the first half of a head and their 8 partners in
 // the second half; a row has 16 of them, and epilogue thread e (of 256) takes item e % 16 of the rows
 // e / 16 + 16 k, k = 0..7: the same head and columns in eight rows.  What it needs from global memory for
-// that (bias, the rows' positions and cache slots) does not depend on the product and is read while the MMAs
-// of the tile still run (gp_qkv_prepare); the rows' cos and sin are asked for one row ahead.
+// that (bias, the rows' positions and cache slots, and from these where the rows go, and the first rows' cos and sin) does not
+// depend on the product and is read while the MMAs of the tile still run (gp_qkv_prepare); later rows' cos and sin are
+// asked for GP_CS_AHEAD rows ahead.  (One row ahead, and the cache rows' places by a division a row: the eight rows took 6,000 to
+// 7,000 clocks of a tile's 25,000.)
+#define GP_CS_AHEAD 3
 struct GpQkvPrep {
   int pos[8];
-  int slot[8];
+  int at[8];             // the row's place, in rows of `stride` from `dst` on; -1: nothing is written
+  bf16* dst;
+  long stride;
+  bool rotate;           // q or k head (v heads: bias and store)
   float b0[8], b1[8];
+  float4 cs[GP_CS_AHEAD][4];   // cos (2) and sin (2) of the next rows
 };
+__device__ __forceinline__ void gp_qkv_ask(const GpParams& p, const GpQkvPrep& w, int i0, int k, float4 (&t)[4]) {
+  const float* src = p.cos_sin + (size_t)w.pos[k] * p.hd + i0;
+  const int half = p.hd >> 1;
+  t[0] = __ldg(reinterpret_cast<const float4*>(src));
+  t[1] = __ldg(reinterpret_cast<const float4*>(src) + 1);
+  t[2] = __ldg(reinterpret_cast<const float4*>(src + half));
+  t[3] = __ldg(reinterpret_cast<const float4*>(src + half) + 1);
+}
 __device__ __forceinline__ void gp_qkv_prepare(const GpParams& p, int e, int row0, int head0, GpQkvPrep& w) {
   const int hd = p.hd, half = hd >> 1, per_head = half >> 3;
   const int pi = e & 15, hl = pi / per_head, i0 = (pi - hl * per_head) << 3, h = head0 + hl;
+  int slot[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int row = row0 + (e >> 4) + 16 * k;
     w.pos[k] = row < p.M ? p.positions[row] : 0;
-    w.slot[k] = (row < p.M && p.slot_map != nullptr) ? p.slot_map[row] : -1;
+    slot[k] = (row < p.M && p.slot_map != nullptr) ? p.slot_map[row] : -1;
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) w.b0[j] = w.b1[j] = 0.f;
@@ -180,45 +196,47 @@ __device__ __forceinline__ void gp_qkv_prepare(const GpParams& p, int e, int row
       set_status(p.status, LL_ERR_POSITION_RANGE);
       w.pos[k] = 0;
     }
-    if ((long)w.slot[k] >= p.num_slots) {
+    if ((long)slot[k] >= p.num_slots) {
       set_status(p.status, LL_ERR_SLOT_RANGE);
-      w.slot[k] = -1;
+      slot[k] = -1;
     }
   }
+  w.rotate = h < p.nh + p.nkv;
+  const int kv = w.rotate ? h - p.nh : h - p.nh - p.nkv;      // (of the cache plane; q heads: not used)
+  w.dst = h < p.nh ? p.out + (size_t)h * hd : w.rotate ? p.k_cache : p.v_cache;
+  w.stride = h < p.nh ? p.out_stride : hd;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int row = row0 + (e >> 4) + 16 * k;
+    w.at[k] = -1;
+    if (h < p.nh) {
+      w.at[k] = row < p.M ? row : -1;
+    } else if (slot[k] >= 0 && h < p.nh + 2 * p.nkv) {
+      const int page = slot[k] / p.page_size;
+      w.at[k] = (page * p.nkv + kv) * p.page_size + slot[k] - page * p.page_size;
+    }
+  }
+  if (w.rotate) {
+#pragma unroll
+    for (int k = 0; k < GP_CS_AHEAD; ++k) gp_qkv_ask(p, w, i0, k, w.cs[k]);
+  }
 }
-__device__ __forceinline__ void gp_qkv_finish(const GpParams& p, const unsigned char* stg, int e, int row0, int head0,
-                                              const GpQkvPrep& w) {
+__device__ __forceinline__ void gp_qkv_finish(const GpParams& p, const unsigned char* stg, int e, int head0, GpQkvPrep& w) {
   const int hd = p.hd, half = hd >> 1, per_head = half >> 3;
   const int pi = e & 15, hl = pi / per_head, i0 = (pi - hl * per_head) << 3, h = head0 + hl;
   if (h >= p.nh + 2 * p.nkv) return;
-  const bool rotate = h < p.nh + p.nkv;   // q or k head; v heads: bias and store
   const int piece = (hl * hd + i0) >> 3;
-  float4 cs[4];                           // cos (2) and sin (2) of the row in hand
-  auto ask = [&](int k, float4 (&t)[4]) {
-    const float* src = p.cos_sin + (size_t)w.pos[k] * hd + i0;
-    t[0] = __ldg(reinterpret_cast<const float4*>(src));
-    t[1] = __ldg(reinterpret_cast<const float4*>(src) + 1);
-    t[2] = __ldg(reinterpret_cast<const float4*>(src + half));
-    t[3] = __ldg(reinterpret_cast<const float4*>(src + half) + 1);
-  };
-  if (rotate) ask(0, cs);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const int r = (e >> 4) + 16 * k, row = row0 + r;
-    float4 nxt[4];
-    if (rotate && k + 1 < 8) ask(k + 1, nxt);
-    bf16* dst = nullptr;
-    if (row < p.M) {
-      if (h < p.nh) {
-        dst = p.out + (size_t)row * p.out_stride + (size_t)h * hd;
-      } else if (w.slot[k] >= 0) {
-        const int page = w.slot[k] / p.page_size;
-        const int off = w.slot[k] - page * p.page_size;
-        dst = rotate ? p.k_cache + (((size_t)page * p.nkv + (h - p.nh)) * p.page_size + off) * hd
-                     : p.v_cache + (((size_t)page * p.nkv + (h - p.nh - p.nkv)) * p.page_size + off) * hd;
-      }
+    const int r = (e >> 4) + 16 * k;
+    float4 cs[4];
+    if (w.rotate) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cs[j] = w.cs[k % GP_CS_AHEAD][j];
+      if (k + GP_CS_AHEAD < 8) gp_qkv_ask(p, w, i0, k + GP_CS_AHEAD, w.cs[k % GP_CS_AHEAD]);
     }
-    if (dst != nullptr) {
+    if (w.at[k] >= 0) {
+      bf16* dst = w.dst + w.at[k] * w.stride + i0;
       float x0[8], x1[8];
       gp_unpack8(*reinterpret_cast<const uint4*>(stg + gp_stg_offset(r, piece)), x0);
       gp_unpack8(*reinterpret_cast<const uint4*>(stg + gp_stg_offset(r, piece + (half >> 3))), x1);
@@ -227,7 +245,7 @@ __device__ __forceinline__ void gp_qkv_finish(const GpParams& p, const unsigned 
         x0[j] += w.b0[j];
         x1[j] += w.b1[j];
       }
-      if (rotate) {
+      if (w.rotate) {
         const float c[8] = {cs[0].x, cs[0].y, cs[0].z, cs[0].w, cs[1].x, cs[1].y, cs[1].z, cs[1].w};
         const float sn[8] = {cs[2].x, cs[2].y, cs[2].z, cs[2].w, cs[3].x, cs[3].y, cs[3].z, cs[3].w};
         float o0[8], o1[8];
@@ -236,16 +254,12 @@ __device__ __forceinline__ void gp_qkv_finish(const GpParams& p, const unsigned 
           o0[j] = x0[j] * c[j] - x1[j] * sn[j];
           o1[j] = x0[j] * sn[j] + x1[j] * c[j];
         }
-        *reinterpret_cast<uint4*>(dst + i0) = gp_pack8(o0);
-        *reinterpret_cast<uint4*>(dst + i0 + half) = gp_pack8(o1);
+        *reinterpret_cast<uint4*>(dst) = gp_pack8(o0);
+        *reinterpret_cast<uint4*>(dst + half) = gp_pack8(o1);
       } else {
-        *reinterpret_cast<uint4*>(dst + i0) = gp_pack8(x0);
-        *reinterpret_cast<uint4*>(dst + i0 + half) = gp_pack8(x1);
+        *reinterpret_cast<uint4*>(dst) = gp_pack8(x0);
+        *reinterpret_cast<uint4*>(dst + half) = gp_pack8(x1);
       }
-    }
-    if (rotate && k + 1 < 8) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cs[j] = nxt[j];
     }
   }
 }
@@ -377,11 +391,13 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
         if (MODE == GP_MODE_QKV) {
           const int r = 32 * ew + lane;
 #pragma unroll 1
-          for (int c = eh * 4; c < eh * 4 + 4; ++c) {
-            unsigned a[32];
-            gp_ld32_issue(taddr + 32 * c, a);
-            gp_ld_wait(a);
-            gp_stage32(stg, r, 32 * c, a);
+          for (int c = eh * 4; c < eh * 4 + 4; c += 2) {
+            unsigned a0[32], a1[32];
+            gp_ld32_issue(taddr + 32 * c, a0);
+            gp_ld32_issue(taddr + 32 * c + 32, a1);
+            gp_ld_wait2(a0, a1);
+            gp_stage32(stg, r, 32 * c, a0);
+            gp_stage32(stg, r, 32 * c + 32, a1);
           }
         } else {
         bf16* out_row = p.out + (size_t)(row < p.M ? row : 0) * p.out_stride;
@@ -436,7 +452,7 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
         if (lane == 0) gp_mbar_arrive_cluster(acc_empty_lead + 8 * b);
         if (MODE == GP_MODE_QKV) {
           asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps: the staged tile is complete
-          gp_qkv_finish(p, stg, tid - 64, mt * 256 + (int)rank * 128, nt * (256 / p.hd), prep);
+          gp_qkv_finish(p, stg, tid - 64, nt * (256 / p.hd), prep);
           asm volatile("bar.sync 1, 256;" ::: "memory");   // it may be overwritten by the next tile
         }
       }
