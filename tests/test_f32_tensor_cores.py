@@ -55,6 +55,31 @@ def test_gated_product(M, I, K, act):
     assert float((got - want).abs().max()) <= 4e-6 * float(want.abs().max())
 
 
+# more tiles than the device has pairs of blocks: the split terms' buffers go from one tile to the next while both run
+@gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("M,N,K", [(701, 17920, 192), (1030, 10248, 136)])
+def test_several_tiles_a_pair(M, N, K, gated):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") * K ** -0.5
+    want, scale = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    bound = (8 + (K + 63) // 64) * 2.0 ** -24 * scale
+    if gated:     # silu(a) * b: a slope of at most 1.1, and a few roundings of the result
+        a, b = want.chunk(2, dim=1)
+        want = torch.nn.functional.silu(a) * b
+        bound = 1.1 * bound[:, :N // 2] * b.abs() + bound[:, N // 2:] * a.abs() + 2.0 ** -21 * want.abs()
+    first = None
+    for _ in range(5):
+        out = torch.empty(M, N // 2 if gated else N, device="cuda")
+        got = ops.gemm_f32(x, w, out, **(dict(gated=ops.GateAct("silu")) if gated else dict(splits=1)))
+        assert bool(((got.double() - want).abs() <= bound + 1e-12).all())
+        assert first is None or torch.equal(first, got)
+        first = got.clone()
+
+
 def test_which_float32_products_go_to_the_tensor_cores():
     from lite_lang_b200 import ops
     x, w = torch.zeros(2048, 1536), torch.zeros(2048, 1536)
