@@ -1517,7 +1517,7 @@ def delta_out(out: torch.Tensor, o: torch.Tensor, weight: torch.Tensor, gate: to
 # --------------------------------------------------------------------------
 def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, eps: float, freq: torch.Tensor,
                    rot_dims: int, positions: torch.Tensor, slot_map: Optional[torch.Tensor], cache: torch.Tensor,
-                   q_full: torch.Tensor, H: int, d: int, r: int, R: int, status: Optional[torch.Tensor],
+                   q_full: Optional[torch.Tensor], H: int, d: int, r: int, R: int, status: Optional[torch.Tensor],
                    amplitude: float = 1.0, q: Optional[torch.Tensor] = None, half_split: bool = False,
                    inplace_from: Optional[int] = None, turn_q: bool = True, cq: Optional[torch.Tensor] = None,
                    cq_norm: Optional[torch.Tensor] = None) -> None:
@@ -1526,7 +1526,7 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Te
     ``q``: the rows that hold the query heads at ``q_off`` when they are not rows of ``proj`` (queries made by a
     second product); ``amplitude``: a factor on cos and sin; ``half_split``: pairs (i, i + rot_dims / 2) instead of
     neighbours.  ``inplace_from``: tokens from there on have their rotated query parts turned where they lie (``q_full``
-    holds the tokens before).  ``turn_q=False``: the queries are left alone.  ``cq`` [tokens, width] with ``cq_norm``: the RMS
+    holds the tokens before; None where there are none).  ``turn_q=False``: the queries are left alone.  ``cq`` [tokens, width] with ``cq_norm``: the RMS
     norm of the first ``width`` numbers of ``proj``'s rows (the queries' own latent), beside the rest."""
     n = proj.shape[0]
     first = n if inplace_from is None else int(inplace_from)
@@ -1542,7 +1542,8 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Te
     _i32(slot_map, "slot_map")
     _need(proj.stride(1) == 1 and cache.is_contiguous() and cache.dtype == proj.dtype and cache.shape[-1] == R + r
           and cache.shape[1] == 1, "latent_prepare: the cache plane is [pages, 1, page, latent + rotated]")
-    _need(q_full.is_contiguous() and q_full.dtype == proj.dtype and tuple(q_full.shape[1:]) == (H, R + r)
+    _need(first == 0 or not turn_q if q_full is None else
+          q_full.is_contiguous() and q_full.dtype == proj.dtype and tuple(q_full.shape[1:]) == (H, R + r)
           and q_full.shape[0] >= min(first, n), "latent_prepare: q_full is [tokens, H, latent + rotated] of the projections' dtype")
     load_library("latent_attn").call(
         "ll_latent_prepare", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), c_int(q_off), c_int(kv_off),

@@ -254,13 +254,13 @@ class LatentAttention(Mixer):
         qrows = proj
         if self.q_rank is not None:          # the queries' own latent: norm (with the cache rows), then the second product
             cq = torch.empty((n, self.q_rank), dtype=x.dtype, device=dev)
-            self._prepare(proj, proj, step, cache, proj.new_empty((0, H, R + r)), 0, cq)
+            self._prepare(proj, proj, step, cache, None, 0, cq)
             qrows = ops.linear(cq, self.w_uq)
         latent, groups = self._runs(step, qrows)
         # (tokens in front of the first expanded portion, the step's single tokens among them, have their rotated parts put
         # where the products over heads write; everybody else's are turned where they lie)
         na, front = (latent[-1][1], latent[0][1] if latent[0][0] == 0 else 0) if latent else (0, 0)
-        q_full = torch.empty((na, H, R + r), dtype=x.dtype, device=dev)
+        q_full = torch.empty((na, H, R + r), dtype=x.dtype, device=dev) if na else None
         if self.q_rank is None or r:
             self._prepare(proj, qrows, step, cache, q_full, front)
         heads = torch.empty((n, H * self.dv), dtype=x.dtype, device=dev)
