@@ -1149,7 +1149,8 @@ def f32_preferred(m: int, n: int, k: int, sms: int, gated: bool = False) -> bool
     64 to 65,536 features and 72 to 18,944 numbers of k).  Few tiles with a gate (its k is not cut; library / here):
     128 x 4,096 x 1,024 34 / 58 us, 1,024 x 4,096 x 1,024 173 / 63; a short k: 128 x 40,000 x 72 28 / 47, 512 x 40,000 x 72
     90 / 75, 96 x 8,192 x 512 26 / 31, 192 x 8,192 x 512 41 / 32.  Else: 96 x 2,048 x 1,536 32 / 28, 128 x 37,888 x 3,584
-    568 / 342; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395."""
+    568 / 342; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395.  (The kernel has
+    become faster since, 701 x 17,920 x 1,536 170 us; the line is where it was, on the library's side of the new one.)"""
     tiles, boxes = ((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64
     splits = 1 if gated else _f32_parts(tiles, boxes, sms)
     rounds = -(-tiles * splits // (sms // 2))
