@@ -52,6 +52,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "moe_act.cuh"
 
 #define LL_ERR_WAIT_TIMEOUT 5
 
@@ -193,6 +194,10 @@ struct GtParams {
   long res_stride;
   const float* norm_w;     // float32 [N]
   float* sumsq_out;        // float32 [N / 16][64]
+  // WIDE with SPLIT, all experts' first matrices: the first shared_ff features belong to an expert for every token, the rest ff
+  // each to E others; gates [M][E]: their weights for the tokens, 0: not chosen; moe_act: see moe_weighted_activation
+  const float* gates;
+  int shared_ff, ff, E, moe_act;
   const float* sumsq_in;   // float32 [sumsq_units][64]; null: no row factor
   int sumsq_units;
   float norm_eps, norm_inv_n;
@@ -214,6 +219,9 @@ template <int MODE, int MT> struct GtStage {
   static constexpr int STAGES = FIT < S::STAGES ? FIT : S::STAGES;
 };
 
+// SPLIT with WIDE: the experts' activation and routing weights on the result, which is rounded to bfloat16 first (a kernel of its
+// own for it took 4.4 us between two products of 25, 8 tokens; the whole part 65.3 -> 60.3 us).  The weights are asked for
+// before a unit's MMAs.  A variant of its own, as the others are, so that the plain products carry none of it.
 // SPLIT: the kernel's part of a norm that is split between the products around it (see GtParams): the NARROW product
 // before the norm, or the GATED product after it, which then has a sixth warp that makes the rows' factors.
 // BLOCKS: more than 32 tokens (NARROW and QKV_ROPE, up to 64): the tokens in blocks of 32 along grid.y, each block
@@ -437,6 +445,21 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
         fr_w[e] = ok ? p.norm_w[n] : 0.f;
       }
     }
+    constexpr bool EXPERTS = SPLIT && MODE == GT_MODE_WIDE && sizeof(OutT) == 2;
+    float ex_w[EXPERTS ? MT : 1][4];
+    if constexpr (EXPERTS) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int f = u * 64 + 16 * warp + g + 8 * h, own = f - p.shared_ff, e = own >= 0 && f < p.N ? own / p.ff : 0;
+#pragma unroll
+        for (int j = 0; j < MT; ++j)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int t = 8 * j + 2 * c + k;
+            ex_w[j][2 * h + k] = own < 0 ? 1.f : t < p.M && f < p.N ? p.gates[(size_t)t * p.E + e] : 0.f;
+          }
+      }
+    }
     const int kc_end = min(kchunks, (kp + 1) * p.cpp);
     for (int kc = kp * p.cpp; kc < kc_end; ++kc) {
       uint4 xv[MYBOXES][2][MT];
@@ -476,7 +499,14 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
     OutT* out = reinterpret_cast<OutT*>(p.out) + (size_t)kp * p.M * p.out_stride;  // this part's [M, N] block
     if (MODE == GT_MODE_WIDE) {
       const int fa = u * 64 + 16 * warp + g, fb = fa + 8;
-      if (sizeof(OutT) == 2 && p.row_act != 0) {
+      if constexpr (EXPERTS) {      // (an expert that was not chosen contributes an exact zero whatever the product gave)
+#pragma unroll
+        for (int j = 0; j < MT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            acc[j][e] = ex_w[j][e] == 0.f ? 0.f
+                                          : moe_weighted_activation(__bfloat162float(__float2bfloat16_rn(acc[j][e])), ex_w[j][e], p.moe_act);
+      } else if (sizeof(OutT) == 2 && p.row_act != 0) {
 #pragma unroll
         for (int j = 0; j < MT; ++j)
 #pragma unroll
@@ -752,6 +782,34 @@ extern "C" int ll_gemm_stream(void* out, long out_stride, int out_f32, const voi
                    : gt_dispatch_m<GT_MODE_NARROW, bf16>(p, w, sm_count, stream);
   }
   return (int)cudaErrorInvalidValue;
+}
+
+// out[M, N] = the experts' activation and weights on x W^T, N = shared_ff + E * ff (see GtParams): wide units, M <= 32.
+extern "C" int ll_gemm_stream_experts(void* out, long out_stride, const void* x, long x_stride, const void* w, int M, int N, int K,
+                                      const float* gates, int shared_ff, int ff, int E, int act, int sm_count, int* status,
+                                      cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 32 || K <= 0 || K % 128 || (x_stride % 8) != 0 || sm_count <= 0 || shared_ff < 0 || ff < 0 || E < 0 ||
+      (long)shared_ff + (long)E * ff != N || (E > 0 && (ff <= 0 || gates == nullptr)))
+    return (int)cudaErrorInvalidValue;
+  GtParams p = {};
+  p.x = (const bf16*)x;
+  p.out = out;
+  p.x_stride = x_stride;
+  p.out_stride = out_stride;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.status = status;
+  p.gates = gates;
+  p.shared_ff = shared_ff;
+  p.ff = ff;
+  p.E = E;
+  p.moe_act = act;
+  p.cpp = K / 128;
+  p.ksplit = 1;
+  p.units = (N + 63) / 64;
+  return gt_dispatch_m<GT_MODE_WIDE, bf16, true>(p, w, sm_count, stream);
 }
 
 // The product before a norm and the product after it, with the norm split between them (see GtParams).

@@ -2201,6 +2201,29 @@ def linear_act(x: torch.Tensor, weight: torch.Tensor, act: str) -> torch.Tensor:
     return out
 
 
+def expert_hidden(x: torch.Tensor, weight: torch.Tensor, gates: torch.Tensor, shared_ff: int, ff: int, E: int, act: str,
+                  weight_in: bool = False) -> torch.Tensor:
+    """The hidden units of all experts' stacked first matrices ``weight`` [shared_ff + E * ff, in], activation and routing weights
+    on (``moe_act``).  Where the product is one of wide units of the weight-streaming kernel with k whole (the ones of few tokens
+    over many hidden units), that kernel's epilogue makes them; else a product and ``moe_act``."""
+    if (x.dtype == torch.bfloat16 and x.shape[0] <= STREAM_M and stream_mode(x, weight) == 0
+            and not (weight.shape[0] >= 8192 and tc_preferred(x, weight, wide=True))):
+        _need_cuda(x, weight, gates)
+        _f32(gates, "gates")
+        n = shared_ff + E * ff
+        _need(tuple(gates.shape) == (x.shape[0], E) and tuple(weight.shape) == (n, x.shape[1]),
+              "expert_hidden: gates are [tokens, experts], weight [shared + experts * ff, in]")
+        out = torch.empty((x.shape[0], n), dtype=x.dtype, device=x.device)
+        load_library("gemm_stream").call(
+            "ll_gemm_stream_experts", _ptr(out), c_long(n), _ptr(x), c_long(x.stride(0)), _ptr(weight), c_int(x.shape[0]), c_int(n),
+            c_int(x.shape[1]), _ptr(gates), c_int(shared_ff), c_int(ff), c_int(E),
+            c_int(MOE_ACT[act] + (MOE_ACT_WEIGHT_IN if weight_in else 0)), c_int(sm_count(x.device)), _ptr(TIMELINE_STATUS), _stream())
+        return out
+    out = linear(x, weight)
+    moe_act(out, gates, shared_ff, ff, E, act, weight_in)
+    return out
+
+
 def act_rows(x: torch.Tensor, act: str) -> None:
     """x <- act(x) in place (float32 arithmetic, one rounding): the activation of a feed-forward without a gate."""
     _need_cuda(x)

@@ -179,12 +179,12 @@ class RoutedExperts(FeedForward):
         if (self.grouped and x.shape[0] >= self.GROUPED_MIN_TOKENS and ops.TC_ENABLED and not getattr(step, "captured", False)
                 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
             return self._forward_grouped(x, idx, wts, getattr(step, "status", None))
-        hidden = ops.linear(x, self.w_up)
         if self.gated:
+            hidden = ops.linear(x, self.w_up)
             hidden = ops.moe_gated_act(hidden, gates, self._shared_w, self.shared_ff, self.ff, self.E, self.limit,
                                        self.shared_limit, self.swish_alpha)
         else:
-            ops.moe_act(hidden, gates, self.shared_ff, self.ff, self.E, self.activation, self.weight_in)
+            hidden = ops.expert_hidden(x, self.w_up, gates, self.shared_ff, self.ff, self.E, self.activation, self.weight_in)
         # (few tokens and many hidden units: float32 partial sums of a split inner dimension, added up by the norm)
         return ops.linear(hidden, self.w_down, partial_ok=True)
 
