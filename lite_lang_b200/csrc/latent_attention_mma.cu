@@ -67,6 +67,7 @@ __device__ __forceinline__ unsigned lm_pack(float lo, float hi) {
 }
 
 __device__ __forceinline__ void lm_cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // the address of this CTA's shared-memory location `addr` in CTA `rank` of the cluster, a store and a load there
@@ -161,6 +162,9 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
     for (int i = split * LM_THREADS + tid; i < hc * R; i += nsplit * LM_THREADS) orow[i] = __float2bfloat16_rn(0.f);
     return;
   }
+  // The parts' meeting below writes into the other CTAs' shared memory, which needs them to have started: everyone says so
+  // here and waits for it there, behind the tiles (a CTA whose share is no tile at all gets there at once).
+  if (nsplit > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   bool dead = false;
   const int units = R / 16, u0 = warp * UPW;      // (fewer than UPW units for the last warps unless 128 UPW = R)
   float o_acc[2 * UPW][4];
@@ -414,6 +418,8 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
   // (Sums handed over by remote stores instead, in pieces of the products' 8 bytes: 7,400 clocks against 5,000.) ----
   const int opitch = R + 8;
   float* osum = reinterpret_cast<float*>(lm_smem);
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // (the arrive is above the tiles)
   if (warp < LM_WARPS) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
