@@ -34,7 +34,7 @@
 #define LM_LOADERS 4              // warps that bring the rows (TMA: the first of them)
 #define LM_THREADS (32 * (LM_WARPS + LM_LOADERS))
 #define LM_HEADS 16
-#define LM_UNITS 4                // units of 16 columns a warp: R / 128 (UPW: 1, 2 or 4 = 512 columns, without a look at R)
+#define LM_UNITS 4                // units of 16 columns a warp, at most (UPW: 1 to 4; the eight warps have 128 UPW columns, at least R)
 #define LM_PPITCH (2 * LM_TK + 16)      // bytes from one head's row of P to the next
 #define LM_MAX_STAGES 3
 #define LM_LOG2E 1.4426950408889634f
@@ -91,8 +91,9 @@ __device__ __forceinline__ void lm_cp_async16(unsigned dst, const void* src, int
 // q: [tokens, H, KD]; cache: one plane [pages, 1, page_size, KD]; out: [tokens, H, R].  `first`: the launch's first
 // token.  gridDim = (tokens, ceil(H / 16), parts), a cluster the parts of a (token, group of heads).  STEPS: steps of 16 of KD
 // a warp takes, half of KD's, whose queries are kept in registers (0: any number, queries from shared memory).  bw: columns a
-// block of a tile; box_rows: rows a box (64 without TMA); `map`: the plane as [KD / bw][rows][bw].
-template <int STEPS, int UPW, bool TMA>
+// block of a tile; box_rows: rows a box (64 without TMA); `map`: the plane as [KD / bw][rows][bw].  FULL: 128 UPW = R, so that
+// every warp has UPW units, without a look at R.
+template <int STEPS, int UPW, bool FULL, bool TMA>
 __global__ void __launch_bounds__(LM_THREADS, 1)
 latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, const bf16* __restrict__ cache,
                             const int* __restrict__ block_table, int bt_stride, const int* __restrict__ token_req,
@@ -166,7 +167,7 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
   // here and waits for it there, behind the tiles (a CTA whose share is no tile at all gets there at once).
   if (nsplit > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   bool dead = false;
-  const int units = R / 16, u0 = warp * UPW;      // (fewer than UPW units for the last warps unless 128 UPW = R)
+  const int units = R / 16, u0 = warp * UPW;      // (fewer than UPW units for the last warps unless FULL)
   float o_acc[2 * UPW][4];
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // rows g and g + 8 (l: this thread's share)
 
@@ -367,7 +368,7 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
         const unsigned vrow = kt + vrow_at[ks];
 #pragma unroll
         for (int u = 0; u < UPW; ++u) {
-          if (UPW == LM_UNITS || u0 + u < units) {
+          if (FULL || u0 + u < units) {
             unsigned b0, b1, b2, b3;
             lm_ldmatrix_x4_trans(b0, b1, b2, b3, vrow + voff[u]);
             lm_mma(o_acc[2 * u], hi[0], hi[1], hi[2], hi[3], b0, b1);
@@ -528,9 +529,11 @@ struct LmArgs {
   int *status, stages, bw, box_rows;
   const float* sink;
 };
-template <int STEPS, int UPW, bool TMA>
+template <int STEPS, int UPW, bool FULL, bool TMA>
 static int lm_launch(const LmArgs& a, const CUtensorMap& map) {
-  auto kernel = latent_attention_mma_kernel<STEPS, UPW, TMA>;
+  static_assert(UPW >= 1 && UPW <= LM_UNITS, "units a warp");
+  if (a.R > 16 * LM_WARPS * UPW || (FULL && a.R != 16 * LM_WARPS * UPW)) return (int)cudaErrorInvalidValue;
+  auto kernel = latent_attention_mma_kernel<STEPS, UPW, FULL, TMA>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
   if (a.grid.z > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   ll_launch_cluster(kernel, a.grid, dim3(LM_THREADS), a.smem, a.stream, (int)a.grid.z, a.out, a.q, a.cache, a.block_table,
@@ -538,9 +541,25 @@ static int lm_launch(const LmArgs& a, const CUtensorMap& map) {
                     a.scale_log2, a.status, a.stages, a.bw, a.box_rows, a.sink, map);
   return LL_LAUNCH_RESULT();
 }
-template <int STEPS, int UPW>
+template <int STEPS, int UPW, bool FULL>
 static int lm_launch(const LmArgs& a, const CUtensorMap& map, bool tma) {
-  return tma ? lm_launch<STEPS, UPW, true>(a, map) : lm_launch<STEPS, UPW, false>(a, map);
+  return tma ? lm_launch<STEPS, UPW, FULL, true>(a, map) : lm_launch<STEPS, UPW, FULL, false>(a, map);
+}
+// Which variant serves a latent of R numbers and r rotated ones: units a warp, whether all warps have as many (R = 512), and the
+// latents that models have (512, alone or with 32 or 64 rotated numbers, and 256 with them), whose steps are straight code.
+struct LmVariant {
+  int steps, upw;
+  bool full;
+};
+static LmVariant lm_variant(int R, int r) {
+  const int steps = (R + r) % 32 == 0 ? (R + r) / 32 : 0;
+  if (R == 512) return {steps >= 16 && steps <= 18 ? steps : 0, 4, true};
+  if (R == 256) return {steps >= 8 && steps <= 10 ? steps : 0, 2, false};
+  return {0, (R + 16 * LM_WARPS - 1) / (16 * LM_WARPS), false};
+}
+// Columns of the result that the variant for these sizes makes (at least R), 0 where there is none
+extern "C" int ll_latent_attention_mma_columns(int R, int r) {
+  return ll_latent_attention_mma_ok(R, r) ? 16 * LM_WARPS * lm_variant(R, r).upw : 0;
 }
 
 // Clusters of `size` CTAs that are resident at once on the current device, a CTA an SM (an SM's shared memory holds one):
@@ -551,7 +570,7 @@ static int lm_resident(int size) {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int n = known[dev][size].load(std::memory_order_relaxed);
   if (n == 0) {
-    auto kernel = latent_attention_mma_kernel<16, 4, true>;
+    auto kernel = latent_attention_mma_kernel<16, 4, true, true>;
     const int smem = 200 * 1024;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -624,18 +643,16 @@ extern "C" int ll_latent_attention_mma(void* out, const void* q, const void* cac
   a.scale_log2 = scale * LM_LOG2E;
   a.status = status;
   a.sink = sink;
-  // the latents that models have (512, alone or with 32 or 64 rotated numbers, and 256 with them): the steps are straight code
-  if (KD % 32 == 0) {
-    const int steps = KD / 32;
-    if (R == 512 && steps == 16) return lm_launch<16, 4>(a, map, tma);
-    if (R == 512 && steps == 17) return lm_launch<17, 4>(a, map, tma);
-    if (R == 512 && steps == 18) return lm_launch<18, 4>(a, map, tma);
-    if (R == 256 && steps == 8) return lm_launch<8, 2>(a, map, tma);
-    if (R == 256 && steps == 9) return lm_launch<9, 2>(a, map, tma);
-    if (R == 256 && steps == 10) return lm_launch<10, 2>(a, map, tma);
-  }
-  if (R <= 128) return lm_launch<0, 1>(a, map, tma);
-  if (R <= 256) return lm_launch<0, 2>(a, map, tma);
-  if (R < 512) return lm_launch<0, 3>(a, map, tma);      // (UPW 4 is all of 512 columns)
-  return lm_launch<0, 4>(a, map, tma);
+  const LmVariant v = lm_variant(R, r);
+  if (v.steps == 16) return lm_launch<16, 4, true>(a, map, tma);
+  if (v.steps == 17) return lm_launch<17, 4, true>(a, map, tma);
+  if (v.steps == 18) return lm_launch<18, 4, true>(a, map, tma);
+  if (v.steps == 8) return lm_launch<8, 2, false>(a, map, tma);
+  if (v.steps == 9) return lm_launch<9, 2, false>(a, map, tma);
+  if (v.steps == 10) return lm_launch<10, 2, false>(a, map, tma);
+  if (v.full) return lm_launch<0, 4, true>(a, map, tma);
+  if (v.upw == 1) return lm_launch<0, 1, false>(a, map, tma);
+  if (v.upw == 2) return lm_launch<0, 2, false>(a, map, tma);
+  if (v.upw == 3) return lm_launch<0, 3, false>(a, map, tma);
+  return lm_launch<0, 4, false>(a, map, tma);
 }

@@ -16,10 +16,12 @@ gpu = pytest.mark.gpu
 
 @gpu
 # R, r: blocks of 64 columns (512, 512 + 64, 256 + 64, 384), of 32 (512 + 32, 256 + 32), of 16 (64 + 16); 1,024: one stage.
+# 416, 448, 480: four units of 16 columns a warp, not all of which are there.
 # pages of 8 to 128 rows are boxes, of 4 and 12 come row by row.
 @pytest.mark.parametrize("H,R,r,page", [(12, 512, 0, 16), (16, 512, 64, 32), (3, 512, 32, 8), (28, 256, 0, 64), (5, 256, 64, 128),
                                         (17, 256, 32, 16), (2, 384, 0, 16), (4, 64, 16, 16), (2, 512, 512, 16), (3, 512, 0, 12),
-                                        (4, 160, 32, 4)])
+                                        (4, 160, 32, 4), (2, 416, 0, 16), (3, 416, 32, 12), (12, 448, 0, 16), (2, 448, 64, 32),
+                                        (5, 480, 0, 8), (4, 480, 32, 4)])
 def test_keys_shared_out_over_clusters(H, R, r, page):
     from lite_lang_b200 import ops
     assert ops.latent_attention_heads(torch.bfloat16, R, r) == 16
@@ -63,6 +65,20 @@ def test_keys_shared_out_over_clusters(H, R, r, page):
             got = out.float().cpu().numpy().reshape(n + 1, -1)
             assert rel_err(got[:n], want) <= kernel_tol(torch.bfloat16), (window, nsplit)
             assert not got[n].any()
+
+
+def test_every_latent_width_has_warps_for_all_its_columns():
+    from ctypes import c_int
+    from lite_lang_b200.ops import load_library
+    lib = load_library("latent_attn")
+    taken = 0
+    for R in range(16, 528, 16):
+        for r in range(0, 528, 16):
+            if lib.fn("ll_latent_attention_mma_ok")(c_int(R), c_int(r)):
+                taken += 1
+                columns = lib.fn("ll_latent_attention_mma_columns")(c_int(R), c_int(r))
+                assert R <= columns < R + 128, (R, r, columns)
+    assert taken > 400
 
 
 @gpu
