@@ -232,7 +232,8 @@ __device__ __forceinline__ float gf_divide(float x, float d) {
   return fmaf(fmaf(-d, y, x), r, y);
 }
 // The activation of 64 pairs (gate numbers, then up numbers) to dst[0 .. left - 1].  (The divisions of ll_gated, with a branch
-// each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some divisor was above 2^126, or NaN.
+// each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some pair has to be made again by the division: a
+// divisor above 2^126 has no reciprocal in range, an infinite gate's quotient no remainder; or NaN.
 template <int ACT>
 __device__ __forceinline__ bool gf_gate_row(float* dst, const float (&v)[128], int left, const GateAct& k) {
   bool odd = false;
@@ -248,7 +249,7 @@ __device__ __forceinline__ bool gf_gate_row(float* dst, const float (&v)[128], i
         const float a = ACT == 2 ? fminf(g, k.limit) : g;
         const float z = ACT == 2 ? k.alpha * a : ACT == 3 ? 1.5957691216057308f * (a + 0.044715f * a * a * a) : a;
         const float d = 1.0f + expf(-z);
-        odd |= !(d < 8.507059e37f);
+        odd |= !(d < 8.507059e37f && a < INFINITY);
         o[j] = gf_divide(a, d) * (ACT == 2 ? fminf(fmaxf(u, -k.limit), k.limit) + 1.0f : u);
       }
     }

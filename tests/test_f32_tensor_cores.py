@@ -55,6 +55,38 @@ def test_gated_product(M, I, K, act):
     assert float((got - want).abs().max()) <= 4e-6 * float(want.abs().max())
 
 
+# gate sums that are far out: each beside the same product without a gate and the activation's own kernel, whose sums are the same
+# numbers.  Finite inputs whose sums overflow to infinity, gates whose exponential leaves float32, and ordinary ones between them.
+@gpu
+@pytest.mark.parametrize("act", ["silu", "relu", "gelu_tanh", "clamped_swish"])
+def test_gates_that_overflow_and_vanish(act):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    M, I, K = 130, 192, 64
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    x = torch.randn(M, K, generator=g, device="cuda")
+    w = torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5
+    w[:, 1] = 0
+    w[:16, 1] = 1e19                                 # sums of 1e39, whose lower terms' products stay finite: +inf in some rows, -inf
+    x[:20, 1], x[20:40, 1] = 1e20, -1e20             # in others, beside ordinary ones
+    x[40:90, 1:] = 0                                 # one number a row and one a gate: sums of exactly their product, -85 to -105
+    x[40:90, 0] = torch.linspace(85, 105, 50, device="cuda")
+    w[32:40, 0] = -1.0
+    w[40:48, 0] = 1.0
+    kind = ops.GateAct(act, 2.0 if act == "clamped_swish" else 0.0, 1.702)
+    got = ops.gemm_f32(x, w, torch.empty(M, I, device="cuda"), gated=kind)
+    sums = ops.gemm_f32(x, w, splits=1)
+    assert bool(torch.isposinf(sums[:20, :16]).all()) and bool(torch.isneginf(sums[20:40, :16]).all())
+    want = torch.empty(M, I, device="cuda")
+    ops.act_mul(want, sums, kind)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    # (a quotient that is one unit of the last place off, times the same number)
+    assert bool(((got - want)[fine].abs() <= 2.0 ** -22 * want[fine].abs() + 1e-44).all())
+
+
 # more tiles than the device has pairs of blocks: the split terms' buffers go from one tile to the next while both run
 @gpu
 @pytest.mark.parametrize("gated", [False, True])
