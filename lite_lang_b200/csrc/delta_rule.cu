@@ -63,26 +63,6 @@ template <int VEC> __device__ __forceinline__ void dp_store(float* p, const floa
   else p[0] = v[0];
 }
 
-// silu of N numbers, to a unit of the last place, without the branch of the compiler's division: the reciprocal instruction with
-// Newton's iteration and the quotient corrected by its remainder (Markstein's scheme); numbers below -87, whose divisor has no
-// reciprocal in range, and infinities, whose remainder is no number, again by the division
-template <int N> __device__ __forceinline__ void dp_silu(float (&v)[N]) {
-  float y[N];
-  bool odd = false;
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const float d = 1.0f + expf(-v[k]);
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(fmaf(-d, r, 1.f), r, r);
-    const float q = v[k] * r;
-    y[k] = fmaf(fmaf(-d, q, v[k]), r, q);
-    odd |= !(d < 8.507059e37f && v[k] < INFINITY);
-  }
-#pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = odd ? dr_silu(v[k]) : y[k];
-}
-
 // What one token's projections of a unit (a q, k or v head, the betas, or decays) come to, by one warp.
 template <typename T, int VEC, int TAPS>
 __device__ __forceinline__ void delta_prepare_token(
@@ -268,7 +248,7 @@ delta_prepare_kernel(const T* __restrict__ proj, long proj_stride, int q_off, in
 #pragma unroll
           for (int j = 0; j < 4; ++j) y[k] = fmaf(f[k][j], x[i + j][k], y[k]);
         }
-        dp_silu<VEC>(y);
+        ll_silu_all<VEC>(y);
         if (kind == 2) {
           if (on) dp_store<VEC>(vc + (size_t)(t_first + i) * Cv + c0 + c, y);
           continue;

@@ -222,15 +222,6 @@ __device__ __noinline__ float gf_plain(const float* x, const float* w, int k0, i
   return s;
 }
 
-// x / d for d of 1 to 2^126, rounded to within a unit of the last place: the reciprocal instruction, Newton's iteration on it and
-// the quotient corrected by its remainder (Markstein's scheme), without the branch of the compiler's division
-__device__ __forceinline__ float gf_divide(float x, float d) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(fmaf(-d, r, 1.f), r, r);
-  const float y = x * r;
-  return fmaf(fmaf(-d, y, x), r, y);
-}
 // The activation of 64 pairs (gate numbers, then up numbers) to dst[0 .. left - 1].  (The divisions of ll_gated, with a branch
 // each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some pair has to be made again by the division: a
 // divisor above 2^126 has no reciprocal in range, an infinite gate's quotient no remainder; or NaN.
@@ -241,18 +232,7 @@ __device__ __forceinline__ bool gf_gate_row(float* dst, const float (&v)[128], i
   for (int i = 0; i < 64; i += 4) {
     float o[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float g = v[i + j], u = v[64 + i + j];
-      if (ACT == 1) {
-        o[j] = fmaxf(g, 0.f) * u;
-      } else {
-        const float a = ACT == 2 ? fminf(g, k.limit) : g;
-        const float z = ACT == 2 ? k.alpha * a : ACT == 3 ? 1.5957691216057308f * (a + 0.044715f * a * a * a) : a;
-        const float d = 1.0f + expf(-z);
-        odd |= !(d < 8.507059e37f && a < INFINITY);
-        o[j] = gf_divide(a, d) * (ACT == 2 ? fminf(fmaxf(u, -k.limit), k.limit) + 1.0f : u);
-      }
-    }
+    for (int j = 0; j < 4; ++j) o[j] = ll_gated_divide<ACT>(v[i + j], v[64 + i + j], k, odd);
     if (i < left) *reinterpret_cast<float4*>(dst + i) = make_float4(o[0], o[1], o[2], o[3]);      // (N is a multiple of 4)
   }
   return odd;

@@ -59,3 +59,33 @@ def test_runs_of_tokens(dtype, H, Hk, dk, dv, lens):
         inf = torch.isinf(y)
         assert torch.equal(inf, torch.isinf(ours)) and bool(((ours - y).abs()[~inf] <= bound[~inf]).all())
         assert torch.equal(on[slots[e], tail_off:].cpu().view(taps - 1, C), x[-(taps - 1):].float())
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_token_has_the_same_bits_in_a_run_and_alone(dtype):
+    """A prompt's 600 tokens at once (eight a warp) and in portions of 100 (one a warp)."""
+    from lite_lang_b200 import ops
+    g = torch.Generator().manual_seed(2)
+    n, H, Hk, dk, dv, taps = 600, 4, 2, 128, 128, 4
+    Cq, Cv = Hk * dk, H * dv
+    C = 2 * Cq + Cv
+    proj = (3.0 * torch.randn(n, C + H, generator=g)).to(dtype).to(dev())
+    a_in = torch.randn(n, H, generator=g).to(dtype).to(dev())
+    w = [torch.randn(c, taps, generator=g).to(dev()) for c in (Cq, Cq, Cv)]
+    A_log, dt_bias = torch.randn(H, generator=g).to(dev()), torch.randn(H, generator=g).to(dev())
+    tail_off = H * dk * dv
+
+    def made(each):
+        state = torch.zeros(2, tail_off + (taps - 1) * C, device=dev())
+        outs = []
+        for at in range(0, n, each):
+            f32 = dict(dtype=torch.float32, device=dev())
+            o = [torch.empty(each, c, **f32) for c in (Cq, Cq, Cv, H, H)]
+            ops.delta_prepare(proj[at:at + each], 0, Cq, 2 * Cq, C, a_in[at:at + each], *w, A_log, dt_bias, state, tail_off,
+                              _step([each], [at], [1]), *o, H, Hk, dk, dv, taps, False)
+            outs.append(torch.cat(o, dim=1))
+        return torch.cat(outs), state[1, tail_off:].clone()
+
+    (runs, tail), (alone, tail_alone) = made(n), made(100)
+    assert torch.equal(runs, alone) and torch.equal(tail, tail_alone)

@@ -82,9 +82,26 @@ def test_gates_that_overflow_and_vanish(act):
     ops.act_mul(want, sums, kind)
     assert torch.equal(got.isnan(), want.isnan())
     assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
-    fine = want.isfinite()
-    # (a quotient that is one unit of the last place off, times the same number)
-    assert bool(((got - want)[fine].abs() <= 2.0 ** -22 * want[fine].abs() + 1e-44).all())
+    assert torch.equal(got[want.isfinite()], want[want.isfinite()])
+
+
+# the epilogue's quotients are the division's: every number of ordinary gates, and of ones spread over the exponential's range
+@gpu
+@pytest.mark.parametrize("spread", [0.02, 1.0, 30.0])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "clamped_swish"])
+def test_the_gate_has_the_bits_of_its_own_kernel(act, spread):
+    from lite_lang_b200 import ops
+    ops.configure_matmul_precision()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    x = torch.randn(700, 128, generator=g, device="cuda")
+    w = torch.randn(2 * 2048, 128, generator=g, device="cuda") * 128 ** -0.5
+    w[:2048] *= spread
+    kind = ops.GateAct(act, 7.0 if act == "clamped_swish" else 0.0, 1.702)
+    got = ops.gemm_f32(x, w, torch.empty(700, 2048, device="cuda"), gated=kind)
+    want = torch.empty(700, 2048, device="cuda")
+    ops.act_mul(want, ops.gemm_f32(x, w, splits=1), kind)
+    assert torch.equal(got, want)
 
 
 # more tiles than the device has pairs of blocks: the split terms' buffers go from one tile to the next while both run
