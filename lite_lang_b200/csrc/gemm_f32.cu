@@ -223,19 +223,18 @@ __device__ __noinline__ float gf_plain(const float* x, const float* w, int k0, i
 }
 
 // The activation of 64 pairs (gate numbers, then up numbers) to dst[0 .. left - 1].  (The divisions of ll_gated, with a branch
-// each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some pair has to be made again by the division: a
-// divisor above 2^126 has no reciprocal in range, an infinite gate's quotient no remainder; or NaN.
+// each, made a tile's end 26,000 clocks, eight of its 24 steps.)  Returns whether some pair has to be made again by the division.
 template <int ACT>
 __device__ __forceinline__ bool gf_gate_row(float* dst, const float (&v)[128], int left, const GateAct& k) {
-  bool odd = false;
+  DivideMet met;
 #pragma unroll
   for (int i = 0; i < 64; i += 4) {
     float o[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = ll_gated_divide<ACT>(v[i + j], v[64 + i + j], k, odd);
+    for (int j = 0; j < 4; ++j) o[j] = ll_gated_divide<ACT>(v[i + j], v[64 + i + j], k, met);
     if (i < left) *reinterpret_cast<float4*>(dst + i) = make_float4(o[0], o[1], o[2], o[3]);      // (N is a multiple of 4)
   }
-  return odd;
+  return met.far();
 }
 
 template <bool GATED>

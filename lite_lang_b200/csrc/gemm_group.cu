@@ -258,21 +258,17 @@ gemm_group_kernel(const GgParams p, const __grid_constant__ CUtensorMap w_shared
         constexpr int PIECES = GATED ? 8 : 16, STEP = 256 / PIECES, MINE = 128 / STEP;      // 16 bytes of features; a thread's rows
         const int piece = e & (PIECES - 1), j0 = e / PIECES, f = o.ft * FT + (int)rank * (FT / 2) + 8 * piece;
         const bool weigh = GATED || p.act >= 0;
-        float w[2][MINE];           // the thread's rows' weights: asked for while the MMAs run
-        if (weigh) {
-#pragma unroll
-          for (int i = 0; i < 2 * MINE; ++i) {
-            const int j = (i / MINE) * 128 + j0 + (i % MINE) * STEP;
-            w[i / MINE][i % MINE] = (g_w != nullptr && j < o.n) ? g_w[o.row + j] : 1.f;
-          }
-        }
+        // the weight of the thread's r-th row of the tile, asked for a row ahead (the first one while the MMAs run)
+        auto ask = [&](int r) {
+          const int j = r / MINE * 128 + j0 + (r % MINE) * STEP;
+          return weigh && g_w != nullptr && j < o.n ? g_w[o.row + j] : 1.f;
+        };
+        float w_next = ask(0);
         gp_mbar_wait(acc_full0 + 8 * b, (unsigned)((tl >> 1) & 1), p.status, dead);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned taddr = tmem + ((unsigned)(32 * ew) << 16) + (unsigned)(b * 256);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int c0 = 128 * h;
-          if (c0 >= o.nw) break;
+#pragma unroll 1
+        for (int c0 = 0; c0 < o.nw; c0 += 128) {
           {
             unsigned v0[32], v1[32];
             const int c = c0 + 64 * eh;
@@ -295,24 +291,34 @@ gemm_group_kernel(const GgParams p, const __grid_constant__ CUtensorMap w_shared
             if (lane == 0) gp_mbar_arrive_cluster(acc_empty_lead + 8 * b);
           }
           asm volatile("bar.sync 1, 256;" ::: "memory");   // 128 rows are staged
-          if (f < g_N) {
+          if (f < g_N && !weigh) {
 #pragma unroll
             for (int i = 0; i < MINE; ++i) {
               const int j = j0 + i * STEP;
-              if (c0 + j < o.n) {
-                const unsigned char* src = stg + j * 256 + 16 * piece;
-                uint4 out = *reinterpret_cast<const uint4*>(src);
-                if (weigh) {
-                  float z[8], u[8];
-                  gp_unpack8(out, z);
-                  if (GATED) gp_unpack8(*reinterpret_cast<const uint4*>(src + 128), u);
-                  if (GATED) ll_gated_any<8>(z, u, gate);
+              if (c0 + j < o.n)
+                *reinterpret_cast<uint4*>(g_out + (size_t)(o.row + c0 + j) * g_N + f) =
+                    *reinterpret_cast<const uint4*>(stg + j * 256 + 16 * piece);
+            }
+          } else if (f < g_N) {
+#pragma unroll 1
+            for (int i = 0; i < MINE; ++i) {      // (eight or sixteen copies of the activations' code left the instruction cache)
+              const int j = j0 + i * STEP;
+              const float w = w_next;
+              w_next = ask(c0 / 128 * MINE + i + 1);
+              if (c0 + j >= o.n) break;
+              const unsigned char* src = stg + j * 256 + 16 * piece;
+              float z[8];
+              gp_unpack8(*reinterpret_cast<const uint4*>(src), z);
+              if (GATED) {
+                float u[8];
+                gp_unpack8(*reinterpret_cast<const uint4*>(src + 128), u);
+                ll_gated_any<8>(z, u, gate);
 #pragma unroll
-                  for (int k = 0; k < 8; ++k) z[k] = GATED ? z[k] * w[h][i] : moe_weighted_activation(z[k], w[h][i], p.act);
-                  out = gp_pack8(z);
-                }
-                *reinterpret_cast<uint4*>(g_out + (size_t)(o.row + c0 + j) * g_N + f) = out;
+                for (int k = 0; k < 8; ++k) z[k] *= w;
+              } else {
+                moe_weighted_act_any<8>(z, w, p.act);
               }
+              *reinterpret_cast<uint4*>(g_out + (size_t)(o.row + c0 + j) * g_N + f) = gp_pack8(z);
             }
           }
           asm volatile("bar.sync 1, 256;" ::: "memory");   // they may be overwritten

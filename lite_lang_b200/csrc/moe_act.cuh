@@ -19,3 +19,24 @@ __device__ __forceinline__ float moe_activation(float z, int act) {
 __device__ __forceinline__ float moe_weighted_activation(float z, float w, int act) {
   return (act & MOE_ACT_WEIGHT_IN) ? moe_activation(z * w, act & 15) : moe_activation(z, act) * w;
 }
+// N numbers with the same weight, the choice outside: the same bits
+template <int ACT, int N> __device__ __forceinline__ void moe_weighted_act_all(float (&z)[N], float w, bool weight_in) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] * w : z[i];
+  if (ACT == 1) {
+    ll_silu_all<N>(z);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) z[i] = moe_activation(z[i], ACT);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] : z[i] * w;
+}
+template <int N> __device__ __forceinline__ void moe_weighted_act_any(float (&z)[N], float w, int act) {
+  const bool in = (act & MOE_ACT_WEIGHT_IN) != 0;
+  act &= MOE_ACT_WEIGHT_IN - 1;
+  if (act == 0) moe_weighted_act_all<0, N>(z, w, in);
+  else if (act == 1) moe_weighted_act_all<1, N>(z, w, in);
+  else if (act == 2) moe_weighted_act_all<2, N>(z, w, in);
+  else moe_weighted_act_all<3, N>(z, w, in);
+}

@@ -90,6 +90,26 @@ def test_up_and_down_products_of_runs(counts, n, k, shared):
 
 
 @gpu
+@pytest.mark.parametrize("name,weight_in", [("relu2", False), ("silu", True), ("silu", False), ("gelu_tanh", True), ("gelu", False)])
+def test_epilogue_without_a_gate_has_the_bits_of_the_activation_kernel(name, weight_in):
+    """The product as one without an activation makes it, and the kernel for rows behind it; numbers far out among them."""
+    from lite_lang_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(9)
+    counts, n, k = (700, 3, 0, 321), 520, 512
+    ends = torch.cumsum(torch.tensor(counts), 0).to(torch.int32).cuda()
+    total = sum(counts)
+    rows, w = _bf16(total, k, gen=gen), _bf16(len(counts), n, k, gen=gen, std=4 * k ** -0.5)
+    w[0] *= 16.0
+    rows[9, 7] = float("-inf")
+    row_w = torch.rand(total, generator=gen, device="cuda")
+    got, _ = ops.expert_products(rows, w, ends, False, name, row_w, weight_in)
+    want, _ = ops.expert_products(rows, w, ends)
+    ops.moe_row_act(want, row_w, name, weight_in)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~got.isnan()], want[~want.isnan()])
+
+
+@gpu
 def test_many_groups_and_refusals():
     from lite_lang_b200 import ops
     gen = torch.Generator(device="cuda")
