@@ -110,6 +110,29 @@ def test_epilogue_without_a_gate_has_the_bits_of_the_activation_kernel(name, wei
 
 
 @gpu
+@pytest.mark.parametrize("limit,limit_s", [(0.0, 0.0), (7.0, 3.0)])
+def test_gated_epilogue_has_the_bits_of_the_activation_kernel(limit, limit_s):
+    """The gate and up products as a product without an activation makes them, and the kernel for rows behind it."""
+    from lite_lang_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(8)
+    counts, n, k, tokens = (700, 3, 0, 321), 520, 512, 600
+    ends = torch.cumsum(torch.tensor(counts), 0).to(torch.int32).cuda()
+    total, E = sum(counts), len(counts)
+    rows, x = _bf16(total, k, gen=gen), _bf16(tokens, k, gen=gen)
+    w, ws = _bf16(E, 2 * n, k, gen=gen, std=4 * k ** -0.5), _bf16(2 * n, k, gen=gen, std=4 * k ** -0.5)
+    w[0, :n] *= 8.0                                                      # gates of 30 and more: far into the exponential's range
+    x[5, 3], rows[9, 7] = float("inf"), float("-inf")
+    row_w, shared_w = torch.rand(total, generator=gen, device="cuda"), torch.rand(tokens, generator=gen, device="cuda")
+    act = ops.GateAct("clamped_swish", limit, 1.702) if limit else ops.GateAct("silu")
+    out, out_s = ops.expert_products(rows, w, ends, True, act, row_w, x=x, shared=ws, shared_w=shared_w, shared_limit=limit_s)
+    z, z_s = ops.expert_products(rows, w, ends, x=x, shared=ws)
+    for got, two, weight, lim in ((out, z, row_w, limit), (out_s, z_s, shared_w, limit_s)):
+        want = ops.moe_row_gated_act(two, weight, lim, 1.702)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~got.isnan()], want[~want.isnan()])
+
+
+@gpu
 def test_many_groups_and_refusals():
     from lite_lang_b200 import ops
     gen = torch.Generator(device="cuda")
