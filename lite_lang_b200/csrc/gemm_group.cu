@@ -319,7 +319,8 @@ gemm_group_kernel(const GgParams p, const __grid_constant__ CUtensorMap w_shared
 #pragma unroll
                 for (int k = 0; k < 8; ++k) z[k] *= w;
               } else {
-                moe_weighted_act_any<8>(z, w, p.act);
+                const float ws[8] = {w, w, w, w, w, w, w, w};
+                moe_weighted_act_any<8>(z, ws, p.act);
               }
               *reinterpret_cast<uint4*>(g_out + (size_t)(o.row + c0 + j) * g_N + f) = gp_pack8(z);
             }

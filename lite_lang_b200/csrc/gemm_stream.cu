@@ -501,11 +501,14 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
       const int fa = u * 64 + 16 * warp + g, fb = fa + 8;
       if constexpr (EXPERTS) {      // (an expert that was not chosen contributes an exact zero whatever the product gave)
 #pragma unroll
-        for (int j = 0; j < MT; ++j)
+        for (int j = 0; j < MT; ++j) {
+          float z[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            acc[j][e] = ex_w[j][e] == 0.f ? 0.f
-                                          : moe_weighted_activation(__bfloat162float(__float2bfloat16_rn(acc[j][e])), ex_w[j][e], p.moe_act);
+          for (int e = 0; e < 4; ++e) z[e] = __bfloat162float(__float2bfloat16_rn(acc[j][e]));
+          moe_weighted_act_any<4>(z, ex_w[j], p.moe_act);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] = ex_w[j][e] == 0.f ? 0.f : z[e];
+        }
       } else if (sizeof(OutT) == 2 && p.row_act != 0) {
 #pragma unroll
         for (int j = 0; j < MT; ++j)

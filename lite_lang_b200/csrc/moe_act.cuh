@@ -19,10 +19,11 @@ __device__ __forceinline__ float moe_activation(float z, int act) {
 __device__ __forceinline__ float moe_weighted_activation(float z, float w, int act) {
   return (act & MOE_ACT_WEIGHT_IN) ? moe_activation(z * w, act & 15) : moe_activation(z, act) * w;
 }
-// N numbers with the same weight, the choice outside: the same bits
-template <int ACT, int N> __device__ __forceinline__ void moe_weighted_act_all(float (&z)[N], float w, bool weight_in) {
+// N numbers and their weights, the choice outside: the same bits from a quarter of the code (an epilogue runs it once a unit of work,
+// from memory that the instruction cache does not hold yet)
+template <int ACT, int N> __device__ __forceinline__ void moe_weighted_act_all(float (&z)[N], const float (&w)[N], bool weight_in) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] * w : z[i];
+  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] * w[i] : z[i];
   if (ACT == 1) {
     ll_silu_all<N>(z);
   } else {
@@ -30,9 +31,9 @@ template <int ACT, int N> __device__ __forceinline__ void moe_weighted_act_all(f
     for (int i = 0; i < N; ++i) z[i] = moe_activation(z[i], ACT);
   }
 #pragma unroll
-  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] : z[i] * w;
+  for (int i = 0; i < N; ++i) z[i] = weight_in ? z[i] : z[i] * w[i];
 }
-template <int N> __device__ __forceinline__ void moe_weighted_act_any(float (&z)[N], float w, int act) {
+template <int N> __device__ __forceinline__ void moe_weighted_act_any(float (&z)[N], const float (&w)[N], int act) {
   const bool in = (act & MOE_ACT_WEIGHT_IN) != 0;
   act &= MOE_ACT_WEIGHT_IN - 1;
   if (act == 0) moe_weighted_act_all<0, N>(z, w, in);
