@@ -428,9 +428,8 @@ gemm_pair_kernel(const GpParams p, const __grid_constant__ CUtensorMap wmap, con
                 // u = sqrt(2/pi) (z + 0.044715 z^3)
                 float z[32];
                 ll_round_bf16<32>(z, a);
-                if (p.act == 3) {
-#pragma unroll
-                  for (int i = 0; i < 32; ++i) z[i] *= ll_sigmoid_fast(z[i]);
+                if (p.act == 3) {      // to the bit of the kernels for rows: expf and the division's quotient
+                  ll_silu_all<32>(z);
                 } else if (p.act == 1) {
 #pragma unroll
                   for (int i = 0; i < 32; ++i) z[i] *= ll_sigmoid_fast(1.5957691216057308f * (z[i] + 0.044715f * z[i] * z[i] * z[i]));

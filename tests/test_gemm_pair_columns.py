@@ -50,3 +50,22 @@ def test_product_with_silu_on_its_first_columns(dtype, m):
     want[:, :136] = torch.nn.functional.silu(want[:, :136])
     got = ops.linear_silu(x, w, 136).double()
     assert float((got - want).norm() / want.norm()) <= (1e-5 if dtype == torch.float32 else 2 ** -7)
+
+
+@gpu
+@pytest.mark.parametrize("cols", [128, 192, 256])
+def test_silu_in_the_epilogue_has_the_bits_of_its_own_kernel(cols):
+    """Beside the product alone and the kernel for rows; numbers far out and infinities among them."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    m, n, k, first = 1100, 1544, 256, 1201
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=g, device="cuda") * 4 * k ** -0.5).to(torch.bfloat16)
+    w[:64] *= 16.0
+    x[700, 3], x[701, 3] = float("inf"), float("-inf")
+    got, want = (torch.empty(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.gemm_pair(x, w, got, row_act="silu", act_cols=first, cols=cols)
+    ops.gemm_pair(x, w, want, cols=cols)
+    ops.silu_rows(want[:, :first])
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~got.isnan()], want[~want.isnan()])
