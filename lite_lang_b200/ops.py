@@ -1271,11 +1271,20 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, activation="silu") ->
     return act
 
 
+def silu_preferred(m: int, n: int, k: int) -> bool:
+    """Whether SiLU goes into the epilogue of ``gemm_pair`` rather than behind the library's product: where the product is long
+    enough to hide it and its rows fill their tiles of 256.  Measured on a B200, three quarters of the columns activated (product
+    and kernel / epilogue, us): 128 x 6,144 x 1,536 8.1 / 9.5, 512 12.9 / 13.9, 1,000 21.1 / 20.1, 1,025 21.7 / 23.8, 1,280
+    26.7 / 24.1, 2,048 39.5 / 31.2; 769 x 14,336 x 3,584 66 / 80, 1,000 84 / 82, 2,048 192 / 157; 1,280 x 3,072 x 1,024
+    13.8 / 14.1, 2,048 18.8 / 17.4; 4,096 x 1,536 x 512 15.2 / 15.0."""
+    return m > 768 and 20 * m >= 17 * ((m + 255) // 256 * 256) and m * n * k >= 1 << 32
+
+
 def linear_silu(x: torch.Tensor, weight: torch.Tensor, cols: int) -> torch.Tensor:
     """x @ weight.T with SiLU on the first ``cols`` columns, applied to the product as its dtype holds it: in the product's
-    epilogue for portions of prompts in bfloat16 (``gemm_pair``; measured on a B200, 6,144 columns of which 4,608, k 1,536,
-    product and kernel / here: 2,048 tokens 30.2 + 11.7 / 31 us, 128 tokens 6.3 + 3 / 9.7), else by a kernel behind it."""
-    if TC_ENABLED and x.shape[0] >= PAIR_MIN_M and pair_supported(x, weight):
+    epilogue for long portions of prompts in bfloat16 (``gemm_pair``; see ``silu_preferred``), else by a kernel behind it, to
+    the same bits of the same product."""
+    if TC_ENABLED and silu_preferred(x.shape[0], weight.shape[0], x.shape[1]) and pair_supported(x, weight):
         out = torch.empty((x.shape[0], weight.shape[0]), dtype=x.dtype, device=x.device)
         return gemm_pair(x, weight, out, row_act="silu", act_cols=cols)
     out = linear(x, weight)

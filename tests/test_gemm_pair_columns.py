@@ -38,6 +38,34 @@ def test_columns_of_a_tile():
     assert ops.pair_columns(2048, 6144, 148) == 256 and ops.pair_columns(2048, 1536, 148) == 192
 
 
+def test_where_silu_goes_into_the_epilogue():
+    """Nowhere where it was measured slower (product and kernel, epilogue; us), and where it was faster by a tenth on long ones."""
+    from lite_lang_b200 import ops
+    for m, n, k, two, one in [(65, 8192, 2048, 9.5, 10.6), (128, 6144, 1536, 8.1, 9.5), (512, 6144, 1536, 12.9, 13.9),
+                              (769, 6144, 1536, 18.9, 19.8), (1025, 6144, 1536, 21.7, 23.8), (513, 14336, 3584, 50.0, 61.4),
+                              (769, 14336, 3584, 66.4, 79.8), (2048, 1536, 512, 10.0, 10.4), (1280, 3072, 1024, 13.8, 14.1),
+                              (1280, 6144, 1536, 26.7, 24.1), (2048, 6144, 1536, 39.5, 31.2), (2049, 14336, 3584, 189.1, 159.0),
+                              (8192, 1536, 512, 25.4, 23.5), (2048, 4608, 1024, 24.2, 20.9)]:
+        assert ops.silu_preferred(m, n, k) == (one < two), (m, n, k)
+
+
+@gpu
+def test_long_portions_have_silu_in_the_epilogue(monkeypatch):
+    from lite_lang_b200 import ops
+    calls, real = [], ops.gemm_pair
+    monkeypatch.setattr(ops, "gemm_pair", lambda *a, **k: (calls.append(k), real(*a, **k))[1])
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    x, w = torch.randn(1030, 1024, generator=g, device="cuda"), torch.randn(4200, 1024, generator=g, device="cuda") / 32
+    x, w = x.to(torch.bfloat16), w.to(torch.bfloat16)
+    for m, taken in ((1000, True), (300, False), (1030, False)):
+        want = (x[:m].double() @ w.double().T).to(x.dtype).double()
+        want[:, :3000] = torch.nn.functional.silu(want[:, :3000])
+        got = ops.linear_silu(x[:m], w, 3000).double()
+        assert float((got - want).norm() / want.norm()) <= 2 ** -7 and bool(calls) == taken
+        calls.clear()
+
+
 @gpu
 @pytest.mark.parametrize("dtype,m", [(torch.bfloat16, 300), (torch.bfloat16, 40), (torch.float32, 70)])
 def test_product_with_silu_on_its_first_columns(dtype, m):
