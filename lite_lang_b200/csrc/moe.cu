@@ -26,9 +26,10 @@
 // each) with the largest best choice score can be chosen.  A place that finds nothing left gets top_idx -1 and weight 0.
 //
 // Two kernels.  `moe_router_tc_kernel`: portions of bfloat16 rows and at most 32 outputs (experts and the shared one's gate), 16 tokens a
-// block on tensor cores.  `moe_router_kernel`: a block takes TOK tokens: one, with a warp an output, which has asked for the first
-// pieces of its row before the token's was there; or eight in long portions, four a warp: the router's matrix is then read
-// once for four tokens.  Its warps share out the outputs, and then the tokens, whose scores a warp each makes and picks from.  Bound by
+// block on tensor cores.  `moe_router_kernel`: a block takes TOK tokens: one, with a warp an output for at most 24 of them (AWARP),
+// which has asked for the first pieces of its row before the token's was there (more outputs keep their warps' loads in flight
+// anyway, and were 8 % slower with it: 64 outputs of 2,048 9.2 and 10.0 us, 32 6.4 and 7.0); or eight in long portions, four a warp: the router's
+// matrix is then read once for four tokens.  Its warps share out the outputs, and then the tokens, whose scores a warp each makes and picks from.  Bound by
 // the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row, then the lanes are added up: an
 // order that depends on the sizes only.  In `moe_pick` a lane has one of at most 32 outputs, and a pick is one maximum over the
 // warp and a ballot.
@@ -156,7 +157,7 @@ __device__ __forceinline__ void moe_pick(float* z, int t, float* __restrict__ ga
   }
 }
 
-template <typename T, int TOK>
+template <typename T, int TOK, bool AWARP>
 __global__ void __launch_bounds__(TOK == 1 ? 1024 : 512)
 moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restrict__ Wr, const float* __restrict__ bias,
                   float* __restrict__ gates, int* __restrict__ top_idx, float* __restrict__ top_w,
@@ -170,9 +171,9 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
   const int tok0 = blockIdx.x * TOK, nt = min(TOK, num_tokens - tok0);
   const int zs = 2 * E + 1 + count;
   T* xrow = reinterpret_cast<T*>(moe_smem + (TOK * zs + 3) / 4 * 4);     // the tokens' rows, `pitch` apart
-  const int n_rows = E + (shared_w ? 1 : 0), warps = blockDim.x >> 5;
+  const int n_rows = E + (shared_w ? 1 : 0), threads = AWARP ? (int)blockDim.x : TOK == 1 ? 1024 : 512, warps = threads / 32;
   const bool vec = (hidden & 3) == 0;
-  constexpr int AHEAD = TOK == 1 ? 8 : 0;                 // pieces of the warp's first row that are asked for now
+  constexpr int AHEAD = AWARP ? 8 : 0;                    // pieces of the warp's row that are asked for now
   float4 head[AHEAD > 0 ? AHEAD : 1];
   if (AHEAD > 0 && vec && warp < n_rows) {
 #pragma unroll
@@ -182,14 +183,14 @@ moe_router_kernel(const T* __restrict__ x, long x_stride, const float* __restric
   constexpr int VEC = 16 / (int)sizeof(T);
   if ((hidden % VEC) == 0 && (x_stride % VEC) == 0 && ((uintptr_t)x % 16) == 0) {
     const int per = hidden / VEC;
-    for (int i = threadIdx.x; i < nt * per; i += blockDim.x) {
+    for (int i = threadIdx.x; i < nt * per; i += threads) {
       const int k = i / per, c = (i - k * per) * VEC;
       *reinterpret_cast<uint4*>(xrow + (size_t)k * pitch + c) =
           *reinterpret_cast<const uint4*>(x + (size_t)(tok0 + k) * x_stride + c);
     }
   } else {
     for (int k = 0; k < nt; ++k)
-      for (int i = threadIdx.x; i < hidden; i += blockDim.x) xrow[(size_t)k * pitch + i] = x[(size_t)(tok0 + k) * x_stride + i];
+      for (int i = threadIdx.x; i < hidden; i += threads) xrow[(size_t)k * pitch + i] = x[(size_t)(tok0 + k) * x_stride + i];
   }
   __syncthreads();
   constexpr int PER = TOK < 4 ? TOK : 4;                  // tokens of a warp at a time
@@ -376,14 +377,14 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
   if (E <= 0 || E > MOE_MAX_E || top <= 0 || top > E || hidden <= 0) return (int)cudaErrorInvalidValue;
   const int zs = 2 * E + 1 + count, pitch = (hidden + 7) / 8 * 8;
   const int rows = E + (shared_w != nullptr ? 1 : 0);
-#define MOE_ROUTER_LAUNCH(TOK)                                                                                           \
+#define MOE_ROUTER_LAUNCH(TOK, AWARP)                                                                                    \
   do {                                                                                                                   \
     const size_t smem = sizeof(float) * (size_t)((TOK * zs + 3) / 4 * 4) + sizeof(T) * (size_t)TOK * pitch;              \
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;                                                            \
     if (smem > 48 * 1024)                                                                                                \
-      cudaFuncSetAttribute(moe_router_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
-    const int warps = TOK > 1 ? 16 : rows < 32 ? (rows > 8 ? rows : 8) : 32;                                              \
-    ll_launch(moe_router_kernel<T, TOK>, dim3((num_tokens + TOK - 1) / TOK), dim3(32 * warps), smem, stream, (const T*)x, x_stride, \
+      cudaFuncSetAttribute(moe_router_kernel<T, TOK, AWARP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    const int warps = TOK > 1 ? 16 : !AWARP ? 32 : rows > 8 ? rows : 8;                                                  \
+    ll_launch(moe_router_kernel<T, TOK, AWARP>, dim3((num_tokens + TOK - 1) / TOK), dim3(32 * warps), smem, stream, (const T*)x, x_stride, \
               Wr, bias, gates, top_idx, top_w, shared_w, num_tokens, hidden, E, top, score_fn, renormalize, choice_bias, count, \
               keep, weight_scale, identity_w, real, pitch);                                                              \
   } while (0)
@@ -409,9 +410,11 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
   }
   LL_DISPATCH_DTYPE(dtype, {
     if (num_tokens >= 512 && sizeof(float) * 8 * (size_t)zs + sizeof(T) * 8 * (size_t)pitch <= 100 * 1024)
-      MOE_ROUTER_LAUNCH(8);
+      MOE_ROUTER_LAUNCH(8, false);
+    else if (rows <= 24)
+      MOE_ROUTER_LAUNCH(1, true);
     else
-      MOE_ROUTER_LAUNCH(1);
+      MOE_ROUTER_LAUNCH(1, false);
   });
 #undef MOE_ROUTER_LAUNCH
   return LL_LAUNCH_RESULT();
