@@ -33,8 +33,11 @@
 // the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row, then the lanes are added up: an
 // order that depends on the sizes only.  In `moe_pick` a lane has one of at most 32 outputs, and a pick is one maximum over the
 // warp and a ballot.
-// Measured on a B200, hidden 1,536, 16 outputs and a shared gate, 4 chosen (us; multiply-adds / tensor cores): 100 tokens 6.3 / 10,
-// 256 11.4 / 10.4, 512 14.1 / 10.3, 2,048 17.2 / 11.0, 4,096 31.6 / 19.5: the line is 256.
+// Tensor cores from 512 tokens on, and from 4,096 with at most 8 outputs, of which a tile of the MMA is half empty.  Measured on a
+// B200 (multiply-adds / tensor cores, us): 17 outputs of 1,536, 256 tokens 10.8 / 9.1, 512 13.4 / 9.2, 2,048 15.3 / 9.5; 32 of
+// 7,168, 256 20.5 / 29.7, 512 39.8 / 29.8; 32 of 4,096, 256 15.2 / 19.6, 512 32.5 / 19.6; 9 of 3,584, 384 11.8 / 12.5, 512 16.1 /
+// 12.5; 4 of 1,024, 512 6.1 / 6.0, 2,048 6.5 / 8.1, 4,096 12.1 / 8.6.
+#define MOE_TC_LEAST(rows) ((rows) > 8 ? 512 : 4096)
 __device__ __forceinline__ float4 moe_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 moe_load4(const bf16* p) {
   const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -388,7 +391,7 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
               Wr, bias, gates, top_idx, top_w, shared_w, num_tokens, hidden, E, top, score_fn, renormalize, choice_bias, count, \
               keep, weight_scale, identity_w, real, pitch);                                                              \
   } while (0)
-  if (dtype == LL_DTYPE_BF16 && num_tokens >= 256 && rows <= 32 && hidden % 16 == 0 && x_stride % 2 == 0 && ((uintptr_t)x % 4) == 0 &&
+  if (dtype == LL_DTYPE_BF16 && num_tokens >= MOE_TC_LEAST(rows) && rows <= 32 && hidden % 16 == 0 && x_stride % 2 == 0 && ((uintptr_t)x % 4) == 0 &&
       ((uintptr_t)Wr % 8) == 0) {
     const int tiles = (rows + 7) / 8;
     const size_t smem = sizeof(float) * ((size_t)(MOE_TC_TOKENS * zs + 3) / 4 * 4 + (size_t)MOE_TC_WARPS * MOE_TC_TOKENS * (8 * tiles + 1));

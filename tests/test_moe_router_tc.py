@@ -10,7 +10,8 @@ gpu = pytest.mark.gpu
 @gpu
 @pytest.mark.parametrize("E,top,shared,score", [(8, 2, False, "softmax"), (16, 4, True, "softmax_top"), (32, 3, False, "sigmoid"),
                                                 (31, 5, True, "softmax"), (5, 5, False, "softmax")])
-@pytest.mark.parametrize("tokens,hidden", [(256, 16), (259, 528), (2048, 1536)])
+# (on tensor cores from 512 tokens on, with at most 8 outputs from 4,096)
+@pytest.mark.parametrize("tokens,hidden", [(256, 16), (259, 528), (512, 528), (515, 16), (2048, 1536), (4099, 144)])
 def test_logits_choice_and_weights(E, top, shared, score, tokens, hidden):
     from lite_lang_b200 import ops
     g = torch.Generator(device="cuda")
@@ -40,11 +41,12 @@ def test_logits_choice_and_weights(E, top, shared, score, tokens, hidden):
 
 
 @gpu
-def test_an_infinity_stays_in_its_token():
+@pytest.mark.parametrize("tokens", [300, 600])
+def test_an_infinity_stays_in_its_token(tokens):
     from lite_lang_b200 import ops
     g = torch.Generator(device="cuda")
     g.manual_seed(3)
-    x = torch.randn(300, 64, generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn(tokens, 64, generator=g, device="cuda").to(torch.bfloat16)
     w = torch.randn(16, 64, generator=g, device="cuda")
     x[37, 5] = float("inf")
     out = []
