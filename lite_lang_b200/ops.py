@@ -1836,6 +1836,20 @@ def moe_combine(base: Optional[torch.Tensor], y: torch.Tensor, pair_row: torch.T
     return out
 
 
+def grouped_product(rows: torch.Tensor, weights: torch.Tensor, ends: torch.Tensor) -> torch.Tensor:
+    """Library grouped product: rows [total, k] cut into runs that end at ``ends`` [groups] (int32, on the
+    device), run g times weights[g] [n, k] transposed; bfloat16 with float32 accumulation."""
+    _need_cuda(rows, weights, ends)
+    _i32(ends, "ends")
+    _need(rows.dtype == torch.bfloat16 and weights.dtype == torch.bfloat16 and weights.dim() == 3,
+          "grouped_product: bfloat16 rows and weights [groups, n, k]")
+    return torch.nn.functional.grouped_mm(rows, weights.transpose(1, 2), offs=ends)
+
+
+def grouped_product_available() -> bool:
+    return hasattr(torch.nn.functional, "grouped_mm")
+
+
 def expert_products(rows: torch.Tensor, weights: torch.Tensor, ends: torch.Tensor, gated: bool = False, act=None,
                     row_w: Optional[torch.Tensor] = None, weight_in: bool = False, x: Optional[torch.Tensor] = None,
                     shared: Optional[torch.Tensor] = None, shared_w: Optional[torch.Tensor] = None,

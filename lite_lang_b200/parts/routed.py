@@ -179,9 +179,11 @@ class RoutedExperts(FeedForward):
 
     def _experts(self, x, step):
         gates, idx, wts = self.route(x)
-        if (self.grouped and x.shape[0] >= self.GROUPED_MIN_TOKENS and ops.TC_ENABLED and not getattr(step, "captured", False)
-                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
-            return self._forward_grouped(x, idx, wts, getattr(step, "status", None))
+        if self.grouped and x.shape[0] >= self.GROUPED_MIN_TOKENS and not getattr(step, "captured", False):
+            if ops.TC_ENABLED:
+                return self._forward_grouped(x, idx, wts, getattr(step, "status", None))
+            if ops.grouped_product_available():
+                return self._forward_library(x, idx, wts)
         if self.gated:
             hidden = ops.linear(x, self.w_up)
             hidden = ops.moe_gated_act(hidden, gates, self._shared_w, self.shared_ff, self.ff, self.E, self.limit,
@@ -192,8 +194,30 @@ class RoutedExperts(FeedForward):
         return ops.linear(hidden, self.w_down, partial_ok=True)
 
 
+    def _forward_library(self, x, idx, wts):
+        """The many tokens' way by library products and activation kernels (``ops.TC_ENABLED`` off, for comparisons)."""
+        sff = self.shared_ff
+        base = None
+        if sff and self.gated:
+            hs = ops.linear(x, self.w_up[:2 * sff])
+            hs = ops.moe_row_gated_act(hs, self._shared_w, self.shared_limit, self.swish_alpha)
+            base = ops.linear(hs, self.w_down[:, :sff])
+        elif sff:
+            hs = ops.linear(x, self.w_up[:sff])
+            ops.moe_act(hs, wts, sff, self.ff, 0, self.activation)      # (no routed columns: every weight is 1)
+            base = ops.linear(hs, self.w_down[:, :sff])
+        ends, row_token, row_w, pair_row = ops.moe_sort(idx, wts, self.E)
+        hidden = ops.grouped_product(ops.moe_gather_rows(x, row_token), self.w_up_experts, ends)
+        if self.gated:
+            hidden = ops.moe_row_gated_act(hidden, row_w, self.limit, self.swish_alpha)
+        else:
+            ops.moe_row_act(hidden, row_w, self.activation, self.weight_in)
+        return ops.moe_combine(base, ops.grouped_product(hidden, self.w_down_experts, ends), pair_row)
+
     def _forward_grouped(self, x, idx, wts, status):
         sff = self.shared_ff
+        if sff and (x.stride(0) % 8 or x.data_ptr() % 16):      # (the shared expert's product brings x's rows by TMA)
+            x = x.clone(memory_format=torch.contiguous_format)
         ends, row_token, row_w, pair_row = ops.moe_sort(idx, wts, self.E)
         rows = ops.moe_gather_rows(x, row_token)
         up = dict(x=x, shared=self.w_up[:2 * sff if self.gated else sff]) if sff else {}
