@@ -33,11 +33,18 @@
 // the loads' latency and the warps in flight.  A lane sums its pieces of four numbers of a row, then the lanes are added up: an
 // order that depends on the sizes only.  In `moe_pick` a lane has one of at most 32 outputs, and a pick is one maximum over the
 // warp and a ballot.
-// Tensor cores from 512 tokens on, and from 4,096 with at most 8 outputs, of which a tile of the MMA is half empty.  Measured on a
-// B200 (multiply-adds / tensor cores, us): 17 outputs of 1,536, 256 tokens 10.8 / 9.1, 512 13.4 / 9.2, 2,048 15.3 / 9.5; 32 of
-// 7,168, 256 20.5 / 29.7, 512 39.8 / 29.8; 32 of 4,096, 256 15.2 / 19.6, 512 32.5 / 19.6; 9 of 3,584, 384 11.8 / 12.5, 512 16.1 /
-// 12.5; 4 of 1,024, 512 6.1 / 6.0, 2,048 6.5 / 8.1, 4,096 12.1 / 8.6.
-#define MOE_TC_LEAST(rows) ((rows) > 8 ? 512 : 4096)
+// Fewest tokens that go to tensor cores.  The other kernel has a token a block, of a warp an output for at most 24 outputs (as many
+// blocks an SM as 32 warps hold) and of 32 warps for more: it is the faster one while that is one round of blocks over the 148
+// SMs, with 32 warps two.  With at most 8 outputs a tile of the MMA is half empty.  Measured on a B200 (a token a block / tensor
+// cores, us): 17 outputs of 1,536, 256 tokens 10.5 / 9.1, 384 14.8 / 9.2; 16 of 2,048, 256 6.3 / 10.0, 320 11.2 / 10.1; 9 of
+// 3,584, 384 7.5 / 12.5; 32 of 2,048, 256 11.4 / 12.5, 320 16.8 / 12.5; 32 of 4,096, 256 14.7 / 19.6, 320 21.0 / 19.6; eight
+// tokens a block: 9 of 3,584, 512 16.1 / 12.5; 32 of 7,168, 512 39.8 / 29.8; 4 of 1,024, 2,048 6.1 / 8.1, 4,096 12.1 / 8.5.
+static int moe_tc_least(int rows) {
+  if (rows <= 8) return 4096;
+  if (rows > 24) return 2 * 148 + 1;
+  const int round = 148 * (32 / rows);
+  return round + 1 > 256 ? round + 1 : 256;
+}
 __device__ __forceinline__ float4 moe_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 moe_load4(const bf16* p) {
   const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -391,7 +398,7 @@ extern "C" int ll_moe_router(int dtype, const void* x, long x_stride, const floa
               Wr, bias, gates, top_idx, top_w, shared_w, num_tokens, hidden, E, top, score_fn, renormalize, choice_bias, count, \
               keep, weight_scale, identity_w, real, pitch);                                                              \
   } while (0)
-  if (dtype == LL_DTYPE_BF16 && num_tokens >= MOE_TC_LEAST(rows) && rows <= 32 && hidden % 16 == 0 && x_stride % 2 == 0 && ((uintptr_t)x % 4) == 0 &&
+  if (dtype == LL_DTYPE_BF16 && num_tokens >= moe_tc_least(rows) && rows <= 32 && hidden % 16 == 0 && x_stride % 2 == 0 && ((uintptr_t)x % 4) == 0 &&
       ((uintptr_t)Wr % 8) == 0) {
     const int tiles = (rows + 7) / 8;
     const size_t smem = sizeof(float) * ((size_t)(MOE_TC_TOKENS * zs + 3) / 4 * 4 + (size_t)MOE_TC_WARPS * MOE_TC_TOKENS * (8 * tiles + 1));

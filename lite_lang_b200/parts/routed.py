@@ -20,8 +20,8 @@ Two ways through the experts, both without the host ever knowing who chose whom:
   pairs' results are added per token in the order of the pairs, onto the shared expert's output.
 
 A token's result depends on the other tokens of the step only through their number: it says which of the two ways they take, and
-which kernel makes the router's logits (tensor cores from 512 tokens on, 4,096 with at most 8 outputs, for bfloat16 and at most 32
-outputs).  The kernels' float32 sums are in different orders, so experts whose scores are nearer than those sums' rounding may be
+which kernel makes the router's logits (for bfloat16 and at most 32 outputs tensor cores from 256 to 445 tokens on, 4,096 with at
+most 8 outputs).  The kernels' float32 sums are in different orders, so experts whose scores are nearer than those sums' rounding may be
 chosen differently by a prompt cut into portions on both sides of the line.
 
 Further parameters, for designs that differ:

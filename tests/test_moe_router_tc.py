@@ -9,9 +9,9 @@ gpu = pytest.mark.gpu
 
 @gpu
 @pytest.mark.parametrize("E,top,shared,score", [(8, 2, False, "softmax"), (16, 4, True, "softmax_top"), (32, 3, False, "sigmoid"),
-                                                (31, 5, True, "softmax"), (5, 5, False, "softmax")])
-# (on tensor cores from 512 tokens on, with at most 8 outputs from 4,096)
-@pytest.mark.parametrize("tokens,hidden", [(256, 16), (259, 528), (512, 528), (515, 16), (2048, 1536), (4099, 144)])
+                                                (31, 5, True, "softmax"), (5, 5, False, "softmax"), (9, 2, False, "sigmoid"), (23, 4, True, "softmax")])
+# (on tensor cores from 256 tokens on with 17 to 24 outputs, 297 with 11 to 16 or more than 24, 445 with 9 or 10, 4,096 with fewer)
+@pytest.mark.parametrize("tokens,hidden", [(256, 16), (259, 528), (297, 528), (445, 16), (515, 528), (2048, 1536), (4099, 144)])
 def test_logits_choice_and_weights(E, top, shared, score, tokens, hidden):
     from lite_lang_b200 import ops
     g = torch.Generator(device="cuda")
