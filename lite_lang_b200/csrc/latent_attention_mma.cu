@@ -37,6 +37,7 @@
 #define LM_UNITS 4                // units of 16 columns a warp, at most (UPW: 1 to 4; the eight warps have 128 UPW columns, at least R)
 #define LM_PPITCH (2 * LM_TK + 16)      // bytes from one head's row of P to the next
 #define LM_MAX_STAGES 3
+#define LM_MAX_SMEM (218 * 1024)  // dynamic shared memory of any launch
 #define LM_LOG2E 1.4426950408889634f
 
 __device__ __forceinline__ void lm_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
@@ -45,11 +46,6 @@ __device__ __forceinline__ void lm_mma(float (&d)[4], unsigned a0, unsigned a1, 
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ float lm_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 __device__ __forceinline__ void lm_ldmatrix_x4(unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3, unsigned addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -529,13 +525,19 @@ struct LmArgs {
   int *status, stages, bw, box_rows;
   const float* sink;
 };
+// What a variant needs to be launched with any size: the same for every call, since threads that launch or plan share it.
+template <int STEPS, int UPW, bool FULL, bool TMA>
+static void lm_allow() {
+  auto kernel = latent_attention_mma_kernel<STEPS, UPW, FULL, TMA>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_MAX_SMEM);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
 template <int STEPS, int UPW, bool FULL, bool TMA>
 static int lm_launch(const LmArgs& a, const CUtensorMap& map) {
   static_assert(UPW >= 1 && UPW <= LM_UNITS, "units a warp");
   if (a.R > 16 * LM_WARPS * UPW || (FULL && a.R != 16 * LM_WARPS * UPW)) return (int)cudaErrorInvalidValue;
   auto kernel = latent_attention_mma_kernel<STEPS, UPW, FULL, TMA>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
-  if (a.grid.z > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  lm_allow<STEPS, UPW, FULL, TMA>();
   ll_launch_cluster(kernel, a.grid, dim3(LM_THREADS), a.smem, a.stream, (int)a.grid.z, a.out, a.q, a.cache, a.block_table,
                     a.bt_stride, a.token_req, a.req_slot, a.positions, a.first, a.H, a.R, a.r, a.page_size, a.num_pages, a.window,
                     a.scale_log2, a.status, a.stages, a.bw, a.box_rows, a.sink, map);
@@ -571,13 +573,11 @@ static int lm_resident(int size) {
   int n = known[dev][size].load(std::memory_order_relaxed);
   if (n == 0) {
     auto kernel = latent_attention_mma_kernel<16, 4, true, true>;
-    const int smem = 200 * 1024;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    lm_allow<16, 4, true, true>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, size);
     cfg.blockDim = dim3(LM_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = LM_MAX_SMEM;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
@@ -621,7 +621,7 @@ extern "C" int ll_latent_attention_mma(void* out, const void* q, const void* cac
   }
   const size_t beside = 1024 + (size_t)LM_HEADS * (2 * KD + 16) + 2 * LM_HEADS * LM_PPITCH, tile = (size_t)LM_TK * 2 * KD;
   a.stages = LM_MAX_STAGES;
-  while (a.stages > 1 && beside + a.stages * tile > 218 * 1024) --a.stages;      // (a tile of KD = 1,024 fits once)
+  while (a.stages > 1 && beside + a.stages * tile > LM_MAX_SMEM) --a.stages;      // (a tile of KD = 1,024 fits once)
   a.smem = beside + a.stages * tile;
   a.grid = dim3(num_tokens, (H + LM_HEADS - 1) / LM_HEADS, nsplit < 16 ? nsplit : 16);
   a.stream = stream;

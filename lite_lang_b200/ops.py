@@ -1628,14 +1628,18 @@ def latent_attention_heads(dtype: torch.dtype, R: int, r: int) -> int:
     return int(load_library("latent_attn").fn("ll_latent_attention_heads")(c_int(_DT[dtype]), c_int(R), c_int(r)))
 
 
-@functools.lru_cache(maxsize=4096)
 def latent_attention_splits(pairs: int, longest: int) -> int:
     """CTAs that share the keys of each of ``pairs`` (query, group of 16 heads) on tensor cores, for runs of up to ``longest``
     keys: the largest cluster (16 at most) that lets all of them run at once, since a CTA takes an SM and a second round
     of clusters doubles the time.  Measured on a B200 (12 heads, a latent of 512, context 2,048; us):
     16 tokens with 4, 6 and 8 CTAs 21.6, 17.0 and 25.2, 64 tokens with 1, 2 and 4 60.0, 37.1 and 43.0; one token with 8, 10
-    and 16 14.2, 12.6 and 13.6."""
-    return int(load_library("latent_attn").fn("ll_latent_attention_mma_splits")(c_int(pairs), c_int((longest + 63) // 64 + 1)))
+    and 16 14.2, 12.6 and 13.6.  (Of the current device, whose room for clusters it is.)"""
+    return _latent_splits(pairs, (longest + 63) // 64 + 1, torch.cuda.current_device())
+
+
+@functools.lru_cache(maxsize=4096)
+def _latent_splits(pairs: int, tiles: int, device: int) -> int:
+    return int(load_library("latent_attn").fn("ll_latent_attention_mma_splits")(c_int(pairs), c_int(tiles)))
 
 
 def latent_gather(dst: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, slot: int, lo: int, page_size: int,

@@ -102,3 +102,64 @@ def test_splits_fit_the_device():
         for longest in (10, 300, 9000):
             n = ops.latent_attention_splits(pairs, longest)
             assert 1 <= n <= 16 and n <= (longest + 63) // 64 + 1 and (n == 1 or n * pairs <= sms)
+
+
+def test_a_plan_belongs_to_its_device(monkeypatch):
+    from lite_lang_b200 import ops
+    device = [0]
+
+    class Library:
+        def fn(self, name):
+            return lambda pairs, tiles: 4 + 2 * device[0]
+
+    monkeypatch.setattr(ops, "load_library", lambda name: Library())
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: device[0])
+    ops._latent_splits.cache_clear()
+    try:
+        assert ops.latent_attention_splits(3, 1000) == 4
+        device[0] = 1
+        assert ops.latent_attention_splits(3, 1000) == 6
+        device[0] = 0
+        assert ops.latent_attention_splits(3, 1000) == 4
+    finally:
+        ops._latent_splits.cache_clear()
+
+
+@gpu
+def test_threads_that_plan_and_launch_share_a_kernel():
+    """One variant of the kernel with rows of 496 and of 1,008 numbers, from two threads on streams of their own, beside plans."""
+    import threading
+    from lite_lang_b200 import ops
+    scale, lens = 0.1, [200, 330]
+    step = _step([1, 1], [n - 1 for n in lens], [0, 1])
+    table = torch.arange(2 * 21, dtype=torch.int32, device=dev()).view(2, 21)
+    g = torch.Generator(device=dev())
+    g.manual_seed(2)
+    work = []
+    for R, r in ((480, 16), (480, 528)):
+        q, pool = (torch.randn(*shape, generator=g, device=dev()).to(torch.bfloat16) for shape in ((2, 4, R + r), (42, 1, 16, R + r)))
+        want = torch.empty(2, 4, R, dtype=torch.bfloat16, device=dev())
+        ops.latent_attention(want, q, pool, table, step, 0, 2, 4, R, r, 16, None, scale, 2, 1)
+        work.append((R, r, q, pool, want))
+    torch.cuda.synchronize()
+    failed = []
+
+    def run(R, r, q, pool, want):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(300):
+                    out = torch.empty_like(want)
+                    ops.latent_attention(out, q, pool, table, step, 0, 2, 4, R, r, 16, None, scale, 2, 1)
+                    ops._latent_splits.cache_clear()
+                    ops.latent_attention_splits(1 + i % 20, 3000)
+                torch.cuda.current_stream().synchronize()
+                assert torch.equal(out, want)
+        except Exception as exc:      # (pytest sees no other thread's)
+            failed.append(repr(exc))
+
+    threads = [threading.Thread(target=run, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
