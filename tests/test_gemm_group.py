@@ -27,10 +27,15 @@ def _gate(g, u, limit, alpha):
 
 
 def _close(got, want):
-    """A bfloat16 product, rounded (2^-9 a number), its activation (slopes of a few), rounded again."""
-    want = want.cpu()
-    err = (got.double().cpu() - want).norm() / want.norm()
+    """A bfloat16 product, rounded (2^-9 a number), its activation (slopes of a few), rounded again.  All of it, and every row: a
+    row of few numbers may have several whose product is rounded the other way (2^-8, and twice that behind a square), and one
+    that is small beside the others is held to a part of their mean."""
+    want, diff = want.cpu(), got.double().cpu() - want.cpu()
+    err = diff.norm() / want.norm()
     assert float(err) <= 0.01, float(err)
+    mean = want.norm() / max(1, want.shape[0]) ** 0.5
+    rows = diff.norm(dim=-1) / (want.norm(dim=-1) + 0.1 * mean)
+    assert float(rows.max()) <= 0.03, float(rows.max())
 
 
 COUNTS = [(1, 31, 32, 33), (255, 256, 257, 3), (0, 513, 0, 64), (700, 1, 129, 0)]
