@@ -17,9 +17,9 @@
 //                   as before, and nothing has to be rescaled.
 // Two CTAs fit an SM (half of its shared memory and tensor memory each), so that one's softmax runs
 // beside the other's MMAs.
-// Roles: warp 0 loads (one thread: Q once through a 3-d tensor map [token, head, head size]; K and V
+// Roles: warp 0 loads (one lane a box: Q once through a 3-d tensor map [token, head, head size]; K and V
 // of a block page by page through 2-d maps over the cache plane, into a ring of two stages), warp 1
-// issues the MMAs (one thread; S a whole block ahead of the softmax, so that the tensor cores work
+// issues the MMAs (an elected lane; S a whole block ahead of the softmax, so that the tensor cores work
 // while the softmax threads do), warps 2..5 are the softmax rows.  All hand-offs are mbarriers: TMA
 // completes the "full" ones, tcgen05.commit the ones the tensor cores free, the softmax warps arrive
 // on the rest.  Every wait is bounded; one that runs out records LL_ERR_WAIT_TIMEOUT, stops waiting in

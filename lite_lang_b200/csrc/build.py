@@ -29,7 +29,10 @@ from typing import Dict, Iterable, List, Optional, Sequence, Tuple
 _HERE = os.path.dirname(os.path.abspath(__file__))
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# --use_fast_math is NOT used: expf, division and sqrtf keep their IEEE forms.
+# --use_fast_math is NOT used: expf, division and sqrtf keep their IEEE forms.  Where an epilogue could not hide the division's
+# branch it takes common.cuh's ll_divide, whose numbers are the division's (gemm_f32, gemm_group, linear attention's projection in
+# gemm_pair, the delta rule's convolutions).  The exponential and reciprocal instructions alone (ll_gated_fast) make the dense
+# feed-forward's activation in gemm_pair and gemm_tc, whose result is rounded to bfloat16.
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
 # name -> (sources, definitions)

@@ -20,10 +20,10 @@
 // q|k|v row never goes to memory and one kernel stands for two.
 //
 // Roles in a CTA (320 threads):
-//   warp 0    producer: one thread keeps a ring of six 32 KB stages filled (four in q|k|v mode, whose epilogue
-//             takes the room of two for its staging tile); both CTAs' copies complete on the even CTA's
+//   warp 0    producer: keeps a ring of stages filled: six of 32 KB for tiles of 256 columns (four in q|k|v mode, whose
+//             epilogue takes the room of two for its staging tile), seven of 28 KB for 192, eight of 24 KB for 128; both CTAs' copies complete on the even CTA's
 //             `full` barrier of the stage;
-//   warp 1    MMA: in the even CTA one thread issues the MMAs of a stage when it is full, and a
+//   warp 1    MMA: in the even CTA an elected lane issues the MMAs of a stage when it is full, and a
 //             tcgen05.commit hands the stage back to both producers; the accumulator is double-buffered
 //             (2 x 256 columns), so the MMAs of the next tile run while this one's epilogue reads;
 //   warps 2-9 epilogue: tensor memory -> registers -> activation -> 16-byte stores of the thread's own row

@@ -3,9 +3,9 @@
 //
 // A decode step is a stream of every weight through the SMs, so this kernel is built
 // around the copy engine, not around the tensor core: persistent CTAs, each with one
-// producer warp that keeps a ring of shared-memory stages filled by TMA (tiled
-// cp.async.bulk.tensor.2d through a tensor map of W, boxes of 64 k x 16..64 rows with the
-// 128-byte swizzle, completion counted by an mbarrier per stage; no multicast), and four
+// producer warp that keeps a ring of shared-memory stages filled by TMA (a tiled
+// cp.async.bulk.tensor.4d a stage through a tensor map of W as [k / 64][runs of rows][row][64], 128-byte
+// swizzle, completion counted by an mbarrier per stage; no multicast), and four
 // consumer warps that feed mma.sync.m16n8k16 from the stages and hand them back through a
 // second mbarrier.  Bytes in flight are bounded by shared memory (about 100 KB a CTA, two
 // CTAs an SM), not by registers or occupancy, and the producer runs ahead over the end of a
@@ -17,11 +17,11 @@
 // gemm_smallm.cu the contraction index of an MMA step is mapped to 8 contiguous elements
 // per thread, so a thread's A fragment is one 16-byte read from a stage row and its B
 // fragment one 16-byte read of a token row.  The token rows of a stage's k range travel with
-// its weights: a second tensor map (of x, boxes of 8..32 rows x 64 k) puts them behind the
-// weight boxes of the stage, after griddepcontrol.wait (the weights start before it).
+// its weights: a second tensor map (of x as [k / 64][row][64], a box of 8..32 rows a stage) puts them behind
+// the stage's weights, after griddepcontrol.wait (the weights start before it).
 //
 // Four shapes of work unit:
-//   WIDE    64 output features x all of K; a stage is 64 rows x 128 k (two boxes); warp w
+//   WIDE    64 output features x all of K; a stage is 64 rows x 128 k; warp w
 //           owns rows 16 w .. 16 w + 15.  For wide products (lm_head).
 //   GATED   32 features of the SiLU-gated feed-forward; W is [2 I, K], gate rows first.
 //           Warp w's tile has 8 gate rows and, as rows 8..15, the up rows of the same 8
@@ -29,12 +29,12 @@
 //           and writes silu(gate) * up: the [M, 2 I] intermediate never exists.
 //   QKV_ROPE  the fused q|k|v projection of an attention layer with everything that follows it: a unit
 //           is 8 features of the first half of a head and their 8 rotation partners from the second half
-//           (two TMA boxes of 8 rows), k split over the warps as in NARROW.  After the warps' partial
+//           (two runs of 8 rows in one box), k split over the warps as in NARROW.  After the warps' partial
 //           tiles are added, bias and rotary position encoding are applied in float32 and the results
 //           go where they belong: q into the output rows, k and v into the pages of the cache.  The
 //           [M, (nh + 2 nkv) hd] projection is never written and the rope/store kernel is not launched.
-//   NARROW  16 features x all of K; a stage is 16 rows x 256 k (four boxes) and warp w takes
-//           one box; the four partial tiles are added through shared memory.  For
+//   NARROW  16 features x all of K; a stage is 16 rows x 256 k (four blocks of 64) and warp w takes
+//           one block; the four partial tiles are added through shared memory.  For
 //           products with few output features (q|k|v, o, down), where units, not k, are scarce.
 //
 // Two of them have a variant (template flag SPLIT) that takes over half of an RMS norm that lies between two
@@ -64,7 +64,7 @@
 #define GT_MODE_QKV_ROPE 3
 
 template <int MODE> struct GtShape;
-// ROWS x KC elements a stage, made of boxes of BOX_ROWS rows x 64 k (128 bytes a row).
+// ROWS x KC elements a stage, in blocks of 64 k (128 bytes a row) of runs of BOX_ROWS rows.
 template <> struct GtShape<GT_MODE_WIDE> {
   static constexpr int ROWS = 64, KC = 128, BOX_ROWS = 64, STAGES = 6;
 };
@@ -74,7 +74,7 @@ template <> struct GtShape<GT_MODE_GATED> {
 template <> struct GtShape<GT_MODE_NARROW> {
   static constexpr int ROWS = 16, KC = 256, BOX_ROWS = 16, STAGES = 12;
 };
-// two boxes of 8 rows land exactly where the 16-row box of NARROW does, so the consumers are the same
+// two runs of 8 rows land exactly where the 16 rows of NARROW do, so the consumers are the same
 template <> struct GtShape<GT_MODE_QKV_ROPE> {
   static constexpr int ROWS = 16, KC = 256, BOX_ROWS = 8, STAGES = 12;
 };

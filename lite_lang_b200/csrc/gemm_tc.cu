@@ -3,11 +3,11 @@
 //
 // The weights are the M side of the MMA (128 output features a tile), the tokens the N side (64 or
 // 128 columns).  One persistent CTA per SM with three roles:
-//   warp 0    producer: one thread keeps a ring of shared-memory stages filled by TMA
-//             (cp.async.bulk.tensor.2d, 128-byte swizzle, no multicast): a box of 128 features x 64 k of
-//             W (for the gated feed-forward two boxes of 64 rows, the gate rows and the up rows of the same
-//             64 features, stacked into one 128-row tile) and a box of the tokens' rows;
-//   warp 1    MMA: one thread issues tcgen05.mma.cta_group::1.kind::f16 (128 x NT x 16) straight from
+//   warp 0    producer: keeps a ring of shared-memory stages filled by TMA (the whole warp runs the loop, one
+//             elected lane issues; 128-byte swizzle, no multicast): a 3d box of 128 features x 64 k of
+//             W (for the gated feed-forward the gate rows and the up rows of the same 64 features, stacked
+//             into one 128-row tile by the map's third dimension) and a 2d box of the tokens' rows;
+//   warp 1    MMA: an elected lane issues tcgen05.mma.cta_group::1.kind::f16 (128 x NT x 16) straight from
 //             the stages through shared-memory descriptors, accumulating in tensor memory; a
 //             tcgen05.commit hands each stage back to the producer when the MMAs that read it are done;
 //   warps 2-5 epilogue: when a unit's last MMA has completed they read the accumulator from tensor

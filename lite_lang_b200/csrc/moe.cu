@@ -524,7 +524,7 @@ moe_sort_kernel(const int* __restrict__ top_idx, const float* __restrict__ top_w
 template <typename T>
 __global__ void moe_gather_rows_kernel(T* __restrict__ dst, const T* __restrict__ x, long x_stride,
                                        const int* __restrict__ row_token, int hidden) {
-  LL_PDL_WAIT();      // (no early release: what runs next may be a library kernel that does not wait itself)
+  LL_PDL_WAIT();      // (no early release: a library product may run next, which does not wait itself; see grouped_product)
   const int row = blockIdx.x;
   const T* src = x + (size_t)row_token[row] * x_stride;
   T* d = dst + (size_t)row * hidden;
