@@ -1438,7 +1438,7 @@ CHUNK = 64                 # tokens of a chunk (csrc/chunk_scan.cu)
 #     87 / 95, x 160 105 / 91; 28 heads: 1 x 128 85 / 94, x 160 92 / 92, x 192 101 / 91; 4 x 48 99 / 91
 #   delta rule        12 heads: 1 x 192 105 / 117, x 256 140 / 117; 2 x 96 105 / 117, x 128 130 / 118; 4 x 48 105 / 117, x 64
 #     124 / 118; 28 heads: 1 x 96 116 / 120, x 128 143 / 119; 2 x 48 118 / 120, x 64 143 / 120; 4 x 48 193 / 135
-#   2,048 tokens of 12 heads, the kernels alone: decay scan 320 / 53, delta rule 872 / 185
+#   2,048 tokens of 12 heads, the kernels alone: decay scan 320 / 53, delta rule 872 / 135 (two portions of together 2,047: 122)
 DECAY_CHUNKED_MIN = 275
 DELTA_CHUNKED_MIN = 178
 
@@ -1476,17 +1476,19 @@ def _cut(step, tokens: int, heads: int, dk: int, dv: int, minimum) -> Optional[T
 
 def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, cut) -> None:
     single, rest, items = cut
-    # scratch of one allocation: states in front of the chunks, u, w, decays to the chunks' ends and of whole chunks
-    n = items * H
-    base = torch.empty(n * (dv * dk + CHUNK * (dv + dk + 1) + 1), dtype=torch.float32, device=qn.device)
-    u = n * dv * dk
-    w = u + n * CHUNK * dv
-    suf = w + n * CHUNK * dk
+    # scratch of one allocation: states in front of the chunks, u, the terms of w and of k (six bytes a number), the scores of q and
+    # k, decays to the chunks' ends and from their starts, and of whole chunks
+    n, at, ptrs = items * H, 0, []
+    sizes = (n * dv * dk, n * CHUNK * dv, n * CHUNK * dk * 3 // 2, items * Hk * CHUNK * dk * 3 // 2, n * CHUNK * CHUNK, n * CHUNK,
+             n * CHUNK, n)
+    base = torch.empty(sum(sizes), dtype=torch.float32, device=qn.device)
+    for size in sizes:
+        ptrs.append(_ptr_at(base, at))
+        at += size
     load_library("chunk_scan").call(
         "ll_chunk_delta_scan", _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(g), _ptr(state), c_long(state.stride(0)),
         c_int(state.shape[0]), _ptr_at(step.cu_q, single), _ptr_at(step.req_slot, single), _ptr(o), c_int(rest), c_int(H),
-        c_int(Hk), c_int(dk), c_int(dv), _ptr(base), _ptr_at(base, u), _ptr_at(base, w), _ptr_at(base, suf),
-        _ptr_at(base, suf + n * CHUNK), c_int(items), _stream())
+        c_int(Hk), c_int(dk), c_int(dv), *ptrs, c_int(items), _ptr(getattr(step, "status", None)), _stream())
 
 
 def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta: torch.Tensor, g: torch.Tensor,
