@@ -10,8 +10,9 @@
 // [(taps - 1), channels] for the last taps - 1 inputs of the convolutions (oldest first;
 // channels = q | k | v), so that a request can go on in a later step from where it stopped.
 //
-// Four kernels (a long portion's recurrence with one decay a head goes by chunks instead: chunk_scan.cu), all reading the
-// step's device arrays only (so that a step of single tokens can be captured and replayed):
+// Four kernels (a long portion's recurrence with one decay a head goes by chunks instead: delta_chunks.cu; a step of single tokens
+// takes one launch for all of them, delta_step, where its sizes allow it), all reading the step's device arrays only (so that
+// a step of single tokens can be captured and replayed):
 //   delta_prepare      per token: convolution + SiLU, unit vectors, beta, decay -> float32 buffers
 //   delta_conv_update  per entry of several tokens: the new last taps - 1 inputs of the record
 //   delta_recurrence   per (entry, head, 16 value columns): the scan over the entry's tokens
@@ -596,6 +597,270 @@ extern "C" int ll_delta_out(int dtype, void* out, const float* o, const float* w
     else
       ll_launch(delta_out_kernel<T, 1>, dim3((pairs + 3) / 4), dim3(128), 0, stream, (T*)out, o, w, (const T*)gate, gate_stride,
                 eps, pairs, H, dv, gate_act);
+  });
+  return LL_LAUNCH_RESULT();
+}
+
+// A step of single tokens in one launch, a CTA a (token, head): what delta_prepare, delta_recurrence and delta_out do, and the second
+// products of decays and gates that come through a few numbers (decay_rank, gate_rank).  For one token those are five launches in a
+// chain of 1.6 to 3 us each; for many the scan's loop over chunks of 16 tokens is made for more than one.  D: channels of a key and of
+// a value head.  What does not depend on the step (filters, the ranks' matrices) is asked for before the wait; then a thread's part of
+// the state is on its way, all at once, while
+//   warp 0, 1, 2   make the head's q, k and v (four channels a lane, as delta_prepare_token),
+//   the warps from the fifth on the decays of the key channels and (for heads of 128 the first four) the gates, a number a thread.
+// A thread has 16 channels of four columns (heads of 64: of one), which share what it reads of q, k and decays: 1,024 threads with a
+// column each read four times as much of shared memory, and took 9.1 us for a token and 14.4 for 16 (12 heads; this way 7.8 and 8.5).
+// The heads that read the same q and k are a cluster: their inputs in the record move up when all of them have been read.  Every sum
+// but the ranks' has the order that it has in the kernels one by one, so that a token's bits do not depend on what it shares a step
+// with.  Whole layers of 12 heads, launches one by one / this way: 1 token 18.6 / 14.5 us, 16 tokens 35.1 / 18.7, 64 tokens 90 / 43.
+template <typename T> struct DeltaStep {
+  const T *proj, *a_in, *gate;           // a_in, gate: rows of their own numbers, or of the ranks' inputs
+  const T *w_a, *w_g;                    // [H * D or H, a_rank], [H * D, g_rank], or null
+  long stride, a_stride, gate_stride;
+  int q_off, k_off, v_off, b_off, a_rank, g_rank;
+  const float *conv_q, *conv_k, *conv_v, *A_log, *dt_bias, *norm;
+  float* state;
+  long state_stride, tail_off;
+  const int *req_slot, *positions;
+  T* y;
+  float eps;
+  int H, Hk, per_channel, gate_act;
+};
+
+// pieces of 16 bytes from one row of a rank's matrix to the next in shared memory: odd, so that neighbouring threads' rows lie in
+// different banks
+template <typename T> __host__ __device__ __forceinline__ int ds_pitch(int rank) { return (rank * (int)sizeof(T) / 16) | 1; }
+template <typename T> __device__ __forceinline__ float ds_dot(const uint4* row, const float* x, int rank) {
+  constexpr int N = 16 / (int)sizeof(T);
+  float acc[4] = {};
+#pragma unroll 4
+  for (int p = 0; p < rank / N; ++p) {
+    const uint4 w = row[p];
+    const T* v = reinterpret_cast<const T*>(&w);
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const float4 x4 = *reinterpret_cast<const float4*>(x + p * N + i);
+      acc[0] = fmaf(to_f32<T>(v[i]), x4.x, acc[0]);
+      acc[1] = fmaf(to_f32<T>(v[i + 1]), x4.y, acc[1]);
+      acc[2] = fmaf(to_f32<T>(v[i + 2]), x4.z, acc[2]);
+      acc[3] = fmaf(to_f32<T>(v[i + 3]), x4.w, acc[3]);
+    }
+  }
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(256, 2)
+delta_step_kernel(DeltaStep<T> s) {
+  // lanes of delta_recurrence that a thread stands for, threads that share a column, columns a thread and their distance
+  constexpr int VL = 4, TPC = D / 16, THREADS = 256, NC = D * TPC / THREADS, STEP = D / NC;
+  extern __shared__ __align__(16) uint4 mat_a[];               // the rows of w_a, then of w_g
+  __shared__ __align__(16) float qs[D], ks[D], vs[D], gs[D], zs[D], os[D];
+  __shared__ __align__(16) float ax[128], gx[128];
+  __shared__ float beta;
+  LL_PDL_TRIGGER();
+  const int e = blockIdx.x, h = blockIdx.z, hk = h / (s.H / s.Hk);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n_decay = tid - 128, n_gate = D == 128 ? tid : tid - 192;      // the key channel or value column of a thread
+  const bool is_decay = n_decay >= 0 && n_decay < D, is_gate = n_gate >= 0 && n_gate < D;
+  const int drow = s.per_channel ? h * D + n_decay : h;
+  // before the wait: filters and the head's rows of the ranks' matrices
+  float4 f[4];
+  constexpr int width = D / 4;                                 // lanes of warps 0 to 2 with channels
+  const float* filt = warp == 0 ? s.conv_q + (size_t)hk * D * 4 : warp == 1 ? s.conv_k + (size_t)hk * D * 4 : s.conv_v + (size_t)h * D * 4;
+  if (warp < 3 && lane < width) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] = reinterpret_cast<const float4*>(filt)[lane * 4 + k];
+  }
+  const int pitch_a = ds_pitch<T>(s.a_rank), pitch_g = ds_pitch<T>(s.g_rank), rows_a = s.per_channel ? D : 1;
+  uint4* mat_g = mat_a + (s.a_rank > 0 ? rows_a * pitch_a : 0);
+  auto fetch = [&](uint4* dst, int pitch, const T* src, int rank, int rows) {
+    const int pieces = rank * (int)sizeof(T) / 16;
+    for (int i = tid; i < rows * pieces; i += THREADS) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(dst + i / pieces * pitch + i % pieces);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(reinterpret_cast<const uint4*>(src) + i) : "memory");
+    }
+  };
+  if (s.a_rank > 0) fetch(mat_a, pitch_a, s.w_a + (size_t)h * rows_a * s.a_rank, s.a_rank, rows_a);
+  if (s.g_rank > 0) fetch(mat_g, pitch_g, s.w_g + (size_t)h * D * s.g_rank, s.g_rank, D);
+  const int col = tid / TPC, l = tid % TPC;
+  const float a_log = s.A_log[h], bias = is_decay ? s.dt_bias[drow] : 0.f, weight = s.norm[tid % D];
+  LL_PDL_WAIT();
+  const int slot = s.req_slot[e], t = e, p = s.positions[t];   // (an entry a token)
+  T* yrow = s.y + (size_t)t * s.H * D + (size_t)h * D;
+  if (slot < 0) {                                              // a padding entry (the cluster's CTAs have the same one)
+    if (tid < D) yrow[tid] = from_f32<T>(0.f);
+    return;
+  }
+  float* rec = s.state + (size_t)slot * s.state_stride;
+  float* srow = rec + ((size_t)h * D + col) * D + l * VL;
+  float S[NC][4][VL];                                          // columns col + n STEP, key channels j D / 4 + l VL + i
+#pragma unroll
+  for (int n = 0; n < NC; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"      // (in this place: they are the most bytes)
+                   : "=f"(S[n][j][0]), "=f"(S[n][j][1]), "=f"(S[n][j][2]), "=f"(S[n][j][3])
+                   : "l"(srow + (size_t)n * STEP * D + j * (D / 4)));
+  const T* row = s.proj + (size_t)t * s.stride;
+  for (int i = tid; i < s.a_rank; i += THREADS) ax[i] = to_f32<T>(s.a_in[(size_t)t * s.a_stride + i]);
+  for (int i = tid; i < s.g_rank; i += THREADS) gx[i] = to_f32<T>(s.gate[(size_t)t * s.gate_stride + i]);
+  const int Cq = s.Hk * D, C = 2 * Cq + s.H * D;
+  const int c = 4 * lane, chan = warp == 0 ? hk * D + c : warp == 1 ? Cq + hk * D + c : 2 * Cq + h * D + c;      // among the record's inputs
+  if (warp < 3 && lane < width) {
+    const float* tail = rec + s.tail_off + chan;
+    float x[4][4];
+    DpVec<T, 4>::load(row + (warp == 0 ? s.q_off + hk * D : warp == 1 ? s.k_off + hk * D : s.v_off + h * D) + c, x[0]);
+#pragma unroll
+    for (int j = 1; j < 4; ++j) DpVec<float, 4>::load(tail + (size_t)(3 - j) * C, x[j]);      // inputs of earlier steps
+#pragma unroll
+    for (int j = 1; j < 4; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[j][k] = p - j >= 0 ? x[j][k] : 0.f;
+    float acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {                              // oldest input first
+      acc[k] = fmaf(f[k].x, x[3][k], 0.f);
+      acc[k] = fmaf(f[k].y, x[2][k], acc[k]);
+      acc[k] = fmaf(f[k].z, x[1][k], acc[k]);
+      acc[k] = dr_silu(fmaf(f[k].w, x[0][k], acc[k]));
+    }
+    if (warp < 2) {                                            // unit vectors
+      float ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ss = fmaf(acc[k], acc[k], ss);
+#pragma unroll
+      for (int o = width / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(D == 128 ? 0xffffffffu : 0xffffu, ss, o);
+      float inv = 1.0f / sqrtf(ss + 1e-6f);
+      if (warp == 0) inv *= 1.0f / sqrtf((float)D);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[k] *= inv;
+    }
+    float* dst = warp == 0 ? qs : warp == 1 ? ks : vs;
+    *reinterpret_cast<float4*>(dst + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  } else if (tid == 96) {
+    beta = dr_sigmoid(to_f32<T>(row[s.b_off + h]));
+  }
+  if (s.a_rank > 0 || s.g_rank > 0) {                          // the ranks' rows and inputs
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
+  if (is_decay) {
+    const float a = s.a_rank > 0 ? round_to<T>(ds_dot<T>(mat_a + (s.per_channel ? n_decay * pitch_a : 0), ax, s.a_rank))
+                                 : to_f32<T>(s.a_in[(size_t)t * s.a_stride + drow]);
+    gs[n_decay] = expf(-expf(a_log) * dr_softplus(a + bias));
+  }
+  if (is_gate) {
+    const float z = s.g_rank > 0 ? round_to<T>(ds_dot<T>(mat_g + n_gate * pitch_g, gx, s.g_rank))
+                                 : to_f32<T>(s.gate[(size_t)t * s.gate_stride + (size_t)h * D + n_gate]);
+    zs[n_gate] = s.gate_act == 0 ? dr_silu(z) : dr_sigmoid(z);
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive;" ::: "memory");        // this CTA has read the record's inputs of q and k
+  // the token, as delta_recurrence has it and with its sums in its order: S^T (g . k) and S^T (g . q) side by side, then the write
+  float dot[NC][VL] = {}, oq[NC][VL] = {}, d1[NC][VL] = {}, o1[NC][VL] = {}, kq[VL] = {};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int ch = j * (D / 4) + l * VL;
+    const float4 k4 = *reinterpret_cast<const float4*>(ks + ch), q4 = *reinterpret_cast<const float4*>(qs + ch);
+    const float4 g4 = *reinterpret_cast<const float4*>(gs + ch);
+    const float kv[VL] = {k4.x, k4.y, k4.z, k4.w}, qv[VL] = {q4.x, q4.y, q4.z, q4.w}, gv[VL] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+    for (int i = 0; i < VL; ++i) {
+      const float gk = gv[i] * kv[i], gq = gv[i] * qv[i];
+      kq[i] = fmaf(kv[i], qv[i], kq[i]);
+#pragma unroll
+      for (int n = 0; n < NC; ++n) {
+        if (j & 1) {
+          d1[n][i] = fmaf(S[n][j][i], gk, d1[n][i]);
+          o1[n][i] = fmaf(S[n][j][i], gq, o1[n][i]);
+        } else {
+          dot[n][i] = fmaf(S[n][j][i], gk, dot[n][i]);
+          oq[n][i] = fmaf(S[n][j][i], gq, oq[n][i]);
+        }
+      }
+    }
+  }
+  float k_q = (kq[0] + kq[1]) + (kq[2] + kq[3]), u[NC];
+#pragma unroll
+  for (int w = 1; w < TPC; w <<= 1) k_q += __shfl_xor_sync(0xffffffffu, k_q, w);
+#pragma unroll
+  for (int n = 0; n < NC; ++n) {
+#pragma unroll
+    for (int i = 0; i < VL; ++i) {
+      dot[n][i] += d1[n][i];
+      oq[n][i] += o1[n][i];
+    }
+    float d = (dot[n][0] + dot[n][1]) + (dot[n][2] + dot[n][3]), o = (oq[n][0] + oq[n][1]) + (oq[n][2] + oq[n][3]);
+#pragma unroll
+    for (int w = 1; w < TPC; w <<= 1) {
+      d += __shfl_xor_sync(0xffffffffu, d, w);
+      o += __shfl_xor_sync(0xffffffffu, o, w);
+    }
+    u[n] = beta * (vs[col + n * STEP] - d);
+    if (l == 0) os[col + n * STEP] = fmaf(u[n], k_q, o);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int ch = j * (D / 4) + l * VL;
+    const float4 k4 = *reinterpret_cast<const float4*>(ks + ch), g4 = *reinterpret_cast<const float4*>(gs + ch);
+#pragma unroll
+    for (int n = 0; n < NC; ++n)
+      *reinterpret_cast<float4*>(srow + (size_t)n * STEP * D + j * (D / 4)) =
+          make_float4(fmaf(g4.x, S[n][j][0], k4.x * u[n]), fmaf(g4.y, S[n][j][1], k4.y * u[n]), fmaf(g4.z, S[n][j][2], k4.z * u[n]),
+                      fmaf(g4.w, S[n][j][3], k4.w * u[n]));
+  }
+  __syncthreads();
+  if (tid < D) {      // norm and gate, as delta_out: every warp adds the squares up
+    float ss = 0.f;
+    if (lane < width) {
+      const float4 v = *reinterpret_cast<const float4*>(os + 4 * lane);
+      ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+    }
+    ss = warp_sum(ss);
+    yrow[tid] = from_f32<T>(os[tid] * (1.0f / sqrtf(ss / (float)D + s.eps)) * weight * zs[tid]);
+  }
+  asm volatile("barrier.cluster.wait;" ::: "memory");          // every head of the cluster has read them
+  if (lane < width && (warp == 2 || (warp < 2 && h == hk * (s.H / s.Hk)))) {      // a place holds the input behind it from now on
+    float* tail = rec + s.tail_off + chan;
+    float own[4], old[4] = {};
+    if (p >= 2) DpVec<float, 4>::load(tail + C, old);
+    dp_store<4>(tail, old);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) old[k] = 0.f;
+    if (p >= 1) DpVec<float, 4>::load(tail + 2 * C, old);
+    dp_store<4>(tail + C, old);
+    DpVec<T, 4>::load(row + (warp == 0 ? s.q_off + hk * D : warp == 1 ? s.k_off + hk * D : s.v_off + h * D) + c, own);
+    dp_store<4>(tail + 2 * C, own);
+  }
+}
+
+// A step of one token an entry (which brings position ctx_len) with key and value heads of 64 or 128, four taps and at most eight
+// heads that read the same q and k; a_in and gate: the ranks' inputs where w_a, w_g are not null.  Rows at multiples of four numbers,
+// records, filters and ranks' rows at multiples of 16 bytes; the head's rows of w_a and w_g together at most DS_ROOM bytes.
+#define DS_ROOM 40960
+extern "C" int ll_delta_step(int dtype, const void* proj, long stride, int q_off, int k_off, int v_off, int b_off, const void* a_in,
+                             long a_stride, const void* w_a, int a_rank, const void* gate, long gate_stride, const void* w_g,
+                             int g_rank, const float* conv_q, const float* conv_k, const float* conv_v, const float* A_log,
+                             const float* dt_bias, const float* norm, float* state, long state_stride, long tail_off,
+                             const int* req_slot, const int* positions, void* y, float eps, int num_entries, int H,
+                             int Hk, int d, int per_channel, int gate_act, cudaStream_t stream) {
+  if (num_entries <= 0) return 0;
+  const int esz = dtype == LL_DTYPE_F32 ? 4 : 2;
+  if (H <= 0 || Hk <= 0 || H % Hk || H / Hk > 8 || H > 65535 || (d != 64 && d != 128) || a_rank < 0 || g_rank < 0 || a_rank > 128 ||
+      g_rank > 128 || a_rank % 8 || g_rank % 8 || state_stride % 4 || tail_off % 4 || stride % 4 || (q_off | k_off | v_off) % 4 ||
+      (uintptr_t)proj % (4 * esz) || ((uintptr_t)conv_q | (uintptr_t)conv_k | (uintptr_t)conv_v | (uintptr_t)state) % 16 ||
+      ((uintptr_t)w_a | (uintptr_t)w_g) % 16)
+    return (int)cudaErrorInvalidValue;
+  LL_DISPATCH_DTYPE(dtype, {
+    const size_t smem = 16 * ((a_rank > 0 ? (size_t)(per_channel ? d : 1) * ds_pitch<T>(a_rank) : 0) +
+                              (g_rank > 0 ? (size_t)d * ds_pitch<T>(g_rank) : 0));
+    if (smem > DS_ROOM) return (int)cudaErrorInvalidValue;
+    const DeltaStep<T> s{(const T*)proj, (const T*)a_in, (const T*)gate, (const T*)w_a, (const T*)w_g, stride, a_stride, gate_stride,
+                         q_off, k_off, v_off, b_off, a_rank, g_rank, conv_q, conv_k, conv_v, A_log, dt_bias, norm, state,
+                         state_stride, tail_off, req_slot, positions, (T*)y, eps, H, Hk, per_channel, gate_act};
+    if (d == 128) ll_launch_cluster(delta_step_kernel<T, 128>, dim3(num_entries, 1, H), dim3(256), smem, stream, H / Hk, s);
+    else ll_launch_cluster(delta_step_kernel<T, 64>, dim3(num_entries, 1, H), dim3(256), smem, stream, H / Hk, s);
   });
   return LL_LAUNCH_RESULT();
 }

@@ -1524,6 +1524,49 @@ def delta_out(out: torch.Tensor, o: torch.Tensor, weight: torch.Tensor, gate: to
         c_float(eps), c_int(out.shape[0]), c_int(H), c_int(dv), c_int(gate_act), _stream())
 
 
+def delta_step_supported(proj: torch.Tensor, step, H: int, Hk: int, dk: int, dv: int, taps: int, offsets, a_w: Optional[torch.Tensor],
+                         g_w: Optional[torch.Tensor], per_channel: bool, state: torch.Tensor, tail_off: int, constants) -> bool:
+    """Whether a step is one of single tokens that ``delta_step`` takes (see ``ll_delta_step``, csrc/delta_rule.cu)."""
+    if proj.shape[0] != step.num_entries or dk != dv or dk not in (64, 128) or taps != 4 or H // Hk > 8:
+        return False
+    size, room = proj.element_size(), 0
+    for w, rows in ((a_w, dk if per_channel else 1), (g_w, dk)):
+        if w is not None:
+            rank = w.shape[1]
+            if rank % 8 or rank > 128 or not w.is_contiguous() or w.data_ptr() % 16:
+                return False
+            room += 16 * rows * (rank * size // 16 | 1)
+    return (room <= DELTA_STEP_ROOM and proj.stride(1) == 1 and state.stride(0) % 4 == 0 and tail_off % 4 == 0
+            and proj.stride(0) % 4 == 0 and all(o % 4 == 0 for o in offsets) and proj.data_ptr() % (4 * size) == 0
+            and all(t.data_ptr() % 16 == 0 for t in (state, *constants)))
+
+
+DELTA_STEP_ROOM = 40960      # bytes of shared memory for a head's rows of the ranks' matrices
+
+
+def delta_step(out: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int, b_off: int, a_in: torch.Tensor,
+               a_w: Optional[torch.Tensor], gate: torch.Tensor, g_w: Optional[torch.Tensor], conv_q: torch.Tensor,
+               conv_k: torch.Tensor, conv_v: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor, weight: torch.Tensor,
+               state: torch.Tensor, tail_off: int, step, eps: float, H: int, Hk: int, d: int, per_channel: bool, gate_act: int) -> None:
+    """A step of one token an entry: ``delta_prepare``, ``delta_recurrence`` and ``delta_out`` in one launch, with the second
+    products of decays (``a_in`` times ``a_w`` transposed) and gates (``gate`` times ``g_w``) where these are not None."""
+    _need_cuda(out, proj, a_in, gate, conv_q, conv_k, conv_v, A_log, dt_bias, weight, state, a_w, g_w)
+    for t, nm in ((conv_q, "conv_q"), (conv_k, "conv_k"), (conv_v, "conv_v"), (A_log, "A_log"), (dt_bias, "dt_bias"),
+                  (state, "state"), (weight, "weight")):
+        _f32(t, nm)
+    _need(out.is_contiguous() and a_in.stride(1) == 1 and gate.stride(1) == 1 and out.dtype == proj.dtype == a_in.dtype == gate.dtype
+          and all(w is None or w.dtype == proj.dtype for w in (a_w, g_w)), "delta_step: rows of one dtype")
+    _need(state.dim() == 2 and state.shape[1] == tail_off + 3 * (2 * Hk + H) * d,
+          "delta_step: the state record is S followed by the convolutions' last inputs")
+    load_library("delta_rule").call(
+        "ll_delta_step", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off),
+        c_int(b_off), _ptr(a_in), c_long(a_in.stride(0)), _ptr(a_w), c_int(0 if a_w is None else a_w.shape[1]), _ptr(gate),
+        c_long(gate.stride(0)), _ptr(g_w), c_int(0 if g_w is None else g_w.shape[1]), _ptr(conv_q), _ptr(conv_k), _ptr(conv_v),
+        _ptr(A_log), _ptr(dt_bias), _ptr(weight), _ptr(state), c_long(state.stride(0)), c_long(tail_off),
+        _ptr(step.req_slot), _ptr(step.positions), _ptr(out), c_float(eps), c_int(step.num_entries), c_int(H), c_int(Hk), c_int(d),
+        c_int(1 if per_channel else 0), c_int(gate_act), _stream())
+
+
 # --------------------------------------------------------------------------
 # latent attention
 # --------------------------------------------------------------------------

@@ -146,9 +146,18 @@ class GatedDeltaRule(Mixer):
         n, dev = x.shape[0], x.device
         proj = ops.linear(x, self.w_in)
         a_in = proj[:, self.off["a"]:self.off["a"] + self.width["a"]]
+        gate = proj[:, self.off["g"]:self.off["g"] + self.width["g"]]
+        per_channel, act = self.decay == "channel", 0 if self.gate == "silu" else 1
+        at = tuple(self.off[name] for name in "qkvb")
+        if ops.delta_step_supported(proj, step, self.H, self.Hk, self.dk, self.dv, self.taps, at[:3], self.w_a2, self.w_g2, per_channel,
+                                    cache.state, self.state_floats, (self.conv_q, self.conv_k, self.conv_v)):
+            y = torch.empty((n, self.Cv), dtype=x.dtype, device=dev)
+            ops.delta_step(y, proj, *at, a_in, self.w_a2, gate, self.w_g2, self.conv_q, self.conv_k, self.conv_v, self.A_log,
+                           self.dt_bias, self.norm_w, cache.state, self.state_floats, step, self.eps, self.H, self.Hk, self.dk,
+                           per_channel, act)
+            return ops.linear(y, self.w_o)
         if self.w_a2 is not None:
             a_in = ops.linear(a_in, self.w_a2)
-        gate = proj[:, self.off["g"]:self.off["g"] + self.width["g"]]
         if self.w_g2 is not None:
             gate = ops.linear(gate, self.w_g2)
         f32 = dict(dtype=torch.float32, device=dev)
@@ -158,14 +167,13 @@ class GatedDeltaRule(Mixer):
         beta = torch.empty((n, self.H), **f32)
         g = torch.empty((n, self.n_decay), **f32)
         o = torch.empty((n, self.Cv), **f32)
-        per_channel = self.decay == "channel"
         ops.delta_prepare(proj, self.off["q"], self.off["k"], self.off["v"], self.off["b"], a_in, self.conv_q,
                           self.conv_k, self.conv_v, self.A_log, self.dt_bias, cache.state, self.state_floats, step,
                           qn, kn, vc, beta, g, self.H, self.Hk, self.dk, self.dv, self.taps, per_channel)
         ops.delta_recurrence(qn, kn, vc, beta, g, cache.state, step, o, self.H, self.Hk, self.dk, self.dv,
                              per_channel)
         y = torch.empty((n, self.Cv), dtype=x.dtype, device=dev)
-        ops.delta_out(y, o, self.norm_w, gate, self.eps, self.H, self.dv, 0 if self.gate == "silu" else 1)
+        ops.delta_out(y, o, self.norm_w, gate, self.eps, self.H, self.dv, act)
         return ops.linear(y, self.w_o)
 
 
