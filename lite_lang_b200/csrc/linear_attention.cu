@@ -21,6 +21,7 @@
 // group): `tok_decay` and `tok_scale` [tokens, H] replace the constant decay and scale the written values,
 // `skip` [H] adds the token's own value to its read-out.
 //
+// `decay_step`: a step of single tokens with heads of 64 or 128, all between the products (but the norm over all heads) in one launch.
 // `rotate_rows_f32`: the operands of such a scan when q and k are rotated by the token's position: float32 rows q | k | v
 // from the projections, nothing of them rounded after the rotation.
 // `head_norm_gate_out`: y = (o of a head / its root mean square) * act(gate), act SiLU or sigmoid, heads side by side.
@@ -561,6 +562,193 @@ extern "C" int ll_head_norm_gate_out(int dtype, void* y, const float* o, const v
     else
       ll_launch(head_norm_gate_out_kernel<T, 1>, grid, dim3(threads), 0, stream, (T*)y, o, (const T*)gate, gate_stride,
                 eps, pairs, H, dv, act);
+  });
+  return LL_LAUNCH_RESULT();
+}
+
+// A step of single tokens in one launch, a CTA a (token, head): `silu_rows` (act 1) or `rotate_rows_f32` (act 0; rot_dim may be 0),
+// the scan, and, where y is asked for and not o, `head_norm_gate_out`.  The scan's loop over chunks of 16 tokens is made for more than
+// one (16 tokens of 12 heads 15.4 us).  Whole layers of 12 heads, launches one by one / this way: retention 1 token 18.7 / 14.6 us, 16
+// tokens 33.0 / 18.7, 64 tokens 72 / 28; linear attention, whose norm is over all heads, 17.7 / 16.6, 31.8 / 20.7, 72 / 30.  D: channels of a key and of a value head.  A thread has
+// 16 channels of four columns (heads of 64: of one), on their way while warps 0, 1 and 2 make the head's q, k and v, four numbers
+// a lane; it stands for the scan's lanes that the exchange there adds up first, so every sum has the scan's order and a token's
+// bits do not depend on what it shares a step with.
+template <typename T> struct DecayStep {
+  const T *proj, *gate;
+  long stride, gate_stride;
+  int q_off, k_off, v_off, act;
+  const int* positions;
+  const float* freq;
+  int rot_dim, interleaved;
+  float q_scale, k_scale;
+  const float* decay;
+  float* state;
+  long slot_stride;
+  int num_slots;
+  const int* req_slot;
+  float* o;
+  T* y;
+  float eps;
+  int gate_act, H, write_state;
+  int* status;
+};
+template <typename T> __device__ __forceinline__ float4 ls_load4(const T* p);
+template <> __device__ __forceinline__ float4 ls_load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 ls_load4<bf16>(const bf16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(256, 2)
+decay_step_kernel(DecayStep<T> s) {
+  // threads that share a column, columns a thread and their distance; width: lanes of warps 0 to 2 with numbers
+  constexpr int TPC = D / 16, NC = D * TPC / 256, STEP = D / NC, width = D / 4;
+  __shared__ __align__(16) float qs[D], ks[D], vs[D], os[D], cs[D / 2], sn[D / 2];
+  LL_PDL_TRIGGER();
+  const int t = blockIdx.x, h = blockIdx.y;                    // (an entry a token)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = s.rot_dim >> 1;
+  const int col = tid / TPC, l = tid % TPC;
+  const float d = s.decay[h], freq = tid >= 96 && tid - 96 < half ? s.freq[tid - 96] : 0.f;
+  LL_PDL_WAIT();
+  const int slot = s.req_slot[t];
+  float* orow = s.o != nullptr ? s.o + ((size_t)t * s.H + h) * D : nullptr;
+  T* yrow = s.y != nullptr ? s.y + ((size_t)t * s.H + h) * D : nullptr;
+  if (slot < 0 || slot >= s.num_slots) {                       // a padding entry: defined output, nothing read
+    if (slot >= s.num_slots && tid == 0) set_status(s.status, LL_ERR_SLOT_RANGE);
+    if (tid < D) {
+      if (orow != nullptr) orow[tid] = 0.f;
+      else yrow[tid] = from_f32<T>(0.f);
+    }
+    return;
+  }
+  float* srow = s.state + (size_t)slot * s.slot_stride + ((size_t)h * D + col) * D + 4 * l;
+  float S[NC][4][4];                                           // columns col + n STEP, key channels p D / 4 + 4 l + i
+#pragma unroll
+  for (int n = 0; n < NC; ++n)
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+      asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"      // (in this place: they are the most bytes)
+                   : "=f"(S[n][p][0]), "=f"(S[n][p][1]), "=f"(S[n][p][2]), "=f"(S[n][p][3])
+                   : "l"(srow + (size_t)n * STEP * D + p * (D / 4)));
+  const int c = 4 * lane;
+  float x[4] = {}, other[4] = {};
+  if (warp < 3 && lane < width) {
+    const T* src = s.proj + (size_t)t * s.stride + (warp == 0 ? s.q_off : warp == 1 ? s.k_off : s.v_off) + (size_t)h * D;
+    const float4 v = ls_load4<T>(src + c);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    if (warp < 2 && c < s.rot_dim && !s.interleaved) {         // the other half's numbers (half is a multiple of four)
+      const float4 w = ls_load4<T>(src + (c < half ? c + half : c - half));
+      other[0] = w.x; other[1] = w.y; other[2] = w.z; other[3] = w.w;
+    }
+  }
+  if (s.rot_dim > 0) {
+    if (tid >= 96 && tid - 96 < half) sincosf((float)s.positions[t] * freq, &sn[tid - 96], &cs[tid - 96]);
+    __syncthreads();
+  }
+  if (warp < 3 && lane < width) {
+    if (s.act == 1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = round_to<T>(la_silu(x[k]));
+    } else if (warp < 2) {
+      if (c < s.rot_dim) {
+        if (s.interleaved) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) other[k] = x[k ^ 1];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int i = (c + k) >> 1;
+            x[k] = ((c + k) & 1) ? x[k] * cs[i] + other[k] * sn[i] : x[k] * cs[i] - other[k] * sn[i];
+          }
+        } else {
+          const bool low = c < half;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int i = (low ? c : c - half) + k;
+            x[k] = low ? x[k] * cs[i] - other[k] * sn[i] : x[k] * cs[i] + other[k] * sn[i];
+          }
+        }
+      }
+      const float scale = warp == 0 ? s.q_scale : s.k_scale;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] *= scale;
+    }
+    *reinterpret_cast<float4*>((warp == 0 ? qs : warp == 1 ? ks : vs) + c) = make_float4(x[0], x[1], x[2], x[3]);
+  }
+  __syncthreads();
+  float v[NC], part[NC][4];                                    // part[.][m]: the scan's lane that has the channels of place m
+#pragma unroll
+  for (int n = 0; n < NC; ++n) v[n] = vs[col + n * STEP];
+  float a[NC][4][4];                                           // [column][scan's lane][number of four]
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float4 k4 = *reinterpret_cast<const float4*>(ks + p * (D / 4) + 4 * l), q4 = *reinterpret_cast<const float4*>(qs + p * (D / 4) + 4 * l);
+    const float kv[4] = {k4.x, k4.y, k4.z, k4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+    const int m = D == 128 ? p & 1 : p;
+    const bool first = D == 128 ? p < 2 : true;
+#pragma unroll
+    for (int n = 0; n < NC; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        S[n][p][i] = fmaf(d, S[n][p][i], kv[i] * v[n]);
+        a[n][m][i] = fmaf(S[n][p][i], qv[i], first ? 0.f : a[n][m][i]);
+      }
+  }
+#pragma unroll
+  for (int n = 0; n < NC; ++n) {
+#pragma unroll
+    for (int m = 0; m < (D == 128 ? 2 : 4); ++m) part[n][m] = (a[n][m][0] + a[n][m][1]) + (a[n][m][2] + a[n][m][3]);
+    float sum = D == 128 ? part[n][0] + part[n][1] : (part[n][0] + part[n][2 % 4]) + (part[n][1] + part[n][3 % 4]);
+#pragma unroll
+    for (int w = TPC / 2; w >= 1; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+    if (l == 0) {
+      if (orow != nullptr) orow[col + n * STEP] = sum;
+      else os[col + n * STEP] = sum;
+    }
+  }
+  if (s.write_state) {
+#pragma unroll
+    for (int n = 0; n < NC; ++n)
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+        *reinterpret_cast<float4*>(srow + (size_t)n * STEP * D + p * (D / 4)) = make_float4(S[n][p][0], S[n][p][1], S[n][p][2], S[n][p][3]);
+  }
+  if (orow != nullptr) return;
+  __syncthreads();
+  if (tid < D) {                                               // as head_norm_gate_out; every warp adds the squares up
+    const float z = to_f32<T>(s.gate[(size_t)t * s.gate_stride + (size_t)h * D + tid]);
+    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < width) w = *reinterpret_cast<const float4*>(os + c);
+    float ss = 0.f;
+    ss += (w.x * w.x + w.y * w.y) + (w.z * w.z + w.w * w.w);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)D + s.eps);
+    const float sig = 1.0f / (1.0f + expf(-z));
+    yrow[tid] = from_f32<T>(os[tid] * inv * (s.gate_act == 0 ? z * sig : sig));
+  }
+}
+
+// A step of one token an entry with key and value heads of 64 or 128; either o (float32 [tokens, H * d]) or y.  Rows and offsets at
+// multiples of four numbers, records at multiples of 16 bytes; rot_dim a multiple of 8, or of 4 in pairs.
+extern "C" int ll_decay_step(int dtype, const void* proj, long stride, int q_off, int k_off, int v_off, int act, const int* positions,
+                             const float* freq, int rot_dim, int interleaved, float q_scale, float k_scale, const float* decay,
+                             float* state, long slot_stride, int num_slots, const int* req_slot, float* o, void* y, const void* gate,
+                             long gate_stride, float eps, int gate_act, int num_entries, int H, int d, int write_state, int* status,
+                             cudaStream_t stream) {
+  if (num_entries <= 0) return 0;
+  const int esz = dtype == LL_DTYPE_F32 ? 4 : 2;
+  if (H <= 0 || H > 65535 || (d != 64 && d != 128) || act < 0 || act > 1 || rot_dim < 0 || rot_dim > d || rot_dim % 4 ||
+      (!interleaved && rot_dim % 8) || (rot_dim > 0 && freq == nullptr) || (act == 1 && rot_dim > 0) || (o == nullptr) == (y == nullptr) ||
+      (y != nullptr && gate == nullptr) || stride % 4 || (q_off | k_off | v_off) % 4 || (uintptr_t)proj % (4 * esz) ||
+      slot_stride % 4 || (uintptr_t)state % 16)
+    return (int)cudaErrorInvalidValue;
+  LL_DISPATCH_DTYPE(dtype, {
+    const DecayStep<T> s{(const T*)proj, (const T*)gate, stride, gate_stride, q_off, k_off, v_off, act, positions, freq, rot_dim,
+                         interleaved, q_scale, k_scale, decay, state, slot_stride, num_slots, req_slot, o, (T*)y, eps, gate_act, H,
+                         write_state, status};
+    if (d == 128) ll_launch(decay_step_kernel<T, 128>, dim3(num_entries, H), dim3(256), 0, stream, s);
+    else ll_launch(decay_step_kernel<T, 64>, dim3(num_entries, H), dim3(256), 0, stream, s);
   });
   return LL_LAUNCH_RESULT();
 }

@@ -2106,6 +2106,38 @@ def ssd_gated_norm(out: torch.Tensor, y: torch.Tensor, z: torch.Tensor, weight: 
                              c_int(parts), _stream())
 
 
+def decay_step_supported(proj: torch.Tensor, offsets, step, H: int, dk: int, dv: int, state: torch.Tensor, rot: int = 0,
+                         interleaved: bool = True) -> bool:
+    """Whether a step is one of single tokens that ``decay_step`` takes (see ``ll_decay_step``, csrc/linear_attention.cu)."""
+    return (proj.shape[0] == step.num_entries and dk == dv and dk in (64, 128) and proj.stride(1) == 1 and proj.stride(0) % 4 == 0
+            and all(o % 4 == 0 for o in offsets) and proj.data_ptr() % (4 * proj.element_size()) == 0 and state.stride(0) % 4 == 0
+            and state.data_ptr() % 16 == 0 and rot <= dk and rot % (4 if interleaved else 8) == 0)
+
+
+def decay_step(proj: torch.Tensor, offsets, decay: torch.Tensor, state: torch.Tensor, step, H: int, d: int, o: Optional[torch.Tensor] = None,
+               y: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, eps: float = 0.0, gate_act: str = "silu",
+               silu: bool = False, freq: Optional[torch.Tensor] = None, interleaved: bool = True, q_scale: float = 1.0,
+               k_scale: float = 1.0, write_state: bool = True) -> None:
+    """A step of one token an entry in one launch, from its projections as they come out of their product: SiLU of q, k and v
+    (``silu``), or q and k turned and scaled (``rotate_rows_f32``); ``decay_scan``; and the read-outs to ``o``, or with
+    ``head_norm_gate_out`` to ``y``."""
+    _need_cuda(proj, decay, state, o, y, gate, freq)
+    for t, nm in ((decay, "decay"), (state, "state"), (o, "o"), (freq, "freq")):
+        _f32(t, nm)
+    n = proj.shape[0]
+    _need((o is None) != (y is None) and decay.numel() == H and state.shape[1] >= H * d * d and max(offsets) + H * d <= proj.shape[1]
+          and all(t is None or (t.is_contiguous() and tuple(t.shape) == (n, H * d)) for t in (o, y)), "decay_step: shapes")
+    _need(y is None or (gate is not None and tuple(gate.shape) == (n, H * d) and gate.dtype == y.dtype == proj.dtype
+                        and gate.stride(1) == 1), "decay_step: gate")
+    load_library("linear_attn").call(
+        "ll_decay_step", c_int(_dtype_code(proj)), _ptr(proj), c_long(proj.stride(0)), *(c_int(x) for x in offsets),
+        c_int(1 if silu else 0), _ptr(step.positions), _ptr(freq), c_int(0 if freq is None else 2 * freq.numel()),
+        c_int(1 if interleaved else 0), c_float(q_scale), c_float(k_scale), _ptr(decay), _ptr(state), c_long(state.stride(0)),
+        c_int(state.shape[0]), _ptr(step.req_slot), _ptr(o), _ptr(y), _ptr(gate), c_long(0 if gate is None else gate.stride(0)),
+        c_float(eps), c_int(HEAD_GATE_ACT[gate_act]), c_int(n), c_int(H), c_int(d), c_int(1 if write_state else 0), _ptr(step.status),
+        _stream())
+
+
 def linear_attn_out(y: torch.Tensor, o: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, eps: float) -> None:
     """y = o / rms(o over the whole row) * weight * sigmoid(gate), in y's dtype."""
     _need_cuda(y, o, weight, gate)

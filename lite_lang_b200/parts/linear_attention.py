@@ -84,10 +84,18 @@ class DecayLinearAttention(Mixer):
 
     def forward(self, x, step, cache):
         n, dev = x.shape[0], x.device
-        proj = ops.linear_silu(x, self.w_in, self.off["g"])        # q | k | v (and the zero columns that pad them)
         o = torch.empty((n, self.Cv), dtype=torch.float32, device=dev)
-        ops.decay_scan(proj, self.off["q"], self.off["k"], self.off["v"], self.decay, cache.state, step, o,
-                       self.H, self.dk, self.dv, cache.writable)
+        at = tuple(self.off[name] for name in "qkv")
+        if n == step.num_entries:                                  # single tokens: SiLU and scan in one launch
+            proj = ops.linear(x, self.w_in)
+            if ops.decay_step_supported(proj, at, step, self.H, self.dk, self.dv, cache.state):
+                ops.decay_step(proj, at, self.decay, cache.state, step, self.H, self.dk, o=o, silu=True, write_state=cache.writable)
+            else:
+                ops.silu_rows(proj[:, :self.off["g"]])
+                ops.decay_scan(proj, *at, self.decay, cache.state, step, o, self.H, self.dk, self.dv, cache.writable)
+        else:
+            proj = ops.linear_silu(x, self.w_in, self.off["g"])    # q | k | v (and the zero columns that pad them)
+            ops.decay_scan(proj, *at, self.decay, cache.state, step, o, self.H, self.dk, self.dv, cache.writable)
         y = torch.empty((n, self.Cv), dtype=x.dtype, device=dev)
         ops.linear_attn_out(y, o, self.norm_w, proj[:, self.off["g"]:self.off["g"] + self.Cv], self.eps)
         return ops.linear(y, self.w_o, partial_ok=self.partial_ok)
@@ -157,15 +165,20 @@ class Retention(Mixer):
     def forward(self, x, step, cache):
         n, dev = x.shape[0], x.device
         proj = ops.linear(x, self.w_in)
+        pos, at = self.position, tuple(self.off[name] for name in "qkv")
+        freq, interleaved = None if pos is None else pos.freq, bool(pos is None or pos.interleaved)
+        gate = proj[:, self.off["g"]:self.off["g"] + self.Cv]
+        y = torch.empty((n, self.Cv), dtype=x.dtype, device=dev)
+        if ops.decay_step_supported(proj, at, step, self.H, self.dk, self.dv, cache.state, 0 if freq is None else 2 * freq.numel(),
+                                    interleaved):                  # single tokens: everything between the products in one launch
+            ops.decay_step(proj, at, self.decay, cache.state, step, self.H, self.dk, y=y, gate=gate, eps=self.eps, freq=freq,
+                           interleaved=interleaved, k_scale=self.key_scale, write_state=cache.writable)
+            return ops.linear(y, self.w_o, partial_ok=self.partial_ok)
         rows = torch.empty((n, self.row_width), dtype=torch.float32, device=dev)
-        pos = self.position
-        ops.rotate_rows_f32(rows, self.row, proj, (self.off["q"], self.off["k"], self.off["v"]), step.positions,
-                            None if pos is None else pos.freq, bool(pos is None or pos.interleaved), self.H, self.dk, self.Cv,
-                            1.0, self.key_scale)
+        ops.rotate_rows_f32(rows, self.row, proj, at, step.positions, freq, interleaved, self.H, self.dk, self.Cv, 1.0, self.key_scale)
         o = torch.empty((n, self.Cv), dtype=torch.float32, device=dev)
         ops.decay_scan(rows, *self.row, self.decay, cache.state, step, o, self.H, self.dk, self.dv, cache.writable)
-        y = torch.empty((n, self.Cv), dtype=x.dtype, device=dev)
-        ops.head_norm_gate_out(y, o, proj[:, self.off["g"]:self.off["g"] + self.Cv], self.eps, self.H, self.dv, "silu")
+        ops.head_norm_gate_out(y, o, gate, self.eps, self.H, self.dv, "silu")
         return ops.linear(y, self.w_o, partial_ok=self.partial_ok)
 
 
