@@ -9,17 +9,22 @@ There is no fallback: without nvcc, or on a compile error, loading raises.
 
 The launchers are plain C functions (raw pointers, sizes, a ``cudaStream_t``)
 that return a ``cudaError_t`` as an int; ``Library.call`` raises on non-zero.
+They are called through a small extension module (launch.c) where it can be
+built, else by ctypes.
 """
 
 from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.util
 import os
+import platform
 import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -227,14 +232,67 @@ def build_library(name: str, verbose: bool = True) -> str:
     return target
 
 
+def _by_ctypes(f, args) -> int:
+    """A launcher called by ctypes: integers and pointers in 64 bits, whose low half an int parameter reads."""
+    return f(*[ctypes.c_long(a) if isinstance(a, int) else ctypes.c_float(a) if isinstance(a, float)
+               else ctypes.c_void_p(0) if a is None else a for a in args])
+
+
+def _launch_path() -> Optional[str]:
+    """Where the native call (launch.c) is built, or None where it is not: another machine than x86-64 Linux, no Python headers."""
+    include = sysconfig.get_paths()["include"]
+    if platform.machine() != "x86_64" or sys.platform != "linux" or not os.path.isfile(os.path.join(include, "Python.h")):
+        return None
+    h = hashlib.sha256(open(_src_path("launch.c"), "rb").read() + sys.version.encode()).hexdigest()[:16]
+    return os.path.join(_build_dir(), f"ll_launch_{h}.so")
+
+
+def build_launch() -> Optional[str]:
+    """Compile launch.c if needed; its path, or None where launchers are called by ctypes."""
+    target = _launch_path()
+    if target is None or os.path.isfile(target):
+        return target
+    cc = next((c for c in (shutil.which(n) for n in ("cc", "gcc", "g++")) if c), None)
+    if cc is None:
+        return None
+    tmp = f"{target}.{os.getpid()}.tmp"
+    try:
+        _run([cc, "-x", "c", "-O2", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], _src_path("launch.c"), "-o", tmp], "launch.c")
+    except BuildError as exc:
+        _say(f"{exc}; launchers are called by ctypes")
+        return None
+    os.replace(tmp, target)
+    for old in os.listdir(_build_dir()):
+        path = os.path.join(_build_dir(), old)
+        if re.fullmatch(r"ll_launch_[0-9a-f]{16}\.so", old) and path != target:
+            try:
+                os.remove(path)
+            except OSError:
+                pass
+    return target
+
+
+def _native_call():
+    """``call(address, *args)`` of launch.c, or None."""
+    path = build_launch()
+    if path is None:
+        return None
+    spec = importlib.util.spec_from_file_location("_ll_launch", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module.call
+
+
 class Library:
-    """A loaded kernel library; ``call(symbol, *args)`` checks the returned cudaError_t."""
+    """A loaded kernel library; ``call(symbol, *args)`` (ints, floats, None, or ctypes objects) checks the returned cudaError_t."""
 
     def __init__(self, name: str, path: str):
         self.name = name
         self.path = path
         self._dll = ctypes.CDLL(path)
         self._fns: Dict[str, ctypes._CFuncPtr] = {}
+        self._addresses: Dict[str, int] = {}
+        self._native = _native_call()
 
     def fn(self, symbol: str):
         f = self._fns.get(symbol)
@@ -250,7 +308,13 @@ class Library:
     def call(self, symbol: str, *args) -> None:
         global LAUNCHES
         LAUNCHES += 1
-        err = self.fn(symbol)(*args)
+        if self._native is not None:
+            address = self._addresses.get(symbol)
+            if address is None:
+                address = self._addresses[symbol] = ctypes.cast(self.fn(symbol), ctypes.c_void_p).value
+            err = self._native(address, *args)
+        else:
+            err = _by_ctypes(self.fn(symbol), args)
         if err != 0:
             raise RuntimeError(f"{symbol} failed with CUDA error {err} "
                                f"(1 = invalid value: a size this kernel does not take)")
@@ -258,6 +322,9 @@ class Library:
 
 def load_library(name: str) -> Library:
     """Build (if needed) and load a kernel library.  Raises if that is not possible."""
+    lib = _loaded.get(name)
+    if lib is not None:
+        return lib
     with _lock:
         lib = _loaded.get(name)
         if lib is None:
@@ -268,4 +335,5 @@ def load_library(name: str) -> Library:
 
 def build_all(verbose: bool = True) -> List[str]:
     """Compile every declared library (used by the repository's build check)."""
-    return [build_library(n, verbose) for n in sorted(LIBRARIES)]
+    native = build_launch()
+    return [build_library(n, verbose) for n in sorted(LIBRARIES)] + ([native] if native else [])

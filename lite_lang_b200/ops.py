@@ -13,11 +13,10 @@ float32 path TF32 is switched off so that it is a true 32-bit product.
 
 from __future__ import annotations
 
-import ctypes
 import functools
 import os
 import threading
-from ctypes import c_float, c_int, c_long, c_void_p
+from ctypes import c_void_p
 from typing import NamedTuple, Optional, Tuple
 
 import torch
@@ -25,6 +24,9 @@ import torch
 from .csrc.build import load_library
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
+# What a launcher's parameters are: integers and pointers go over as Python's, floats as floats (csrc/launch.c)
+c_int = c_long = int
+c_float = float
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -35,23 +37,24 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _ptr_at(t: torch.Tensor, first: int):
     """Number ``first`` of a contiguous tensor of 32-bit numbers (a slice is another tensor object: 1.5 us)."""
-    return c_void_p(t.data_ptr() + 4 * first)
+    return t.data_ptr() + 4 * first
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)      # (without asking whether CUDA has been started)
 
 
 def _stream():
     """The current CUDA stream's handle.  (``torch.cuda.current_stream()`` builds a Python object through
     several layers, 15 us a call, with well over a hundred launches in a step that is not captured.)"""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(torch.cuda.current_device()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _need_cuda(*ts: Optional[torch.Tensor]) -> None:
@@ -1223,7 +1226,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         "ll_gemm_f32", _ptr(out), c_long(N if out is None else out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight),
         c_long(weight.stride(0)), c_int(M), c_int(N), c_int(K), _ptr(terms), _ptr(parts), c_int(splits),
         c_int(1 if accumulate else 0), c_int(0 if gated is None else GATE_ACT[act.kind] + 1), c_float(act.limit),
-        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(status), _stream())
+        c_float(act.alpha), c_int(sm_count(x.device)), c_void_p(_ptr(status)), _stream())
     return parts if hand_on else out
 
 
@@ -2264,13 +2267,13 @@ def layernorm_into_residual(residual: torch.Tensor, y: torch.Tensor, weight: tor
         _need(y.dtype == torch.float32 and y.is_contiguous() and tuple(y.shape[1:]) == (n, hidden),
               "layernorm_into_residual: partial sums are float32 [parts, tokens, hidden]")
         dt = _dtype_code(copy) if copy is not None else 0
-        core().call("ll_layernorm_into_residual", c_int(dt), _ptr(copy), _ptr(residual), c_void_p(0), _ptr(y),
+        core().call("ll_layernorm_into_residual", c_int(dt), _ptr(copy), _ptr(residual), 0, _ptr(y),
                     c_int(y.shape[0]), c_long(n * hidden), _ptr(weight), c_float(eps), c_int(n), c_int(hidden),
                     _stream())
         return
     _need(y.is_contiguous() and tuple(y.shape) == (n, hidden) and (copy is None or copy.dtype == y.dtype),
           "layernorm_into_residual: y is [tokens, hidden] of the copy's dtype")
-    core().call("ll_layernorm_into_residual", c_int(_dtype_code(y)), _ptr(copy), _ptr(residual), _ptr(y), c_void_p(0),
+    core().call("ll_layernorm_into_residual", c_int(_dtype_code(y)), _ptr(copy), _ptr(residual), _ptr(y), 0,
                 c_int(0), c_long(0), _ptr(weight), c_float(eps), c_int(n), c_int(hidden), _stream())
 
 
