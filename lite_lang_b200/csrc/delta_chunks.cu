@@ -485,6 +485,7 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
   bool dead = false;
   auto copy = [&](const unsigned* dst, const unsigned* src, int place) {      // by one thread
     const unsigned bar = at_smem(full + place);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // what has been read from the place, then the copy
     at_mbar_expect_tx(bar, BYTES);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(ms_smem(dst)),
                  "l"(src), "r"(BYTES), "r"(bar)

@@ -350,6 +350,7 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
     unsigned ph = 0;            // (early < STAGES: nothing is left)
     while (w.uu < p.units) {
       gt_mbar_wait(empty0 + 8 * s, ph, p.status);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the consumers' loads, then the copies
       if (gt_elect()) {
         gt_mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
         gt_tma_w(stage0 + s * STAGE_BYTES, &wmap, w.y, w.kc * KBOXES, full0 + 8 * s);
@@ -463,6 +464,7 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
     const int kc_end = min(kchunks, (kp + 1) * p.cpp);
     for (int kc = kp * p.cpp; kc < kc_end; ++kc) {
       uint4 xv[MYBOXES][2][MT];
+      unsigned held = 0;
       gt_mbar_wait(full0 + 8 * s, ph, p.status);
       // token row 8 j + g of the stage's x box: its 16-byte chunk 4 i + c sits at chunk (4 i + c) ^ g
 #pragma unroll
@@ -481,6 +483,7 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
           const unsigned chunk = ((unsigned)(4 * i + c) ^ sw) * 16;
           const uint4 wa = gt_lds16(box + row_off[0] + chunk);
           const uint4 wb = gt_lds16(box + row_off[1] + chunk);
+          held = wb.x;
 #pragma unroll
           for (int j = 0; j < MT; ++j) {
             gt_mma(acc[j], wa.x, wb.x, wa.y, wb.y, xv[b][i][j].x, xv[b][i][j].y);
@@ -488,8 +491,13 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
           }
         }
       }
+      // The stage goes back when its values are here, not when they have been asked for: the arrival's address takes (no) part of
+      // the last load, and the producer has a proxy fence between the arrivals and the next copy.  An arrival behind the loads and
+      // no more overtook them, and the copy of the ring's next round was in their place: a line of a weight or token row in one
+      // product out of two, K = 2,048 and 12 tokens, beside a kernel of many CTAs that had started early.  (A part of every load:
+      // a decode step at batch 8 989 -> 1,000 us; this way 991.)
       __syncwarp();
-      if (lane == 0) gt_mbar_arrive(empty0 + 8 * s);
+      if (lane == 0) gt_mbar_arrive(empty0 + 8 * s + (held & (unsigned)(p.M >> 31)));
       if (++s == STAGES) {
         s = 0;
         ph ^= 1;
