@@ -180,8 +180,8 @@ attn_prefill_tc_kernel(const AttnTcParams p, const __grid_constant__ CUtensorMap
   const int keep = SHAPED && p.mask == 1 ? p.keep : 0;
   const int kept = min((keep + AT_KB - 1) / AT_KB, lo_min / AT_KB);
   const int nblk_all = kept + hi / AT_KB - lo_min / AT_KB + 1;
-  // splits that have work: about split_len blocks each (the host chooses that length so that the step's CTAs
-  // just fit the SMs at once), none empty; the same for every CTA of the row block
+  // splits that have work: about split_len blocks each (the host chooses that length so that the longest is short and
+  // all find room on the SMs at once), none empty; the same for every CTA of the row block
   int eff = min(p.nsplit, max(1, (nblk_all + p.split_len - 1) / p.split_len));
   const int per = (nblk_all + eff - 1) / eff;
   eff = (nblk_all + per - 1) / per;

@@ -541,38 +541,57 @@ def _attn_tc_scratch_for(device, row_blocks: int, num_kv_heads: int, nsplit: int
 
 
 def attn_prefill_tc_plan(entries, group: int, window: Optional[int], num_kv_heads: int = 1, slots: int = 0,
-                         chunk: Optional[int] = None, keep_first: int = 0):
+                         chunk: Optional[int] = None, keep_first: int = 0, shaped: bool = False):
     """(row blocks, nsplit, split_len) of a step for ``attn_prefill_tc``.  ``entries``: (cached tokens, new tokens)
     per entry; a row block takes floor(128 / group) tokens and walks n key blocks of 64.
 
-    A CTA's blocks are a chain (scores, softmax, P V: about 1.4 us a block), so a step lasts as long as its
-    longest CTA, and a CTA that finds no room on the SMs at once waits for a whole one to end (the hardware hands
-    CTAs out in order).  So row blocks are cut into splits of at most ``split_len`` blocks, with the smallest
-    ``split_len`` for which all CTAs of the step fit the ``slots`` (two an SM) at once: a whole causal prompt of
-    2,048 tokens (row blocks of 1..32 blocks, 2 kv heads) gets 16, i.e. its longer half is cut in two.  Not below
-    4 blocks a split or over 8 splits (every split's partial result goes through scratch memory); when the
-    unsplit row blocks already exceed the slots, nothing is cut.  ``chunk``, ``keep_first``: the masks of shaped scores."""
+    A CTA's blocks are a chain (scores, softmax, P V), so a step lasts as long as its longest CTA, and a CTA that finds no room on
+    the SMs at once waits for a whole one to end (the hardware hands CTAs out in order, and those without work, the splits that a
+    short row block does not have, go through the same door).  So row blocks are cut into splits of at most ``split_len`` blocks
+    where that is shorter by this count, fitted to a hundred steps each cut in several ways: 1.1 us a block (shaped scores 4.5), up to
+    15% more where SMs have two CTAs, 2.2 us a split (shaped 5; a third of one less in all), and only cuts whose CTAs, with those without
+    work that come before the last one with work, find room in the ``slots`` (two an SM).  Measured on a B200 (whole / cut as here /
+    cut to the shortest that has room by itself, longest CTA in blocks and us): 12 heads on 2, 1,400 tokens 22 31.4 / 8 24.7 /
+    7 33.7; 128 behind 4,096: 66 81.9 / 11 28.6 / 9 29.8; 16 on 2, 1,400: 22 31.3 / 11 28.2 / 10 35.2; 12 on 12 with a window of 512,
+    2,048 in three portions: 10 21.0 (whole here) / 8 28.7; 28 on 4, 700: 11 19.6 / 6 19.6 / 5 23.3; shaped scores, 12 on 2, 1,400:
+    11 48.9 / 6 47.5 / 5 59.2; 28 on 4, 700: 11 66.9 / 6 48.1 / 5 55.1.  ``chunk``, ``keep_first``: the masks of shaped scores."""
     tpb = 128 // group
-    lengths = []
+    lengths: dict = {}
+    blocks = 0
     for ctx, q in entries:
         for first in range(0, q, tpb):
             hi = ctx + min(first + tpb, q) - 1
             lo = max(0, ctx + first - window + 1) if window else (ctx + first) // chunk * chunk if chunk else 0
-            lengths.append(hi // 64 - lo // 64 + 1 + min((keep_first + 63) // 64, lo // 64))
-    blocks = len(lengths)
+            n = hi // 64 - lo // 64 + 1 + min((keep_first + 63) // 64, lo // 64)
+            lengths[n] = lengths.get(n, 0) + num_kv_heads
+            blocks += 1
     if not lengths or slots <= 0 or blocks * num_kv_heads > slots:
         return blocks, 1, 1 << 20
     longest = max(lengths)
-    best = longest
-    for t in range(max(4, (longest + 7) // 8), longest + 1):
-        if sum((n + t - 1) // t for n in lengths) * num_kv_heads <= slots:
-            best = t
-            break
-    if best * 5 > longest * 4:      # cutting off less than a fifth of the longest chain does not pay for the merges
-        return blocks, 1, 1 << 20   # (four portions of 512 behind 1,536 tokens: 49 us uncut, 52.5 us cut at 29 of 32)
+    a_block, a_part, slower = (4.5, 5.0, 0.15) if shaped else (1.1, 2.2, 0.15)
+
+    def time(t: int, parts: int, ctas: int) -> float:
+        return a_block * t * (1 + slower * max(0.0, 2 * ctas / slots - 1)) + (a_part * (parts - 0.33) if parts > 1 else 0.0)
+
+    best, least = longest, time(longest, 1, blocks * num_kv_heads)
+    over, above = [0] * (longest + 1), 0             # over[m]: CTAs of row blocks of more than m blocks
+    for n in range(longest, 0, -1):
+        above += lengths.get(n, 0)
+        over[n - 1] = above
+    for t in range(max(5, (longest + 7) // 8), longest, 1 + longest // 64):
+        parts = (longest + t - 1) // t
+        if time(t, parts, 0) >= least:
+            continue
+        ctas = sum(over[:longest:t])                                            # with work; then without, in front of the last round's
+        idle = parts * over[0] - over[0] - (ctas - over[(parts - 1) * t])
+        if ctas <= slots and ctas + idle <= slots * 21 // 20:
+            took = time(t, parts, ctas)
+            if took < least:
+                best, least = t, took
+    if best == longest:
+        return blocks, 1, 1 << 20
     most = (longest + best - 1) // best
-    nsplit = 1 if most <= 1 else 2 if most <= 2 else 4 if most <= 4 else 8
-    return blocks, nsplit, best
+    return blocks, 2 if most <= 2 else 4 if most <= 4 else 8, best
 
 
 def attn_prefill_tc_splits(row_blocks: int, num_kv_heads: int, device) -> int:

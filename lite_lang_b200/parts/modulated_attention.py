@@ -392,8 +392,8 @@ class ModulatedAttention(Mixer):
             spans = [(c, len(e.tokens)) for c, e in zip(step.entry_ctx[n_single:], step.entries[n_single:])]
             plan = step.scratch[key] = ops.attn_prefill_tc_plan(
                 spans, group, self.mask_size if self.mask == "window" else None, self.num_kv_heads, 2 * ops.sm_count(q.device),
-                self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0
-            ) if (ops.attn_prefill_tc_supported(q.dtype, self.key_dim, page_size, q.stride(0), group)
+                self.mask_size if self.mask == "chunk" else None, self.keep_first if self.mask == "window" else 0,
+                shaped=True) if (ops.attn_prefill_tc_supported(q.dtype, self.key_dim, page_size, q.stride(0), group)
                   and self._tc_preferred(spans, group)) else None
         return plan
 
