@@ -1,4 +1,5 @@
-// The gated delta rule of prompt portions with one decay a head, 64 tokens at a time (what a chunk is: chunk_scan.cu).
+// The gated delta rule of prompt portions, 64 tokens at a time (what a chunk is: chunk_scan.cu), with one decay a head as written here or
+// one a key channel (delta_solve_channels).
 //
 //     S <- a_t S;   u_t = beta_t (v_t - S^T k_t);   S <- S + k_t u_t^T;   o_t = S^T q_t
 // With L(t, s) = beta_t G(t, s) (k_t . k_s), s < t, the values that a chunk writes are u = U - W S0 with
@@ -128,6 +129,109 @@ template <int DK> __device__ __noinline__ void dc_again_w(const bf16* Lp, const 
 }
 __device__ __noinline__ void dc_again_u(const bf16* Lp, const float* rhs, long rs, int n, const float* bt, float* u) {
   dc_again(Lp, rhs, rs, n, bt, nullptr, [&](int t) { return u[t]; }, [&](int t, float x) { u[t] = x; });
+}
+
+// The inverse of a block 1 + L_ii of the four in Ld, a column a thread (tid < 64): x_i = [i = j] - sum over m < i of L(i, m) x_m, its
+// terms without the ones.
+__device__ __forceinline__ void dc_invert(const float* Ld, bf16* Tp, int tid) {
+  const int blk = tid >> 4, j = tid & 15;
+  const float* l = Ld + blk * 16 * 20;
+  float x[DC_BLOCK];
+#pragma unroll
+  for (int i = 0; i < DC_BLOCK; ++i) {
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int m = 0; m < i; m += 4) {
+      const float4 l4 = *reinterpret_cast<const float4*>(l + i * 20 + m);
+      s0 = fmaf(-l4.x, x[m], s0);
+      if (m + 1 < i) s1 = fmaf(-l4.y, x[m + 1], s1);
+      if (m + 2 < i) s0 = fmaf(-l4.z, x[m + 2], s0);
+      if (m + 3 < i) s1 = fmaf(-l4.w, x[m + 3], s1);
+    }
+    x[i] = j < i ? s0 + s1 : j == i ? 1.f : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < DC_BLOCK; ++i) {
+    unsigned p0, p1, p2;
+    ms_split(i == j ? 0.f : x[i], 0.f, p0, p1, p2);
+    unsigned short* d = reinterpret_cast<unsigned short*>(Tp + (blk * 16 + i) * DC_TP + j);
+    d[0] = (unsigned short)p0;
+    d[CS_C * DC_TP] = (unsigned short)p1;
+    d[2 * CS_C * DC_TP] = (unsigned short)p2;
+  }
+}
+
+// 16 columns (tile `tile`: W's, or U's behind them) of the system: X^T block by block, rhs(i, nt, j) the right-hand side's number of the
+// lane, next(i) what is asked for behind the i-th.  W's terms go to wrow, U's numbers to urow.  Whether a number is not finite.
+template <int TILES, typename R, typename N>
+__device__ __forceinline__ bool dc_columns(unsigned Lp_b, unsigned Tp_b, bool is_k, int tile, unsigned* wrow, float* urow, R rhs, N next) {
+  const int lane = threadIdx.x & 31, mt = lane >> 3, r = lane & 7, c = lane & 3;
+  unsigned xa[3][3][4];                               // the terms of X^T's first three blocks
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float acc[2][4] = {}, low[2][4] = {};
+#pragma unroll
+    for (int m = 0; m < i; ++m) {
+      unsigned b[2][3][2];
+      ms_load_b<3, false>(b, Lp_b + 2 * ((i * 16 + (mt >> 1) * 8 + r) * DC_LP + m * 16 + (mt & 1) * 8), 2 * CS_C * DC_LP);
+      ms_terms<2, 3, 3>(acc, low, xa[m], b);
+    }
+    unsigned ra[3][4];
+    float y[2][4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y[nt][j] = rhs(i, nt, j) - (acc[nt][j] + low[nt][j]);
+      }
+      ms_split(y[nt][0], y[nt][1], ra[0][2 * nt], ra[1][2 * nt], ra[2][2 * nt]);
+      ms_split(y[nt][2], y[nt][3], ra[0][2 * nt + 1], ra[1][2 * nt + 1], ra[2][2 * nt + 1]);
+    }
+    next(i);
+    unsigned b[2][3][2];
+    ms_load_b<3, false>(b, Tp_b + 2 * ((i * 16 + (mt >> 1) * 8 + r) * DC_TP + (mt & 1) * 8), 2 * CS_C * DC_TP);
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[nt][j] = low[nt][j] = 0.f;
+    ms_terms<2, 3, 3>(acc, low, ra, b);
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[nt][j] = y[nt][j] + (acc[nt][j] + low[nt][j]);
+        odd |= !(fabsf(acc[nt][j]) < INFINITY);
+      }
+      const int t = i * 16 + nt * 8 + 2 * c;
+      unsigned lo[3], hi[3];                          // the terms of columns gr and gr + 8
+      if (i < 3 || is_k) {
+        ms_split(acc[nt][0], acc[nt][1], lo[0], lo[1], lo[2]);
+        ms_split(acc[nt][2], acc[nt][3], hi[0], hi[1], hi[2]);
+      }
+      if (i < 3) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          xa[i][p][2 * nt] = lo[p];
+          xa[i][p][2 * nt + 1] = hi[p];
+        }
+      }
+      if (is_k) {
+        DcFrag f;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          f.b[p][0] = dc_turned(lo[p]);
+          f.b[p][1] = dc_turned(hi[p]);
+        }
+        dc_frag_put<TILES>(wrow, tile * 8 + 2 * i + nt, lane, f);
+      } else {
+        float* d = urow + t;
+        *reinterpret_cast<float2*>(d) = make_float2(acc[nt][0], acc[nt][1]);
+        *reinterpret_cast<float2*>(d + 8 * CS_C) = make_float2(acc[nt][2], acc[nt][3]);
+      }
+    }
+  }
+  return odd;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -300,34 +404,7 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
     }
   }
   __syncthreads();
-  // the inverse of a block 1 + L_ii, a column a thread: x_i = [i = j] - sum over m < i of L(i, m) x_m, without the ones
-  if (tid < CS_C) {
-    const int blk = tid >> 4, j = tid & 15;
-    const float* l = Ld + blk * 16 * 20;
-    float x[DC_BLOCK];
-#pragma unroll
-    for (int i = 0; i < DC_BLOCK; ++i) {
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-      for (int m = 0; m < i; m += 4) {
-        const float4 l4 = *reinterpret_cast<const float4*>(l + i * 20 + m);
-        s0 = fmaf(-l4.x, x[m], s0);
-        if (m + 1 < i) s1 = fmaf(-l4.y, x[m + 1], s1);
-        if (m + 2 < i) s0 = fmaf(-l4.z, x[m + 2], s0);
-        if (m + 3 < i) s1 = fmaf(-l4.w, x[m + 3], s1);
-      }
-      x[i] = j < i ? s0 + s1 : j == i ? 1.f : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < DC_BLOCK; ++i) {
-      unsigned p0, p1, p2;
-      ms_split(i == j ? 0.f : x[i], 0.f, p0, p1, p2);
-      unsigned short* d = reinterpret_cast<unsigned short*>(Tp + (blk * 16 + i) * DC_TP + j);
-      d[0] = (unsigned short)p0;
-      d[CS_C * DC_TP] = (unsigned short)p1;
-      d[2 * CS_C * DC_TP] = (unsigned short)p2;
-    }
-  }
+  if (tid < CS_C) dc_invert(Ld, Tp, tid);
   if (h == hk * group) {                                // k's terms, once for the heads that read it
     unsigned* dst = kp + ((size_t)item * Hk + hk) * TILES * 192;
     for (int tile = 2 * warp; tile < TILES; tile += CS_THREADS / 16) {
@@ -347,72 +424,15 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
     const bool is_k = tile < DK / 16;
     const int c0 = is_k ? tile * 16 : tile * 16 - DK;
     unsigned* wrow = wt + ih * TILES * 192;
-    unsigned xa[3][3][4];                               // the terms of X^T's first three blocks
-    bool odd = false;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float acc[2][4] = {}, low[2][4] = {};
-#pragma unroll
-      for (int m = 0; m < i; ++m) {
-        unsigned b[2][3][2];
-        ms_load_b<3, false>(b, Lp_b + 2 * ((i * 16 + (mt >> 1) * 8 + r) * DC_LP + m * 16 + (mt & 1) * 8), 2 * CS_C * DC_LP);
-        ms_terms<2, 3, 3>(acc, low, xa[m], b);
-      }
-      unsigned ra[3][4];
-      float y[2][4];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
+    const bool odd = dc_columns<TILES>(
+        Lp_b, Tp_b, is_k, tile, wrow, ut + (ih * DV + c0 + gr) * CS_C,
+        [&](int i, int nt, int j) {
           const int t = i * 16 + nt * 8 + 2 * c + (j & 1);
-          y[nt][j] = bx[i][nt][j] * (is_k ? bt[t] * pre[t] : bt[t]) - (acc[nt][j] + low[nt][j]);
-        }
-        ms_split(y[nt][0], y[nt][1], ra[0][2 * nt], ra[1][2 * nt], ra[2][2 * nt]);
-        ms_split(y[nt][2], y[nt][3], ra[0][2 * nt + 1], ra[1][2 * nt + 1], ra[2][2 * nt + 1]);
-      }
-      if (tile + CS_THREADS / 32 < (DK + DV) / 16) ask_b(tile + CS_THREADS / 32, i);
-      unsigned b[2][3][2];
-      ms_load_b<3, false>(b, Tp_b + 2 * ((i * 16 + (mt >> 1) * 8 + r) * DC_TP + (mt & 1) * 8), 2 * CS_C * DC_TP);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[nt][j] = low[nt][j] = 0.f;
-      ms_terms<2, 3, 3>(acc, low, ra, b);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[nt][j] = y[nt][j] + (acc[nt][j] + low[nt][j]);
-          odd |= !(fabsf(acc[nt][j]) < INFINITY);
-        }
-        const int t = i * 16 + nt * 8 + 2 * c;
-        unsigned lo[3], hi[3];                          // the terms of columns gr and gr + 8
-        if (i < 3 || is_k) {
-          ms_split(acc[nt][0], acc[nt][1], lo[0], lo[1], lo[2]);
-          ms_split(acc[nt][2], acc[nt][3], hi[0], hi[1], hi[2]);
-        }
-        if (i < 3) {
-#pragma unroll
-          for (int p = 0; p < 3; ++p) {
-            xa[i][p][2 * nt] = lo[p];
-            xa[i][p][2 * nt + 1] = hi[p];
-          }
-        }
-        if (is_k) {
-          DcFrag f;
-#pragma unroll
-          for (int p = 0; p < 3; ++p) {
-            f.b[p][0] = dc_turned(lo[p]);
-            f.b[p][1] = dc_turned(hi[p]);
-          }
-          dc_frag_put<TILES>(wrow, tile * 8 + 2 * i + nt, lane, f);
-        } else {
-          float* d = ut + (ih * DV + c0 + gr) * CS_C + t;
-          *reinterpret_cast<float2*>(d) = make_float2(acc[nt][0], acc[nt][1]);
-          *reinterpret_cast<float2*>(d + 8 * CS_C) = make_float2(acc[nt][2], acc[nt][3]);
-        }
-      }
-    }
+          return bx[i][nt][j] * (is_k ? bt[t] * pre[t] : bt[t]);
+        },
+        [&](int i) {
+          if (tile + CS_THREADS / 32 < (DK + DV) / 16) ask_b(tile + CS_THREADS / 32, i);
+        });
     // columns gr and gr + 8 of the tile have a number that is not finite in some lane of the four: its first lane makes them again
     const unsigned bad = __ballot_sync(0xffffffffu, odd);
     __syncwarp();
@@ -422,6 +442,276 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
         const int col = c0 + gr + 8 * q;
         if (is_k) dc_again_w<DK>(Lp, krow + col, Cq, n, bt, pre, wrow, col);
         else dc_again_u(Lp, vc + (size_t)base * Cv + (size_t)h * DV + col, Cv, n, bt, ut + (ih * DV + col) * CS_C);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The same with a decay a key channel: L(t, s) = beta_t sum over the channels of k_t G(t, s) k_s, and so on.  A quotient of running
+// products would overflow, so G is made of factors that are at most one: within a block of 16 tokens (s, t of the same) a thread has
+// 8 or 16 channels of k_s and multiplies decay by decay while it adds up the products with the tokens behind; between blocks
+// G(t, s) = R(t) B Y(s), R from t's block's start, Y to s's block's end, B the blocks between, and k_t R(t), q_t R(t) and k_s Y(s) B are
+// the operands of products on the tensor cores.  What the walk multiplies the state by is rounded once (DcProduct).
+// qd [items][H][64][DK] = G(t, -) q_t, kp [items][H] = the terms of G(C, s) k_s, gam [items][H][DK] = G(C, -); the rest as above.
+// One CTA an SM (191 KB of shared memory).  Two entries of together 2,047 tokens, 12 heads: the three kernels 153 us, the walk by tokens
+// 857; its error against 64 bits is half the walk's.
+// ---------------------------------------------------------------------------------------------------------------
+#define DC_CH_THREADS 512
+template <int DK, int DV>
+__global__ void __launch_bounds__(DC_CH_THREADS, 1)
+delta_solve_channels_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
+                            const float* __restrict__ beta, const float* __restrict__ g, const int* __restrict__ cu_q,
+                            const int* __restrict__ req_slot, int E, float* __restrict__ ut, unsigned* __restrict__ wt,
+                            unsigned* __restrict__ kp, float* __restrict__ mm, float* __restrict__ qd, float* __restrict__ gam, int H,
+                            int Hk) {
+  constexpr int FP = DK + 8, TILES = DK / 2, WARPS = DC_CH_THREADS / 32, PIECES = DK / 4;
+  extern __shared__ __align__(16) unsigned char cs_smem[];
+  float* kf = reinterpret_cast<float*>(cs_smem);                 // [64][FP] each: k, q
+  float* qf = kf + CS_C * FP;
+  float* rf = qf + CS_C * FP;                                    // decays, R, at last k G(t, -)
+  float* yf = rf + CS_C * FP;                                    // Y, at last k G(C, s)
+  bf16* Lp = reinterpret_cast<bf16*>(yf + CS_C * FP);            // [3][64][DC_LP]
+  bf16* Tp = Lp + 3 * CS_C * DC_LP;                              // [3][64][DC_TP]
+  float* Ld = reinterpret_cast<float*>(Tp + 3 * CS_C * DC_TP);   // [64][20]
+  DcProduct* blk = reinterpret_cast<DcProduct*>(Ld + CS_C * 20);      // [4][DK]: whole blocks
+  float* front = reinterpret_cast<float*>(blk + 4 * DK);         // [4][DK]: the blocks in front of a block
+  float* behind = front + 4 * DK;                                // [4][DK]: behind it
+  float* mid = behind + 4 * DK;                                  // [4][DK]: between blocks 0 and 2, 1 and 3, 0 and 3; ones
+  __shared__ float bt[CS_C];
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int item = blockIdx.x, h = blockIdx.y, hk = h / (H / Hk);
+  int e, chunk;
+  if (!cs_item(item, cu_q, E, e, chunk)) return;
+  if (req_slot[e] < 0) return;
+  const int base = cu_q[e] + chunk * CS_C, n = min(CS_C, cu_q[e + 1] - base);
+  const long Cq = (long)Hk * DK, Cv = (long)H * DV;
+  const size_t ih = (size_t)item * H + h;
+  const int gr = lane >> 2, c = lane & 3;
+  {
+    const float* krow = kn + (size_t)base * Cq + hk * DK;
+    const float* qrow = qn + (size_t)base * Cq + hk * DK;
+    const float* arow = g + ((size_t)base * H + h) * DK;
+    constexpr int N = CS_C * PIECES / DC_CH_THREADS;
+    float4 v[3][N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int i = j * DC_CH_THREADS + tid, t = i / PIECES, ch = i % PIECES * 4;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0][j] = t < n ? *reinterpret_cast<const float4*>(krow + (size_t)t * Cq + ch) : z;
+      v[1][j] = t < n ? *reinterpret_cast<const float4*>(qrow + (size_t)t * Cq + ch) : z;
+      v[2][j] = t < n ? *reinterpret_cast<const float4*>(arow + (size_t)t * H * DK + ch) : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    if (tid < CS_C) bt[tid] = tid < n ? beta[(size_t)(base + tid) * H + h] : 0.f;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int i = j * DC_CH_THREADS + tid, at = i / PIECES * FP + i % PIECES * 4;
+      *reinterpret_cast<float4*>(kf + at) = v[0][j];
+      *reinterpret_cast<float4*>(qf + at) = v[1][j];
+      *reinterpret_cast<float4*>(rf + at) = v[2][j];
+    }
+  }
+  __syncthreads();
+  float* mrow = mm + ih * CS_C * CS_C;
+  auto put_l = [&](int t, int s, float x, float y) {             // L(t, s) and L(t, s + 1)
+    unsigned p0, p1, p2;
+    ms_split(x, y, p0, p1, p2);
+    unsigned* d = reinterpret_cast<unsigned*>(Lp + t * DC_LP + s);
+    d[0] = p0;
+    d[CS_C * DC_LP / 2] = p1;
+    d[CS_C * DC_LP] = p2;
+  };
+  // the blocks on the diagonal: eight threads a token s, channels 4 (tid % 8) + 32 j
+  {
+    const int s = tid >> 3, cg = tid & 7, b0 = s & ~15;
+    float kg[DK / 8], v[32];
+#pragma unroll
+    for (int j = 0; j < DK / 32; ++j) *reinterpret_cast<float4*>(kg + 4 * j) = *reinterpret_cast<const float4*>(kf + s * FP + cg * 4 + 32 * j);
+#pragma unroll
+    for (int tt = 0; tt < 16; ++tt) {
+      const int t = b0 + tt;
+      float dk = 0.f, dq = 0.f;
+#pragma unroll
+      for (int j = 0; j < DK / 32; ++j) {
+        const int at = t * FP + cg * 4 + 32 * j;
+        const float4 a4 = *reinterpret_cast<const float4*>(rf + at), k4 = *reinterpret_cast<const float4*>(kf + at);
+        const float4 q4 = *reinterpret_cast<const float4*>(qf + at);
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, kv[4] = {k4.x, k4.y, k4.z, k4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (t > s) kg[4 * j + i] *= av[i];
+          dk = fmaf(kv[i], kg[4 * j + i], dk);
+          dq = fmaf(qv[i], kg[4 * j + i], dq);
+        }
+      }
+      v[2 * tt] = dk;
+      v[2 * tt + 1] = dq;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)                              // a lane keeps half of what it has at each step: two tokens t at last
+#pragma unroll
+      for (int i = 0; i < 4 * o; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, cg & o ? v[i] : v[i + 4 * o], o);
+        v[i] = (cg & o ? v[i + 4 * o] : v[i]) + other;
+      }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = b0 + 2 * cg + i;
+      const float x = s < t ? bt[t] * v[2 * i] : 0.f;
+      unsigned p0, p1, p2;
+      ms_split(x, 0.f, p0, p1, p2);
+      unsigned short* d = reinterpret_cast<unsigned short*>(Lp + t * DC_LP + s);
+      d[0] = (unsigned short)p0;
+      d[CS_C * DC_LP] = (unsigned short)p1;
+      d[2 * CS_C * DC_LP] = (unsigned short)p2;
+      Ld[t * 20 + (s & 15)] = x;
+      mrow[t * CS_C + s] = s <= t ? v[2 * i + 1] : 0.f;
+    }
+  }
+  __syncthreads();
+  // R, Y and whole blocks: a thread a channel and block
+  if (tid < 4 * DK) {
+    const int ch = tid % DK, b = tid / DK;
+    float* a = rf + b * 16 * FP + ch;
+    float* y = yf + b * 16 * FP + ch;
+    float av[16];
+    DcProduct p;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      av[t] = a[t * FP];
+      p.times(av[t]);
+      a[t * FP] = p.value();
+    }
+    blk[b * DK + ch] = p;
+    p = DcProduct();
+#pragma unroll
+    for (int t = 15; t >= 0; --t) {
+      y[t * FP] = p.value();
+      p.times(av[t]);
+    }
+  }
+  __syncthreads();
+  if (tid < DK) {
+    const DcProduct b0 = blk[tid], b1 = blk[DK + tid], b2 = blk[2 * DK + tid], b3 = blk[3 * DK + tid];
+    DcProduct f = b0, w = b3;
+    front[tid] = 1.f;
+    front[DK + tid] = f.value();
+    f.times(b1);
+    front[2 * DK + tid] = f.value();
+    f.times(b2);
+    front[3 * DK + tid] = f.value();
+    f.times(b3);
+    gam[ih * DK + tid] = f.value();
+    behind[3 * DK + tid] = 1.f;
+    behind[2 * DK + tid] = w.value();
+    w.times(b2);
+    behind[DK + tid] = w.value();
+    w.times(b1);
+    behind[tid] = w.value();
+    mid[tid] = b1.value();
+    mid[DK + tid] = b2.value();
+    DcProduct m = b1;
+    m.times(b2);
+    mid[2 * DK + tid] = m.value();
+    mid[3 * DK + tid] = 1.f;
+  }
+  __syncthreads();
+  // the blocks below the diagonal, L's and M's, a warp each; two more warps invert the ones on it
+  if (warp < 12) {
+    const int pair = warp >> 1, I = pair < 1 ? 1 : pair < 3 ? 2 : 3, J = pair - (I * (I - 1)) / 2;
+    const float* row = (warp & 1 ? qf : kf) + (I * 16 + gr) * FP + 2 * c;
+    const float* fac = rf + (I * 16 + gr) * FP + 2 * c;
+    const float* col = kf + (J * 16 + gr) * FP + 2 * c;
+    const float* yac = yf + (J * 16 + gr) * FP + 2 * c;
+    const float* between = mid + (I - J == 1 ? 3 : I - J == 3 ? 2 : J) * DK + 2 * c;
+    float acc[2][4] = {}, low[2][4] = {};
+#pragma unroll 2
+    for (int kt = 0; kt < DK / 16; ++kt) {
+      unsigned a[3][4], b[2][3][2];
+      auto two = [](const float* p, const float* q) {
+        const float2 x = *reinterpret_cast<const float2*>(p), y = *reinterpret_cast<const float2*>(q);
+        return make_float2(x.x * y.x, x.y * y.y);
+      };
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int at = kt * 16 + (j & 1) * 8 * FP + (j >> 1) * 8;
+        const float2 x = two(row + at, fac + at);
+        ms_split(x.x, x.y, a[0][j], a[1][j], a[2][j]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int at = kt * 16 + nt * 8 * FP + q * 8;
+          const float2 x = two(col + at, yac + at), y = *reinterpret_cast<const float2*>(between + kt * 16 + q * 8);
+          ms_split(x.x * y.x, x.y * y.y, b[nt][0][q], b[nt][1][q], b[nt][2][q]);
+        }
+      ms_terms<2, 3, 3>(acc, low, a, b);
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int t = I * 16 + gr + 8 * q, s = J * 16 + nt * 8 + 2 * c;
+        const float x = acc[nt][2 * q] + low[nt][2 * q], y = acc[nt][2 * q + 1] + low[nt][2 * q + 1];
+        if (warp & 1) *reinterpret_cast<float2*>(mrow + t * CS_C + s) = make_float2(x, y);
+        else put_l(t, s, bt[t] * x, bt[t] * y);
+      }
+  } else if (warp < 14) {
+    dc_invert(Ld, Tp, tid - 12 * 32);
+  }
+  __syncthreads();
+  // k from the chunk's start and to its end in the factors' places, q from its start for the read-outs
+  for (int i = tid; i < CS_C * PIECES; i += DC_CH_THREADS) {
+    const int t = i / PIECES, ch = i % PIECES * 4, at = t * FP + ch;
+    const float4 k4 = *reinterpret_cast<const float4*>(kf + at), q4 = *reinterpret_cast<const float4*>(qf + at);
+    const float4 f4 = *reinterpret_cast<const float4*>(front + (t >> 4) * DK + ch), b4 = *reinterpret_cast<const float4*>(behind + (t >> 4) * DK + ch);
+    float4 r4 = *reinterpret_cast<const float4*>(rf + at), y4 = *reinterpret_cast<const float4*>(yf + at);
+    r4 = make_float4(r4.x * f4.x, r4.y * f4.y, r4.z * f4.z, r4.w * f4.w);
+    y4 = make_float4(y4.x * b4.x, y4.y * b4.y, y4.z * b4.z, y4.w * b4.w);
+    *reinterpret_cast<float4*>(rf + at) = make_float4(k4.x * r4.x, k4.y * r4.y, k4.z * r4.z, k4.w * r4.w);
+    *reinterpret_cast<float4*>(yf + at) = make_float4(k4.x * y4.x, k4.y * y4.y, k4.z * y4.z, k4.w * y4.w);
+    *reinterpret_cast<float4*>(qd + (ih * CS_C + t) * DK + ch) = make_float4(q4.x * r4.x, q4.y * r4.y, q4.z * r4.z, q4.w * r4.w);
+  }
+  __syncthreads();
+  unsigned* kdst = kp + ih * TILES * 192;
+  for (int tile = warp; tile < TILES; tile += WARPS) {
+    DcFrag f;
+    const float* src = yf + (tile / (DK / 8) * 16 + 2 * c) * FP + tile % (DK / 8) * 8 + gr;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) ms_split(src[8 * q * FP], src[(8 * q + 1) * FP], f.b[0][q], f.b[1][q], f.b[2][q]);
+    dc_frag_put<TILES>(kdst, tile, lane, f);
+  }
+  const unsigned Lp_b = ms_smem(Lp), Tp_b = ms_smem(Tp);
+#pragma unroll 1
+  for (int tile = warp; tile < (DK + DV) / 16; tile += WARPS) {
+    const bool is_k = tile < DK / 16;
+    const int c0 = is_k ? tile * 16 : tile * 16 - DK;
+    const float* vrow = vc + (size_t)base * Cv + (size_t)h * DV + c0 + gr;
+    unsigned* wrow = wt + ih * TILES * 192;
+    float bx[4][2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int t = i * 16 + nt * 8 + 2 * c + (j & 1);
+          bx[i][nt][j] = is_k ? rf[t * FP + c0 + gr + 8 * (j >> 1)] : t < n ? vrow[(size_t)t * Cv + 8 * (j >> 1)] : 0.f;
+        }
+    const bool odd = dc_columns<TILES>(
+        Lp_b, Tp_b, is_k, tile, wrow, ut + (ih * DV + c0 + gr) * CS_C,
+        [&](int i, int nt, int j) { return bx[i][nt][j] * bt[i * 16 + nt * 8 + 2 * c + (j & 1)]; }, [](int) {});
+    const unsigned bad = __ballot_sync(0xffffffffu, odd);
+    __syncwarp();
+    if (((bad >> (lane & 28)) & 15) != 0 && c == 0) {
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        const int col = c0 + gr + 8 * q;
+        if (is_k) dc_again_w<DK>(Lp, rf + col, FP, n, bt, nullptr, wrow, col);
+        else dc_again_u(Lp, vrow + 8 * q, Cv, n, bt, ut + (ih * DV + col) * CS_C);
       }
     }
   }
@@ -439,7 +729,7 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
 // terms made here from float32, 1,180 instructions a warp and chunk; 55 with four warps, or eight that all read all of the state's
 // terms; 59 with W's and k's terms straight from L2 and two CTAs an SM.)  The longest entries' CTAs come first.
 // ---------------------------------------------------------------------------------------------------------------
-template <int DK>
+template <int DK, bool CH>
 __global__ void __launch_bounds__(CS_THREADS)
 delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const unsigned* __restrict__ kp,
                   const float* __restrict__ suf_in, const float* __restrict__ gam, float* __restrict__ s0,
@@ -495,7 +785,7 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
     if (chunk < chunks && tid == 0) copy(wb + (chunk & 1) * WORDS, wt + ((size_t)(first + chunk) * H + h) * WORDS, chunk & 1);
   };
   auto fetch_k = [&](int chunk) {
-    if (chunk < chunks && tid == 0) copy(kb + (chunk & 1) * WORDS, kp + ((size_t)(first + chunk) * Hk + hk) * WORDS, 2 + (chunk & 1));
+    if (chunk < chunks && tid == 0) copy(kb + (chunk & 1) * WORDS, kp + ((size_t)(first + chunk) * (CH ? H : Hk) + (CH ? h : hk)) * WORDS, 2 + (chunk & 1));
   };
   fetch_w(0);
   fetch_k(0);
@@ -555,8 +845,13 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
     for (int p = 0; p < 3; ++p) ms_ldm4(a[0][p], ss_at + 2 * p * 16 * SP);
     float* urow = ut + (ih * dv + c0 + g) * CS_C + tw + 2 * c;
     const float2 u0 = *reinterpret_cast<const float2*>(urow), u1 = *reinterpret_cast<const float2*>(urow + 8 * CS_C);
-    const float2 f2 = *reinterpret_cast<const float2*>(suf_in + ih * CS_C + tw + 2 * c);
-    const float gc = gam[ih];
+    float2 f2 = make_float2(1.f, 1.f), gc[NT];            // (CH: the decays to the chunk's end are in k's terms)
+    if (!CH) f2 = *reinterpret_cast<const float2*>(suf_in + ih * CS_C + tw + 2 * c);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      if (CH) gc[nt] = *reinterpret_cast<const float2*>(gam + ih * DK + kw + nt * 8 + 2 * c);
+      else gc[nt].x = gc[nt].y = gam[ih];
+    }
     put_state(s0 + (ih * dv + c0) * DK + kw);
 #pragma unroll
     for (int i = 0; i < KH; ++i) {
@@ -619,7 +914,7 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) S[nt][j] *= gc;
+      for (int j = 0; j < 4; ++j) S[nt][j] *= j & 1 ? gc[nt].y : gc[nt].x;
 #pragma unroll
     for (int kt = 0; kt < 4; ++kt) {
       const int now = kt & 1, then = now ^ 1;
@@ -661,12 +956,14 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
 }
 
 // The read-out of one token and value column again, token by token from the state in front of the chunk
+// (token j's decay of channel ch: decay[j * step + ch * per_channel])
 template <int DK>
-__device__ __noinline__ float dc_number(const float* q, const float* k, long stride, const float* u, const float* state, const float* av,
-                                        int t) {
+__device__ __noinline__ float dc_number(const float* q, const float* k, long stride, const float* u, const float* state, const float* decay,
+                                        long step, int per_channel, int t) {
   float a = 0.f;
   for (int ch = 0; ch < DK && a == a; ++ch)
-    a = fmaf(cs_again<float>(state + ch, k + ch, stride, u, 1, t, [&](int j) { return av[j]; }, [](int) { return 1.f; }),
+    a = fmaf(cs_again<float>(state + ch, k + ch, stride, u, 1, t, [&](int j) { return decay[j * step + ch * per_channel]; },
+                             [](int) { return 1.f; }),
              q[(size_t)t * stride + ch], a);
   return a;
 }
@@ -681,7 +978,7 @@ __device__ __noinline__ float dc_number(const float* q, const float* k, long str
 // time and one CTA an SM: 46 us for 384 (chunk, head) pairs; norm and gate behind the products here: 43 us instead of 27 and a kernel
 // of 10.)
 // ---------------------------------------------------------------------------------------------------------------
-template <int DK, int DV>
+template <int DK, int DV, bool CH>
 __global__ void __launch_bounds__(CS_THREADS, 2)
 delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ g,
                   const int* __restrict__ cu_q, const int* __restrict__ req_slot, int E, int num_slots,
@@ -712,9 +1009,10 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   {
     CsTile<float, DK, KP, CS_THREADS> qt;
     CsTile<float, CS_C, DC_LP, CS_THREADS> m_;
-    qt.ask(qrow, Cq, n);
+    if (CH) qt.ask(pre_in + ih * CS_C * DK, DK, n);
+    else qt.ask(qrow, Cq, n);
     m_.ask(mm + ih * CS_C * CS_C, CS_C, CS_C);
-    if (tid < CS_C) {
+    if (!CH && tid < CS_C) {
       av[tid] = tid < n ? g[(size_t)(base + tid) * H + h] : 1.f;
       pre[tid] = pre_in[ih * CS_C + tid];
     }
@@ -760,7 +1058,7 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float f0 = pre[i * 16 + gr], f1 = pre[i * 16 + gr + 8];
+    const float f0 = CH ? 1.f : pre[i * 16 + gr], f1 = CH ? 1.f : pre[i * 16 + gr + 8];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -804,7 +1102,8 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
           const int t = i * 16 + gr + 8 * (j >> 1);
           const size_t v = ih * DV + v0 + nt * 8 + 2 * c + (j & 1);
           if (t < n && !(fabsf(acc[i][nt][j]) < INFINITY))
-            acc[i][nt][j] = dc_number<DK>(qrow, krow, Cq, ut + v * CS_C, s0 + v * DK, av, t);
+            acc[i][nt][j] = CH ? dc_number<DK>(qrow, krow, Cq, ut + v * CS_C, s0 + v * DK, g + ((size_t)base * H + h) * DK, (long)H * DK, 1, t)
+                               : dc_number<DK>(qrow, krow, Cq, ut + v * CS_C, s0 + v * DK, av, 1, 0, t);
         }
   }
 #pragma unroll
@@ -819,48 +1118,59 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     }
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool CH>
 static int dc_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* g, float* state,
                    long state_stride, int num_slots, const int* cu_q, const int* req_slot, float* o, int E, int H, int Hk,
                    float* s0, float* ut, unsigned* wt, unsigned* kp, float* m, float* suf, float* pre, float* gam, int items, int* status,
                    cudaStream_t stream) {
-  const size_t solve = 2 * (size_t)3 * CS_C * (DK + 8 + DC_LP + DC_TP) + 4 * (size_t)CS_C * (20 + DC_GP);
+  const size_t solve = CH ? 4 * (size_t)CS_C * (4 * (DK + 8) + 20) + 2 * (size_t)3 * CS_C * (DC_LP + DC_TP) + 4 * (size_t)20 * DK
+                          : 2 * (size_t)3 * CS_C * (DK + 8 + DC_LP + DC_TP) + 4 * (size_t)CS_C * (20 + DC_GP);
   const size_t walk = 2 * (size_t)4 * 3 * CS_C * DK + 2 * (size_t)3 * 16 * (DK + 8 + CS_C + 8) + 16 * (size_t)CS_THREADS;
   const size_t read = 2 * (size_t)3 * CS_C * (DK + 8 + DC_LP);
-  cudaError_t rc = cs_room<delta_solve_kernel<DK, DV>>(solve);
+  cudaError_t rc;
+  if constexpr (CH) rc = cs_room<delta_solve_channels_kernel<DK, DV>>(solve);
+  else rc = cs_room<delta_solve_kernel<DK, DV>>(solve);
   if (rc != cudaSuccess) return (int)rc;
-  rc = cs_room<delta_walk_kernel<DK>>(walk);
+  rc = cs_room<delta_walk_kernel<DK, CH>>(walk);
   if (rc != cudaSuccess) return (int)rc;
-  rc = cs_room<delta_read_kernel<DK, DV>>(read);
+  rc = cs_room<delta_read_kernel<DK, DV, CH>>(read);
   if (rc != cudaSuccess) return (int)rc;
-  ll_launch(delta_solve_kernel<DK, DV>, dim3(items, H), dim3(CS_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q, req_slot, E, ut,
-            wt, kp, m, suf, pre, gam, H, Hk);
-  ll_launch(delta_walk_kernel<DK>, dim3(DV / 16, H, E), dim3(CS_THREADS), walk, stream, ut, (const unsigned*)wt, (const unsigned*)kp,
+  if constexpr (CH)
+    ll_launch(delta_solve_channels_kernel<DK, DV>, dim3(items, H), dim3(DC_CH_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q,
+              req_slot, E, ut, wt, kp, m, pre, gam, H, Hk);
+  else
+    ll_launch(delta_solve_kernel<DK, DV>, dim3(items, H), dim3(CS_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q, req_slot, E, ut,
+              wt, kp, m, suf, pre, gam, H, Hk);
+  ll_launch(delta_walk_kernel<DK, CH>, dim3(DV / 16, H, E), dim3(CS_THREADS), walk, stream, ut, (const unsigned*)wt, (const unsigned*)kp,
             (const float*)suf, (const float*)gam, s0, state, state_stride, num_slots, cu_q, req_slot, E, H, Hk, DV, status);
-  ll_launch(delta_read_kernel<DK, DV>, dim3(items, H), dim3(CS_THREADS), read, stream, qn, kn, g, cu_q, req_slot, E, num_slots,
+  ll_launch(delta_read_kernel<DK, DV, CH>, dim3(items, H), dim3(CS_THREADS), read, stream, qn, kn, g, cu_q, req_slot, E, num_slots,
             (const float*)s0, (const float*)ut, (const float*)m, (const float*)pre, o, H, Hk);
   return LL_LAUNCH_RESULT();
 }
 
-// The recurrence of ll_delta_recurrence (delta_rule.cu) with one decay a head, by chunks: three launches.  `items`: at least the
-// number of chunks of 64 tokens of the step's entries.  Scratch, 32 bits a number, at multiples of 16 bytes: s0 [items][H][dv][dk],
-// ut [items][H][dv][64], wt [items][H][96 dk], kp [items][Hk][96 dk], m [items][H][64][64], suf and pre [items][H][64],
-// gam [items][H].
+// The recurrence of ll_delta_recurrence (delta_rule.cu) by chunks: three launches.  `items`: at least the number of chunks of 64 tokens
+// of the step's entries.  Scratch, 32 bits a number, at multiples of 16 bytes: s0 [items][H][dv][dk], ut [items][H][dv][64], wt
+// [items][H][96 dk], m [items][H][64][64]; with one decay a head kp [items][Hk][96 dk], suf and pre [items][H][64], gam [items][H];
+// with one a channel kp [items][H][96 dk], pre [items][H][64][dk], gam [items][H][dk] and no suf.
 extern "C" int ll_chunk_delta_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* g,
                                    float* state, long state_stride, int num_slots, const int* cu_q, const int* req_slot,
-                                   float* o, int num_entries, int H, int Hk, int dk, int dv, float* s0, float* ut,
+                                   float* o, int num_entries, int H, int Hk, int dk, int dv, int per_channel, float* s0, float* ut,
                                    void* wt, void* kp, float* m, float* suf, float* pre, float* gam, int items, int* status,
                                    cudaStream_t stream) {
   if (num_entries <= 0 || items <= 0) return 0;
   if (H <= 0 || Hk <= 0 || H % Hk || H > 65535 || num_entries > 65535 || ((uintptr_t)wt | (uintptr_t)kp | (uintptr_t)ut) % 16 != 0)
     return (int)cudaErrorInvalidValue;
-#define DC_SCAN(DK, DV)                                                                                                        \
-  return dc_scan<DK, DV>(qn, kn, vc, beta, g, state, state_stride, num_slots, cu_q, req_slot, o, num_entries, H, Hk, s0, ut,   \
-                         (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, items, status, stream)
-  if (dk == 128 && dv == 128) DC_SCAN(128, 128);
-  if (dk == 128 && dv == 64) DC_SCAN(128, 64);
-  if (dk == 64 && dv == 128) DC_SCAN(64, 128);
-  if (dk == 64 && dv == 64) DC_SCAN(64, 64);
+  if (per_channel && ((uintptr_t)g | (uintptr_t)pre | (uintptr_t)gam) % 16 != 0) return (int)cudaErrorInvalidValue;
+#define DC_SCAN(DK, DV)                                                                                                              \
+  if (dk == DK && dv == DV)                                                                                                          \
+  return per_channel ? dc_scan<DK, DV, true>(qn, kn, vc, beta, g, state, state_stride, num_slots, cu_q, req_slot, o, num_entries, H, \
+                                             Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, items, status, stream)      \
+                     : dc_scan<DK, DV, false>(qn, kn, vc, beta, g, state, state_stride, num_slots, cu_q, req_slot, o, num_entries, H, \
+                                              Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, items, status, stream)
+  DC_SCAN(128, 128);
+  DC_SCAN(128, 64);
+  DC_SCAN(64, 128);
+  DC_SCAN(64, 64);
 #undef DC_SCAN
   return (int)cudaErrorInvalidValue;
 }

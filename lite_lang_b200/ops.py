@@ -1476,6 +1476,14 @@ def delta_chunked_min(heads: int, dk: int, dv: int) -> float:
     return DELTA_CHUNKED_MIN * 0.482 / max(0.32 + 0.012 * states, 0.2 + 0.0235 * states)
 
 
+def delta_channels_chunked_min(heads: int, dk: int, dv: int) -> float:
+    """As above with a decay a channel, whose chunks cost a third more and whose walk takes as long: whole layers, walk / chunks, us,
+    12 heads 1 x 192 tokens 125 / 131, x 256 158 / 130; 2 x 96 120 / 129, x 128 148 / 129; 4 x 48 117 / 130, x 64 141 / 130; 28 heads
+    1 x 96 129 / 130, x 128 160 / 131; 2 x 48 129 / 129; 4 x 32 159 / 133."""
+    states = heads * dk * dv / 16384
+    return min(1.15 * delta_chunked_min(heads, dk, dv), DELTA_CHUNKED_MIN * 15.2 / (states + 1.2))
+
+
 def chunked_scan(step, tokens: int, dk: int, dv: int, least: float) -> Optional[Tuple[int, int, int]]:
     """How a step's recurrences are cut: None (all entries token by token), or (entries at the front that stay with the
     walk by tokens, entries behind them that go by chunks, an upper bound of their chunks).
@@ -1496,13 +1504,14 @@ def _cut(step, tokens: int, heads: int, dk: int, dv: int, minimum) -> Optional[T
     return chunked_scan(step, tokens, dk, dv, minimum(heads * rest, dk, dv)) if rest > 0 else None
 
 
-def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, cut) -> None:
+def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, per_channel: bool, cut) -> None:
     single, rest, items = cut
     # scratch of one allocation: states in front of the chunks, u, the terms of w and of k (six bytes a number), the scores of q and
-    # k, decays to the chunks' ends and from their starts, and of whole chunks
+    # k, decays to the chunks' ends and from their starts, and of whole chunks; with a decay a channel the second of these are in
+    # the terms of k and the third are q times them
     n, at, ptrs = items * H, 0, []
-    sizes = (n * dv * dk, n * CHUNK * dv, n * CHUNK * dk * 3 // 2, items * Hk * CHUNK * dk * 3 // 2, n * CHUNK * CHUNK, n * CHUNK,
-             n * CHUNK, n)
+    sizes = (n * dv * dk, n * CHUNK * dv, n * CHUNK * dk * 3 // 2, (n if per_channel else items * Hk) * CHUNK * dk * 3 // 2,
+             n * CHUNK * CHUNK, *((0, n * CHUNK * dk, n * dk) if per_channel else (n * CHUNK, n * CHUNK, n)))
     base = torch.empty(sum(sizes), dtype=torch.float32, device=qn.device)
     for size in sizes:
         ptrs.append(_ptr_at(base, at))
@@ -1510,7 +1519,7 @@ def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: i
     load_library("chunk_scan").call(
         "ll_chunk_delta_scan", _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(g), _ptr(state), c_long(state.stride(0)),
         c_int(state.shape[0]), _ptr_at(step.cu_q, single), _ptr_at(step.req_slot, single), _ptr(o), c_int(rest), c_int(H),
-        c_int(Hk), c_int(dk), c_int(dv), *ptrs, c_int(items), _ptr(getattr(step, "status", None)), _stream())
+        c_int(Hk), c_int(dk), c_int(dv), c_int(1 if per_channel else 0), *ptrs, c_int(items), _ptr(getattr(step, "status", None)), _stream())
 
 
 def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta: torch.Tensor, g: torch.Tensor,
@@ -1520,11 +1529,11 @@ def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta:
     _need_cuda(qn, kn, vc, beta, g, state, o)
     _need(dk <= 256, f"delta rule: key heads of {dk} channels are wider than the scan kernel takes (256)")
     entries = step.num_entries
-    if not per_channel and dv <= 128:
-        cut = _cut(step, qn.shape[0], H, dk, dv, delta_chunked_min)
+    if dv <= 128:
+        cut = _cut(step, qn.shape[0], H, dk, dv, delta_channels_chunked_min if per_channel else delta_chunked_min)
         if cut is not None and state.stride(0) % 4 == 0 and (
-                qn.data_ptr() | kn.data_ptr() | vc.data_ptr() | state.data_ptr() | o.data_ptr()) % 16 == 0:
-            _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H, Hk, dk, dv, cut)
+                qn.data_ptr() | kn.data_ptr() | vc.data_ptr() | state.data_ptr() | o.data_ptr() | (g.data_ptr() if per_channel else 0)) % 16 == 0:
+            _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H, Hk, dk, dv, per_channel, cut)
             entries = cut[0]
     if entries == 0:
         return
