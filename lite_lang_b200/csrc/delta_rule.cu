@@ -10,7 +10,7 @@
 // [(taps - 1), channels] for the last taps - 1 inputs of the convolutions (oldest first;
 // channels = q | k | v), so that a request can go on in a later step from where it stopped.
 //
-// Four kernels (a long portion's recurrence with one decay a head goes by chunks instead: delta_chunks.cu; a step of single tokens
+// Four kernels (a long portion's recurrence goes by chunks instead: delta_chunks.cu; a step of single tokens
 // takes one launch for all of them, delta_step, where its sizes allow it), all reading the step's device arrays only (so that
 // a step of single tokens can be captured and replayed):
 //   delta_prepare      per token: convolution + SiLU, unit vectors, beta, decay -> float32 buffers
