@@ -1,11 +1,10 @@
-// Paged attention in true float32 on tensor cores (head size 64 or 128, any page size and group): prompt portions and single
-// tokens.
+// Paged attention in true float32 on tensor cores (head size 64 or 128, any page size and group): prompt portions, and single tokens
+// (groups of up to 16 heads have a kernel of their own, attn_f32_few).
 //
 // The float32 path's general kernel (attention_generic.cu) gives a block a (token, kv head) pair and reads the keys once for
-// its group of heads only: 337 us for two prompts of 262 and 439 tokens with 12 heads of 128 on 2 kv heads (50 us here), and
-// 704 us for 64 single tokens at contexts of 500 to 1,000 (106 here), whose blocks walk their keys alone.  Here a CTA takes 64 rows
-// (a row = a (token, query head of the kv head's group) pair, token-major), so the keys are read once for 64 rows, and both
-// products run on mma.sync with every float32 operand as three bfloat16 terms that hold its 24 bits (mma_split.cuh):
+// its group of heads only: 337 us for two prompts of 262 and 439 tokens with 12 heads of 128 on 2 kv heads (50 us here).  Here a CTA
+// takes 64 rows (a row = a (token, query head of the kv head's group) pair, token-major), so the keys are read once for 64 rows, and
+// both products run on mma.sync with every float32 operand as three bfloat16 terms that hold its 24 bits (mma_split.cuh):
 //   S [64 x 32]  = Q K^T     a warp 16 rows, 6 products a step of 16 channels
 //   O [64 x HD] += P V       P from the accumulators' registers
 // Two groups of four warps walk the tiles of 32 keys alternately, each with its own maximum, sum and O, and meet at the end in
@@ -319,18 +318,298 @@ attn_f32_kernel(const AttnF32Params p) {
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Steps of single tokens, groups of at most 16 heads: a warp has all rows (16, those behind the group's are zeros) and tiles of 16
+// keys of its own, so that no row of the other kernel's 64 is multiplied for nothing (its four warps a tile had 16 rows each, and the
+// tensor pipe of a step of single tokens was busy with zeros).  Keys and values come by cp.async as stored, two of a warp's three
+// places on their way, and become terms in the registers of the one warp that needs them.  A cluster of CTAs takes the warps' tiles in
+// turn (tile t to warp t mod 8 C), so that few tokens fill the SMs too; the order of a row's sums depends on C, that is on how many
+// tokens decode together, within rounding.  12 heads on 2, contexts around 2,000 (heads of 128), the other kernel /
+// this one, us: 1 token 194 / 15, 16 tokens 268 / 32, 64 tokens 278 / 96.
+// ---------------------------------------------------------------------------------------------------------------
+#define AF_FEW 16
+template <int HD>
+__global__ void __launch_bounds__(AF_THREADS, 1)
+attn_f32_few_kernel(const AttnF32Params p, int ctas) {
+  constexpr int P = HD + 8, PF = HD + 8, NO = HD / 8, WARPS = AF_THREADS / 32, PLACES = 3, LOADS = AF_FEW * HD / 4 / 32;
+  constexpr int PLACE = AF_FEW * PF;                           // numbers of a place: 16 keys or values
+  extern __shared__ __align__(16) unsigned char af_smem[];
+  __shared__ float top[WARPS][AF_FEW], sum[WARPS][AF_FEW], part[2][AF_FEW];
+  __shared__ int bad[AF_FEW];
+  bf16* qs = reinterpret_cast<bf16*>(af_smem);                 // [3][16][P]
+  float* places = reinterpret_cast<float*>(qs + 3 * AF_FEW * P);
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int entry = blockIdx.x, kvh = blockIdx.y, rank = blockIdx.z;
+  const int slot = p.req_slot[entry], t = p.cu_q[entry], pos = p.ctx_len[entry], head0 = kvh * p.group;
+  float* out = p.out + (size_t)t * p.out_stride + (size_t)head0 * HD;
+  if (slot < 0) {                                              // (the cluster's CTAs have the same entry)
+    if (rank == 0)
+      for (int i = tid; i < p.group * HD; i += AF_THREADS) out[i] = 0.f;
+    return;
+  }
+  const float* qrow = p.q + (size_t)t * p.q_stride + (size_t)head0 * HD;
+  const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0, first = lo / AF_FEW, tiles = pos / AF_FEW - first + 1;
+  const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+  const int step = WARPS * ctas;
+  float* mine = places + warp * PLACES * PLACE;
+  // lane l: where the row of key l % 16 of a tile starts in the planes; -1: not seen
+  auto place = [&](int tile) -> long {
+    const int at = (first + tile) * AF_FEW + (lane & 15);
+    if (tile >= tiles || at < lo || at > pos) return -1;
+    const int lp = at / p.page_size, page = lp < p.bt_stride ? bt[lp] : -1;
+    if (page < 0 || page >= p.num_pages) {
+      set_status(p.status, LL_ERR_PAGE_RANGE);
+      return -1;
+    }
+    return (((long)page * p.nkv + kvh) * p.page_size + at % p.page_size) * HD;
+  };
+  auto ask = [&](const float* plane, long base, int where) {   // 16 rows (zeros for keys that are not seen)
+    const unsigned dst = ms_smem(mine + where * PLACE);
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) {
+      const int i = j * 32 + lane, kk = i / (HD / 4), c = (i % (HD / 4)) * 4;
+      const long at = __shfl_sync(0xffffffffu, base, kk);
+      const int bytes = at < 0 ? 0 : 16;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 4 * (kk * PF + c)), "l"(plane + (at < 0 ? 0 : at) + c), "r"(bytes)
+                   : "memory");
+    }
+  };
+  int tile = rank * WARPS + warp, asked = tile;                // the next tile to ask K of
+  long kbase = place(asked), vbase = -1;
+  int where = 0;                                               // the place that is asked for next
+  auto next_k = [&]() {
+    if (asked < tiles) ask(p.k_cache, kbase, where);
+    ms_commit();
+    vbase = kbase;
+    asked += step;
+    kbase = place(asked);
+    where = where == PLACES - 1 ? 0 : where + 1;
+  };
+  auto next_v = [&]() {
+    if (asked - step < tiles) ask(p.v_cache, vbase, where);
+    ms_commit();
+    where = where == PLACES - 1 ? 0 : where + 1;
+  };
+  next_k();
+  next_v();
+  next_k();
+  for (int i = tid; i < AF_FEW * (HD / 4); i += AF_THREADS) {
+    const int r = i / (HD / 4), c = (i % (HD / 4)) * 4;
+    const float4 v = r < p.group ? *reinterpret_cast<const float4*>(qrow + (size_t)r * HD + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    uint2 t0, t1, t2;
+    ms_split(v.x, v.y, t0.x, t1.x, t2.x);
+    ms_split(v.z, v.w, t0.y, t1.y, t2.y);
+    *reinterpret_cast<uint2*>(qs + r * P + c) = t0;
+    *reinterpret_cast<uint2*>(qs + (AF_FEW + r) * P + c) = t1;
+    *reinterpret_cast<uint2*>(qs + (2 * AF_FEW + r) * P + c) = t2;
+  }
+  if (tid < AF_FEW) bad[tid] = 0;
+  __syncthreads();
+  const int m8 = lane >> 3, r8 = lane & 7, g = lane >> 2, c = lane & 3;
+  const unsigned qs_b = ms_smem(qs) + 2 * (((m8 & 1) * 8 + r8) * P + (m8 >> 1) * 8);
+  float o[NO][4], m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+#pragma unroll
+  for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  int have = 0;                                                // the place that is read next
+  for (; tile < tiles; tile += step) {
+    ms_wait<PLACES - 1>();
+    __syncwarp();
+    const float* kf = mine + have * PLACE + g * PF + 2 * c;
+    float s[2][4] = {}, low[2][4] = {};
+#pragma unroll
+    for (int kt = 0; kt < HD / 16; ++kt) {
+      unsigned a[3][4], b[2][3][2];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) ms_ldm4(a[q], qs_b + 2 * (q * AF_FEW * P + kt * 16));
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 x = *reinterpret_cast<const float2*>(kf + nt * 8 * PF + kt * 16 + q * 8);
+          ms_split(x.x, x.y, b[nt][0][q], b[nt][1][q], b[nt][2][q]);
+        }
+      ms_terms<2, 3, 3>(s, low, a, b);
+    }
+    __syncwarp();
+    next_v();
+    have = have == PLACES - 1 ? 0 : have + 1;
+    const int k0 = (first + tile) * AF_FEW;
+    float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int at = k0 + i * 8 + 2 * c + (j & 1);
+        s[i][j] = at <= pos && at >= lo ? (s[i][j] + low[i][j]) * p.scale : -INFINITY;
+        if (j < 2) x0 = fmaxf(x0, s[i][j]);
+        else x1 = fmaxf(x1, s[i][j]);
+      }
+#pragma unroll
+    for (int w = 1; w < 4; w <<= 1) {
+      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, w));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, w));
+    }
+    const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+    const float u0 = n0 == -INFINITY ? 0.f : n0, u1 = n1 == -INFINITY ? 0.f : n1;
+    const float f0 = expf(m0 - u0), f1 = expf(m1 - u1);          // (-inf: nothing so far, 0)
+    m0 = n0;
+    m1 = n1;
+    float t0 = 0.f, t1 = 0.f;
+    unsigned a[3][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      s[i][0] = expf(s[i][0] - u0);
+      s[i][1] = expf(s[i][1] - u0);
+      s[i][2] = expf(s[i][2] - u1);
+      s[i][3] = expf(s[i][3] - u1);
+      t0 += s[i][0] + s[i][1];
+      t1 += s[i][2] + s[i][3];
+      ms_split(s[i][0], s[i][1], a[0][2 * i], a[1][2 * i], a[2][2 * i]);
+      ms_split(s[i][2], s[i][3], a[0][2 * i + 1], a[1][2 * i + 1], a[2][2 * i + 1]);
+    }
+    l0 = l0 * f0 + t0;
+    l1 = l1 * f1 + t1;
+    ms_wait<PLACES - 1>();
+    __syncwarp();
+    const float* vf = mine + have * PLACE + 2 * c * PF + g;
+#pragma unroll
+    for (int nt = 0; nt < NO; nt += 4) {
+      float d[4][4], small[4][4];
+      unsigned b[4][3][2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[i][j] = small[i][j] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float* at = vf + 8 * q * PF + (nt + i) * 8;
+          ms_split(at[0], at[PF], b[i][0][q], b[i][1][q], b[i][2][q]);
+        }
+      }
+      ms_terms<4, 3, 3>(d, small, a, b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[nt + i][j] = fmaf(o[nt + i][j], j < 2 ? f0 : f1, d[i][j] + small[i][j]);
+    }
+    __syncwarp();
+    next_k();
+    have = have == PLACES - 1 ? 0 : have + 1;
+  }
+  ms_wait<0>();
+#pragma unroll
+  for (int w = 1; w < 4; w <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, w);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+  }
+  __syncwarp();                                                // the warp's first place holds its rows from now on
+  {
+    float* d0 = mine + g * PF + 2 * c;
+#pragma unroll
+    for (int i = 0; i < NO; ++i) {
+      *reinterpret_cast<float2*>(d0 + i * 8) = make_float2(o[i][0], o[i][1]);
+      *reinterpret_cast<float2*>(d0 + 8 * PF + i * 8) = make_float2(o[i][2], o[i][3]);
+    }
+    if (c == 0) {
+      top[warp][g] = m0; sum[warp][g] = l0;
+      top[warp][g + 8] = m1; sum[warp][g + 8] = l1;
+    }
+  }
+  __syncthreads();
+  // the CTA's rows: against their largest score, not divided, in the second place of warp 0
+  float* own = places + PLACE;
+  for (int i = tid; i < p.group * HD; i += AF_THREADS) {
+    const int r = i / HD, ch = i % HD;
+    float m = -INFINITY, l = 0.f, x = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) m = fmaxf(m, top[w][r]);
+    const float u = m == -INFINITY ? 0.f : m;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float f = expf(top[w][r] - u);
+      l = fmaf(sum[w][r], f, l);
+      x = fmaf(places[w * PLACES * PLACE + r * PF + ch], f, x);
+    }
+    if (ctas > 1) {
+      own[r * PF + ch] = x;
+      if (ch == 0) {
+        part[0][r] = m;
+        part[1][r] = l;
+      }
+    } else {
+      const float y = l > 0.f ? x / l : l != l ? l : 0.f;
+      out[i] = y;
+      if (y != y) bad[r] = 1;
+    }
+  }
+  if (ctas > 1) {
+    asm volatile("barrier.cluster.arrive;" ::: "memory");
+    asm volatile("barrier.cluster.wait;" ::: "memory");
+    auto peer = [](const float* x, int z) {                    // CTA z's number of that place
+      unsigned at;
+      float v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(ms_smem(x)), "r"(z));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+      return v;
+    };
+    for (int i = tid; rank + i / HD * ctas < p.group; i += AF_THREADS) {      // every C-th row a CTA
+      const int r = rank + i / HD * ctas, ch = i % HD;
+      float mz[8], m = -INFINITY, l = 0.f, x = 0.f;
+#pragma unroll
+      for (int z = 0; z < 8; ++z) {
+        mz[z] = z < ctas ? peer(&part[0][r], z) : -INFINITY;
+        m = fmaxf(m, mz[z]);
+      }
+      const float u = m == -INFINITY ? 0.f : m;
+#pragma unroll
+      for (int z = 0; z < 8; ++z)
+        if (z < ctas) {
+          const float f = expf(mz[z] - u);
+          l = fmaf(peer(&part[1][r], z), f, l);
+          x = fmaf(peer(own + r * PF + ch, z), f, x);
+        }
+      const float y = l > 0.f ? x / l : l != l ? l : 0.f;
+      out[r * HD + ch] = y;
+      if (y != y) bad[r] = 1;
+    }
+    asm volatile("barrier.cluster.arrive;" ::: "memory");      // the rows have been read
+    asm volatile("barrier.cluster.wait;" ::: "memory");
+  }
+  __syncthreads();
+  for (int r = warp; r < p.group; r += WARPS)
+    if (bad[r]) af_plain_row<HD>(p, bt, kvh, lo, pos, qrow + (size_t)r * HD, out + (size_t)r * HD);
+}
+
 // q: float32, head h of token t at q + t * q_stride + h * hd; out float32 [tokens, nh * hd].  cu_q, ctx_len, req_slot: the
-// entries' arrays (cu_q[e] counts the step's tokens); row_blocks: sum over the entries of ceil(new tokens * group / 64).
+// entries' arrays (cu_q[e] counts the step's tokens); row_blocks: sum over the entries of ceil(new tokens * group / 64).  ctas: 0, or
+// for entries of one token each and groups of at most 16 heads 1, 2, 4 or 8 CTAs a token and kv head.
 extern "C" int ll_attn_f32(float* out, long out_stride, const float* q, long q_stride, const float* k_cache,
                            const float* v_cache, const int* block_table, int bt_stride, const int* cu_q, const int* ctx_len,
                            const int* req_slot, int n_entries, int row_blocks, int nh, int nkv, int hd, int page_size,
-                           int num_pages, int window, float scale, int* status, cudaStream_t stream) {
+                           int num_pages, int window, float scale, int ctas, int* status, cudaStream_t stream) {
   if (row_blocks <= 0 || n_entries <= 0) return 0;
   if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv != 0 || nkv > 65535 || page_size <= 0 || (q_stride % 4) != 0 ||
       (out_stride % 2) != 0 || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16) != 0 || ((uintptr_t)out % 8) != 0)
     return (int)cudaErrorInvalidValue;
   AttnF32Params p{out, out_stride, q, q_stride, k_cache, v_cache, block_table, bt_stride, cu_q, ctx_len, req_slot, n_entries,
                   nkv, nh / nkv, page_size, num_pages, window, row_blocks, scale, status};
+  if (ctas != 0) {
+    if ((ctas != 1 && ctas != 2 && ctas != 4 && ctas != 8) || p.group > AF_FEW || row_blocks != n_entries) return (int)cudaErrorInvalidValue;
+    const size_t few = 2 * (size_t)3 * AF_FEW * (hd + 8) + 4 * (size_t)(AF_THREADS / 32) * 3 * AF_FEW * (hd + 8);
+    const dim3 grid(n_entries, nkv, ctas);
+    if (hd == 128) {
+      const cudaError_t rc = cudaFuncSetAttribute(attn_f32_few_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
+      if (rc != cudaSuccess) return (int)rc;
+      ll_launch_cluster(attn_f32_few_kernel<128>, grid, dim3(AF_THREADS), few, stream, ctas, p, ctas);
+    } else {
+      const cudaError_t rc = cudaFuncSetAttribute(attn_f32_few_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
+      if (rc != cudaSuccess) return (int)rc;
+      ll_launch_cluster(attn_f32_few_kernel<64>, grid, dim3(AF_THREADS), few, stream, ctas, p, ctas);
+    }
+    return LL_LAUNCH_RESULT();
+  }
   const size_t smem = 2 * (size_t)(hd + 8) * 3 * (AF_ROWS + 4 * AF_TK) + 4 * (size_t)hd * 4 * AF_TK;
   if (hd == 128) {
     const cudaError_t rc = cudaFuncSetAttribute(attn_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -245,20 +245,34 @@ def attn_f32_supported(q: torch.Tensor, k_cache: torch.Tensor, head_dim: int, va
 
 
 def attn_f32_preferred(tokens: int, num_kv_heads: int, longest: int, sms: int) -> bool:
-    """Whether a step of single tokens is meant for ``attn_f32``: 64 rows a CTA of which a token fills its group of heads, one
-    CTA an SM.  Measured on a B200 (general kernel / here, us; heads of 128): one token 64 keys 42 / 14, 8,192 keys 3,717 /
+    """Whether a step of single tokens that ``attn_f32_ctas`` leaves is meant for ``attn_f32``'s kernel for portions: 64 rows a CTA of
+    which a token fills its group of heads, one CTA an SM.  Measured on a B200 (general kernel / here, us; heads of 128): one token 64 keys 42 / 14, 8,192 keys 3,717 /
     781; 64 tokens on 2 kv heads 64 keys 43 / 19, 8,192 keys 5,548 / 807; on 8 kv heads (four CTAs an SM in turn) 64 keys
     35 / 62, 512 keys 312 / 232, 2,048 keys 1,198 / 818.  Short contexts of many (token, kv head) pairs stay with the
     general kernel."""
     return tokens * num_kv_heads <= 2 * sms or longest > 192
 
 
+def attn_f32_ctas(tokens: int, num_heads: int, num_kv_heads: int, longest: int, sms: int) -> int:
+    """For a step of single tokens, CTAs that share the keys of a (token, kv head) pair in ``attn_f32``'s kernel for these: as many
+    as find room at once, a CTA an SM (clusters of 8 leave SMs of a GPC over).  0: the step is for the other kernels, with more than
+    16 heads a kv head, or many pairs of a few keys (64 tokens on 8 kv heads, general kernel / one CTA a pair, us: 17 keys
+    21 / 25, 64 keys 57 / 27).  Measured on a B200 (12 heads on 2, contexts around 1,000, 1 / 2 / 4 / 8 CTAs, us): 4 tokens
+    40 / 25 / 17 / 13, 8 tokens 47 / 31 / 19 / 20, 16 tokens 48 / 31 / 19 / 34, 36 tokens 49 / 32 / 46 / 60, 64 tokens 53 / 60."""
+    pairs = tokens * num_kv_heads
+    if num_heads // num_kv_heads > 16 or (pairs > 2 * sms and longest <= 32):
+        return 0
+    return 8 if pairs * 12 <= sms else 4 if pairs * 4 <= sms else 2 if pairs * 2 <= sms else 1
+
+
 def attn_f32(out: torch.Tensor, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
              cu_q: torch.Tensor, ctx_len: torch.Tensor, req_slot: torch.Tensor, q_lens, num_heads: int, num_kv_heads: int,
-             head_dim: int, page_size: int, window: Optional[int], scale: float, status: Optional[torch.Tensor]) -> None:
+             head_dim: int, page_size: int, window: Optional[int], scale: float, status: Optional[torch.Tensor],
+             ctas: int = 0) -> None:
     """Attention of entries over their requests' cached keys in true float32 on tensor cores (csrc/attention_f32.cu).
     ``cu_q``, ``ctx_len``, ``req_slot``: the arrays from the first of these entries on (``q`` and ``out`` hold all of the step's
-    tokens); ``q_lens``: new tokens of each entry (host)."""
+    tokens); ``q_lens``: new tokens of each entry (host).  ``ctas``: from ``attn_f32_ctas`` for single tokens (0: the kernel for
+    portions, whose bits do not depend on how a prompt is cut)."""
     _need_cuda(out, q, k_cache, v_cache, block_table, cu_q, ctx_len, req_slot)
     for t, nm in ((block_table, "block_table"), (cu_q, "cu_q"), (ctx_len, "ctx_len"), (req_slot, "req_slot")):
         _i32(t, nm)
@@ -272,11 +286,12 @@ def attn_f32(out: torch.Tensor, q: torch.Tensor, k_cache: torch.Tensor, v_cache:
     n, group = len(q_lens), num_heads // num_kv_heads
     _need(cu_q.numel() >= n + 1 and ctx_len.numel() >= n and req_slot.numel() >= n, "attn_f32: entry arrays too short")
     blocks = sum((int(x) * group + 63) // 64 for x in q_lens)
+    _need(ctas == 0 or (group <= 16 and all(int(x) == 1 for x in q_lens)), "attn_f32: several CTAs a pair are for single tokens")
     load_library("attn_f32").call(
         "ll_attn_f32", _ptr(out), c_long(out.stride(0)), _ptr(q), c_long(q.stride(0)), _ptr(k_cache), _ptr(v_cache),
         _ptr(block_table), c_int(block_table.stride(0)), _ptr(cu_q), _ptr(ctx_len), _ptr(req_slot), c_int(n), c_int(blocks),
         c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(page_size), c_int(k_cache.shape[0]), c_int(window or 0),
-        c_float(scale), _ptr(status), _stream())
+        c_float(scale), c_int(ctas), _ptr(status), _stream())
 
 
 def bias_rotate_store(qkv: torch.Tensor, bias: Optional[torch.Tensor], positions: Optional[torch.Tensor],

@@ -302,18 +302,20 @@ class GQAttention(Mixer):
                                      *args, step.status)
             return
         if ops.attn_f32_supported(qkv, cache.k, self.head_dim, self.vdim):
-            # true float32: 64 (token, head) rows a CTA share the keys, products of float32 terms on tensor cores
+            # true float32, products of float32 terms on tensor cores: 64 (token, head) rows a CTA share the keys, or a single
+            # token's CTAs share out its keys
             captured = getattr(step, "captured", False)
             entries = None if captured else getattr(step, "entries", None)
             lens = [1] * step.num_entries if step.num_single == step.num_entries else \
                 None if entries is None else [len(e.tokens) for e in entries]
+            single = lens is not None and len(lens) == sum(lens) == qkv.shape[0]
+            longest, sms = min(step.max_kv_len, self.window or step.max_kv_len), ops.sm_count(qkv.device)
+            ctas = ops.attn_f32_ctas(len(lens), self.num_heads, self.num_kv_heads, longest, sms) if single else 0
             if lens is not None and sum(lens) == qkv.shape[0] and (
-                    len(lens) != sum(lens) or ops.attn_f32_preferred(
-                        len(lens), self.num_kv_heads, min(step.max_kv_len, self.window or step.max_kv_len),
-                        ops.sm_count(qkv.device))):
+                    not single or ctas or ops.attn_f32_preferred(len(lens), self.num_kv_heads, longest, sms)):
                 ops.attn_f32(out, qkv, cache.k, cache.v, cache.block_table, step.cu_q, step.ctx_len, step.req_slot, lens,
                              self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size, self.window, self.scale,
-                             step.status)
+                             step.status, ctas=ctas)
                 return
         ops.paged_attention_generic(out, qkv, qkv.stride(0), cache.k, cache.v, cache.block_table, step.token_req,
                                     step.req_slot, step.positions, qkv.shape[0], self.num_heads, self.num_kv_heads,
