@@ -1159,11 +1159,15 @@ def gemm_pair_qkv_rope(q_out: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor
 ACCUMULATE_MIN_M = 129   # more tokens than any of the hand-written plain products takes: library territory
 
 
-# Rows, and multiply-adds, from which on a float32 product may go to the tensor cores (``gemm_f32``): below them its launches
-# count.  Measured on a B200 (library / here): 64 x 17,920 x 1,536 72 / 81 us, 64 x 2,048 x 1,536 31 / 39, 300 x 132 x 72
-# 11 / 24.  Above them `f32_preferred` says which is the faster.
+# Rows, and multiply-adds, from which on a float32 product may go to the tensor cores (``gemm_f32``); steps of few tokens, 2 to 64
+# rows, have a line of their own (one row is a product of a matrix and a vector, which the library reads at the memory's rate).
+# Where a line allows it `f32_preferred` says which is the faster.  (Between the two the library keeps what it had, as the tests of
+# this dispatch have it: 83 x 17,920 x 1,536 116 us, 63 here.)
 F32_MIN_M = 96
 F32_MIN_WORK = 1 << 28
+F32_FEW_M = (2, 64)
+F32_FEW_WORK = 1 << 22
+F32_FEW_N = 1024       # (64 x 256 x 2,048 20 / 23 us, 28 x 1,024 x 4,096 31 / 25)
 
 
 def f32_supported(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
@@ -1171,7 +1175,12 @@ def f32_supported(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) ->
     if x.dtype != torch.float32 or x.dim() != 2 or weight.dim() != 2:
         return False
     (m, k), n = x.shape, weight.shape[0]      # (first what most products of a decode step or a small model fail)
-    if m < F32_MIN_M or m * k * n < F32_MIN_WORK or k % 8 or n % 4 or n < 64 or not (TC_ENABLED and x.is_cuda):
+    if F32_FEW_M[0] <= m <= F32_FEW_M[1]:
+        if m * k * n < F32_FEW_WORK or n < F32_FEW_N:
+            return False
+    elif m < F32_MIN_M or m * k * n < F32_MIN_WORK:
+        return False
+    if k % 8 or n % 4 or n < 64 or not (TC_ENABLED and x.is_cuda):
         return False
     return (f32_preferred(m, n, k, sm_count(x.device), gated) and weight.dtype == torch.float32 and x.stride(1) == 1
             and weight.stride(1) == 1 and x.stride(0) % 4 == 0 and weight.stride(0) % 4 == 0
@@ -1180,19 +1189,22 @@ def f32_supported(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) ->
 
 @functools.lru_cache(maxsize=1024)
 def f32_preferred(m: int, n: int, k: int, sms: int, gated: bool = False) -> bool:
-    """Whether ``gemm_f32`` is expected to be faster than the library.  A step of 64 numbers of k takes a pair of SMs 3.1 us
-    and a tile's end 4, however many of the tile's 256 rows and columns are there, and tiles are handed out in rounds; the
-    library takes 12 us, 0.009 for a number of k and its operations at 68 TFLOP/s (measured on a B200 over 96 to 1,024 rows,
-    64 to 65,536 features and 72 to 18,944 numbers of k).  Few tiles with a gate (its k is not cut; library / here):
-    128 x 4,096 x 1,024 34 / 58 us, 1,024 x 4,096 x 1,024 173 / 63; a short k: 128 x 40,000 x 72 28 / 47, 512 x 40,000 x 72
-    90 / 75, 96 x 8,192 x 512 26 / 31, 192 x 8,192 x 512 41 / 32.  Else: 96 x 2,048 x 1,536 32 / 28, 128 x 37,888 x 3,584
-    568 / 342; 701 x 1,536 x 1,536 70 / 44, 701 x 17,920 x 1,536 684 / 224, 2,048 x 1,536 x 8,960 1,169 / 395.  (The kernel has
-    become faster since, 701 x 17,920 x 1,536 170 us; the line is where it was, on the library's side of the new one.)"""
+    """Whether ``gemm_f32`` is expected to be faster than the library.  A step of 64 numbers of k takes a pair of SMs 1.9 us (2.3
+    with 256 rows) and a tile's end 4 to 5.4, tiles are handed out in rounds, and parts of k are added up at the end.  The library
+    takes 12 us, 0.009 for a number of k and its operations at 68 TFLOP/s (over 96 to 1,024 rows, 64 to 65,536 features and 72 to
+    18,944 numbers of k); up to 64 rows at least 7 us and 0.0064 for a number of k, a little more with the rows.  Measured on a
+    B200 (library / here, us): 4 x 1,536 x 1,536 17 / 21, 33 x 1,536 x 1,536 39 / 23, 4 x 1,536 x 8,960 65 / 36, 4 x 17,920 x 1,536
+    53 / 58, 32 x 2,048 x 1,536 40 / 22, 32 x 17,920 x 1,536 54 / 58, 24 x 2,048 x 11,008 111 / 54, 64 x 3,584 x 18,944 492 / 140;
+    96 x 22,016 x 2,048 211 / 147, 128 x 37,888 x 3,584 551 / 282, 400 x 17,920 x 1,536 436 / 126; few tiles with a gate (its k is
+    not cut) 128 x 4,096 x 1,024 34 / 58, 1,024 x 4,096 x 1,024 173 / 63; a short k 128 x 40,000 x 72 28 / 47, 700 x 40,000 x 72
+    121 / 87, 100 x 8,192 x 512 25 / 27, 300 x 8,192 x 512 63 / 32."""
     tiles, boxes = ((m + 255) // 256) * ((n + 255) // 256), (k + 63) // 64
     splits = 1 if gated else _f32_parts(tiles, boxes, sms)
     rounds = -(-tiles * splits // (sms // 2))
-    here = 8 + rounds * (-(-boxes // splits) * 3.1 + 4)
-    return here < 12 + 0.009 * k + 2 * m * n * k / 68e6
+    end = 0.02 * min(m, 100)
+    here = 6 + 2.2 * end + rounds * (-(-boxes // splits) * (1.9 + 0.0017 * min(m, 256)) + 4 + 0.7 * end) + (0.25 * splits if splits > 1 else 0)
+    library = 12 + 0.009 * k + 2 * m * n * k / 68e6 if m > F32_FEW_M[1] else (7.2 + 0.0064 * k) * (1 + m / 64)
+    return here < library
 
 
 def _f32_parts(tiles: int, boxes: int, sms: int) -> int:
