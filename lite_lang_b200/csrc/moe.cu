@@ -792,3 +792,202 @@ extern "C" int ll_moe_row_gated_act(int dtype, void* out, const void* in, const 
   });
   return LL_LAUNCH_RESULT();
 }
+
+// ---------------------------------------------------------------------------------------------------------------
+// Experts of one or two tokens: only the matrices of experts that one of the tokens has chosen (and the one for every token) are
+// read.  The products over all experts' stacked matrices read every one of them: for a token of four out of sixteen experts 3.4 times
+// the bytes.  A warp makes a hidden unit (moe_few_up: a row of the first matrix, or a gate row and an up row), or a part of an output
+// (moe_few_down: a row of the second matrix at the chosen experts' columns), 16 bytes a lane and load, float32 sums.  Which experts:
+// every CTA looks through the gates.  Hidden units of experts that were not chosen are neither made nor read; those of
+// a token for an expert that only another one has chosen are zeros.  Bound by the weights and, from two
+// tokens on, by the multiply-adds on the CUDA cores.  Whole parts, all experts' products / this way, us: one token 1.5B sizes 59 / 37,
+// 3B 88 / 50, 7B 191 / 108, gated 60 / 33, 86 / 46, 196 / 95; two tokens gated 60 / 49, 86 / 63, 196 / 129, without a gate 59 / 65,
+// 89 / 81, 191 / 175, which stay with the other kernels, as do three (60 / 80).
+// ---------------------------------------------------------------------------------------------------------------
+#define MOE_FEW_THREADS 256
+#define MOE_FEW_EXPERTS 256
+struct MoeFew {
+  const float* gates;        // [M][E]
+  const float* shared_w;     // [M] or null: 1
+  int shared_ff, ff, E;
+};
+// the chosen experts in order, by all threads; behind it all of them may read `list`
+__device__ __forceinline__ int moe_few_list(const MoeFew& p, int M, unsigned char* list, int* count) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    int n = 0;
+    for (int e0 = 0; e0 < p.E; e0 += 32) {
+      bool live = false;
+      if (e0 + lane < p.E)
+        for (int t = 0; t < M; ++t) live |= p.gates[(size_t)t * p.E + e0 + lane] != 0.f;
+      const unsigned hit = __ballot_sync(0xffffffffu, live);
+      if (live) list[n + __popc(hit & ((1u << lane) - 1))] = (unsigned char)(e0 + lane);
+      n += __popc(hit);
+    }
+    if (lane == 0) *count = n;
+  }
+  __syncthreads();
+  return *count;
+}
+__device__ __forceinline__ void moe_few_eight(const uint4& v, float (&x)[8]) {
+  const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[2 * i] = __uint_as_float(w[i] << 16);
+    x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+template <int M, bool GATED>
+__global__ void __launch_bounds__(MOE_FEW_THREADS)
+moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_stride, const bf16* __restrict__ w, int K, MoeFew p, int act,
+                  float limit, float shared_limit, float alpha) {
+  constexpr int R = GATED ? 2 : 1, DEPTH = GATED ? 4 : 8;
+  extern __shared__ __align__(16) unsigned char mf_smem[];
+  uint4* xs = reinterpret_cast<uint4*>(mf_smem);                 // [M][K / 8]
+  __shared__ unsigned char list[MOE_FEW_EXPERTS];
+  __shared__ int count;
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int lane = threadIdx.x & 31, pieces = K / 8, width = p.shared_ff + p.E * p.ff;
+  for (int i = threadIdx.x; i < M * pieces; i += MOE_FEW_THREADS)
+    xs[i] = reinterpret_cast<const uint4*>(x + (size_t)(i / pieces) * x_stride)[i % pieces];
+  const int units = p.shared_ff + moe_few_list(p, M, list, &count) * p.ff;
+  for (int r = blockIdx.x * (MOE_FEW_THREADS / 32) + (threadIdx.x >> 5); r < units; r += gridDim.x * (MOE_FEW_THREADS / 32)) {
+    const bool own = r >= p.shared_ff;
+    const int slot = own ? (r - p.shared_ff) / p.ff : 0, f = own ? r - p.shared_ff - slot * p.ff : r, e = own ? list[slot] : 0;
+    const int col = own ? p.shared_ff + e * p.ff + f : f, apart = own ? p.ff : p.shared_ff;
+    const size_t first = GATED ? (own ? 2 * (size_t)p.shared_ff + (size_t)e * 2 * p.ff + f : f) : col;
+    const uint4* row = reinterpret_cast<const uint4*>(w + first * K);
+    const uint4* row2 = row + (size_t)(GATED ? apart : 0) * pieces;
+    float acc[R][M] = {};
+    for (int c0 = lane; c0 < pieces; c0 += 32 * DEPTH) {
+      uint4 v[R][DEPTH];
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        const int c = c0 + 32 * d;
+        v[0][d] = c < pieces ? __ldcs(row + c) : make_uint4(0, 0, 0, 0);
+        if (GATED) v[R - 1][d] = c < pieces ? __ldcs(row2 + c) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        const int c = min(c0 + 32 * d, pieces - 1);              // (behind the end the weights are zeros, and the token's numbers finite
+                                                                 //  or in the sum anyway)
+        float a[R][8];
+#pragma unroll
+        for (int q = 0; q < R; ++q) moe_few_eight(v[q][d], a[q]);
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+          float b[8];
+          moe_few_eight(xs[t * pieces + c], b);
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[q][t] = fmaf(a[q][i], b[i], acc[q][t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) acc[q][t] = warp_sum(acc[q][t]);
+      if (lane == t) {
+        const float weight = own ? p.gates[(size_t)t * p.E + e] : p.shared_w != nullptr ? p.shared_w[t] : 1.f;
+        const float z = to_f32<bf16>(from_f32<bf16>(acc[0][t]));
+        float y;
+        if (GATED) y = moe_gate(z, to_f32<bf16>(from_f32<bf16>(acc[R - 1][t])), own ? limit : shared_limit, alpha) * weight;
+        else y = moe_weighted_activation(z, weight, act);
+        out[(size_t)t * width + col] = from_f32<bf16>(own && weight == 0.f ? 0.f : y);
+      }
+    }
+  }
+}
+
+// out [M][N] float32; w [N][shared_ff + E ff]; a row of w by four warps
+template <int M>
+__global__ void __launch_bounds__(MOE_FEW_THREADS)
+moe_few_down_kernel(float* __restrict__ out, const bf16* __restrict__ h, const bf16* __restrict__ w, int N, MoeFew p) {
+  constexpr int PARTS = 4, DEPTH = 4, ROWS = MOE_FEW_THREADS / 32 / PARTS;
+  __shared__ unsigned char list[MOE_FEW_EXPERTS];
+  __shared__ int count;
+  __shared__ float sums[MOE_FEW_THREADS / 32][M];
+  LL_PDL_TRIGGER();
+  LL_PDL_WAIT();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % PARTS;
+  const int width = p.shared_ff + p.E * p.ff, f8 = p.ff / 8, s8 = p.shared_ff / 8;
+  const int pieces = s8 + moe_few_list(p, M, list, &count) * f8;
+  for (int n0 = blockIdx.x * ROWS; n0 < N; n0 += gridDim.x * ROWS) {
+    const int n = n0 + warp / PARTS;
+    float acc[M] = {};
+    if (n < N) {
+      const uint4* row = reinterpret_cast<const uint4*>(w + (size_t)n * width);
+      const uint4* rows = reinterpret_cast<const uint4*>(h);
+      for (int c0 = part * 32 + lane; c0 < pieces; c0 += 32 * PARTS * DEPTH) {
+        uint4 v[DEPTH], b[DEPTH][M];
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+          const int c = c0 + 32 * PARTS * d;
+          const int slot = c < s8 ? 0 : (c - s8) / f8;
+          const int at = c < s8 ? c : c < pieces ? s8 + list[slot] * f8 + (c - s8 - slot * f8) : -1;
+          v[d] = at >= 0 ? __ldcs(row + at) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int t = 0; t < M; ++t) b[d][t] = at >= 0 ? rows[(size_t)t * (width / 8) + at] : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+          float a[8];
+          moe_few_eight(v[d], a);
+#pragma unroll
+          for (int t = 0; t < M; ++t) {
+            float z[8];
+            moe_few_eight(b[d][t], z);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[t] = fmaf(a[i], z[i], acc[t]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      acc[t] = warp_sum(acc[t]);
+      if (lane == 0) sums[warp][t] = acc[t];
+    }
+    __syncthreads();
+    if (threadIdx.x < ROWS * M) {
+      const int q = threadIdx.x / M, t = threadIdx.x % M;
+      if (n0 + q < N) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < PARTS; ++i) s += sums[q * PARTS + i][t];
+        out[(size_t)t * N + n0 + q] = s;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// out float32 [M][N] = the experts' outputs for one row of x, or two with gated experts, bfloat16; hidden: bfloat16 [M][shared_ff + E ff], scratch.
+// gated: limits and alpha as in ll_moe_gated_act, else act as in ll_gemm_stream_experts.  K, ff, shared_ff: multiples of 8; rows of x
+// and matrices at multiples of 16 bytes; E at most 256.
+extern "C" int ll_moe_few(float* out, void* hidden, const void* x, long x_stride, const void* w_up, const void* w_down, int M, int K, int N,
+                          const float* gates, const float* shared_w, int shared_ff, int ff, int E, int gated, int act, float limit,
+                          float shared_limit, float alpha, int sms, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > (gated ? 2 : 1) || K <= 0 || K % 8 || ff <= 0 || ff % 8 || shared_ff < 0 || shared_ff % 8 || E <= 0 || E > MOE_FEW_EXPERTS || x_stride % 8 ||
+      (long)M * K * 2 > 49152 || ((uintptr_t)x | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)hidden) % 16)
+    return (int)cudaErrorInvalidValue;
+  const MoeFew p{gates, shared_w, shared_ff, ff, E};
+  const size_t smem = (size_t)M * K * 2;
+  const dim3 grid(4 * sms);
+#define MOE_FEW(MM, GATED)                                                                                                         \
+  if (M == MM && (gated != 0) == GATED) {                                                                                          \
+    ll_launch(moe_few_up_kernel<MM, GATED>, grid, dim3(MOE_FEW_THREADS), smem, stream, (bf16*)hidden, (const bf16*)x, x_stride,      \
+              (const bf16*)w_up, K, p, act, limit, shared_limit, alpha);                                                            \
+    ll_launch(moe_few_down_kernel<MM>, grid, dim3(MOE_FEW_THREADS), 0, stream, out, (const bf16*)hidden, (const bf16*)w_down, N, p); \
+  }
+  MOE_FEW(1, false)
+  MOE_FEW(1, true)
+  MOE_FEW(2, true)
+#undef MOE_FEW
+  return LL_LAUNCH_RESULT();
+}

@@ -2386,6 +2386,42 @@ def expert_hidden(x: torch.Tensor, weight: torch.Tensor, gates: torch.Tensor, sh
     return out
 
 
+def experts_few_preferred(tokens: int, top: int, E: int, gated: bool) -> bool:
+    """Whether few enough of the experts are expected to be chosen by a step's tokens for ``experts_few``: one token, or two with
+    gated experts (see csrc/moe.cu for both sides), and at most half of the experts."""
+    return tokens <= (2 if gated else 1) and 1.0 - (1.0 - top / E) ** tokens <= 0.5
+
+
+def experts_few_supported(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, shared_ff: int, ff: int, E: int) -> bool:
+    return (x.dtype == w_up.dtype == w_down.dtype == torch.bfloat16 and x.is_cuda and 0 < x.shape[0] <= 2 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.shape[1] % 8 == 0 and x.shape[0] * x.shape[1] <= 24576 and ff % 8 == 0 and shared_ff % 8 == 0
+            and E <= 256 and w_up.is_contiguous() and w_down.is_contiguous()
+            and (x.data_ptr() | w_up.data_ptr() | w_down.data_ptr()) % 16 == 0)
+
+
+def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, gates: torch.Tensor, shared_w: Optional[torch.Tensor],
+                shared_ff: int, ff: int, E: int, act: Optional[str], weight_in: bool = False, limit: float = 0.0,
+                shared_limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+    """The experts' outputs for one token, or two with gated experts, float32 [1, tokens, out] (one part of a sum), from the matrices of the chosen
+    experts only.  ``act`` None: experts with a gate, as ``moe_gated_act``; else as ``expert_hidden``."""
+    _need_cuda(x, w_up, w_down, gates, shared_w)
+    _f32(gates, "gates")
+    _f32(shared_w, "shared_w")
+    m, width = x.shape[0], shared_ff + E * ff
+    _need(experts_few_supported(x, w_up, w_down, shared_ff, ff, E) and (m == 1 or act is None) and tuple(gates.shape) == (m, E) and gates.is_contiguous()
+          and tuple(w_up.shape) == ((2 if act is None else 1) * width, x.shape[1]) and w_down.shape[1] == width
+          and (shared_w is None or (act is None and shared_w.numel() == m)), "experts_few: shapes")
+    n = w_down.shape[0]
+    hidden = torch.empty((m, width), dtype=x.dtype, device=x.device)
+    out = torch.empty((1, m, n), dtype=torch.float32, device=x.device)
+    code = 0 if act is None else MOE_ACT[act] + (MOE_ACT_WEIGHT_IN if weight_in else 0)
+    load_library("moe").call(
+        "ll_moe_few", _ptr(out), _ptr(hidden), _ptr(x), c_long(x.stride(0)), _ptr(w_up), _ptr(w_down), c_int(m), c_int(x.shape[1]),
+        c_int(n), _ptr(gates), _ptr(shared_w), c_int(shared_ff), c_int(ff), c_int(E), c_int(1 if act is None else 0), c_int(code),
+        c_float(limit), c_float(shared_limit), c_float(alpha), c_int(sm_count(x.device)), _stream())
+    return out
+
+
 def act_rows(x: torch.Tensor, act: str) -> None:
     """x <- act(x) in place (float32 arithmetic, one rounding): the activation of a feed-forward without a gate."""
     _need_cuda(x)

@@ -184,6 +184,11 @@ class RoutedExperts(FeedForward):
                 return self._forward_grouped(x, idx, wts, getattr(step, "status", None))
             if ops.grouped_product_available():
                 return self._forward_library(x, idx, wts)
+        if ops.experts_few_preferred(x.shape[0], self.top, self.E + self.identity, self.gated) and ops.experts_few_supported(
+                x, self.w_up, self.w_down, self.shared_ff, self.ff, self.E):
+            return ops.experts_few(x, self.w_up, self.w_down, gates, self._shared_w if self.gated else None, self.shared_ff, self.ff, self.E,
+                                   None if self.gated else self.activation, self.weight_in, self.limit, self.shared_limit,
+                                   self.swish_alpha)
         if self.gated:
             hidden = ops.linear(x, self.w_up)
             hidden = ops.moe_gated_act(hidden, gates, self._shared_w, self.shared_ff, self.ff, self.E, self.limit,
