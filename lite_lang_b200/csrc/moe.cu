@@ -800,9 +800,10 @@ extern "C" int ll_moe_row_gated_act(int dtype, void* out, const void* in, const 
 // (moe_few_down: a row of the second matrix at the chosen experts' columns), 16 bytes a lane and load, float32 sums.  Which experts:
 // every CTA looks through the gates.  Hidden units of experts that were not chosen are neither made nor read; those of
 // a token for an expert that only another one has chosen are zeros.  Bound by the weights and, from two
-// tokens on, by the multiply-adds on the CUDA cores.  Whole parts, all experts' products / this way, us: one token 1.5B sizes 59 / 37,
-// 3B 88 / 50, 7B 191 / 108, gated 60 / 33, 86 / 46, 196 / 95; two tokens gated 60 / 49, 86 / 63, 196 / 129, without a gate 59 / 65,
-// 89 / 81, 191 / 175, which stay with the other kernels, as do three (60 / 80).
+// tokens on, by the multiply-adds on the CUDA cores.  Whole parts, all experts' products / this way, us: one token 1.5B sizes 59 / 35,
+// 3B 88 / 41, 7B 191 / 88, gated 60 / 32, 86 / 39, 196 / 84; two tokens gated 60 / 51, 87 / 65, 196 / 134, without a gate 59 / 65,
+// 89 / 81, 191 / 175, which stay with the other kernels, as do three (60 / 80).  (Loads eight deep, or without the branch behind the
+// end: 37 to 39, 50, 108 and 33, 46, 95.)
 // ---------------------------------------------------------------------------------------------------------------
 #define MOE_FEW_THREADS 256
 #define MOE_FEW_EXPERTS 256
@@ -842,7 +843,7 @@ template <int M, bool GATED>
 __global__ void __launch_bounds__(MOE_FEW_THREADS)
 moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_stride, const bf16* __restrict__ w, int K, MoeFew p, int act,
                   float limit, float shared_limit, float alpha) {
-  constexpr int R = GATED ? 2 : 1, DEPTH = GATED ? 4 : 8;
+  constexpr int R = GATED ? 2 : 1, DEPTH = 4;
   extern __shared__ __align__(16) unsigned char mf_smem[];
   uint4* xs = reinterpret_cast<uint4*>(mf_smem);                 // [M][K / 8]
   __shared__ unsigned char list[MOE_FEW_EXPERTS];
@@ -871,8 +872,7 @@ moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_str
       }
 #pragma unroll
       for (int d = 0; d < DEPTH; ++d) {
-        const int c = min(c0 + 32 * d, pieces - 1);              // (behind the end the weights are zeros, and the token's numbers finite
-                                                                 //  or in the sum anyway)
+        const int c = min(c0 + 32 * d, pieces - 1);
         float a[R][8];
 #pragma unroll
         for (int q = 0; q < R; ++q) moe_few_eight(v[q][d], a[q]);
@@ -880,6 +880,7 @@ moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_str
         for (int t = 0; t < M; ++t) {
           float b[8];
           moe_few_eight(xs[t * pieces + c], b);
+          if (c0 + 32 * d >= pieces) continue;
 #pragma unroll
           for (int q = 0; q < R; ++q)
 #pragma unroll
