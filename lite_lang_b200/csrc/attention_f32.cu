@@ -328,6 +328,18 @@ attn_f32_kernel(const AttnF32Params p) {
 // this one, us: 1 token 194 / 15, 16 tokens 268 / 32, 64 tokens 278 / 96.
 // ---------------------------------------------------------------------------------------------------------------
 #define AF_FEW 16
+__device__ __forceinline__ void af_cluster_sync() {
+  asm volatile("barrier.cluster.arrive;" ::: "memory");
+  asm volatile("barrier.cluster.wait;" ::: "memory");
+}
+__device__ __forceinline__ float af_peer(const float* x, int z) {      // CTA z's number of that place
+  unsigned at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(ms_smem(x)), "r"(z));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
 template <int HD>
 __global__ void __launch_bounds__(AF_THREADS, 1)
 attn_f32_few_kernel(const AttnF32Params p, int ctas) {
@@ -545,21 +557,13 @@ attn_f32_few_kernel(const AttnF32Params p, int ctas) {
     }
   }
   if (ctas > 1) {
-    asm volatile("barrier.cluster.arrive;" ::: "memory");
-    asm volatile("barrier.cluster.wait;" ::: "memory");
-    auto peer = [](const float* x, int z) {                    // CTA z's number of that place
-      unsigned at;
-      float v;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(ms_smem(x)), "r"(z));
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-      return v;
-    };
+    af_cluster_sync();
     for (int i = tid; rank + i / HD * ctas < p.group; i += AF_THREADS) {      // every C-th row a CTA
       const int r = rank + i / HD * ctas, ch = i % HD;
       float mz[8], m = -INFINITY, l = 0.f, x = 0.f;
 #pragma unroll
       for (int z = 0; z < 8; ++z) {
-        mz[z] = z < ctas ? peer(&part[0][r], z) : -INFINITY;
+        mz[z] = z < ctas ? af_peer(&part[0][r], z) : -INFINITY;
         m = fmaxf(m, mz[z]);
       }
       const float u = m == -INFINITY ? 0.f : m;
@@ -567,15 +571,14 @@ attn_f32_few_kernel(const AttnF32Params p, int ctas) {
       for (int z = 0; z < 8; ++z)
         if (z < ctas) {
           const float f = expf(mz[z] - u);
-          l = fmaf(peer(&part[1][r], z), f, l);
-          x = fmaf(peer(own + r * PF + ch, z), f, x);
+          l = fmaf(af_peer(&part[1][r], z), f, l);
+          x = fmaf(af_peer(own + r * PF + ch, z), f, x);
         }
       const float y = l > 0.f ? x / l : l != l ? l : 0.f;
       out[r * HD + ch] = y;
       if (y != y) bad[r] = 1;
     }
-    asm volatile("barrier.cluster.arrive;" ::: "memory");      // the rows have been read
-    asm volatile("barrier.cluster.wait;" ::: "memory");
+    af_cluster_sync();                                         // the rows have been read
   }
   __syncthreads();
   for (int r = warp; r < p.group; r += WARPS)
