@@ -239,11 +239,14 @@ def _by_ctypes(f, args) -> int:
 
 
 def _launch_path() -> Optional[str]:
-    """Where the native call (launch.c) is built, or None where it is not: another machine than x86-64 Linux, no Python headers."""
-    include = sysconfig.get_paths()["include"]
-    if platform.machine() != "x86_64" or sys.platform != "linux" or not os.path.isfile(os.path.join(include, "Python.h")):
+    """Where the native call (launch.c) is built, or None where it is not: another machine than x86-64 Linux, no Python headers, no
+    launch.c."""
+    include, source = sysconfig.get_paths()["include"], _src_path("launch.c")
+    if (platform.machine() != "x86_64" or sys.platform != "linux" or not os.path.isfile(os.path.join(include, "Python.h"))
+            or not os.path.isfile(source)):
         return None
-    h = hashlib.sha256(open(_src_path("launch.c"), "rb").read() + sys.version.encode()).hexdigest()[:16]
+    with open(source, "rb") as fh:
+        h = hashlib.sha256(fh.read() + sys.version.encode()).hexdigest()[:16]
     return os.path.join(_build_dir(), f"ll_launch_{h}.so")
 
 
