@@ -160,7 +160,7 @@ def _run(cmd: List[str], what: str) -> None:
                 _say(f"... still compiling {what} ({time.time() - t0:.0f} s)")
                 last = time.time()
     if proc.returncode != 0:
-        raise BuildError(f"nvcc failed on {what}:\n{' '.join(cmd)}\n{out}")
+        raise BuildError(f"{os.path.basename(cmd[0])} failed on {what}:\n{' '.join(cmd)}\n{out}")
     if os.environ.get("LITE_LANG_B200_VERBOSE_BUILD") and out.strip():
         _say(out)
 
@@ -240,14 +240,14 @@ def _by_ctypes(f, args) -> int:
 
 def _launch_path() -> Optional[str]:
     """Where the native call (launch.c) is built, or None where it is not: another machine than x86-64 Linux, no Python headers, no
-    launch.c."""
+    launch.c.  Named by the interpreter and by the source, so that several interpreters on one tree have one each."""
     include, source = sysconfig.get_paths()["include"], _src_path("launch.c")
     if (platform.machine() != "x86_64" or sys.platform != "linux" or not os.path.isfile(os.path.join(include, "Python.h"))
             or not os.path.isfile(source)):
         return None
     with open(source, "rb") as fh:
-        h = hashlib.sha256(fh.read() + sys.version.encode()).hexdigest()[:16]
-    return os.path.join(_build_dir(), f"ll_launch_{h}.so")
+        digest = hashlib.sha256(fh.read()).hexdigest()[:16]
+    return os.path.join(_build_dir(), f"ll_launch_{hashlib.sha256(sys.version.encode()).hexdigest()[:8]}_{digest}.so")
 
 
 def build_launch() -> Optional[str]:
@@ -261,13 +261,14 @@ def build_launch() -> Optional[str]:
     tmp = f"{target}.{os.getpid()}.tmp"
     try:
         _run([cc, "-x", "c", "-O2", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], _src_path("launch.c"), "-o", tmp], "launch.c")
-    except BuildError as exc:
+        os.replace(tmp, target)
+    except (BuildError, OSError) as exc:
         _say(f"{exc}; launchers are called by ctypes")
         return None
-    os.replace(tmp, target)
-    for old in os.listdir(_build_dir()):
+    prefix = os.path.basename(target)[:-len("0123456789abcdef.so")]
+    for old in os.listdir(_build_dir()):      # this interpreter's, built from older sources
         path = os.path.join(_build_dir(), old)
-        if re.fullmatch(r"ll_launch_[0-9a-f]{16}\.so", old) and path != target:
+        if re.fullmatch(re.escape(prefix) + r"[0-9a-f]{16}\.so", old) and path != target:
             try:
                 os.remove(path)
             except OSError:
@@ -280,9 +281,13 @@ def _native_call():
     path = build_launch()
     if path is None:
         return None
-    spec = importlib.util.spec_from_file_location("_ll_launch", path)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
+    try:
+        spec = importlib.util.spec_from_file_location("_ll_launch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except (ImportError, OSError) as exc:      # (removed since, or made for another interpreter or machine)
+        _say(f"{exc}; launchers are called by ctypes")
+        return None
     return module.call
 
 

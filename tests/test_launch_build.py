@@ -5,6 +5,7 @@ import glob
 import os
 import shutil
 import subprocess
+import sys
 
 import pytest
 
@@ -61,3 +62,42 @@ def test_libraries_load_without_the_source(library, folder, monkeypatch):
     real = build._src_path
     monkeypatch.setattr(build, "_src_path", lambda s: str(folder / "none.c") if s == "launch.c" else real(s))
     assert build.build_launch() is None and _answers(library)._native is None
+
+
+def test_libraries_load_where_the_module_does_not(library, folder):
+    path = build._launch_path()
+    if path is None:
+        pytest.skip("launchers are called by ctypes here")
+    with open(path, "w") as fh:
+        fh.write("not a shared object")
+    assert _answers(library)._native is None
+
+
+def test_libraries_load_where_the_compiler_fails(library, folder, monkeypatch, capfd):
+    if build._launch_path() is None:
+        pytest.skip("launchers are called by ctypes here")
+    (folder / "bad.c").write_text("#error no\n")
+    real = build._src_path
+    monkeypatch.setattr(build, "_src_path", lambda s: str(folder / "bad.c") if s == "launch.c" else real(s))
+    assert _answers(library)._native is None
+    said = capfd.readouterr().err
+    assert "failed on launch.c" in said and "nvcc" not in said
+
+
+def test_interpreters_keep_their_modules(folder, monkeypatch):
+    """Two interpreters on one tree build one each, and neither removes the other's; an older source's goes."""
+    if build._launch_path() is None:
+        pytest.skip("launchers are called by ctypes here")
+    mine = build.build_launch()
+    older = mine[:-len("0123456789abcdef.so")] + "0123456789abcdef.so"
+    open(older, "w").close()
+    monkeypatch.setattr(sys, "version", "another interpreter")
+    theirs = build.build_launch()
+    assert theirs != mine and os.path.isfile(mine) and os.path.isfile(theirs) and os.path.isfile(older)
+    monkeypatch.undo()
+    os.environ["LITE_LANG_B200_BUILD_DIR"] = str(folder)
+    try:
+        os.remove(mine)
+        assert build.build_launch() == mine and not os.path.isfile(older) and os.path.isfile(theirs)
+    finally:
+        del os.environ["LITE_LANG_B200_BUILD_DIR"]
