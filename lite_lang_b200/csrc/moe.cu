@@ -980,8 +980,12 @@ extern "C" int ll_moe_few(float* out, void* hidden, const void* x, long x_stride
   const MoeFew p{gates, shared_w, shared_ff, ff, E};
   const size_t smem = (size_t)M * K * 2;
   const dim3 grid(4 * sms);
+  const size_t own = 48 * 1024 - 512;      // (the kernel has 272 bytes beside the rows: more than 48 KB together has to be asked for)
 #define MOE_FEW(MM, GATED)                                                                                                         \
   if (M == MM && (gated != 0) == GATED) {                                                                                          \
+    const cudaError_t rc = smem <= own ? cudaSuccess : cudaFuncSetAttribute(moe_few_up_kernel<MM, GATED>,                          \
+                                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (rc != cudaSuccess) return (int)rc;                                                                                         \
     ll_launch(moe_few_up_kernel<MM, GATED>, grid, dim3(MOE_FEW_THREADS), smem, stream, (bf16*)hidden, (const bf16*)x, x_stride,      \
               (const bf16*)w_up, K, p, act, limit, shared_limit, alpha);                                                            \
     ll_launch(moe_few_down_kernel<MM>, grid, dim3(MOE_FEW_THREADS), 0, stream, out, (const bf16*)hidden, (const bf16*)w_down, N, p); \

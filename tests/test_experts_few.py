@@ -55,3 +55,28 @@ def test_experts_of_few_tokens(M, K, N, shared, ff, E, top, gated):
     # roundings of products and hidden units to bfloat16 on both sides, which may differ by one of 2^-8 where a float32 sum lies near
     # the middle: a small share of them
     assert float((out[0].double() - want).norm()) <= 2.0 ** -9 * float(want.norm())
+
+
+@gpu
+@pytest.mark.parametrize("M,K,gated", [(1, 24576, False), (1, 24440, True), (2, 12288, True), (2, 12208, True)])
+def test_the_widest_rows(M, K, gated):
+    """Rows that fill the shared memory of a block: the sizes that `experts_few_supported` ends at."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(K)
+    E, ff, N = 8, 16, 24
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w_up = (torch.randn((2 if gated else 1) * E * ff, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    w_down = torch.randn(N, E * ff, generator=g, device="cuda").bfloat16()
+    gates = torch.zeros(M, E, device="cuda")
+    gates[:, 2], gates[:, 5] = 0.75, 0.5
+    assert ops.experts_few_supported(x, w_up, w_down, 0, ff, E)
+    kind = dict(act=None, limit=7.0, alpha=1.702) if gated else dict(act="silu")
+    out = ops.experts_few(x, w_up, w_down, gates, None, 0, ff, E, **kind)
+    y = (x.double() @ w_up.double().t()).bfloat16().double().view(M, E, -1)
+    if gated:
+        left, right = y[..., :ff].clamp(max=7.0), y[..., ff:].clamp(-7.0, 7.0)
+        h = left * torch.sigmoid(1.702 * left) * (right + 1)
+    else:
+        h = torch.nn.functional.silu(y)
+    want = (h * gates.double()[..., None]).bfloat16().double().view(M, -1) @ w_down.double().t()
+    assert float((out[0].double() - want).norm()) <= 2.0 ** -9 * float(want.norm())      # (as above)
