@@ -799,11 +799,12 @@ extern "C" int ll_moe_row_gated_act(int dtype, void* out, const void* in, const 
 // the bytes.  A warp makes a hidden unit (moe_few_up: a row of the first matrix, or a gate row and an up row), or a part of an output
 // (moe_few_down: a row of the second matrix at the chosen experts' columns), 16 bytes a lane and load, float32 sums.  Which experts:
 // every CTA looks through the gates.  Hidden units of experts that were not chosen are neither made nor read; those of
-// a token for an expert that only another one has chosen are zeros.  Bound by the weights and, from two
-// tokens on, by the multiply-adds on the CUDA cores.  Whole parts, all experts' products / this way, us: one token 1.5B sizes 59 / 35,
-// 3B 88 / 41, 7B 191 / 88, gated 60 / 32, 86 / 39, 196 / 84; two tokens gated 60 / 51, 87 / 65, 196 / 134, without a gate 59 / 65,
-// 89 / 81, 191 / 175, which stay with the other kernels, as do three (60 / 80).  (Loads eight deep, or without the branch behind the
-// end: 37 to 39, 50, 108 and 33, 46, 95.)
+// a token for an expert that only another one has chosen are zeros, and the second product leaves them out.  Bound by the weights and,
+// from two tokens on, by the multiply-adds on the CUDA cores.  Whole parts, all experts' products / this way, us: one token 1.5B sizes
+// 59 / 32, 3B 88 / 40, 7B 191 / 85, gated 60 / 31, 86 / 38, 196 / 82; two tokens gated 60 / 50, 87 / 63, 196 / 132.  (With the pieces of
+// all chosen experts in one row, shared out by their place in it: 34, 41, 88, 32, 39, 85; 54, 67, 142; a token's order of sums then
+// depended on the other one's experts.)  That way two tokens without a gate took 59 / 65, 89 / 81, 191 / 175, which stay with the
+// other kernels, as do three (60 / 80).  Loads for the second product that are asked for on a condition, one after the other: 38, 48, 113.
 // ---------------------------------------------------------------------------------------------------------------
 #define MOE_FEW_THREADS 256
 #define MOE_FEW_EXPERTS 256
@@ -812,17 +813,25 @@ struct MoeFew {
   const float* shared_w;     // [M] or null: 1
   int shared_ff, ff, E;
 };
-// the chosen experts in order, by all threads; behind it all of them may read `list`
-__device__ __forceinline__ int moe_few_list(const MoeFew& p, int M, unsigned char* list, int* count) {
+// the chosen experts in order, by all threads; behind it all of them may read `list`, and (several tokens) `takers`: who chose it, a bit
+// a token
+template <int M>
+__device__ __forceinline__ int moe_few_list(const MoeFew& p, unsigned char* list, unsigned char* takers, int* count) {
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) {
     int n = 0;
     for (int e0 = 0; e0 < p.E; e0 += 32) {
-      bool live = false;
-      if (e0 + lane < p.E)
-        for (int t = 0; t < M; ++t) live |= p.gates[(size_t)t * p.E + e0 + lane] != 0.f;
-      const unsigned hit = __ballot_sync(0xffffffffu, live);
-      if (live) list[n + __popc(hit & ((1u << lane) - 1))] = (unsigned char)(e0 + lane);
+      unsigned who = 0;
+      if (e0 + lane < p.E) {
+#pragma unroll
+        for (int t = 0; t < M; ++t) who |= (p.gates[(size_t)t * p.E + e0 + lane] != 0.f ? 1u : 0u) << t;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, who != 0);
+      if (who != 0) {
+        const int at = n + __popc(hit & ((1u << lane) - 1));
+        list[at] = (unsigned char)(e0 + lane);
+        if (M > 1) takers[at] = (unsigned char)who;
+      }
       n += __popc(hit);
     }
     if (lane == 0) *count = n;
@@ -846,14 +855,14 @@ moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_str
   constexpr int R = GATED ? 2 : 1, DEPTH = 4;
   extern __shared__ __align__(16) unsigned char mf_smem[];
   uint4* xs = reinterpret_cast<uint4*>(mf_smem);                 // [M][K / 8]
-  __shared__ unsigned char list[MOE_FEW_EXPERTS];
+  __shared__ unsigned char list[MOE_FEW_EXPERTS], takers[M > 1 ? MOE_FEW_EXPERTS : 1];
   __shared__ int count;
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int lane = threadIdx.x & 31, pieces = K / 8, width = p.shared_ff + p.E * p.ff;
   for (int i = threadIdx.x; i < M * pieces; i += MOE_FEW_THREADS)
     xs[i] = reinterpret_cast<const uint4*>(x + (size_t)(i / pieces) * x_stride)[i % pieces];
-  const int units = p.shared_ff + moe_few_list(p, M, list, &count) * p.ff;
+  const int units = p.shared_ff + moe_few_list<M>(p, list, takers, &count) * p.ff;
   for (int r = blockIdx.x * (MOE_FEW_THREADS / 32) + (threadIdx.x >> 5); r < units; r += gridDim.x * (MOE_FEW_THREADS / 32)) {
     const bool own = r >= p.shared_ff;
     const int slot = own ? (r - p.shared_ff) / p.ff : 0, f = own ? r - p.shared_ff - slot * p.ff : r, e = own ? list[slot] : 0;
@@ -904,35 +913,50 @@ moe_few_up_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long x_str
   }
 }
 
-// out [M][N] float32; w [N][shared_ff + E ff]; a row of w by four warps
+// out [M][N] float32; w [N][shared_ff + E ff]; a row of w by four warps: block b of 32 pieces of expert e's columns goes to warp
+// (b + e + 1) mod 4 (the columns for every token: b mod 4), whose lanes add up in the order of the experts.  So the order of a token's sum
+// depends on its own experts alone, not on what the other token has chosen.
 template <int M>
 __global__ void __launch_bounds__(MOE_FEW_THREADS)
 moe_few_down_kernel(float* __restrict__ out, const bf16* __restrict__ h, const bf16* __restrict__ w, int N, MoeFew p) {
-  constexpr int PARTS = 4, DEPTH = 4, ROWS = MOE_FEW_THREADS / 32 / PARTS;
-  __shared__ unsigned char list[MOE_FEW_EXPERTS];
+  constexpr int PARTS = 4, DEPTH = M == 1 ? 4 : 3, ROWS = MOE_FEW_THREADS / 32 / PARTS;
+  __shared__ unsigned char list[MOE_FEW_EXPERTS], takers[M > 1 ? MOE_FEW_EXPERTS : 1];
   __shared__ int count;
   __shared__ float sums[MOE_FEW_THREADS / 32][M];
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % PARTS;
   const int width = p.shared_ff + p.E * p.ff, f8 = p.ff / 8, s8 = p.shared_ff / 8;
-  const int pieces = s8 + moe_few_list(p, M, list, &count) * f8;
+  const int live = moe_few_list<M>(p, list, takers, &count);
   for (int n0 = blockIdx.x * ROWS; n0 < N; n0 += gridDim.x * ROWS) {
     const int n = n0 + warp / PARTS;
     float acc[M] = {};
     if (n < N) {
       const uint4* row = reinterpret_cast<const uint4*>(w + (size_t)n * width);
       const uint4* rows = reinterpret_cast<const uint4*>(h);
-      for (int c0 = part * 32 + lane; c0 < pieces; c0 += 32 * PARTS * DEPTH) {
+      int run = -1, c = 32 * part + lane, len = s8, first = 0;      // the columns for every token, then the chosen experts'
+      int next = list[0];
+      unsigned who = (1u << M) - 1;
+      while (run < live) {
         uint4 v[DEPTH], b[DEPTH][M];
+        unsigned take[DEPTH];
 #pragma unroll
         for (int d = 0; d < DEPTH; ++d) {
-          const int c = c0 + 32 * PARTS * d;
-          const int slot = c < s8 ? 0 : (c - s8) / f8;
-          const int at = c < s8 ? c : c < pieces ? s8 + list[slot] * f8 + (c - s8 - slot * f8) : -1;
-          v[d] = at >= 0 ? __ldcs(row + at) : make_uint4(0, 0, 0, 0);
+          if (c - lane >= len) {                                    // (the same for all lanes; an expert may have no block for the warp)
+            ++run;
+            c = 32 * ((part - next - 1) & (PARTS - 1)) + lane;
+            len = f8;
+            first = s8 + next * f8;
+            if (M > 1) who = takers[run & (MOE_FEW_EXPERTS - 1)];
+            next = list[(run + 1) & (MOE_FEW_EXPERTS - 1)];
+          }
+          const bool there = run < live && c < len;
+          const int at = there ? first + c : 0;                     // (behind the end: some piece that is not used)
+          take[d] = there ? who : 0;
+          v[d] = __ldcs(row + at);
 #pragma unroll
-          for (int t = 0; t < M; ++t) b[d][t] = at >= 0 ? rows[(size_t)t * (width / 8) + at] : make_uint4(0, 0, 0, 0);
+          for (int t = 0; t < M; ++t) b[d][t] = rows[(size_t)t * (width / 8) + at];
+          c += 32 * PARTS;
         }
 #pragma unroll
         for (int d = 0; d < DEPTH; ++d) {
@@ -940,6 +964,7 @@ moe_few_down_kernel(float* __restrict__ out, const bf16* __restrict__ h, const b
           moe_few_eight(v[d], a);
 #pragma unroll
           for (int t = 0; t < M; ++t) {
+            if (((take[d] >> t) & 1) == 0) continue;
             float z[8];
             moe_few_eight(b[d][t], z);
 #pragma unroll
@@ -980,7 +1005,7 @@ extern "C" int ll_moe_few(float* out, void* hidden, const void* x, long x_stride
   const MoeFew p{gates, shared_w, shared_ff, ff, E};
   const size_t smem = (size_t)M * K * 2;
   const dim3 grid(4 * sms);
-  const size_t own = 48 * 1024 - 512;      // (the kernel has 272 bytes beside the rows: more than 48 KB together has to be asked for)
+  const size_t own = 48 * 1024 - 1024;      // (the kernel has up to 528 bytes beside the rows: more than 48 KB together has to be asked for)
 #define MOE_FEW(MM, GATED)                                                                                                         \
   if (M == MM && (gated != 0) == GATED) {                                                                                          \
     const cudaError_t rc = smem <= own ? cudaSuccess : cudaFuncSetAttribute(moe_few_up_kernel<MM, GATED>,                          \

@@ -80,3 +80,30 @@ def test_the_widest_rows(M, K, gated):
         h = torch.nn.functional.silu(y)
     want = (h * gates.double()[..., None]).bfloat16().double().view(M, -1) @ w_down.double().t()
     assert float((out[0].double() - want).norm()) <= 2.0 ** -9 * float(want.norm())      # (as above)
+
+
+@gpu
+@pytest.mark.parametrize("K,N,shared,ff,E,top", [(1536, 1536, 1792, 1792, 16, 4), (512, 40, 0, 264, 16, 2), (256, 33, 40, 24, 64, 8)])
+def test_a_token_beside_others(K, N, shared, ff, E, top):
+    """One token's numbers are the same, whatever the other token of the step has chosen, and alone."""
+    from lite_lang_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(K + E)
+    width = shared + E * ff
+    x = torch.randn(2, K, generator=g, device="cuda").bfloat16()
+    w_up = (torch.randn(2 * width, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    w_down = (torch.randn(N, width, generator=g, device="cuda") * 0.1).bfloat16()
+    weights = torch.rand(E, generator=g, device="cuda") + 0.1
+    kind = dict(act=None, limit=7.0, shared_limit=7.0, alpha=1.702)
+
+    def run(rows, chosen):
+        gates = torch.stack([weights * torch.tensor([float(e in c) for e in range(E)], device="cuda") for c in chosen])
+        return ops.experts_few(rows, w_up, w_down, gates, None, shared, ff, E, **kind)[0]
+
+    own = set(range(E // 3, E // 3 + top))
+    alone = run(x[:1], [own])
+    low, high, some = set(range(top)), set(range(E - top, E)), set(range(0, E, E // top))
+    for other in (low, high, some, own, set()):
+        assert torch.equal(run(x, [own, other])[:1], alone)
+        assert torch.equal(run(x.flip(0), [other, own])[1:], alone)
+    w_down[:, shared + (E - 1) * ff:] = float("inf")      # of an expert that this token has not chosen
+    assert torch.equal(run(x, [own, high])[:1], alone)
