@@ -274,6 +274,9 @@ chunk_read_kernel(CsRows<T> in, const int* __restrict__ cu_q, const int* __restr
   const T* prow = in.proj + (size_t)base * in.stride;
   const T *vrow = prow + in.v_off + (size_t)h * dv, *krow = prow + in.k_off;
   const long vstride = in.stride;
+  // (float32: an address of its own.  As an offset from the row's, the compiler moved loads forward into 255 registers and a spill:
+  // 57.8 us for 2,048 tokens of 12 heads of 128, 56.0 this way with 179; heads of 64, 128 registers and two CTAs an SM, 34.6 / 30.4.)
+  if (sizeof(T) == 4) asm("" : "+l"(vrow));
   if (tid < CS_C) {
     av[tid] = tid >= n ? 1.f : in.tok_decay ? in.tok_decay[(size_t)(base + tid) * H + h] : in.decay[h];
     sc[tid] = (in.tok_scale && tid < n) ? in.tok_scale[(size_t)(base + tid) * H + h] : 1.f;
