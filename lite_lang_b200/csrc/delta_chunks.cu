@@ -20,26 +20,19 @@
 #define DC_TP (DC_BLOCK + 8)
 #define DC_GP (CS_C + 4)
 
-// A running product of decays as the sum of two float32 numbers (the rounding of each step by a fused multiply-add; Dekker's product),
-// 2^-47 off after 64 steps and rounded once, as float64 would be, whose multiplications take ten times as long.
+// A running product of decays: float64, rounded once, so that neither the steps' roundings nor products below 2^-100 lose bits.  (The sum
+// of two float32 numbers, whose error term underflows there, is as fast in delta_solve and takes 1 us of 70 less in
+// delta_solve_channels.)
 struct DcProduct {
-  float hi = 1.f, lo = 0.f;
-  __device__ __forceinline__ void times(float a) {
-    const float p = hi * a;
-    lo = fmaf(lo, a, fmaf(hi, a, -p));
-    hi = p;
-  }
-  __device__ __forceinline__ void times(const DcProduct& a) {
-    const float p = hi * a.hi;
-    lo = fmaf(hi, a.lo, fmaf(lo, a.hi, fmaf(hi, a.hi, -p)));
-    hi = p;
-  }
-  __device__ __forceinline__ float value() const { return hi + lo; }
+  double p = 1.0;
+  __device__ __forceinline__ void times(double a) { p *= a; }
+  __device__ __forceinline__ void times(const DcProduct& a) { p *= a.p; }
+  __device__ __forceinline__ float value() const { return (float)p; }
 };
 
 // G(t, s) for s <= t of a chunk's tokens in gs [64][DC_GP], and pre[t] = a_0 ... a_t, by 256 threads: thread (s, quarter) makes 16
 // tokens' products, from the products of s's own quarter and of whole quarters between.  av: the decays.
-__device__ __forceinline__ void dc_gaps(const float* av, float* gs, float* pre, DcProduct* tail, DcProduct* whole) {
+__device__ __forceinline__ void dc_gaps(const double* av, float* gs, float* pre, DcProduct* tail, DcProduct* whole) {
   const int s = threadIdx.x & 63, quarter = threadIdx.x >> 6, own = s >> 4;
   if (quarter == own) {
     DcProduct p;
@@ -259,7 +252,8 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
   bf16* Tp = Lp + 3 * CS_C * DC_LP;                              // [3][64][DC_TP]: (1 + L_ii)^-1 - 1 of the blocks on the diagonal
   float* Ld = reinterpret_cast<float*>(Tp + 3 * CS_C * DC_TP);   // [64][20]: these blocks of L
   float* gs = Ld + CS_C * 20;                                    // [64][DC_GP]
-  __shared__ float av[CS_C], bt[CS_C], pre[CS_C];
+  __shared__ float bt[CS_C], pre[CS_C];
+  __shared__ double av[CS_C];
   __shared__ DcProduct tail[CS_C], whole[4];
   LL_PDL_TRIGGER();
   LL_PDL_WAIT();
@@ -576,7 +570,7 @@ delta_solve_channels_kernel(const float* __restrict__ qn, const float* __restric
     const int ch = tid % DK, b = tid / DK;
     float* a = rf + b * 16 * FP + ch;
     float* y = yf + b * 16 * FP + ch;
-    float av[16];
+    double av[16];
     DcProduct p;
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
