@@ -242,9 +242,9 @@ template <int DK, int DV>
 __global__ void __launch_bounds__(CS_THREADS, 2)
 delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
                    const float* __restrict__ beta, const float* __restrict__ g, const int* __restrict__ cu_q,
-                   const int* __restrict__ req_slot, int E, float* __restrict__ ut, unsigned* __restrict__ wt, unsigned* __restrict__ kp,
-                   float* __restrict__ mm, float* __restrict__ suf_out, float* __restrict__ pre_out, float* __restrict__ gam, int H,
-                   int Hk) {
+                   const int* __restrict__ req_slot, int E, int item0, float* __restrict__ ut, unsigned* __restrict__ wt,
+                   unsigned* __restrict__ kp, float* __restrict__ mm, float* __restrict__ suf_out, float* __restrict__ pre_out,
+                   float* __restrict__ gam, int H, int Hk) {
   constexpr int KP = DK + 8, TILES = DK / 2;                     // tiles of 16 by 8 of 64 tokens' k or W
   extern __shared__ __align__(16) unsigned char cs_smem[];
   bf16* ks = reinterpret_cast<bf16*>(cs_smem);                   // [3][64][KP]
@@ -260,7 +260,7 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int item = blockIdx.x, h = blockIdx.y, group = H / Hk, hk = h / group;
   int e, chunk;
-  if (!cs_item(item, cu_q, E, e, chunk)) return;
+  if (!cs_item(item0 + item, cu_q, E, e, chunk)) return;
   if (req_slot[e] < 0) return;
   const int base = cu_q[e] + chunk * CS_C, n = min(CS_C, cu_q[e + 1] - base);
   const long Cq = (long)Hk * DK, Cv = (long)H * DV;
@@ -456,7 +456,7 @@ template <int DK, int DV>
 __global__ void __launch_bounds__(DC_CH_THREADS, 1)
 delta_solve_channels_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
                             const float* __restrict__ beta, const float* __restrict__ g, const int* __restrict__ cu_q,
-                            const int* __restrict__ req_slot, int E, float* __restrict__ ut, unsigned* __restrict__ wt,
+                            const int* __restrict__ req_slot, int E, int item0, float* __restrict__ ut, unsigned* __restrict__ wt,
                             unsigned* __restrict__ kp, float* __restrict__ mm, float* __restrict__ qd, float* __restrict__ gam, int H,
                             int Hk) {
   constexpr int FP = DK + 8, TILES = DK / 2, WARPS = DC_CH_THREADS / 32, PIECES = DK / 4;
@@ -478,7 +478,7 @@ delta_solve_channels_kernel(const float* __restrict__ qn, const float* __restric
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int item = blockIdx.x, h = blockIdx.y, hk = h / (H / Hk);
   int e, chunk;
-  if (!cs_item(item, cu_q, E, e, chunk)) return;
+  if (!cs_item(item0 + item, cu_q, E, e, chunk)) return;
   if (req_slot[e] < 0) return;
   const int base = cu_q[e] + chunk * CS_C, n = min(CS_C, cu_q[e + 1] - base);
   const long Cq = (long)Hk * DK, Cv = (long)H * DV;
@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(CS_THREADS)
 delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const unsigned* __restrict__ kp,
                   const float* __restrict__ suf_in, const float* __restrict__ gam, float* __restrict__ s0,
                   float* __restrict__ state, long state_stride, int num_slots, const int* __restrict__ cu_q,
-                  const int* __restrict__ req_slot, int E, int H, int Hk, int dv, int* status) {
+                  const int* __restrict__ req_slot, int E, int item0, int items, int H, int Hk, int dv, int* status) {
   constexpr int WARPS = CS_THREADS / 32, KW = DK / WARPS;      // key channels a warp: 16, or 8 of heads of 64
   constexpr int SP = DK + 8, UP = CS_C + 8;
   constexpr int NT = KW / 8, KH = DK / 32, TILES = DK / 2;     // KH: steps of 16 channels a team
@@ -761,8 +761,10 @@ delta_walk_kernel(float* __restrict__ ut, const unsigned* __restrict__ wt, const
   }
   const int slot = req_slot[e];
   if (slot < 0 || slot >= num_slots) return;
-  const int first = cs_first_item(e, cu_q), chunks = (cu_q[e + 1] - cu_q[e] + CS_C - 1) / CS_C;
-  if (chunks == 0) return;
+  // of the entry's chunks those of the call: `first`, the place of their first one in the call's scratch, and their number
+  const int at = cs_first_item(e, cu_q) - item0, first = max(at, 0);
+  const int chunks = min(at + (cu_q[e + 1] - cu_q[e] + CS_C - 1) / CS_C, items) - first;
+  if (chunks <= 0) return;
   const int m = lane >> 3, r = lane & 7, g = lane >> 2, c = lane & 3;
   const int team = warp >> 2, kw = warp * KW;           // the warp's first key channel in the second product
   const int tw = (warp & 3) * 16 + team * 8;            // the first of the eight tokens whose u it makes
@@ -975,7 +977,7 @@ __device__ __noinline__ float dc_number(const float* q, const float* k, long str
 template <int DK, int DV, bool CH>
 __global__ void __launch_bounds__(CS_THREADS, 2)
 delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ g,
-                  const int* __restrict__ cu_q, const int* __restrict__ req_slot, int E, int num_slots,
+                  const int* __restrict__ cu_q, const int* __restrict__ req_slot, int E, int item0, int num_slots,
                   const float* __restrict__ s0, const float* __restrict__ ut, const float* __restrict__ mm,
                   const float* __restrict__ pre_in, float* __restrict__ o, int H, int Hk) {
   constexpr int KP = DK + 8;
@@ -988,7 +990,7 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int item = blockIdx.x, h = blockIdx.y, hk = h / (H / Hk);
   int e, chunk;
-  if (!cs_item(item, cu_q, E, e, chunk)) return;
+  if (!cs_item(item0 + item, cu_q, E, e, chunk)) return;
   const int slot = req_slot[e];
   const int base = cu_q[e] + chunk * CS_C, n = min(CS_C, cu_q[e + 1] - base);
   const long Cq = (long)Hk * DK, Cv = (long)H * DV;
@@ -1115,8 +1117,8 @@ delta_read_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 template <int DK, int DV, bool CH>
 static int dc_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* g, float* state,
                    long state_stride, int num_slots, const int* cu_q, const int* req_slot, float* o, int E, int H, int Hk,
-                   float* s0, float* ut, unsigned* wt, unsigned* kp, float* m, float* suf, float* pre, float* gam, int items, int* status,
-                   cudaStream_t stream) {
+                   float* s0, float* ut, unsigned* wt, unsigned* kp, float* m, float* suf, float* pre, float* gam, int items, int most,
+                   int* status, cudaStream_t stream) {
   const size_t solve = CH ? 4 * (size_t)CS_C * (4 * (DK + 8) + 20) + 2 * (size_t)3 * CS_C * (DC_LP + DC_TP) + 4 * (size_t)20 * DK
                           : 2 * (size_t)3 * CS_C * (DK + 8 + DC_LP + DC_TP) + 4 * (size_t)CS_C * (20 + DC_GP);
   const size_t walk = 2 * (size_t)4 * 3 * CS_C * DK + 2 * (size_t)3 * 16 * (DK + 8 + CS_C + 8) + 16 * (size_t)CS_THREADS;
@@ -1129,38 +1131,43 @@ static int dc_scan(const float* qn, const float* kn, const float* vc, const floa
   if (rc != cudaSuccess) return (int)rc;
   rc = cs_room<delta_read_kernel<DK, DV, CH>>(read);
   if (rc != cudaSuccess) return (int)rc;
-  if constexpr (CH)
-    ll_launch(delta_solve_channels_kernel<DK, DV>, dim3(items, H), dim3(DC_CH_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q,
-              req_slot, E, ut, wt, kp, m, pre, gam, H, Hk);
-  else
-    ll_launch(delta_solve_kernel<DK, DV>, dim3(items, H), dim3(CS_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q, req_slot, E, ut,
-              wt, kp, m, suf, pre, gam, H, Hk);
-  ll_launch(delta_walk_kernel<DK, CH>, dim3(DV / 16, H, E), dim3(CS_THREADS), walk, stream, ut, (const unsigned*)wt, (const unsigned*)kp,
-            (const float*)suf, (const float*)gam, s0, state, state_stride, num_slots, cu_q, req_slot, E, H, Hk, DV, status);
-  ll_launch(delta_read_kernel<DK, DV, CH>, dim3(items, H), dim3(CS_THREADS), read, stream, qn, kn, g, cu_q, req_slot, E, num_slots,
-            (const float*)s0, (const float*)ut, (const float*)m, (const float*)pre, o, H, Hk);
+  for (int item0 = 0; item0 < items; item0 += most) {
+    const int part = items - item0 < most ? items - item0 : most;
+    if constexpr (CH)
+      ll_launch(delta_solve_channels_kernel<DK, DV>, dim3(part, H), dim3(DC_CH_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q,
+                req_slot, E, item0, ut, wt, kp, m, pre, gam, H, Hk);
+    else
+      ll_launch(delta_solve_kernel<DK, DV>, dim3(part, H), dim3(CS_THREADS), solve, stream, qn, kn, vc, beta, g, cu_q, req_slot, E,
+                item0, ut, wt, kp, m, suf, pre, gam, H, Hk);
+    ll_launch(delta_walk_kernel<DK, CH>, dim3(DV / 16, H, E), dim3(CS_THREADS), walk, stream, ut, (const unsigned*)wt, (const unsigned*)kp,
+              (const float*)suf, (const float*)gam, s0, state, state_stride, num_slots, cu_q, req_slot, E, item0, part, H, Hk, DV, status);
+    ll_launch(delta_read_kernel<DK, DV, CH>, dim3(part, H), dim3(CS_THREADS), read, stream, qn, kn, g, cu_q, req_slot, E, item0,
+              num_slots, (const float*)s0, (const float*)ut, (const float*)m, (const float*)pre, o, H, Hk);
+  }
   return LL_LAUNCH_RESULT();
 }
 
-// The recurrence of ll_delta_recurrence (delta_rule.cu) by chunks: three launches.  `items`: at least the number of chunks of 64 tokens
-// of the step's entries.  Scratch, 32 bits a number, at multiples of 16 bytes: s0 [items][H][dv][dk], ut [items][H][dv][64], wt
+// The recurrence of ll_delta_recurrence (delta_rule.cu) by chunks: three launches.  `chunks`: at least the number of chunks of 64 tokens
+// of the step's entries.  More than `items` of them are done `items` at a time, the states go on in the records (the same bits).
+// Scratch, 32 bits a number, at multiples of 16 bytes: s0 [items][H][dv][dk], ut [items][H][dv][64], wt
 // [items][H][96 dk], m [items][H][64][64]; with one decay a head kp [items][Hk][96 dk], suf and pre [items][H][64], gam [items][H];
 // with one a channel kp [items][H][96 dk], pre [items][H][64][dk], gam [items][H][dk] and no suf.
 extern "C" int ll_chunk_delta_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* g,
                                    float* state, long state_stride, int num_slots, const int* cu_q, const int* req_slot,
                                    float* o, int num_entries, int H, int Hk, int dk, int dv, int per_channel, float* s0, float* ut,
-                                   void* wt, void* kp, float* m, float* suf, float* pre, float* gam, int items, int* status,
-                                   cudaStream_t stream) {
-  if (num_entries <= 0 || items <= 0) return 0;
+                                   void* wt, void* kp, float* m, float* suf, float* pre, float* gam, int items, int chunks,
+                                   int* status, cudaStream_t stream) {
+  if (num_entries <= 0 || chunks <= 0) return 0;
+  if (items <= 0) return (int)cudaErrorInvalidValue;
   if (H <= 0 || Hk <= 0 || H % Hk || H > 65535 || num_entries > 65535 || ((uintptr_t)wt | (uintptr_t)kp | (uintptr_t)ut) % 16 != 0)
     return (int)cudaErrorInvalidValue;
   if (per_channel && ((uintptr_t)g | (uintptr_t)pre | (uintptr_t)gam) % 16 != 0) return (int)cudaErrorInvalidValue;
 #define DC_SCAN(DK, DV)                                                                                                              \
   if (dk == DK && dv == DV)                                                                                                          \
   return per_channel ? dc_scan<DK, DV, true>(qn, kn, vc, beta, g, state, state_stride, num_slots, cu_q, req_slot, o, num_entries, H, \
-                                             Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, items, status, stream)      \
+                                             Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, chunks, items, status, stream)      \
                      : dc_scan<DK, DV, false>(qn, kn, vc, beta, g, state, state_stride, num_slots, cu_q, req_slot, o, num_entries, H, \
-                                              Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, items, status, stream)
+                                              Hk, s0, ut, (unsigned*)wt, (unsigned*)kp, m, suf, pre, gam, chunks, items, status, stream)
   DC_SCAN(128, 128);
   DC_SCAN(128, 64);
   DC_SCAN(64, 128);

@@ -1531,22 +1531,29 @@ def _cut(step, tokens: int, heads: int, dk: int, dv: int, minimum) -> Optional[T
     return chunked_scan(step, tokens, dk, dv, minimum(heads * rest, dk, dv)) if rest > 0 else None
 
 
+# Memory that a call's chunks of the delta rule may take at a time: 160 to 250 KB a chunk and head of 128 x 128 (165 MB for 2,048
+# tokens of 28 heads, 237 with a decay a channel).  More chunks are done in parts that stay below it, one at least.
+DELTA_CHUNK_BYTES = 256 << 20
+
+
 def _delta_by_chunks(qn, kn, vc, beta, g, state, step, o, H: int, Hk: int, dk: int, dv: int, per_channel: bool, cut) -> None:
-    single, rest, items = cut
-    # scratch of one allocation: states in front of the chunks, u, the terms of w and of k (six bytes a number), the scores of q and
-    # k, decays to the chunks' ends and from their starts, and of whole chunks; with a decay a channel the second of these are in
-    # the terms of k and the third are q times them
-    n, at, ptrs = items * H, 0, []
-    sizes = (n * dv * dk, n * CHUNK * dv, n * CHUNK * dk * 3 // 2, (n if per_channel else items * Hk) * CHUNK * dk * 3 // 2,
-             n * CHUNK * CHUNK, *((0, n * CHUNK * dk, n * dk) if per_channel else (n * CHUNK, n * CHUNK, n)))
-    base = torch.empty(sum(sizes), dtype=torch.float32, device=qn.device)
+    single, rest, chunks = cut
+    # scratch of one allocation, numbers a chunk: states in front of the chunks, u, the terms of w and of k (six bytes a number), the
+    # scores of q and k, decays to the chunks' ends and from their starts, and of whole chunks; with a decay a channel the second of
+    # these are in the terms of k and the third are q times them
+    sizes = (H * dv * dk, H * CHUNK * dv, H * CHUNK * dk * 3 // 2, (H if per_channel else Hk) * CHUNK * dk * 3 // 2,
+             H * CHUNK * CHUNK, *((0, H * CHUNK * dk, H * dk) if per_channel else (H * CHUNK, H * CHUNK, H)))
+    items = min(chunks, max(1, DELTA_CHUNK_BYTES // (4 * sum(sizes))))
+    base = torch.empty(items * sum(sizes), dtype=torch.float32, device=qn.device)
+    at, ptrs = 0, []
     for size in sizes:
         ptrs.append(_ptr_at(base, at))
-        at += size
+        at += items * size
     load_library("chunk_scan").call(
         "ll_chunk_delta_scan", _ptr(qn), _ptr(kn), _ptr(vc), _ptr(beta), _ptr(g), _ptr(state), c_long(state.stride(0)),
         c_int(state.shape[0]), _ptr_at(step.cu_q, single), _ptr_at(step.req_slot, single), _ptr(o), c_int(rest), c_int(H),
-        c_int(Hk), c_int(dk), c_int(dv), c_int(1 if per_channel else 0), *ptrs, c_int(items), _ptr(getattr(step, "status", None)), _stream())
+        c_int(Hk), c_int(dk), c_int(dv), c_int(1 if per_channel else 0), *ptrs, c_int(items), c_int(chunks),
+        _ptr(getattr(step, "status", None)), _stream())
 
 
 def delta_recurrence(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, beta: torch.Tensor, g: torch.Tensor,
