@@ -491,11 +491,13 @@ gemm_stream_kernel(const GtParams p, const __grid_constant__ CUtensorMap wmap, c
           }
         }
       }
-      // The stage goes back when its values are here, not when they have been asked for: the arrival's address takes (no) part of
-      // the last load, and the producer has a proxy fence between the arrivals and the next copy.  An arrival behind the loads and
-      // no more overtook them, and the copy of the ring's next round was in their place: a line of a weight or token row in one
-      // product out of two, K = 2,048 and 12 tokens, beside a kernel of many CTAs that had started early.  (A part of every load:
-      // a decode step at batch 8 989 -> 1,000 us; this way 991.)
+      // The stage goes back when its values are here, not when they have been asked for.  An arrival behind the loads and no more
+      // overtook them, and the copy of the ring's next round was in their place: a line of a weight or token row in one product out
+      // of two, K = 2,048 and 12 tokens, beside a kernel of many CTAs that had started early.  Two things stand against it.  The
+      // producer's proxy fence orders the loads, which it knows of by the arrivals, and its next copies.  And the arrival's address
+      // takes (no) part of the last load: a warp's loads from shared memory have come back in their order, which is what was seen and
+      // is not promised, so this alone would not be relied on.  (A part of every load: a decode step at batch 8 989 -> 1,000 us;
+      // this way 991.)
       __syncwarp();
       if (lane == 0) gt_mbar_arrive(empty0 + 8 * s + (held & (unsigned)(p.M >> 31)));
       if (++s == STAGES) {

@@ -178,7 +178,10 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
           const int s = n % stages, pos = (tile_begin + n) * LM_TK + lane * box_rows;
           const int y = page == -2 ? -1 : page * page_size + pos % page_size;
           if (n + 1 < tiles) look_box(tile_begin + n + 1);
-          if (n >= stages) at_mbar_wait(empty0 + 8 * s, (unsigned)((n / stages - 1) & 1), status, dead);
+          if (n >= stages) {
+            at_mbar_wait(empty0 + 8 * s, (unsigned)((n / stages - 1) & 1), status, dead);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the consumers' loads, then the copies
+          }
           const unsigned live = __ballot_sync(0xffffffffu, y >= 0);
           if (lane == 0) at_mbar_expect_tx(full0 + 8 * s, __popc(live) * box);
           __syncwarp();
@@ -376,8 +379,9 @@ latent_attention_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
           }
         }
       }
-      // the place goes back when its values are here (an arrival behind loads may overtake them, and so may the next copy): its
-      // address takes (no) part of the last one (of every load of the product: 43.2 -> 48.0 us for a decode step of 16)
+      // The place goes back when its values are here (an arrival behind loads may overtake them, and so may the next copy): the
+      // producer's proxy fence stands between the arrivals and its next copy, and the arrival's address takes (no) part of the last
+      // load, behind which a warp's earlier ones have come (seen, not promised; of every load: 43.2 -> 48.0 us for a decode step of 16)
       __syncwarp();
       if (lane == 0) at_mbar_arrive(empty0 + 8 * s_at + (held & (unsigned)(num_pages >> 31)));
     }
