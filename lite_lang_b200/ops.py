@@ -16,7 +16,6 @@ from __future__ import annotations
 import functools
 import os
 import threading
-from ctypes import c_void_p
 from typing import NamedTuple, Optional, Tuple
 
 import torch
@@ -1161,8 +1160,8 @@ ACCUMULATE_MIN_M = 129   # more tokens than any of the hand-written plain produc
 
 # Rows, and multiply-adds, from which on a float32 product may go to the tensor cores (``gemm_f32``); steps of few tokens, 2 to 64
 # rows, have a line of their own (one row is a product of a matrix and a vector, which the library reads at the memory's rate).
-# Where a line allows it `f32_preferred` says which is the faster.  (Between the two the library keeps what it had, as the tests of
-# this dispatch have it: 83 x 17,920 x 1,536 116 us, 63 here.)
+# Where a line allows it `f32_preferred` says which is the faster.  Between the two, 65 to 95 rows, the library keeps every product: no line
+# was measured there but for one size, 83 x 17,920 x 1,536, whose 116 us would be 63 here.
 F32_MIN_M = 96
 F32_MIN_WORK = 1 << 28
 F32_FEW_M = (2, 64)
@@ -1272,7 +1271,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         "ll_gemm_f32", _ptr(out), c_long(N if out is None else out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight),
         c_long(weight.stride(0)), c_int(M), c_int(N), c_int(K), _ptr(terms), _ptr(parts), c_int(splits),
         c_int(1 if accumulate else 0), c_int(0 if gated is None else GATE_ACT[act.kind] + 1), c_float(act.limit),
-        c_float(act.alpha), c_int(sm_count(x.device)), c_void_p(_ptr(status)), _stream())
+        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(status), _stream())
     return parts if hand_on else out
 
 
@@ -1346,8 +1345,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     """x [n, in] times weight [out, in] transposed.
 
     Up to 32 bfloat16 tokens (decode) go to the hand-written TMA weight-streaming kernel
-    (``gemm_stream``), or to ``gemm_smallm`` for shapes that one does not take; large float32 products go to
-    ``gemm_f32``.  Everything else is a library (cuBLAS) product, as in the reference: float32 operands give a true
+    (``gemm_stream``), or to ``gemm_smallm`` for shapes that one does not take; float32 products of 2 to 64 rows
+    and 2^22 multiply-adds, or 96 and 2^28, go to ``gemm_f32`` where ``f32_preferred`` says so.  Everything else is a library (cuBLAS) product, as in the reference: float32 operands give a true
     float32 product (TF32 is off); bfloat16 operands accumulate in float32.
     ``out_dtype=torch.float32`` with bfloat16 operands keeps the float32 accumulator as the
     result (the logits).  ``partial_ok``: the caller's consumer (the fused residual-and-norm
@@ -1483,10 +1482,13 @@ CHUNK = 64                 # tokens of a chunk (csrc/chunk_scan.cu)
 # take the host 9 us longer than one (13 with a delta rule), and while a layer's kernels take less than its launches the walk's
 # time does not show.  So the lines lie where whole calls of a layer with its products are equal.  Measured on a B200 (walk /
 # chunks, us; portions x heads):
-#   linear attention  12 heads: 1 x 256 tokens 80 / 89, x 384 90 / 89, x 512 114 / 90; 2 x 192 81 / 90, x 256 92 / 90; 4 x 128
-#     87 / 95, x 160 105 / 91; 28 heads: 1 x 128 85 / 94, x 160 92 / 92, x 192 101 / 91; 4 x 48 99 / 91
-#   delta rule        12 heads: 1 x 192 105 / 117, x 256 140 / 117; 2 x 96 105 / 117, x 128 130 / 118; 4 x 48 105 / 117, x 64
-#     124 / 118; 28 heads: 1 x 96 116 / 120, x 128 143 / 119; 2 x 48 118 / 120, x 64 143 / 120; 4 x 48 193 / 135
+#   linear attention  12 heads: 1 x 256 tokens 72 / 82, x 384 90 / 81; 2 x 128 72 / 82; 4 x 64 72 / 82, x 128 87 / 83; 28 heads:
+#     1 x 128 79 / 86, x 192 101 / 82; 2 x 48 76 / 86, x 96 99 / 83; 4 x 32 82 / 87, x 48 99 / 85, x 64 116 / 103
+#   delta rule        12 heads: 1 x 160 93 / 107, x 192 111 / 106, x 256 140 / 106; 2 x 96 105 / 106, x 128 130 / 107; 4 x 48
+#     101 / 105, x 64 125 / 106; 28 heads: 1 x 64 99 / 113, x 96 116 / 108, x 128 143 / 108; 2 x 32 100 / 113, x 48 117 / 107; 4 x 32
+#     143 / 118
+# (The lines were set when a launch took the host longer and the chunks' kernels more; they lie up to 8 % behind where these cross, 15 %
+# for linear attention with 28 heads and four portions.)
 #   2,048 tokens of 12 heads, the kernels alone: decay scan 320 / 53, delta rule 872 / 135 (two portions of together 2,047: 122)
 DECAY_CHUNKED_MIN = 275
 DELTA_CHUNKED_MIN = 178
