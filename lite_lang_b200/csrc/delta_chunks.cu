@@ -448,7 +448,7 @@ delta_solve_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
 // G(t, s) = R(t) B Y(s), R from t's block's start, Y to s's block's end, B the blocks between, and k_t R(t), q_t R(t) and k_s Y(s) B are
 // the operands of products on the tensor cores.  What the walk multiplies the state by is rounded once (DcProduct).
 // qd [items][H][64][DK] = G(t, -) q_t, kp [items][H] = the terms of G(C, s) k_s, gam [items][H][DK] = G(C, -); the rest as above.
-// One CTA an SM (191 KB of shared memory).  Two entries of together 2,047 tokens, 12 heads: the three kernels 153 us, the walk by tokens
+// One CTA an SM (191 KB of shared memory).  Two entries of together 2,047 tokens, 12 heads: the three kernels 154 us, the walk by tokens
 // 857; its error against 64 bits is half the walk's.
 // ---------------------------------------------------------------------------------------------------------------
 #define DC_CH_THREADS 512

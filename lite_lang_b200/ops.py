@@ -16,6 +16,7 @@ from __future__ import annotations
 import functools
 import os
 import threading
+from ctypes import c_void_p
 from typing import NamedTuple, Optional, Tuple
 
 import torch
@@ -1271,7 +1272,8 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         "ll_gemm_f32", _ptr(out), c_long(N if out is None else out.stride(0)), _ptr(x), c_long(x.stride(0)), _ptr(weight),
         c_long(weight.stride(0)), c_int(M), c_int(N), c_int(K), _ptr(terms), _ptr(parts), c_int(splits),
         c_int(1 if accumulate else 0), c_int(0 if gated is None else GATE_ACT[act.kind] + 1), c_float(act.limit),
-        c_float(act.alpha), c_int(sm_count(x.device)), _ptr(status), _stream())
+        c_float(act.alpha), c_int(sm_count(x.device)), c_void_p(_ptr(status)),      # (its value: the word's address or None)
+        _stream())
     return parts if hand_on else out
 
 
